@@ -1,17 +1,13 @@
 // Stable LSD radix sort, onesweep style (one upfront histogram pass, then one
-// pass per 8-bit digit whose tile offsets come from a decoupled look-back).
+// pass per digit of at most 8 bits whose tile offsets come from a decoupled
+// look-back).
 //
-// A tile is 256 threads x 16 keys (or 8, a per-context tuning choice).  Keys are ranked inside each warp with
-// __match_any_sync in input order, so equal digits keep their order and the
-// sort is stable; tiles take their index from an atomic ticket in launch
-// order, which guarantees that every look-back predecessor is running.
-// Passes whose digit is the same for every key are skipped (the permutation
-// would be the identity), unless the caller asks for the variant without a
-// host round trip, which scans the bucket bases on the device and runs every
-// pass over [0, end_bit).
+// A tile is 256 threads x 16, 12, 8 or 4 keys; tiles take their index from an
+// atomic ticket in launch order, which guarantees that every look-back
+// predecessor is running.  Passes whose digit is the same for every key are
+// skipped (the permutation would be the identity), unless the caller asks for
+// the variant without a host round trip, which runs every pass.
 #include "vg_sort.h"
-
-#include <vector>
 
 #include "vg_prims.cuh"
 
@@ -19,44 +15,59 @@ namespace vg {
 namespace {
 
 constexpr int kBlock = 256;
-// Keys per thread of a onesweep tile: 16 (tiles of 4096 keys) or 8 (2048),
-// chosen per context (Ctx::tune.sort_items).
-constexpr int kItemsMax = 16;
-constexpr int kRadix = 256;
-constexpr int kMaxPasses = 8;
+constexpr int kRadix = 256;   // bases and counts are kept for 256 digit values whatever the digit's width
+constexpr int kMaxPasses = kRadixMaxPasses;
 
+struct DigitList {
+  uint32_t n;
+  RadixDigit d[kMaxPasses];
+};
+
+// Digit counts of every pass in one read of the keys, then (the last block to
+// finish) each pass's exclusive scan: bases[p][v] = first output row of value
+// v.  Shared-memory counters, 16-byte loads.
 template <typename K>
-__global__ void __launch_bounds__(kBlock) radix_hist_kernel(const K* __restrict__ keys, uint64_t n,
-                                                            uint32_t passes, uint32_t begin_bit,
-                                                            unsigned long long* __restrict__ hist) {
-  __shared__ uint32_t sh[kMaxPasses * kRadix];
-  for (uint32_t i = threadIdx.x; i < kMaxPasses * kRadix; i += kBlock) sh[i] = 0;
+__global__ void __launch_bounds__(kBlock) radix_hist_kernel(const K* __restrict__ keys, uint64_t n, DigitList dl,
+                                                            unsigned long long* __restrict__ hist,
+                                                            uint64_t* __restrict__ bases, uint32_t* done) {
+  extern __shared__ uint32_t sh[];   // [dl.n][kRadix]
+  __shared__ uint64_t s_scan[kBlock / 32 + 1];
+  __shared__ bool s_last;
+  for (uint32_t i = threadIdx.x; i < dl.n * kRadix; i += kBlock) sh[i] = 0;
   __syncthreads();
+  auto count = [&](K k) {
+    for (uint32_t p = 0; p < dl.n; ++p)
+      atomicAdd(&sh[p * kRadix + (static_cast<uint32_t>(k >> dl.d[p].shift) & ((1u << dl.d[p].bits) - 1u))], 1u);
+  };
+  constexpr uint32_t kVec = 16 / sizeof(K);
+  const uint64_t t = static_cast<uint64_t>(blockIdx.x) * kBlock + threadIdx.x;
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * kBlock;
-  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * kBlock + threadIdx.x; i < n; i += stride) {
-    K k = keys[i];
-    for (uint32_t p = 0; p < passes; ++p)
-      atomicAdd(&sh[p * kRadix + (static_cast<uint32_t>(k >> (begin_bit + 8 * p)) & 0xFFu)], 1u);
+  if ((reinterpret_cast<uintptr_t>(keys) & 15u) == 0) {
+    const uint64_t nv = n / kVec;
+    for (uint64_t i = t; i < nv; i += stride) {
+      K k[kVec];
+      *reinterpret_cast<uint4*>(k) = reinterpret_cast<const uint4*>(keys)[i];
+#pragma unroll
+      for (uint32_t q = 0; q < kVec; ++q) count(k[q]);
+    }
+    for (uint64_t i = nv * kVec + t; i < n; i += stride) count(keys[i]);
+  } else {
+    for (uint64_t i = t; i < n; i += stride) count(keys[i]);
   }
   __syncthreads();
-  for (uint32_t i = threadIdx.x; i < passes * kRadix; i += kBlock)
+  for (uint32_t i = threadIdx.x; i < dl.n * kRadix; i += kBlock)
     if (sh[i]) atomicAdd(&hist[i], static_cast<unsigned long long>(sh[i]));
-}
-
-// Exclusive scan of each pass's 256 digit counts (one block per pass).
-__global__ void __launch_bounds__(kRadix) radix_bases_kernel(const unsigned long long* __restrict__ hist,
-                                                              uint64_t* __restrict__ bases) {
-  __shared__ uint64_t s[kRadix];
-  const uint32_t p = blockIdx.x, d = threadIdx.x;
-  s[d] = hist[p * kRadix + d];
+  __threadfence();
   __syncthreads();
-  for (uint32_t off = 1; off < kRadix; off <<= 1) {
-    const uint64_t v = d >= off ? s[d - off] : 0;
-    __syncthreads();
-    s[d] += v;
-    __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  for (uint32_t p = 0; p < dl.n; ++p) {
+    const uint64_t c = ld_status_u64(reinterpret_cast<const uint64_t*>(&hist[p * kRadix + threadIdx.x]));
+    uint64_t tot;
+    bases[p * kRadix + threadIdx.x] = block_excl_scan64<kBlock>(c, tot, s_scan);
   }
-  bases[p * kRadix + d] = s[d] - hist[p * kRadix + d];
 }
 
 __global__ void iota_kernel(uint32_t* out, uint64_t n) {
@@ -65,246 +76,347 @@ __global__ void iota_kernel(uint32_t* out, uint64_t n) {
     out[i] = static_cast<uint32_t>(i);
 }
 
-template <typename K, bool HAS_V, bool IOTA, int kItems, int kLook>
-__global__ void __launch_bounds__(kBlock, kItems <= 12 ? 4 : 3) onesweep_kernel(
+// Look-back words: 32 bits (two of them flags) while every prefix fits 30
+// bits, else 64.
+template <bool WIDE>
+struct Status;
+template <>
+struct Status<false> {
+  using T = uint32_t;
+  static constexpr T kAgg = 1u << 30, kInc = 2u << 30, kValue = (1u << 30) - 1;
+  static __device__ __forceinline__ T load(const T* p) {
+    T v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+  }
+  static __device__ __forceinline__ void store(T* p, T v) {
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+  }
+};
+template <>
+struct Status<true> {
+  using T = uint64_t;
+  static constexpr T kAgg = kFlagAgg, kInc = kFlagInc, kValue = kValueMask;
+  static __device__ __forceinline__ T load(const T* p) { return ld_status_u64(p); }
+  static __device__ __forceinline__ void store(T* p, T v) { st_status_u64(p, v); }
+};
+
+// One digit pass.  What bounds it is the ranking (about 100 instructions per
+// key and warp, four blocks of 64 registers per SM), not memory: 100M 64-bit
+// keys take 0.49 ms with 7-bit digits and 0.55 with 8-bit ones (3.3 and 2.9
+// TB/s), where ranking with __match_any_sync took 0.89 (its cost grows with
+// the number of distinct digits in the warp).
+// 1. the warps count their digits with shared atomics, so the tile's counts
+//    are published before anything is ranked and the look-back of later tiles
+//    finds them (publishing after the ranking: 0.53 ms);
+// 2. every key's place in the tile: the lanes with the same digit from one
+//    ballot per digit bit, the first of them takes their places off the
+//    warp's running counter (which starts at the warp's first place) with one
+//    shared atomic, four keys' atomics in flight.  Lanes and keys are taken in
+//    input order, so the sort is stable;
+// 3. keys (and values) go to their places in shared memory and leave from
+//    there in digit order, mostly coalesced.
+// Keys past the end are all ones: the tile's highest digit, placed after every
+// real key, never stored, and counted only by the last tile.
+template <typename K, bool HAS_V, bool IOTA, int BITS, int ITEMS, bool WIDE>
+__global__ void __launch_bounds__(kBlock, HAS_V && sizeof(K) == 8 && ITEMS > 8 ? 3 : 4) onesweep_kernel(
     const K* __restrict__ kin, K* __restrict__ kout, const uint32_t* __restrict__ vin,
-    uint32_t* __restrict__ vout, uint64_t n, uint32_t shift, const uint64_t* __restrict__ bucket_base,
-    uint64_t* status, uint32_t* ticket, DeviceErrors* err) {
-  constexpr int kTile = kBlock * kItems;
+    uint32_t* __restrict__ vout, uint64_t n, uint32_t shift, uint32_t mask, uint32_t look,
+    const uint64_t* __restrict__ bucket_base, typename Status<WIDE>::T* status, uint32_t* ticket,
+    DeviceErrors* err) {
+  using S = Status<WIDE>;
+  using Word = typename S::T;
+  constexpr int kTile = kBlock * ITEMS, kWarps = kBlock / 32, R = 1 << BITS, kGroup = 4;
+  static_assert(R <= kBlock, "one thread per digit value");
+  static_assert(ITEMS % kGroup == 0, "keys are ranked in groups");
   extern __shared__ __align__(16) unsigned char smem[];
   K* s_keys = reinterpret_cast<K*>(smem);
   uint32_t* s_vals = reinterpret_cast<uint32_t*>(smem + kTile * sizeof(K));
-  __shared__ uint32_t s_whist[8 * kRadix];
-  __shared__ uint32_t s_dstart[kRadix];
-  __shared__ uint64_t s_dglob[kRadix];
-  __shared__ uint32_t s_scan[9];
+  __shared__ uint32_t s_whist[kWarps * R];
+  __shared__ Word s_glob[R];
+  __shared__ uint32_t s_scan[kWarps + 1];
   __shared__ uint32_t s_tile;
 
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   if (tid == 0) s_tile = atomicAdd(ticket, 1u);
-  for (uint32_t i = tid; i < 8 * kRadix; i += kBlock) s_whist[i] = 0;
+#pragma unroll
+  for (int i = 0; i < kWarps * R / kBlock; ++i) s_whist[i * kBlock + tid] = 0;
   __syncthreads();
   const uint32_t tile = s_tile;
   const uint64_t base = static_cast<uint64_t>(tile) * kTile;
-  const uint64_t wbase = base + warp * (32u * kItems);
+  const uint32_t tile_n = static_cast<uint32_t>(n - base < kTile ? n - base : kTile);
+  const uint32_t w0 = warp * (32u * ITEMS) + lane;
+  kin += base;
+  if (HAS_V && !IOTA) vin += base;
 
-  K key[kItems];
-  uint32_t val[kItems];
-  uint32_t rank[kItems];
+  K key[ITEMS];
+  uint32_t val[HAS_V ? ITEMS : 1];
+  if (tile_n == kTile) {
 #pragma unroll
-  for (int i = 0; i < kItems; ++i) {
-    const uint64_t idx = wbase + i * 32u + lane;
-    const bool ok = idx < n;
-    key[i] = ok ? kin[idx] : K(0);
-    if (HAS_V) val[i] = IOTA ? static_cast<uint32_t>(idx) : (ok ? vin[idx] : 0u);
-  }
-  // Rank every key among the equal digits before it in this warp's chunk.
-  uint32_t* wh = s_whist + warp * kRadix;
+    for (int i = 0; i < ITEMS; ++i) key[i] = kin[w0 + i * 32u];
+    if (HAS_V) {
 #pragma unroll
-  for (int i = 0; i < kItems; ++i) {
-    const bool ok = wbase + i * 32u + lane < n;
-    const uint32_t d = static_cast<uint32_t>(key[i] >> shift) & 0xFFu;
-    const uint32_t peers = __match_any_sync(0xffffffffu, ok ? d : 0x100u);
-    uint32_t prior = 0;
-    if (ok) prior = wh[d];
-    __syncwarp();
-    rank[i] = prior + __popc(peers & lanemask_lt());
-    if (ok && lane == static_cast<uint32_t>(__ffs(peers) - 1)) wh[d] = prior + __popc(peers);
-    __syncwarp();
+      for (int i = 0; i < ITEMS; ++i)
+        val[i] = IOTA ? static_cast<uint32_t>(base) + w0 + i * 32u : vin[w0 + i * 32u];
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+      const uint32_t q = w0 + i * 32u;
+      key[i] = q < tile_n ? kin[q] : ~K(0);
+      if (HAS_V) val[i] = IOTA ? static_cast<uint32_t>(base) + q : (q < tile_n ? vin[q] : 0u);
+    }
   }
+  uint32_t* wh = s_whist + warp * R;
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i) atomicAdd(&wh[static_cast<uint32_t>(key[i] >> shift) & mask], 1u);
   __syncthreads();
 
-  // Thread d owns digit d: per-warp exclusive offsets and the tile count.
-  const uint32_t d = tid;
-  uint32_t run = 0;
+  // Thread d owns digit value d: the tile's count, published for later tiles,
+  // and each warp's first place.
+  uint32_t run = 0, cnt[kWarps];
+  Word* my = status + static_cast<uint64_t>(tile) * R + tid;
+  if (tid < R) {
 #pragma unroll
-  for (int w = 0; w < 8; ++w) {
-    uint32_t c = s_whist[w * kRadix + d];
-    s_whist[w * kRadix + d] = run;
-    run += c;
-  }
-  // Decoupled look-back for digit d over earlier tiles ([tile][digit] layout):
-  // kLook earlier tiles' words are loaded at once, then summed in order until
-  // one holds an inclusive prefix (a word not yet published is waited for).
-  uint64_t prefix = 0;
-  uint64_t* my = status + static_cast<uint64_t>(tile) * kRadix + d;
-  if (tile == 0) {
-    st_status_u64(my, kFlagInc | run);
-  } else {
-    st_status_u64(my, kFlagAgg | run);
-    int64_t j = static_cast<int64_t>(tile) - 1;
-    bool found = false;
-    while (!found) {
-      uint64_t w[kLook];
-#pragma unroll
-      for (int q = 0; q < kLook; ++q)
-        w[q] = (j - q >= 0) ? ld_status_u64(status + static_cast<uint64_t>(j - q) * kRadix + d) : kFlagInc;
-#pragma unroll
-      for (int q = 0; q < kLook; ++q) {
-        if (found) break;
-        uint64_t v = w[q];
-        if ((v & ~kValueMask) == 0) v = wait_status(status + static_cast<uint64_t>(j - q) * kRadix + d, err);
-        prefix += v & kValueMask;
-        found = (v & kFlagInc) != 0;
-      }
-      j -= kLook;
+    for (int w = 0; w < kWarps; ++w) {
+      cnt[w] = s_whist[w * R + tid];
+      run += cnt[w];
     }
-    st_status_u64(my, kFlagInc | (prefix + run));
+    S::store(my, (tile == 0 ? S::kInc : S::kAgg) | run);
   }
   uint32_t tot;
   const uint32_t excl = block_excl_scan<kBlock>(run, tot, s_scan);
-  s_dstart[d] = excl;
-  s_dglob[d] = bucket_base[d] + prefix - excl;
-  __syncthreads();
-
-  // Local scatter into digit order, then a mostly-coalesced global write.
+  if (tid < R) {
+    uint32_t x = excl;
 #pragma unroll
-  for (int i = 0; i < kItems; ++i) {
-    if (wbase + i * 32u + lane < n) {
-      const uint32_t dd = static_cast<uint32_t>(key[i] >> shift) & 0xFFu;
-      const uint32_t pos = s_dstart[dd] + wh[dd] + rank[i];
-      s_keys[pos] = key[i];
-      if (HAS_V) s_vals[pos] = val[i];
+    for (int w = 0; w < kWarps; ++w) {
+      s_whist[w * R + tid] = x;
+      x += cnt[w];
     }
   }
   __syncthreads();
-  const uint32_t tile_n = static_cast<uint32_t>(n - base < kTile ? n - base : kTile);
-  for (uint32_t p = tid; p < tile_n; p += kBlock) {
+
+#pragma unroll
+  for (int g = 0; g < ITEMS; g += kGroup) {
+    uint32_t peers[kGroup], first[kGroup];
+#pragma unroll
+    for (int q = 0; q < kGroup; ++q) {
+      const uint32_t d = static_cast<uint32_t>(key[g + q] >> shift) & mask;
+      uint32_t p = 0xffffffffu;
+#pragma unroll
+      for (int b = 0; b < BITS; ++b) {
+        const bool bit = (d >> b) & 1u;
+        const uint32_t v = __ballot_sync(0xffffffffu, bit);
+        p &= bit ? v : ~v;
+      }
+      peers[q] = p;
+    }
+#pragma unroll
+    for (int q = 0; q < kGroup; ++q) {
+      const uint32_t d = static_cast<uint32_t>(key[g + q] >> shift) & mask;
+      first[q] = 0;
+      if ((peers[q] & lanemask_lt()) == 0) first[q] = atomicAdd(&wh[d], __popc(peers[q]));
+    }
+#pragma unroll
+    for (int q = 0; q < kGroup; ++q) {
+      const uint32_t pos =
+          __shfl_sync(0xffffffffu, first[q], __ffs(peers[q]) - 1) + __popc(peers[q] & lanemask_lt());
+      s_keys[pos] = key[g + q];
+      if (HAS_V) s_vals[pos] = val[g + q];
+    }
+  }
+
+  // Decoupled look-back for digit value d over earlier tiles ([tile][value]
+  // layout): `look` (1 or 4) earlier tiles' words are loaded at once, then
+  // summed in order until one holds an inclusive prefix (a word not yet
+  // published is waited for, a bounded number of polls).
+  if (tid < R) {
+    Word prefix = 0;
+    if (tile > 0) {
+      constexpr int kLook = 4;
+      int64_t j = static_cast<int64_t>(tile) - 1;
+      bool found = false;
+      while (!found) {
+        Word w[kLook];
+#pragma unroll
+        for (int q = 0; q < kLook; ++q)
+          w[q] = (j - q >= 0 && q < static_cast<int>(look)) ? S::load(status + static_cast<uint64_t>(j - q) * R + tid)
+                                                            : S::kInc;
+#pragma unroll
+        for (int q = 0; q < kLook; ++q) {
+          if (found || q >= static_cast<int>(look)) break;
+          Word v = w[q];
+          for (uint32_t spins = 0; (v & ~S::kValue) == 0;) {
+            if (++spins > kSpinLimit) {
+              atomicExch(&err->timeout, 1u);
+              v = S::kInc;
+              break;
+            }
+            __nanosleep(20);
+            v = S::load(status + static_cast<uint64_t>(j - q) * R + tid);
+          }
+          prefix += v & S::kValue;
+          found = (v & S::kInc) != 0;
+        }
+        j -= look;
+      }
+      S::store(my, S::kInc | (prefix + run));
+    }
+    // + a place in the tile gives the output row (modulo the word: n fits it)
+    s_glob[tid] = static_cast<Word>(bucket_base[tid]) + prefix - excl;
+  }
+  __syncthreads();
+  // (after a wait that gave up in an earlier pass the keys no longer match
+  // the counts: the row is checked, the caller sees the recorded timeout)
+  auto store = [&](uint32_t p) {
     const K k = s_keys[p];
-    const uint32_t dd = static_cast<uint32_t>(k >> shift) & 0xFFu;
-    const uint64_t o = s_dglob[dd] + p;
-    kout[o] = k;
-    if (HAS_V) vout[o] = s_vals[p];
+    const Word o = s_glob[static_cast<uint32_t>(k >> shift) & mask] + p;
+    if (o < static_cast<Word>(n)) {
+      kout[o] = k;
+      if (HAS_V) vout[o] = s_vals[p];
+    }
+  };
+  if (tile_n == kTile) {
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) store(i * kBlock + tid);
+  } else {
+    for (uint32_t p = tid; p < tile_n; p += kBlock) store(p);
   }
 }
 
-template <typename K, bool HAS_V, bool IOTA, int kItems, int kLook>
-void launch_pass_items(Ctx& ctx, const K* kin, K* kout, const uint32_t* vin, uint32_t* vout, uint64_t n,
-                       uint32_t shift, const uint64_t* bases, uint64_t* status, uint32_t* ticket) {
-  constexpr int kTile = kBlock * kItems;
+struct PassArgs {
+  const uint32_t* vin;
+  uint32_t* vout;
+  uint64_t n;
+  RadixDigit digit;
+  const uint64_t* bases;
+  void* status;
+  uint32_t* ticket;
+};
+
+template <typename K, bool HAS_V, bool IOTA, int BITS, int ITEMS, bool WIDE>
+void launch_pass_as(Ctx& ctx, const K* kin, K* kout, const PassArgs& a) {
+  constexpr int kTile = kBlock * ITEMS;
   const size_t smem = kTile * sizeof(K) + (HAS_V ? kTile * sizeof(uint32_t) : 0);
+  auto kernel = onesweep_kernel<K, HAS_V, IOTA, BITS, ITEMS, WIDE>;
   // once per instantiation (thread-safe static initialisation)
-  static const bool attr_set = [smem] {
-    VG_CUDA(cudaFuncSetAttribute(onesweep_kernel<K, HAS_V, IOTA, kItems, kLook>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  static const bool attr_set = [&] {
+    VG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     // all of the unified L1/shared storage as shared memory: three or more
     // blocks of a tile's keys (and values) per SM
-    VG_CUDA(cudaFuncSetAttribute(onesweep_kernel<K, HAS_V, IOTA, kItems, kLook>,
-                                 cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    VG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 cudaSharedmemCarveoutMaxShared));
     return true;
   }();
   (void)attr_set;
-  const uint64_t tiles = div_up(n, kTile);
-  const double bytes = static_cast<double>(n) * (2 * sizeof(K) + (HAS_V ? (IOTA ? 4 : 8) : 0));
+  const uint64_t tiles = div_up(a.n, kTile);
+  const double bytes = static_cast<double>(a.n) * (2 * sizeof(K) + (HAS_V ? (IOTA ? 4 : 8) : 0));
   ctx.launch("radix_onesweep", bytes, [&] {
-    onesweep_kernel<K, HAS_V, IOTA, kItems, kLook><<<static_cast<unsigned>(tiles), kBlock, smem, ctx.stream>>>(
-        kin, kout, vin, vout, n, shift, bases, status, ticket, ctx.d_err);
+    kernel<<<static_cast<unsigned>(tiles), kBlock, smem, ctx.stream>>>(
+        kin, kout, a.vin, a.vout, a.n, a.digit.shift, (1u << a.digit.bits) - 1u, ctx.tune.sort_lookback, a.bases,
+        static_cast<typename Status<WIDE>::T*>(a.status), a.ticket, ctx.d_err);
   });
   VG_CUDA(cudaGetLastError());
 }
 
+// Digits of up to 7 bits have 128 counters a warp instead of 256 and one
+// ballot a key less.
+constexpr uint32_t status_row(uint32_t bits) { return bits <= 7 ? 128 : 256; }
+// Prefixes of 2^30 rows and more take 64-bit look-back words.
+constexpr bool wide_status(uint64_t n) { return n >= (1ull << 30); }
+
+template <typename K, bool HAS_V, bool IOTA, int ITEMS, bool WIDE>
+void launch_pass_bits(Ctx& ctx, const K* kin, K* kout, const PassArgs& a) {
+  if (a.digit.bits <= 7) launch_pass_as<K, HAS_V, IOTA, 7, ITEMS, WIDE>(ctx, kin, kout, a);
+  else launch_pass_as<K, HAS_V, IOTA, 8, ITEMS, WIDE>(ctx, kin, kout, a);
+}
+
 template <typename K, bool HAS_V, bool IOTA>
-void launch_pass(Ctx& ctx, int items, const K* kin, K* kout, const uint32_t* vin, uint32_t* vout, uint64_t n,
-                 uint32_t shift, const uint64_t* bases, uint64_t* status, uint32_t* ticket) {
-  const bool look4 = ctx.tune.sort_lookback == 4;
-  if (items == 12) {
-    if (look4) launch_pass_items<K, HAS_V, IOTA, 12, 4>(ctx, kin, kout, vin, vout, n, shift, bases, status, ticket);
-    else launch_pass_items<K, HAS_V, IOTA, 12, 1>(ctx, kin, kout, vin, vout, n, shift, bases, status, ticket);
-  } else if (items == 8) {
-    if (look4) launch_pass_items<K, HAS_V, IOTA, 8, 4>(ctx, kin, kout, vin, vout, n, shift, bases, status, ticket);
-    else launch_pass_items<K, HAS_V, IOTA, 8, 1>(ctx, kin, kout, vin, vout, n, shift, bases, status, ticket);
-  } else {
-    if (look4)
-      launch_pass_items<K, HAS_V, IOTA, kItemsMax, 4>(ctx, kin, kout, vin, vout, n, shift, bases, status, ticket);
-    else
-      launch_pass_items<K, HAS_V, IOTA, kItemsMax, 1>(ctx, kin, kout, vin, vout, n, shift, bases, status, ticket);
-  }
+void launch_pass(Ctx& ctx, int items, const K* kin, K* kout, const PassArgs& a) {
+  if (wide_status(a.n)) launch_pass_bits<K, HAS_V, IOTA, 16, true>(ctx, kin, kout, a);
+  else if (items == 16) launch_pass_bits<K, HAS_V, IOTA, 16, false>(ctx, kin, kout, a);
+  else if (items == 12) launch_pass_bits<K, HAS_V, IOTA, 12, false>(ctx, kin, kout, a);
+  else if (items == 8) launch_pass_bits<K, HAS_V, IOTA, 8, false>(ctx, kin, kout, a);
+  else launch_pass_bits<K, HAS_V, IOTA, 4, false>(ctx, kin, kout, a);
+}
+
+// Keys per thread: the context's choice (16 by default), or fewer while that
+// leaves less than two tiles per SM.
+int items_for(const Ctx& ctx, uint64_t n) {
+  if (wide_status(n)) return 16;
+  const int most = (ctx.tune.sort_items == 8 || ctx.tune.sort_items == 12) ? static_cast<int>(ctx.tune.sort_items) : 16;
+  const uint64_t two = 2ull * ctx.num_sms * kBlock;
+  if (n >= two * most) return most;
+  return n >= two * 8 && most > 8 ? 8 : 4;
 }
 
 template <typename K>
 bool radix_sort_impl(Ctx& ctx, K* keys, K* keys_alt, uint32_t* vals, uint32_t* vals_alt, uint64_t n,
-                     int begin_bit, int end_bit, bool vals_iota, bool host_skip) {
+                     const std::vector<RadixDigit>& digits, bool vals_iota, bool host_skip) {
   const bool has_v = vals != nullptr;
   if (n == 0) return false;
   if (n > 0xFFFFFFFFull && has_v) fail(VG_ERR_OVERFLOW, "radix sort values are 32-bit row ids");
-  if (begin_bit < 0 || begin_bit >= end_bit) begin_bit = 0;
-  int passes = (end_bit - begin_bit + 7) / 8;
-  if (passes < 1) passes = 1;
-  // the last pass may read bits above end_bit; it must not shift past the key
-  while (passes > 1 && begin_bit + 8 * (passes - 1) >= static_cast<int>(8 * sizeof(K))) --passes;
+  const uint32_t passes = static_cast<uint32_t>(digits.size());
+  if (passes > kMaxPasses) fail(VG_ERR_INVALID, "radix sort: too many digits");
+  DigitList dl{};
+  dl.n = passes;
+  for (uint32_t p = 0; p < passes; ++p) dl.d[p] = digits[p];
 
-  Scratch<unsigned long long> hist(ctx, passes * kRadix);
-  VG_CUDA(cudaMemsetAsync(hist.get(), 0, passes * kRadix * sizeof(unsigned long long), ctx.stream));
+  const int items = items_for(ctx, n);
+  const uint64_t tiles = div_up(n, static_cast<uint64_t>(kBlock) * items);
+  const size_t word = wide_status(n) ? sizeof(uint64_t) : sizeof(uint32_t);
+  // counts, tickets and every pass's look-back words in one block, zeroed by
+  // one memset; the bases behind them
+  const size_t hist_bytes = passes * kRadix * sizeof(uint64_t);
+  const size_t ticket_bytes = (kMaxPasses + 1) * sizeof(uint32_t) + 60;   // 128: tickets, then the histogram's
+  size_t zero_bytes = hist_bytes + ticket_bytes;
+  std::vector<size_t> status_at(passes);
+  for (uint32_t p = 0; p < passes; ++p) {
+    status_at[p] = zero_bytes;
+    zero_bytes += tiles * status_row(digits[p].bits) * word;
+  }
+  Scratch<char> scratch(ctx, zero_bytes + hist_bytes);
+  char* sc = scratch.get();
+  auto* hist = reinterpret_cast<unsigned long long*>(sc);
+  auto* ticket = reinterpret_cast<uint32_t*>(sc + hist_bytes);
+  auto* bases = reinterpret_cast<uint64_t*>(sc + zero_bytes);
+  VG_CUDA(cudaMemsetAsync(sc, 0, zero_bytes, ctx.stream));
   uint64_t grid = div_up(n, kBlock * 16);
   const uint64_t gmax = static_cast<uint64_t>(ctx.num_sms) * 8;
   if (grid > gmax) grid = gmax;
   if (grid < 1) grid = 1;
   ctx.launch("radix_histogram", static_cast<double>(n) * sizeof(K), [&] {
-    radix_hist_kernel<K><<<static_cast<unsigned>(grid), kBlock, 0, ctx.stream>>>(keys, n, passes, begin_bit,
-                                                                                hist.get());
+    radix_hist_kernel<K><<<static_cast<unsigned>(grid), kBlock, (passes ? passes : 1) * kRadix * sizeof(uint32_t),
+                           ctx.stream>>>(keys, n, dl, hist, bases, ticket + kMaxPasses);
   });
   VG_CUDA(cudaGetLastError());
-  Scratch<uint64_t> d_bases(ctx, passes * kRadix);
-  std::vector<int> todo;
+  std::vector<uint32_t> todo;
   if (host_skip) {
     std::vector<unsigned long long> h(passes * kRadix);
-    VG_CUDA(cudaMemcpyAsync(h.data(), hist.get(), h.size() * sizeof(unsigned long long),
-                            cudaMemcpyDeviceToHost, ctx.stream));
+    VG_CUDA(cudaMemcpyAsync(h.data(), hist, hist_bytes, cudaMemcpyDeviceToHost, ctx.stream));
     ctx.sync();
-    std::vector<uint64_t> bases(passes * kRadix);
-    for (int p = 0; p < passes; ++p) {
-      uint64_t run = 0;
+    for (uint32_t p = 0; p < passes; ++p) {
       bool trivial = false;
-      for (int d = 0; d < kRadix; ++d) {
-        const uint64_t c = h[p * kRadix + d];
-        if (c == n) trivial = true;
-        bases[p * kRadix + d] = run;
-        run += c;
-      }
+      for (int d = 0; d < kRadix; ++d) trivial = trivial || h[p * kRadix + d] == n;
       if (!trivial) todo.push_back(p);
     }
-    if (todo.empty()) {
-      if (has_v && vals_iota) {
-        ctx.launch("iota", 4.0 * n, [&] { iota_kernel<<<static_cast<unsigned>(grid), kBlock, 0, ctx.stream>>>(vals, n); });
-        VG_CUDA(cudaGetLastError());
-      }
-      return false;
-    }
-    VG_CUDA(cudaMemcpyAsync(d_bases.get(), bases.data(), bases.size() * sizeof(uint64_t),
-                            cudaMemcpyHostToDevice, ctx.stream));
   } else {
-    // no host round trip: bases scanned on the device and every pass runs
-    ctx.launch("radix_bases", 0.0, [&] {
-      radix_bases_kernel<<<static_cast<unsigned>(passes), kRadix, 0, ctx.stream>>>(hist.get(), d_bases.get());
-    });
-    VG_CUDA(cudaGetLastError());
-    for (int p = 0; p < passes; ++p) todo.push_back(p);
+    for (uint32_t p = 0; p < passes; ++p) todo.push_back(p);
   }
-  const int items = (ctx.tune.sort_items == 8 || ctx.tune.sort_items == 12) ? static_cast<int>(ctx.tune.sort_items)
-                                                                            : kItemsMax;
-  const uint64_t tiles = div_up(n, static_cast<uint64_t>(kBlock) * items);
-  Scratch<uint64_t> status(ctx, tiles * kRadix);
-  Scratch<uint32_t> ticket(ctx, todo.size());
-  VG_CUDA(cudaMemsetAsync(ticket.get(), 0, todo.size() * sizeof(uint32_t), ctx.stream));
-
+  if (todo.empty()) {
+    if (has_v && vals_iota) fill_iota(ctx, vals, n);
+    return false;
+  }
   K* kin = keys;
   K* kout = keys_alt;
   uint32_t* vin = vals;
   uint32_t* vout = vals_alt;
   for (size_t t = 0; t < todo.size(); ++t) {
-    const int p = todo[t];
-    VG_CUDA(cudaMemsetAsync(status.get(), 0, tiles * kRadix * sizeof(uint64_t), ctx.stream));
-    const uint64_t* pb = d_bases.get() + p * kRadix;
-    const uint32_t shift = static_cast<uint32_t>(begin_bit + 8 * p);
-    if (!has_v)
-      launch_pass<K, false, false>(ctx, items, kin, kout, nullptr, nullptr, n, shift, pb, status.get(),
-                                   ticket.get() + t);
-    else if (t == 0 && vals_iota)
-      launch_pass<K, true, true>(ctx, items, kin, kout, nullptr, vout, n, shift, pb, status.get(),
-                                 ticket.get() + t);
-    else
-      launch_pass<K, true, false>(ctx, items, kin, kout, vin, vout, n, shift, pb, status.get(),
-                                  ticket.get() + t);
+    const uint32_t p = todo[t];
+    const PassArgs a{vin, vout, n, digits[p], bases + p * kRadix, sc + status_at[p], ticket + p};
+    if (!has_v) launch_pass<K, false, false>(ctx, items, kin, kout, a);
+    else if (t == 0 && vals_iota) launch_pass<K, true, true>(ctx, items, kin, kout, a);
+    else launch_pass<K, true, false>(ctx, items, kin, kout, a);
     std::swap(kin, kout);
     std::swap(vin, vout);
   }
@@ -313,18 +425,43 @@ bool radix_sort_impl(Ctx& ctx, K* keys, K* keys_alt, uint32_t* vals, uint32_t* v
 
 }  // namespace
 
+void radix_plan(std::vector<RadixDigit>& digits, int begin, int end) {
+  const int passes = (end - begin + 7) / 8;
+  for (int p = 0, at = begin; p < passes; ++p) {
+    const int left = passes - p, bits = (end - at + left - 1) / left;
+    digits.push_back({static_cast<uint32_t>(at), static_cast<uint32_t>(bits)});
+    at += bits;
+  }
+}
+
+bool radix_sort_u32(Ctx& ctx, uint32_t* keys, uint32_t* keys_alt, uint32_t* vals, uint32_t* vals_alt,
+                    uint64_t n, const std::vector<RadixDigit>& digits, bool vals_iota, bool host_skip) {
+  return radix_sort_impl<uint32_t>(ctx, keys, keys_alt, vals, vals_alt, n, digits, vals_iota, host_skip);
+}
+
+bool radix_sort_u64(Ctx& ctx, uint64_t* keys, uint64_t* keys_alt, uint32_t* vals, uint32_t* vals_alt,
+                    uint64_t n, const std::vector<RadixDigit>& digits, bool vals_iota, bool host_skip) {
+  return radix_sort_impl<uint64_t>(ctx, keys, keys_alt, vals, vals_alt, n, digits, vals_iota, host_skip);
+}
+
 bool radix_sort_u32(Ctx& ctx, uint32_t* keys, uint32_t* keys_alt, uint32_t* vals, uint32_t* vals_alt,
                     uint64_t n, int end_bit, bool vals_iota, bool host_skip) {
-  return radix_sort_impl<uint32_t>(ctx, keys, keys_alt, vals, vals_alt, n, 0, end_bit, vals_iota, host_skip);
+  std::vector<RadixDigit> digits;
+  radix_plan(digits, 0, end_bit);
+  return radix_sort_impl<uint32_t>(ctx, keys, keys_alt, vals, vals_alt, n, digits, vals_iota, host_skip);
 }
 
 bool radix_sort_u64(Ctx& ctx, uint64_t* keys, uint64_t* keys_alt, uint32_t* vals, uint32_t* vals_alt,
                     uint64_t n, int end_bit, bool vals_iota, bool host_skip) {
-  return radix_sort_impl<uint64_t>(ctx, keys, keys_alt, vals, vals_alt, n, 0, end_bit, vals_iota, host_skip);
+  std::vector<RadixDigit> digits;
+  radix_plan(digits, 0, end_bit);
+  return radix_sort_impl<uint64_t>(ctx, keys, keys_alt, vals, vals_alt, n, digits, vals_iota, host_skip);
 }
 
 bool radix_sort_u64_bits(Ctx& ctx, uint64_t* keys, uint64_t* keys_alt, uint64_t n, int begin_bit, int end_bit) {
-  return radix_sort_impl<uint64_t>(ctx, keys, keys_alt, nullptr, nullptr, n, begin_bit, end_bit, false, true);
+  std::vector<RadixDigit> digits;
+  radix_plan(digits, begin_bit, end_bit);
+  return radix_sort_impl<uint64_t>(ctx, keys, keys_alt, nullptr, nullptr, n, digits, false, true);
 }
 
 void fill_iota(Ctx& ctx, uint32_t* out, uint64_t n) {

@@ -1,16 +1,35 @@
 #pragma once
 
+#include <vector>
+
 #include "vg_ctx.h"
 
 namespace vg {
 
-// Stable LSD radix sort of n keys over bits [0, end_bit).  When `vals` is
-// non-null the uint32 values move with their keys; with vals_iota the values
-// are generated as 0..n-1 (the input value buffer is not read).  Double
-// buffered: returns true when the result is in (keys_alt, vals_alt).  With
-// host_skip the digit histogram is read on the host (one synchronisation)
-// and passes with a single digit value are skipped; without it nothing
-// waits on the device.
+// One radix pass: the digit (key >> shift) & (2^bits - 1), bits <= 8.
+struct RadixDigit {
+  uint32_t shift;
+  uint32_t bits;
+};
+// Appends the digits that cover key bits [begin, end) from the lowest up, as
+// few as 8-bit digits allow and of widths as equal as can be.
+void radix_plan(std::vector<RadixDigit>& digits, int begin, int end);
+
+constexpr int kRadixMaxPasses = 16;
+
+
+// Stable LSD radix sort of n keys by the given digits, in order; what lies
+// outside the digits travels with the key.  When `vals` is non-null the
+// uint32 values move with their keys; with vals_iota the values are generated
+// as 0..n-1 (the input value buffer is not read).  Double buffered: returns
+// true when the result is in (keys_alt, vals_alt).  With host_skip the digit
+// counts are read on the host (one synchronisation) and passes with a single
+// digit value are skipped; without it nothing waits on the device.
+bool radix_sort_u32(Ctx& ctx, uint32_t* keys, uint32_t* keys_alt, uint32_t* vals, uint32_t* vals_alt,
+                    uint64_t n, const std::vector<RadixDigit>& digits, bool vals_iota, bool host_skip);
+bool radix_sort_u64(Ctx& ctx, uint64_t* keys, uint64_t* keys_alt, uint32_t* vals, uint32_t* vals_alt,
+                    uint64_t n, const std::vector<RadixDigit>& digits, bool vals_iota, bool host_skip);
+// The digits of bits [0, end_bit).
 bool radix_sort_u32(Ctx& ctx, uint32_t* keys, uint32_t* keys_alt, uint32_t* vals, uint32_t* vals_alt,
                     uint64_t n, int end_bit, bool vals_iota, bool host_skip = true);
 bool radix_sort_u64(Ctx& ctx, uint64_t* keys, uint64_t* keys_alt, uint32_t* vals, uint32_t* vals_alt,
