@@ -1,62 +1,145 @@
 // Permutation-index construction (hot path a).
 //
-// For each permutation (k0, k1, k2) of (s, p, o) the three uint32 columns are
-// packed into one 64-bit key (k0 | k1 | k2 at their measured bit widths),
-// radix-sorted, and a single fused pass unpacks the sorted keys into the data
-// columns and run-length encodes the level-1 (k0) and level-2 (k0, k1)
-// boundaries into (value, first row) arrays -- the reduce_by_key + exclusive
-// scan pair of the reference -- with a decoupled look-back for the output
-// positions.
+// The three uint32 columns of the triples are packed into one 64-bit key,
+// whose fields every sort takes as they lie: a permutation is the result of
+// stable radix sorts by single fields, each starting from the last one's
+// order.  (p, s) order comes first, from the digits of s and p only; the
+// objects of each (p, s) group, usually a few, are put in order by the kernel
+// that unpacks PSO.  From there
+//   by o: (o, p, s) = OPS,  by p: (p, o, s) = POS,  by s: (s, p, o) = SPO,
+//   by o: (o, s, p) = OSP,  by s: (s, o, p) = SOP.
+// Sorting each permutation by its whole key took 12 passes over 100M triples
+// (7 for PSO, 5 for POS from PSO) where this takes 8, and 40 where it takes
+// 15 for the full index of 3M triples.
+//
+// One fused pass per permutation unpacks the sorted keys into the data
+// columns and run-length encodes the level-1 and level-2 boundaries into
+// (value, first row) arrays -- the reduce_by_key + exclusive scan pair of the
+// reference -- with a decoupled look-back for the output positions.
 #include "vg_index.h"
 
 #include <algorithm>
+#include <optional>
 
 #include "vg_prims.cuh"
+#include "vg_radix.cuh"
 #include "vg_sort.h"
 
 namespace vg {
 namespace {
 
 constexpr int kBlock = 256;
-constexpr int kRows = 8;                 // rows per thread (blocked)
+constexpr int kRows = 8;                 // rows per thread, 32 apart
 constexpr int kTileRows = kBlock * kRows;
-static_assert(kRows % 4 == 0, "unpack_rle_kernel moves a thread's rows in 16-byte pieces");
+constexpr uint32_t kGroupMax = 64;       // groups of more rows are sorted apart (big_* below)
 
-__global__ void max3_kernel(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b,
-                            const uint32_t* __restrict__ c, uint64_t n, uint32_t* out3) {
-  uint32_t ma = 0, mb = 0, mc = 0;
+// Ids from this one on are literals (src/vedas.h:31); between the largest
+// entity id and them lies an unused range, which the packed keys leave out.
+constexpr uint32_t kLiteralStart = 50000000u;
+
+// out4: the maxima of a, b and c, and c's among the ids below the literals,
+// plus one (0: none).  Columns are read in 16-byte pieces where they are
+// aligned.
+__global__ void max4_kernel(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b,
+                            const uint32_t* __restrict__ c, uint64_t n, uint32_t* out4) {
+  uint32_t ma = 0, mb = 0, mc = 0, ml = 0;
+  auto low = [&](uint32_t v) {
+    if (v < kLiteralStart) ml = max(ml, v + 1);
+  };
+  const uint64_t t = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
+  uint64_t nv = 0;
+  if (((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15u) == 0) {
+    nv = n / 4;
+    for (uint64_t i = t; i < nv; i += stride) {
+      const uint4 x = reinterpret_cast<const uint4*>(a)[i];
+      const uint4 y = reinterpret_cast<const uint4*>(b)[i];
+      const uint4 z = reinterpret_cast<const uint4*>(c)[i];
+      ma = max(ma, max(max(x.x, x.y), max(x.z, x.w)));
+      mb = max(mb, max(max(y.x, y.y), max(y.z, y.w)));
+      mc = max(mc, max(max(z.x, z.y), max(z.z, z.w)));
+      low(z.x), low(z.y), low(z.z), low(z.w);
+    }
+  }
+  for (uint64_t i = nv * 4 + t; i < n; i += stride) {
     ma = max(ma, a[i]);
     mb = max(mb, b[i]);
     mc = max(mc, c[i]);
+    low(c[i]);
   }
   for (int d = 16; d > 0; d >>= 1) {
     ma = max(ma, __shfl_xor_sync(0xffffffffu, ma, d));
     mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, d));
     mc = max(mc, __shfl_xor_sync(0xffffffffu, mc, d));
+    ml = max(ml, __shfl_xor_sync(0xffffffffu, ml, d));
   }
   if ((threadIdx.x & 31) == 0) {
-    atomicMax(&out3[0], ma);
-    atomicMax(&out3[1], mb);
-    atomicMax(&out3[2], mc);
+    atomicMax(&out4[0], ma);
+    atomicMax(&out4[1], mb);
+    atomicMax(&out4[2], mc);
+    atomicMax(&out4[3], ml);
   }
 }
 
-__global__ void pack_kernel(const uint32_t* __restrict__ k0, const uint32_t* __restrict__ k1,
-                            const uint32_t* __restrict__ k2, uint64_t n, uint32_t sh0, uint32_t sh1,
-                            uint64_t* __restrict__ keys) {
-  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
-    keys[i] = (static_cast<uint64_t>(k0[i]) << sh0) | (static_cast<uint64_t>(k1[i]) << sh1) |
-              static_cast<uint64_t>(k2[i]);
+// A field of the packed key: (key >> shift) & mask is the column's value,
+// less `add` from `thr` on (the objects' unused range left out).
+struct Field {
+  uint32_t shift, mask, thr, add;
+  __host__ __device__ uint64_t bits_of() const { return static_cast<uint64_t>(mask) << shift; }
+  __device__ __forceinline__ uint32_t get(uint64_t key) const {
+    const uint32_t v = static_cast<uint32_t>(key >> shift) & mask;
+    return v >= thr ? v + add : v;
+  }
+  __device__ __forceinline__ uint64_t put(uint32_t v) const {
+    return static_cast<uint64_t>(add && v >= kLiteralStart ? v - add : v) << shift;
+  }
+};
+
+// Packed keys and the digit counts of every sort that follows (counts do not
+// depend on the order of the keys): one read of the columns instead of a
+// second one of the keys.
+__global__ void __launch_bounds__(kBlock) pack_count_kernel(const uint32_t* __restrict__ s,
+                                                            const uint32_t* __restrict__ p,
+                                                            const uint32_t* __restrict__ o, uint64_t n, Field fs,
+                                                            Field fp, Field fo, uint64_t* __restrict__ keys,
+                                                            DigitList dl, unsigned long long* __restrict__ hist,
+                                                            uint64_t* __restrict__ bases, uint32_t* done) {
+  extern __shared__ uint32_t sh[];   // [dl.n][kRadixValues]
+  digit_counts_init<kBlock>(dl, sh);
+  auto pack = [&](uint32_t vs, uint32_t vp, uint32_t vo) { return fs.put(vs) | fp.put(vp) | fo.put(vo); };
+  const uint64_t t = static_cast<uint64_t>(blockIdx.x) * kBlock + threadIdx.x;
+  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * kBlock;
+  uint64_t nv = 0;
+  if (((reinterpret_cast<uintptr_t>(s) | reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(o)) & 15u) == 0) {
+    nv = n / 4;
+    for (uint64_t i = t; i < nv; i += stride) {
+      const uint4 x = reinterpret_cast<const uint4*>(s)[i];
+      const uint4 y = reinterpret_cast<const uint4*>(p)[i];
+      const uint4 z = reinterpret_cast<const uint4*>(o)[i];
+      const uint64_t k0 = pack(x.x, y.x, z.x), k1 = pack(x.y, y.y, z.y);
+      const uint64_t k2 = pack(x.z, y.z, z.z), k3 = pack(x.w, y.w, z.w);
+      ulonglong2* out = reinterpret_cast<ulonglong2*>(keys + 4 * i);
+      out[0] = make_ulonglong2(k0, k1);
+      out[1] = make_ulonglong2(k2, k3);
+      digit_counts_add(dl, sh, k0);
+      digit_counts_add(dl, sh, k1);
+      digit_counts_add(dl, sh, k2);
+      digit_counts_add(dl, sh, k3);
+    }
+  }
+  for (uint64_t i = nv * 4 + t; i < n; i += stride) {
+    const uint64_t k = pack(s[i], p[i], o[i]);
+    keys[i] = k;
+    digit_counts_add(dl, sh, k);
+  }
+  digit_counts_finish<kBlock>(dl, sh, hist, bases, done);
 }
 
 struct UnpackArgs {
   const uint64_t* keys;
   uint64_t n;
-  uint32_t sh0, sh1;       // k0 = key >> sh0, k1 = (key >> sh1) & m1, k2 = key & m2
-  uint64_t m1, m2;
+  Field f0, f1, f2;
+  uint64_t m1, m2;         // key bits of (k0) and of (k0, k1): equal within a level-1 / level-2 run
   uint32_t* col1;          // k1 per row (nullable)
   uint32_t* col2;          // k2 per row (nullable)
   uint32_t* l1_vals;       // level-1 run values (k0) (nullable)
@@ -66,256 +149,442 @@ struct UnpackArgs {
   uint64_t* status1;
   uint64_t* status2;
   uint32_t* ticket;
-  uint64_t* counts;        // [0] level-1 runs, [1] level-2 runs
+  uint64_t* counts;        // [0] level-1 runs, [1] level-2 runs, [2] not 0: a group of more than kGroupMax rows
   uint64_t tiles;
   DeviceErrors* err;
 };
 
+// A tile is 2048 rows; a warp takes 256 consecutive ones, 32 at a time, so
+// loads, column stores and (as nearly every row starts a level-2 run) run
+// stores are all coalesced: 100M PSO + POS rows took 1.86 ms with eight
+// consecutive rows per thread and the column stores behind the look-back.
+// While warp 0 looks back the other warps store their columns.
+//
+// GROUPS: the rows of a level-2 group come in any order of k2 and col2 gets
+// them in ascending order, for groups of at most kGroupMax rows: k2 and the
+// run heads of the tile and of 64 rows on either side lie in shared memory,
+// and a row's place is the number of rows of its group that go before it.
+// Groups average a few rows (the objects of one subject and predicate); a
+// longer one keeps its order and sets counts[2].
+template <bool GROUPS>
 __global__ void __launch_bounds__(kBlock) unpack_rle_kernel(UnpackArgs a) {
-  __shared__ uint32_t s_scan[kBlock / 32 + 1];
-  __shared__ uint64_t s_b;
+  constexpr uint32_t kHalo = kGroupMax, kWarps = kBlock / 32;
+  __shared__ uint32_t s_cnt[kWarps];
+  __shared__ uint64_t s_b[2];
   __shared__ uint32_t s_tile;
+  __shared__ uint32_t s_k2[GROUPS ? kTileRows + 2 * kHalo : 1];
+  __shared__ uint32_t s_head[GROUPS ? (kTileRows + 2 * kHalo) / 32 : 1];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) s_tile = atomicAdd(a.ticket, 1u);
   __syncthreads();
   const uint32_t tile = s_tile;
-  const uint64_t r0 = static_cast<uint64_t>(tile) * kTileRows + threadIdx.x * kRows;
+  const uint64_t t0 = static_cast<uint64_t>(tile) * kTileRows;
+  const uint64_t r0 = t0 + warp * (32u * kRows) + lane;
 
   uint64_t key[kRows];
-  if (r0 + kRows <= a.n) {
-    // the thread's rows are consecutive and 64-byte aligned (r0 is a multiple
-    // of kRows, the keys an arena block): 16-byte loads
 #pragma unroll
-    for (int i = 0; i < kRows; i += 2) {
-      const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(a.keys + r0 + i);
-      key[i] = v.x;
-      key[i + 1] = v.y;
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < kRows; ++i) key[i] = (r0 + i < a.n) ? a.keys[r0 + i] : 0ull;
-  }
-  uint64_t prev = (r0 > 0 && r0 - 1 < a.n) ? a.keys[r0 - 1] : 0ull;
-  uint32_t f1 = 0, f2 = 0;
-#pragma unroll
-  for (int i = 0; i < kRows; ++i) {
-    const uint64_t r = r0 + i;
-    if (r < a.n) {
-      const uint64_t pv = (i == 0) ? prev : key[i - 1];
-      if (r == 0 || (key[i] >> a.sh0) != (pv >> a.sh0)) f1 |= 1u << i;
-      if (r == 0 || (key[i] >> a.sh1) != (pv >> a.sh1)) f2 |= 1u << i;
-    }
-  }
-  // both levels' run counts in one scan (a tile has at most kTileRows < 2^16
-  // of each) and, when the row count allows, one look-back over both
-  // (level 1 above bit 31, level 2 below)
-  uint32_t tt;
-  const uint32_t ee = block_excl_scan<kBlock>((__popc(f1) << 16) | __popc(f2), tt, s_scan);
-  const uint32_t e1 = ee >> 16, e2 = ee & 0xFFFFu, t1 = tt >> 16, t2 = tt & 0xFFFFu;
-  uint64_t g1 = 0, g2 = 0;
-  if (a.l1_vals && a.l2_vals && a.n < (1ull << 31)) {
-    const uint64_t g = block_lookback(a.status1, tile, (static_cast<uint64_t>(t1) << 31) | t2, a.err, &s_b);
-    g1 = g >> 31;
-    g2 = g & ((1ull << 31) - 1);
-  } else {
-    g1 = a.l1_vals ? block_lookback(a.status1, tile, t1, a.err, &s_b) : 0;
-    g2 = a.l2_vals ? block_lookback(a.status2, tile, t2, a.err, &s_b) : 0;
-  }
-  static_assert(kTileRows < (1 << 16), "a tile's run counts fit 16 bits each");
-  if (tile == a.tiles - 1 && threadIdx.x == 0) {
-    a.counts[0] = g1 + t1;
-    a.counts[1] = g2 + t2;
-  }
-  if (r0 + kRows <= a.n) {
-    // the columns' words of the thread's rows: 16-byte stores (32-byte aligned)
-    uint32_t w1[kRows], w2[kRows];
-#pragma unroll
-    for (int i = 0; i < kRows; ++i) {
-      w1[i] = static_cast<uint32_t>((key[i] >> a.sh1) & a.m1);
-      w2[i] = static_cast<uint32_t>(key[i] & a.m2);
-    }
-#pragma unroll
-    for (int i = 0; i < kRows; i += 4) {
-      if (a.col1) *reinterpret_cast<uint4*>(a.col1 + r0 + i) = make_uint4(w1[i], w1[i + 1], w1[i + 2], w1[i + 3]);
-      if (a.col2) *reinterpret_cast<uint4*>(a.col2 + r0 + i) = make_uint4(w2[i], w2[i + 1], w2[i + 2], w2[i + 3]);
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < kRows; ++i) {
-      const uint64_t r = r0 + i;
-      if (r >= a.n) break;
-      if (a.col1) a.col1[r] = static_cast<uint32_t>((key[i] >> a.sh1) & a.m1);
-      if (a.col2) a.col2[r] = static_cast<uint32_t>(key[i] & a.m2);
-    }
-  }
+  for (int i = 0; i < kRows; ++i) key[i] = r0 + i * 32u < a.n ? a.keys[r0 + i * 32u] : 0ull;
+  uint64_t before = (lane == 0 && r0 > 0 && r0 <= a.n) ? a.keys[r0 - 1] : 0ull;
+  uint32_t h1[kRows], h2[kRows];   // the warp's run heads, bit = lane
   uint32_t c1 = 0, c2 = 0;
 #pragma unroll
   for (int i = 0; i < kRows; ++i) {
-    const uint64_t r = r0 + i;
-    if (r >= a.n) break;
-    const uint32_t v0 = static_cast<uint32_t>(key[i] >> a.sh0);
-    const uint32_t v1 = static_cast<uint32_t>((key[i] >> a.sh1) & a.m1);
-    if (a.l1_vals && (f1 >> i & 1u)) {
-      const uint64_t o = g1 + e1 + c1++;
-      a.l1_vals[o] = v0;
-      a.l1_offs[o] = static_cast<uint32_t>(r);
+    const uint64_t r = r0 + i * 32u;
+    uint64_t pv = __shfl_up_sync(0xffffffffu, key[i], 1);
+    if (lane == 0) pv = before;
+    before = __shfl_sync(0xffffffffu, key[i], 31);
+    const uint64_t x = key[i] ^ pv;
+    h1[i] = __ballot_sync(0xffffffffu, r < a.n && (r == 0 || (x & a.m1)));
+    h2[i] = __ballot_sync(0xffffffffu, r < a.n && (r == 0 || (x & a.m2)));
+    c1 += __popc(h1[i]);
+    c2 += __popc(h2[i]);
+  }
+  static_assert(kTileRows < (1 << 16), "a tile's run counts fit 16 bits each");
+  if (lane == 0) s_cnt[warp] = (c1 << 16) | c2;
+  if (GROUPS) {
+    // rows past the end count as heads (they end the last group)
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      const uint32_t x = kHalo + warp * (32u * kRows) + i * 32u;
+      s_k2[x + lane] = static_cast<uint32_t>(key[i] >> a.f2.shift) & a.f2.mask;
+      const uint32_t past = __ballot_sync(0xffffffffu, r0 + i * 32u >= a.n);
+      if (lane == 0) s_head[x / 32] = h2[i] | past;
     }
-    if (a.l2_vals && (f2 >> i & 1u)) {
-      const uint64_t o = g2 + e2 + c2++;
-      a.l2_vals[o] = v1;
-      a.l2_offs[o] = static_cast<uint32_t>(r);
+    if (warp < 4) {
+      // two warps for the 64 rows before the tile, two for those after it
+      const uint32_t x = warp < 2 ? warp * 32u : kHalo + kTileRows + (warp - 2) * 32u;
+      const bool in = t0 + x + lane >= kHalo && t0 + x + lane - kHalo < a.n;
+      const uint64_t r = t0 + x + lane - kHalo;
+      const uint64_t k = in ? a.keys[r] : 0ull;
+      const uint64_t pv = in && r > 0 ? a.keys[r - 1] : 0ull;
+      s_k2[x + lane] = static_cast<uint32_t>(k >> a.f2.shift) & a.f2.mask;
+      const uint32_t h = __ballot_sync(0xffffffffu, !in || r == 0 || ((k ^ pv) & a.m2));
+      if (lane == 0) s_head[x / 32] = h;
     }
+  }
+  __syncthreads();
+  uint32_t pre = 0, all = 0;
+#pragma unroll
+  for (uint32_t w = 0; w < kWarps; ++w) {
+    if (w < warp) pre += s_cnt[w];
+    all += s_cnt[w];
+  }
+  const uint32_t t1 = all >> 16, t2 = all & 0xFFFFu;
+  if (warp == 0) {
+    // one look-back over both levels where the row count allows it (level 1
+    // above bit 31, level 2 below)
+    uint64_t g1 = 0, g2 = 0;
+    if (a.l1_vals && a.l2_vals && a.n < (1ull << 31)) {
+      const uint64_t g = warp_lookback(a.status1, tile, (static_cast<uint64_t>(t1) << 31) | t2, a.err);
+      g1 = g >> 31;
+      g2 = g & ((1ull << 31) - 1);
+    } else {
+      if (a.l1_vals) g1 = warp_lookback(a.status1, tile, t1, a.err);
+      if (a.l2_vals) g2 = warp_lookback(a.status2, tile, t2, a.err);
+    }
+    if (lane == 0) {
+      s_b[0] = g1;
+      s_b[1] = g2;
+      if (tile == a.tiles - 1) {
+        a.counts[0] = g1 + t1;
+        a.counts[1] = g2 + t2;
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) {
+    const uint64_t r = r0 + i * 32u;
+    if (r < a.n && a.col1) a.col1[r] = a.f1.get(key[i]);
+    if (!GROUPS && r < a.n && a.col2) a.col2[r] = a.f2.get(key[i]);
+  }
+  if (GROUPS) {
+#pragma unroll 1
+    for (int i = 0; i < kRows; ++i) {
+      const uint64_t r = t0 + warp * (32u * kRows) + i * 32u + lane;
+      if (r >= a.n) break;
+      const uint32_t x = kHalo + warp * (32u * kRows) + i * 32u + lane, w = x >> 5;
+      const uint32_t upto = 0xffffffffu >> (31u - lane);   // bits 0..lane (x & 31 == lane)
+      // [b, e): the group, as far as it lies within 64 rows of this one
+      uint32_t b = 0, e = 0xffffffffu;
+      if (s_head[w] & upto) b = w * 32 + 31 - __clz(s_head[w] & upto);
+      else if (s_head[w - 1]) b = w * 32 - 1 - __clz(s_head[w - 1]);
+      else if (s_head[w - 2]) b = w * 32 - 33 - __clz(s_head[w - 2]);
+      if (s_head[w] & ~upto) e = w * 32 + __ffs(s_head[w] & ~upto) - 1;
+      else if (s_head[w + 1]) e = w * 32 + 31 + __ffs(s_head[w + 1]);
+      else if (s_head[w + 2]) e = w * 32 + 63 + __ffs(s_head[w + 2]);
+      const uint32_t mine = s_k2[x];
+      uint32_t at = x;
+      // (b == 0 is not a found head: a group that starts there and holds this
+      // row, 64 rows on or more, is too long)
+      if (b != 0 && e != 0xffffffffu && e - b <= kGroupMax) {
+        at = b;
+        for (uint32_t j = b; j < e; ++j) {
+          const uint32_t v = s_k2[j];
+          at += (v < mine || (v == mine && j < x)) ? 1u : 0u;
+        }
+      } else {
+        a.counts[2] = 1;
+      }
+      if (a.col2) a.col2[t0 + at - kHalo] = mine >= a.f2.thr ? mine + a.f2.add : mine;
+    }
+  }
+  __syncthreads();
+  uint64_t o1 = s_b[0] + (pre >> 16), o2 = s_b[1] + (pre & 0xFFFFu);
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) {
+    const uint64_t r = r0 + i * 32u;
+    if (a.l1_vals && (h1[i] >> lane & 1u)) {
+      const uint64_t q = o1 + __popc(h1[i] & lanemask_lt());
+      a.l1_vals[q] = a.f0.get(key[i]);
+      a.l1_offs[q] = static_cast<uint32_t>(r);
+    }
+    if (a.l2_vals && (h2[i] >> lane & 1u)) {
+      const uint64_t q = o2 + __popc(h2[i] & lanemask_lt());
+      a.l2_vals[q] = a.f1.get(key[i]);
+      a.l2_offs[q] = static_cast<uint32_t>(r);
+    }
+    o1 += __popc(h1[i]);
+    o2 += __popc(h2[i]);
   }
 }
 
-// (k0, k1, k2) keys packed at widths (b0, b1, b2) repacked as (k0, k2, k1).
-__global__ void repack_swap12_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, uint64_t n,
-                                     uint32_t b1, uint32_t b2) {
-  const uint64_t m1 = (1ull << b1) - 1, m2 = (1ull << b2) - 1;
+// Groups of more than kGroupMax rows: listed (start row, first row among the
+// rows of all such groups), their values sorted by (list position, value) and
+// put back.  The packed counter (groups above bit 36, rows below) makes list
+// order and row order agree.
+struct BigGroups {
+  unsigned long long* packed;
+  uint32_t* start;
+  uint64_t* at;
+};
+
+__global__ void big_list_kernel(const uint32_t* __restrict__ offs, uint64_t runs, uint64_t n, BigGroups g) {
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
-    const uint64_t k = in[i];
-    const uint64_t k2 = k & m2, k1 = (k >> b2) & m1, k0 = k >> (b1 + b2);
-    out[i] = (k0 << (b1 + b2)) | (k2 << b1) | k1;
+  for (uint64_t r = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; r < runs; r += stride) {
+    const uint64_t b = offs[r], e = r + 1 < runs ? offs[r + 1] : n;
+    if (e - b <= kGroupMax) continue;
+    const unsigned long long old = atomicAdd(g.packed, (1ull << 36) | (e - b));
+    g.start[old >> 36] = static_cast<uint32_t>(b);
+    g.at[old >> 36] = old & ((1ull << 36) - 1);
   }
 }
 
-int bits_for(uint32_t maxv) { return maxv == 0 ? 1 : 32 - __builtin_clz(maxv); }
+// SCATTER: the sorted values back to the column; else the keys from it.
+template <bool SCATTER>
+__global__ void big_move_kernel(const uint32_t* __restrict__ start, const uint64_t* __restrict__ at, uint64_t groups,
+                                uint64_t rows, uint32_t bits, uint32_t* __restrict__ col,
+                                uint64_t* __restrict__ keys) {
+  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < rows; i += stride) {
+    const uint64_t g = upper_bound_dev(at, 0, groups, i) - 1;
+    uint32_t* c = col + start[g] + (i - at[g]);
+    if (SCATTER) *c = static_cast<uint32_t>(keys[i] & ((1ull << bits) - 1));
+    else keys[i] = (g << bits) | *c;
+  }
+}
 
-unsigned grid_for(const Ctx& ctx, uint64_t n, int per_thread) {
+int bits_for(uint64_t maxv) { return maxv == 0 ? 1 : 64 - __builtin_clzll(maxv); }
+int passes_for(int bits) { return (bits + 7) / 8; }
+
+unsigned grid_for(const Ctx& ctx, uint64_t n, int per_thread, int per_sm = 16) {
   uint64_t g = div_up(n, static_cast<uint64_t>(kBlock) * per_thread);
-  const uint64_t gmax = static_cast<uint64_t>(ctx.num_sms) * 16;
+  const uint64_t gmax = static_cast<uint64_t>(ctx.num_sms) * per_sm;
   if (g > gmax) g = gmax;
   return static_cast<unsigned>(g < 1 ? 1 : g);
 }
+
+void column_max4(Ctx& ctx, const uint32_t* a, const uint32_t* b, const uint32_t* c, uint64_t n, uint32_t out[4]) {
+  Scratch<uint32_t> d(ctx, 4);
+  VG_CUDA(cudaMemsetAsync(d.get(), 0, 4 * sizeof(uint32_t), ctx.stream));
+  if (n) {
+    ctx.launch("column_max", 12.0 * n,
+               [&] { max4_kernel<<<grid_for(ctx, n, 16, 8), kBlock, 0, ctx.stream>>>(a, b, c, n, d.get()); });
+    VG_CUDA(cudaGetLastError());
+  }
+  VG_CUDA(cudaMemcpyAsync(ctx.h_small, d.get(), 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx.stream));
+  ctx.sync();
+  for (int i = 0; i < 4; ++i) out[i] = reinterpret_cast<const uint32_t*>(ctx.h_small)[i];
+}
+
+// The packed keys of one build and the sorts and unpackings over them.
+class Permuter {
+ public:
+  enum Col { S, P, O };
+
+  Permuter(Ctx& ctx, const uint32_t* s, const uint32_t* p, const uint32_t* o, uint64_t n, const uint32_t mx[4],
+           bool full)
+      : ctx_(ctx), n_(n), max_o_(mx[2]) {
+    // objects without the unused range below the literals
+    const bool lits = mx[2] >= kLiteralStart;
+    const uint32_t cut = lits ? kLiteralStart - mx[3] : 0;
+    const int bs = bits_for(mx[0]), bp = bits_for(mx[1]), bo = bits_for(mx[2] - cut);
+    // p on top; whichever of s and o lies below it shares its digits with p
+    // where that saves a pass of a two-column sort
+    const int apart = passes_for(bp);
+    const int with_s = passes_for(bs + bp) + passes_for(bo) + apart, with_o = passes_for(bs) + apart + passes_for(bo + bp);
+    const bool s_next = full || with_s <= with_o;
+    const int at_s = s_next ? bo : 0, at_o = s_next ? 0 : bs, at_p = bs + bo;
+    auto mask = [](int bits) { return static_cast<uint32_t>((1ull << bits) - 1); };
+    f_[S] = {static_cast<uint32_t>(at_s), mask(bs), 0xffffffffu, 0};
+    f_[P] = {static_cast<uint32_t>(at_p), mask(bp), 0xffffffffu, 0};
+    f_[O] = {static_cast<uint32_t>(at_o), mask(bo), lits ? mx[3] : 0xffffffffu, cut};
+    plan({S}, at_s, at_s + bs);
+    plan({P}, at_p, at_p + bp);
+    plan({O}, at_o, at_o + bo);
+    const Col low = s_next ? S : O;
+    const int at_low = s_next ? at_s : at_o, b_low = s_next ? bs : bo;
+    if (passes_for(b_low + bp) < passes_for(b_low) + apart) plan({low, P}, at_low, at_p + bp);
+
+    DigitList dl{};
+    for (const Sort& q : sorts_)
+      for (const RadixDigit& d : q.digits) dl.d[dl.n++] = d;
+    const size_t hist_bytes = dl.n * kRadixValues * sizeof(uint64_t);
+    counts_.emplace(ctx, 2 * hist_bytes + 128);
+    char* sc = counts_->get();
+    auto* hist = reinterpret_cast<unsigned long long*>(sc + 128);
+    auto* bases = reinterpret_cast<uint64_t*>(sc + 128 + hist_bytes);
+    VG_CUDA(cudaMemsetAsync(sc, 0, 128 + hist_bytes, ctx.stream));
+    uint32_t at = 0;
+    for (Sort& q : sorts_)
+      for (size_t d = 0; d < q.digits.size(); ++d) q.bases.push_back(bases + kRadixValues * at++);
+    keys_.emplace(ctx, n);
+    ctx.launch("index_pack", 20.0 * n, [&] {
+      pack_count_kernel<<<grid_for(ctx, n, 16, 8), kBlock, dl.n * kRadixValues * sizeof(uint32_t), ctx.stream>>>(
+          s, p, o, n, f_[S], f_[P], f_[O], keys_->get(), dl, hist, bases, reinterpret_cast<uint32_t*>(sc));
+    });
+    VG_CUDA(cudaGetLastError());
+  }
+  Permuter(const Permuter&) = delete;
+  Permuter& operator=(const Permuter&) = delete;
+
+  // Stable sort of the keys by the columns, the last named counting most.
+  void sort_by(const std::vector<Col>& cols) {
+    std::vector<RadixDigit> digits;
+    std::vector<const uint64_t*> bases;
+    auto take = [&](const std::vector<Col>& c) {
+      for (const Sort& q : sorts_)
+        if (q.cols == c) {
+          digits.insert(digits.end(), q.digits.begin(), q.digits.end());
+          bases.insert(bases.end(), q.bases.begin(), q.bases.end());
+          return true;
+        }
+      return false;
+    };
+    if (!take(cols))
+      for (Col c : cols) take({c});
+    Scratch<uint64_t> alt(ctx_, n_);
+    if (radix_sort_u64_counted(ctx_, keys_->get(), alt.get(), n_, digits, bases)) std::swap(keys_->p, alt.p);
+  }
+
+  // The requested outputs of the keys as (c0, c1, c2); groups: the keys are
+  // in (c0, c1) order only.
+  void unpack(Col c0, Col c1, Col c2, PermOutputs& out, bool groups = false) {
+    Ctx& ctx = ctx_;
+    const uint64_t n = n_;
+    UnpackArgs a{};
+    a.keys = keys_->get();
+    a.n = n;
+    a.f0 = f_[c0];
+    a.f1 = f_[c1];
+    a.f2 = f_[c2];
+    a.m1 = a.f0.bits_of();
+    a.m2 = a.m1 | a.f1.bits_of();
+    a.col1 = out.want_col1 ? ctx.alloc<uint32_t>(n) : nullptr;
+    a.col2 = out.want_col2 ? ctx.alloc<uint32_t>(n) : nullptr;
+    a.l1_vals = out.want_l1 ? ctx.alloc<uint32_t>(n) : nullptr;
+    a.l1_offs = out.want_l1 ? ctx.alloc<uint32_t>(n) : nullptr;
+    a.l2_vals = out.want_l2 ? ctx.alloc<uint32_t>(n) : nullptr;
+    a.l2_offs = out.want_l2 ? ctx.alloc<uint32_t>(n) : nullptr;
+    a.tiles = div_up(n, kTileRows);
+    // counts, ticket and both levels' look-back words, zeroed together
+    Scratch<uint64_t> z(ctx, 4 + 2 * a.tiles);
+    VG_CUDA(cudaMemsetAsync(z.get(), 0, (4 + 2 * a.tiles) * sizeof(uint64_t), ctx.stream));
+    a.counts = z.get();
+    a.ticket = reinterpret_cast<uint32_t*>(z.get() + 3);
+    a.status1 = z.get() + 4;
+    a.status2 = z.get() + 4 + a.tiles;
+    a.err = ctx.d_err;
+    const double ub = 8.0 * n + 4.0 * n * ((a.col1 ? 1 : 0) + (a.col2 ? 1 : 0));
+    ctx.launch("index_unpack_rle", ub, [&] {
+      if (groups) unpack_rle_kernel<true><<<static_cast<unsigned>(a.tiles), kBlock, 0, ctx.stream>>>(a);
+      else unpack_rle_kernel<false><<<static_cast<unsigned>(a.tiles), kBlock, 0, ctx.stream>>>(a);
+    });
+    VG_CUDA(cudaGetLastError());
+    VG_CUDA(cudaMemcpyAsync(ctx.h_small, z.get(), 3 * sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx.stream));
+    ctx.sync();
+    const uint64_t hc[3] = {ctx.h_small[0], ctx.h_small[1], ctx.h_small[2]};
+    ctx.check_device_errors();
+    out.col1 = DevArray(a.col1, a.col1 ? n : 0);
+    out.col2 = DevArray(a.col2, a.col2 ? n : 0);
+    if (a.l1_vals) {
+      ctx.arena.shrink(a.l1_vals, hc[0] * 4);
+      ctx.arena.shrink(a.l1_offs, hc[0] * 4);
+      out.l1_vals = DevArray(a.l1_vals, hc[0]);
+      out.l1_offs = DevArray(a.l1_offs, hc[0]);
+    }
+    if (a.l2_vals) {
+      ctx.arena.shrink(a.l2_vals, hc[1] * 4);
+      ctx.arena.shrink(a.l2_offs, hc[1] * 4);
+      out.l2_vals = DevArray(a.l2_vals, hc[1]);
+      out.l2_offs = DevArray(a.l2_offs, hc[1]);
+    }
+    if (groups && hc[2]) sort_big_groups(out);
+  }
+
+ private:
+  struct Sort {
+    std::vector<Col> cols;
+    std::vector<RadixDigit> digits;
+    std::vector<const uint64_t*> bases;
+  };
+  Ctx& ctx_;
+  uint64_t n_;
+  uint32_t max_o_;
+  Field f_[3];
+  std::vector<Sort> sorts_;
+  std::optional<Scratch<char>> counts_;     // digit counts and bases of every sort
+  std::optional<Scratch<uint64_t>> keys_;   // the packed keys in their present order
+
+  void plan(const std::vector<Col>& cols, int begin, int end) {
+    Sort q;
+    q.cols = cols;
+    radix_plan(q.digits, begin, end);
+    sorts_.push_back(std::move(q));
+  }
+
+  // Orders col2 (objects) within the level-2 runs of more than kGroupMax rows.
+  void sort_big_groups(PermOutputs& out) {
+    Ctx& ctx = ctx_;
+    const uint64_t runs = out.l2_offs.len;
+    const uint64_t most = n_ / (kGroupMax + 1) + 1;
+    Scratch<uint32_t> start(ctx, most);
+    Scratch<uint64_t> at(ctx, most);
+    Scratch<unsigned long long> packed(ctx, 1);
+    VG_CUDA(cudaMemsetAsync(packed.get(), 0, sizeof(unsigned long long), ctx.stream));
+    ctx.launch("index_big_groups", 4.0 * runs, [&] {
+      big_list_kernel<<<grid_for(ctx, runs, 4), kBlock, 0, ctx.stream>>>(out.l2_offs.ptr, runs, n_,
+                                                                        {packed.get(), start.get(), at.get()});
+    });
+    VG_CUDA(cudaGetLastError());
+    VG_CUDA(cudaMemcpyAsync(ctx.h_small, packed.get(), sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx.stream));
+    ctx.sync();
+    const uint64_t groups = ctx.h_small[0] >> 36, rows = ctx.h_small[0] & ((1ull << 36) - 1);
+    if (groups == 0) return;
+    const int bo = bits_for(max_o_);
+    Scratch<uint64_t> kb(ctx, rows), ab(ctx, rows);
+    uint64_t *keys = kb.get(), *alt = ab.get();
+    ctx.launch("index_big_groups", 12.0 * rows, [&] {
+      big_move_kernel<false><<<grid_for(ctx, rows, 4), kBlock, 0, ctx.stream>>>(
+          start.get(), at.get(), groups, rows, static_cast<uint32_t>(bo), out.col2.ptr, keys);
+    });
+    VG_CUDA(cudaGetLastError());
+    if (radix_sort_u64(ctx, keys, alt, nullptr, nullptr, rows, bo + (groups > 1 ? bits_for(groups - 1) : 0), false))
+      std::swap(keys, alt);
+    ctx.launch("index_big_groups", 12.0 * rows, [&] {
+      big_move_kernel<true><<<grid_for(ctx, rows, 4), kBlock, 0, ctx.stream>>>(
+          start.get(), at.get(), groups, rows, static_cast<uint32_t>(bo), out.col2.ptr, keys);
+    });
+    VG_CUDA(cudaGetLastError());
+  }
+};
 
 }  // namespace
 
 void column_max3(Ctx& ctx, const uint32_t* a, const uint32_t* b, const uint32_t* c, uint64_t n,
                  uint32_t out[3]) {
-  Scratch<uint32_t> d(ctx, 3);
-  VG_CUDA(cudaMemsetAsync(d.get(), 0, 3 * sizeof(uint32_t), ctx.stream));
+  uint32_t m[4];
+  column_max4(ctx, a, b, c, n, m);
+  std::copy(m, m + 3, out);
+}
+
+uint32_t build_permutations(Ctx& ctx, const uint32_t* s, const uint32_t* p, const uint32_t* o, uint64_t n,
+                            Permutations& out, bool full) {
+  uint32_t mx[4];
+  column_max4(ctx, s, p, o, n, mx);
+  if (bits_for(mx[0]) + bits_for(mx[1]) + bits_for(mx[2]) > 64)
+    fail(VG_ERR_UNSUPPORTED, "triple ids need more than 64 key bits for the packed index sort");
   if (n) {
-    ctx.launch("column_max", 12.0 * n,
-               [&] { max3_kernel<<<grid_for(ctx, n, 8), kBlock, 0, ctx.stream>>>(a, b, c, n, d.get()); });
-    VG_CUDA(cudaGetLastError());
+    using C = Permuter;
+    Permuter keys(ctx, s, p, o, n, mx, full);
+    keys.sort_by({C::S, C::P});
+    keys.unpack(C::P, C::S, C::O, out.pso, true);
+    if (!full) {
+      keys.sort_by({C::O, C::P});
+      keys.unpack(C::P, C::O, C::S, out.pos);
+    } else {
+      keys.sort_by({C::O});
+      keys.unpack(C::O, C::P, C::S, out.ops);
+      keys.sort_by({C::P});
+      keys.unpack(C::P, C::O, C::S, out.pos);
+      keys.sort_by({C::S});
+      keys.unpack(C::S, C::P, C::O, out.spo);
+      keys.sort_by({C::O});
+      keys.unpack(C::O, C::S, C::P, out.osp);
+      keys.sort_by({C::S});
+      keys.unpack(C::S, C::O, C::P, out.sop);
+    }
   }
-  VG_CUDA(cudaMemcpyAsync(out, d.get(), 3 * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx.stream));
-  ctx.sync();
-}
-
-namespace {
-
-// Run-length encodes and unpacks sorted packed keys (widths b0, b1, b2) into
-// the requested outputs.
-void unpack_outputs(Ctx& ctx, const uint64_t* sorted, uint64_t n, int b0, int b1, int b2, PermOutputs& out) {
-  (void)b0;
-  const uint32_t sh1 = static_cast<uint32_t>(b2), sh0 = static_cast<uint32_t>(b1 + b2);
-  UnpackArgs a{};
-  a.keys = sorted;
-  a.n = n;
-  a.sh0 = sh0;
-  a.sh1 = sh1;
-  a.m1 = (b1 >= 64) ? ~0ull : ((1ull << b1) - 1);
-  a.m2 = (b2 >= 64) ? ~0ull : ((1ull << b2) - 1);
-  a.col1 = out.want_col1 ? ctx.alloc<uint32_t>(n) : nullptr;
-  a.col2 = out.want_col2 ? ctx.alloc<uint32_t>(n) : nullptr;
-  a.l1_vals = out.want_l1 ? ctx.alloc<uint32_t>(n) : nullptr;
-  a.l1_offs = out.want_l1 ? ctx.alloc<uint32_t>(n) : nullptr;
-  a.l2_vals = out.want_l2 ? ctx.alloc<uint32_t>(n) : nullptr;
-  a.l2_offs = out.want_l2 ? ctx.alloc<uint32_t>(n) : nullptr;
-  a.tiles = div_up(n, kTileRows);
-  Scratch<uint64_t> st1(ctx, a.tiles), st2(ctx, a.tiles), counts(ctx, 2);
-  Scratch<uint32_t> ticket(ctx, 1);
-  VG_CUDA(cudaMemsetAsync(st1.get(), 0, a.tiles * sizeof(uint64_t), ctx.stream));
-  VG_CUDA(cudaMemsetAsync(st2.get(), 0, a.tiles * sizeof(uint64_t), ctx.stream));
-  VG_CUDA(cudaMemsetAsync(counts.get(), 0, 2 * sizeof(uint64_t), ctx.stream));
-  VG_CUDA(cudaMemsetAsync(ticket.get(), 0, sizeof(uint32_t), ctx.stream));
-  a.status1 = st1.get();
-  a.status2 = st2.get();
-  a.ticket = ticket.get();
-  a.counts = counts.get();
-  a.err = ctx.d_err;
-  const double ub = 8.0 * n + 4.0 * n * ((a.col1 ? 1 : 0) + (a.col2 ? 1 : 0));
-  ctx.launch("index_unpack_rle", ub,
-             [&] { unpack_rle_kernel<<<static_cast<unsigned>(a.tiles), kBlock, 0, ctx.stream>>>(a); });
-  VG_CUDA(cudaGetLastError());
-  uint64_t hc[2];
-  VG_CUDA(cudaMemcpyAsync(hc, counts.get(), sizeof(hc), cudaMemcpyDeviceToHost, ctx.stream));
-  ctx.sync();
-  ctx.check_device_errors();
-  out.col1 = DevArray(a.col1, a.col1 ? n : 0);
-  out.col2 = DevArray(a.col2, a.col2 ? n : 0);
-  if (a.l1_vals) {
-    ctx.arena.shrink(a.l1_vals, hc[0] * 4);
-    ctx.arena.shrink(a.l1_offs, hc[0] * 4);
-    out.l1_vals = DevArray(a.l1_vals, hc[0]);
-    out.l1_offs = DevArray(a.l1_offs, hc[0]);
-  }
-  if (a.l2_vals) {
-    ctx.arena.shrink(a.l2_vals, hc[1] * 4);
-    ctx.arena.shrink(a.l2_offs, hc[1] * 4);
-    out.l2_vals = DevArray(a.l2_vals, hc[1]);
-    out.l2_offs = DevArray(a.l2_offs, hc[1]);
-  }
-}
-
-// Packs (k0, k1, k2) at widths (b0, b1, b2) and sorts the keys; returns the
-// sorted array (the caller frees it).
-uint64_t* sort_packed(Ctx& ctx, const uint32_t* k0, const uint32_t* k1, const uint32_t* k2, uint64_t n, int b0,
-                      int b1, int b2) {
-  const uint32_t sh1 = static_cast<uint32_t>(b2), sh0 = static_cast<uint32_t>(b1 + b2);
-  uint64_t* keys = ctx.alloc<uint64_t>(n);
-  uint64_t* keys_alt = ctx.alloc<uint64_t>(n);
-  ctx.launch("index_pack", 20.0 * n,
-             [&] { pack_kernel<<<grid_for(ctx, n, 8), kBlock, 0, ctx.stream>>>(k0, k1, k2, n, sh0, sh1, keys); });
-  VG_CUDA(cudaGetLastError());
-  const bool alt = radix_sort_u64(ctx, keys, keys_alt, nullptr, nullptr, n, b0 + b1 + b2, false);
-  ctx.free(alt ? keys : keys_alt);
-  return alt ? keys_alt : keys;
-}
-
-}  // namespace
-
-void build_permutation(Ctx& ctx, const uint32_t* k0, const uint32_t* k1, const uint32_t* k2,
-                       uint64_t n, const uint32_t maxes[3], PermOutputs& out) {
-  const int b0 = bits_for(maxes[0]), b1 = bits_for(maxes[1]), b2 = bits_for(maxes[2]);
-  if (b0 + b1 + b2 > 64)
-    fail(VG_ERR_UNSUPPORTED, "triple ids need more than 64 key bits for the packed index sort");
-  out.col1.clear();
-  out.col2.clear();
-  if (n == 0) return;
-  uint64_t* sorted = sort_packed(ctx, k0, k1, k2, n, b0, b1, b2);
-  unpack_outputs(ctx, sorted, n, b0, b1, b2, out);
-  ctx.free(sorted);
-}
-
-void build_permutation_pair(Ctx& ctx, const uint32_t* k0, const uint32_t* k1, const uint32_t* k2, uint64_t n,
-                            const uint32_t maxes[3], PermOutputs& first, PermOutputs& second) {
-  const int b0 = bits_for(maxes[0]), b1 = bits_for(maxes[1]), b2 = bits_for(maxes[2]);
-  if (b0 + b1 + b2 > 64)
-    fail(VG_ERR_UNSUPPORTED, "triple ids need more than 64 key bits for the packed index sort");
-  first.col1.clear();
-  first.col2.clear();
-  second.col1.clear();
-  second.col2.clear();
-  if (n == 0) return;
-  uint64_t* sorted = sort_packed(ctx, k0, k1, k2, n, b0, b1, b2);
-  unpack_outputs(ctx, sorted, n, b0, b1, b2, first);
-  // (k0, k2, k1) order from (k0, k1, k2) order: a stable sort by (k0, k2)
-  // alone keeps equal (k0, k2) keys in (k0, k1, k2) order, i.e. by k1
-  uint64_t* re = ctx.alloc<uint64_t>(n);
-  uint64_t* re_alt = ctx.alloc<uint64_t>(n);
-  ctx.launch("index_repack", 16.0 * n, [&] {
-    repack_swap12_kernel<<<grid_for(ctx, n, 8), kBlock, 0, ctx.stream>>>(sorted, re, n, static_cast<uint32_t>(b1),
-                                                                         static_cast<uint32_t>(b2));
-  });
-  VG_CUDA(cudaGetLastError());
-  ctx.free(sorted);
-  const bool alt = radix_sort_u64_bits(ctx, re, re_alt, n, b1, b0 + b1 + b2);
-  uint64_t* s2 = alt ? re_alt : re;
-  ctx.free(alt ? re : re_alt);
-  unpack_outputs(ctx, s2, n, b0, b2, b1, second);
-  ctx.free(s2);
+  return std::max(mx[0], std::max(mx[1], mx[2]));
 }
 
 }  // namespace vg

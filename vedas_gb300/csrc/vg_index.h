@@ -29,16 +29,16 @@ struct PermOutputs {
 void column_max3(Ctx& ctx, const uint32_t* a, const uint32_t* b, const uint32_t* c, uint64_t n,
                  uint32_t out[3]);
 
-// Sorts the triples (k0, k1, k2) lexicographically and emits the requested
-// outputs: col1/col2 = k1/k2 in sorted order, level-1 = (k0 run value, first
-// row), level-2 = (k1 of each (k0,k1) run, first row).
-void build_permutation(Ctx& ctx, const uint32_t* k0, const uint32_t* k1, const uint32_t* k2,
-                       uint64_t n, const uint32_t maxes[3], PermOutputs& out);
-// Two permutations sharing their leading column: (k0, k1, k2) into `first`
-// and (k0, k2, k1) into `second`, the second re-sorted from the first's
-// sorted keys by (k0, k2) bits only (fewer radix passes than a full sort).
-void build_permutation_pair(Ctx& ctx, const uint32_t* k0, const uint32_t* k1, const uint32_t* k2, uint64_t n,
-                            const uint32_t maxes[3], PermOutputs& first, PermOutputs& second);
+// The permutations of a build; pxy holds (x, y, z) order: col1/col2 = y/z in
+// sorted order, level-1 = (x run value, first row), level-2 = (y of each
+// (x, y) run, first row), as far as the want_* ask for them.  spo, sop, osp
+// and ops are made with the full index only.
+struct Permutations {
+  PermOutputs pso, pos, spo, sop, osp, ops;
+};
+// Sorts the triples into every permutation; returns the largest id.
+uint32_t build_permutations(Ctx& ctx, const uint32_t* s, const uint32_t* p, const uint32_t* o, uint64_t n,
+                            Permutations& out, bool full);
 
 // The resident permutation indexes in the reference's VedasStorage layout.
 struct Index {

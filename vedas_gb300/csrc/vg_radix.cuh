@@ -1,0 +1,56 @@
+// Digit counts of a radix sort, for kernels that read (or make) the keys
+// anyway: shared-memory counters per digit, added to global counts at the
+// end; the last block to finish turns them into bucket bases.
+#pragma once
+
+#include "vg_prims.cuh"
+#include "vg_sort.h"
+
+namespace vg {
+
+constexpr int kRadixValues = 256;   // counts and bases are kept for 256 values whatever a digit's width
+
+struct DigitList {
+  uint32_t n;
+  RadixDigit d[kRadixMaxPasses];
+};
+
+// s: dl.n * kRadixValues words of shared memory.
+template <int BLOCK>
+__device__ __forceinline__ void digit_counts_init(const DigitList& dl, uint32_t* s) {
+  for (uint32_t i = threadIdx.x; i < dl.n * kRadixValues; i += BLOCK) s[i] = 0;
+  __syncthreads();
+}
+
+template <typename K>
+__device__ __forceinline__ void digit_counts_add(const DigitList& dl, uint32_t* s, K key) {
+  for (uint32_t p = 0; p < dl.n; ++p)
+    atomicAdd(&s[p * kRadixValues + (static_cast<uint32_t>(key >> dl.d[p].shift) & ((1u << dl.d[p].bits) - 1u))], 1u);
+}
+
+// Every thread of every block calls it once, after its last key.  hist (zeroed
+// before the launch) receives the counts, bases[p][v] the first output row of
+// value v; done counts the blocks (zeroed).
+template <int BLOCK>
+__device__ __forceinline__ void digit_counts_finish(const DigitList& dl, const uint32_t* s, unsigned long long* hist,
+                                                    uint64_t* bases, uint32_t* done) {
+  static_assert(BLOCK == kRadixValues, "one thread per digit value");
+  __shared__ uint64_t s_scan[BLOCK / 32 + 1];
+  __shared__ bool s_last;
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < dl.n * kRadixValues; i += BLOCK)
+    if (s[i]) atomicAdd(&hist[i], static_cast<unsigned long long>(s[i]));
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  for (uint32_t p = 0; p < dl.n; ++p) {
+    const uint64_t c = ld_status_u64(reinterpret_cast<const uint64_t*>(&hist[p * kRadixValues + threadIdx.x]));
+    uint64_t tot;
+    bases[p * kRadixValues + threadIdx.x] = block_excl_scan64<BLOCK>(c, tot, s_scan);
+  }
+}
+
+}  // namespace vg

@@ -10,64 +10,44 @@
 #include "vg_sort.h"
 
 #include "vg_prims.cuh"
+#include "vg_radix.cuh"
 
 namespace vg {
 namespace {
 
 constexpr int kBlock = 256;
-constexpr int kRadix = 256;   // bases and counts are kept for 256 digit values whatever the digit's width
+constexpr int kRadix = kRadixValues;
 constexpr int kMaxPasses = kRadixMaxPasses;
 
-struct DigitList {
-  uint32_t n;
-  RadixDigit d[kMaxPasses];
-};
-
-// Digit counts of every pass in one read of the keys, then (the last block to
-// finish) each pass's exclusive scan: bases[p][v] = first output row of value
-// v.  Shared-memory counters, 16-byte loads.
+// Digit counts and bases of every pass in one read of the keys (16-byte
+// loads).
 template <typename K>
 __global__ void __launch_bounds__(kBlock) radix_hist_kernel(const K* __restrict__ keys, uint64_t n, DigitList dl,
                                                             unsigned long long* __restrict__ hist,
                                                             uint64_t* __restrict__ bases, uint32_t* done) {
   extern __shared__ uint32_t sh[];   // [dl.n][kRadix]
-  __shared__ uint64_t s_scan[kBlock / 32 + 1];
-  __shared__ bool s_last;
-  for (uint32_t i = threadIdx.x; i < dl.n * kRadix; i += kBlock) sh[i] = 0;
-  __syncthreads();
-  auto count = [&](K k) {
-    for (uint32_t p = 0; p < dl.n; ++p)
-      atomicAdd(&sh[p * kRadix + (static_cast<uint32_t>(k >> dl.d[p].shift) & ((1u << dl.d[p].bits) - 1u))], 1u);
-  };
+  digit_counts_init<kBlock>(dl, sh);
   constexpr uint32_t kVec = 16 / sizeof(K);
   const uint64_t t = static_cast<uint64_t>(blockIdx.x) * kBlock + threadIdx.x;
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * kBlock;
+  uint64_t nv = 0;
   if ((reinterpret_cast<uintptr_t>(keys) & 15u) == 0) {
-    const uint64_t nv = n / kVec;
+    nv = n / kVec;
     for (uint64_t i = t; i < nv; i += stride) {
+      const uint4 v = reinterpret_cast<const uint4*>(keys)[i];
       K k[kVec];
-      *reinterpret_cast<uint4*>(k) = reinterpret_cast<const uint4*>(keys)[i];
+      if constexpr (sizeof(K) == 8) {
+        k[0] = (static_cast<uint64_t>(v.y) << 32) | v.x;
+        k[1] = (static_cast<uint64_t>(v.w) << 32) | v.z;
+      } else {
+        k[0] = v.x, k[1] = v.y, k[2] = v.z, k[3] = v.w;
+      }
 #pragma unroll
-      for (uint32_t q = 0; q < kVec; ++q) count(k[q]);
+      for (uint32_t q = 0; q < kVec; ++q) digit_counts_add(dl, sh, k[q]);
     }
-    for (uint64_t i = nv * kVec + t; i < n; i += stride) count(keys[i]);
-  } else {
-    for (uint64_t i = t; i < n; i += stride) count(keys[i]);
   }
-  __syncthreads();
-  for (uint32_t i = threadIdx.x; i < dl.n * kRadix; i += kBlock)
-    if (sh[i]) atomicAdd(&hist[i], static_cast<unsigned long long>(sh[i]));
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(done, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  for (uint32_t p = 0; p < dl.n; ++p) {
-    const uint64_t c = ld_status_u64(reinterpret_cast<const uint64_t*>(&hist[p * kRadix + threadIdx.x]));
-    uint64_t tot;
-    bases[p * kRadix + threadIdx.x] = block_excl_scan64<kBlock>(c, tot, s_scan);
-  }
+  for (uint64_t i = nv * kVec + t; i < n; i += stride) digit_counts_add(dl, sh, keys[i]);
+  digit_counts_finish<kBlock>(dl, sh, hist, bases, done);
 }
 
 __global__ void iota_kernel(uint32_t* out, uint64_t n) {
@@ -350,44 +330,80 @@ int items_for(const Ctx& ctx, uint64_t n) {
   return n >= two * 8 && most > 8 ? 8 : 4;
 }
 
+// Tickets and look-back words of a list of passes, to be zeroed before them:
+// the tickets (and one more word for the caller), then each pass's words.
+struct PassScratch {
+  static constexpr size_t kHead = 128;
+  static_assert((kMaxPasses + 1) * sizeof(uint32_t) <= kHead, "tickets and the caller's word");
+  size_t bytes = kHead;
+  size_t at[kMaxPasses];
+  int items;
+  PassScratch(const Ctx& ctx, uint64_t n, const DigitList& dl) : items(items_for(ctx, n)) {
+    const uint64_t tiles = div_up(n, static_cast<uint64_t>(kBlock) * items);
+    const size_t word = wide_status(n) ? sizeof(uint64_t) : sizeof(uint32_t);
+    for (uint32_t p = 0; p < dl.n; ++p) {
+      at[p] = bytes;
+      bytes += tiles * status_row(dl.d[p].bits) * word;
+    }
+  }
+};
+
+DigitList digit_list(const std::vector<RadixDigit>& digits) {
+  if (digits.size() > kMaxPasses) fail(VG_ERR_INVALID, "radix sort: too many digits");
+  DigitList dl{};
+  dl.n = static_cast<uint32_t>(digits.size());
+  for (uint32_t p = 0; p < dl.n; ++p) dl.d[p] = digits[p];
+  return dl;
+}
+
+// The passes (those of `todo`, in order) over zeroed scratch; returns whether
+// the result is in the alternate buffers.
+template <typename K>
+bool run_passes(Ctx& ctx, K* keys, K* keys_alt, uint32_t* vals, uint32_t* vals_alt, uint64_t n, const DigitList& dl,
+                const uint64_t* const* bases, const std::vector<uint32_t>& todo, const PassScratch& ps, char* zeroed,
+                bool vals_iota) {
+  const bool has_v = vals != nullptr;
+  K* kin = keys;
+  K* kout = keys_alt;
+  uint32_t* vin = vals;
+  uint32_t* vout = vals_alt;
+  for (size_t t = 0; t < todo.size(); ++t) {
+    const uint32_t p = todo[t];
+    const PassArgs a{vin, vout, n, dl.d[p], bases[p], zeroed + ps.at[p], reinterpret_cast<uint32_t*>(zeroed) + p};
+    if (!has_v) launch_pass<K, false, false>(ctx, ps.items, kin, kout, a);
+    else if (t == 0 && vals_iota) launch_pass<K, true, true>(ctx, ps.items, kin, kout, a);
+    else launch_pass<K, true, false>(ctx, ps.items, kin, kout, a);
+    std::swap(kin, kout);
+    std::swap(vin, vout);
+  }
+  return kin == keys_alt;
+}
+
 template <typename K>
 bool radix_sort_impl(Ctx& ctx, K* keys, K* keys_alt, uint32_t* vals, uint32_t* vals_alt, uint64_t n,
                      const std::vector<RadixDigit>& digits, bool vals_iota, bool host_skip) {
   const bool has_v = vals != nullptr;
   if (n == 0) return false;
   if (n > 0xFFFFFFFFull && has_v) fail(VG_ERR_OVERFLOW, "radix sort values are 32-bit row ids");
-  const uint32_t passes = static_cast<uint32_t>(digits.size());
-  if (passes > kMaxPasses) fail(VG_ERR_INVALID, "radix sort: too many digits");
-  DigitList dl{};
-  dl.n = passes;
-  for (uint32_t p = 0; p < passes; ++p) dl.d[p] = digits[p];
-
-  const int items = items_for(ctx, n);
-  const uint64_t tiles = div_up(n, static_cast<uint64_t>(kBlock) * items);
-  const size_t word = wide_status(n) ? sizeof(uint64_t) : sizeof(uint32_t);
+  const DigitList dl = digit_list(digits);
+  const uint32_t passes = dl.n;
   // counts, tickets and every pass's look-back words in one block, zeroed by
   // one memset; the bases behind them
+  const PassScratch ps(ctx, n, dl);
   const size_t hist_bytes = passes * kRadix * sizeof(uint64_t);
-  const size_t ticket_bytes = (kMaxPasses + 1) * sizeof(uint32_t) + 60;   // 128: tickets, then the histogram's
-  size_t zero_bytes = hist_bytes + ticket_bytes;
-  std::vector<size_t> status_at(passes);
-  for (uint32_t p = 0; p < passes; ++p) {
-    status_at[p] = zero_bytes;
-    zero_bytes += tiles * status_row(digits[p].bits) * word;
-  }
-  Scratch<char> scratch(ctx, zero_bytes + hist_bytes);
+  Scratch<char> scratch(ctx, ps.bytes + 2 * hist_bytes);
   char* sc = scratch.get();
-  auto* hist = reinterpret_cast<unsigned long long*>(sc);
-  auto* ticket = reinterpret_cast<uint32_t*>(sc + hist_bytes);
-  auto* bases = reinterpret_cast<uint64_t*>(sc + zero_bytes);
-  VG_CUDA(cudaMemsetAsync(sc, 0, zero_bytes, ctx.stream));
+  auto* hist = reinterpret_cast<unsigned long long*>(sc + ps.bytes);
+  auto* bases = reinterpret_cast<uint64_t*>(sc + ps.bytes + hist_bytes);
+  auto* done = reinterpret_cast<uint32_t*>(sc) + kMaxPasses;
+  VG_CUDA(cudaMemsetAsync(sc, 0, ps.bytes + hist_bytes, ctx.stream));
   uint64_t grid = div_up(n, kBlock * 16);
   const uint64_t gmax = static_cast<uint64_t>(ctx.num_sms) * 8;
   if (grid > gmax) grid = gmax;
   if (grid < 1) grid = 1;
   ctx.launch("radix_histogram", static_cast<double>(n) * sizeof(K), [&] {
     radix_hist_kernel<K><<<static_cast<unsigned>(grid), kBlock, (passes ? passes : 1) * kRadix * sizeof(uint32_t),
-                           ctx.stream>>>(keys, n, dl, hist, bases, ticket + kMaxPasses);
+                           ctx.stream>>>(keys, n, dl, hist, bases, done);
   });
   VG_CUDA(cudaGetLastError());
   std::vector<uint32_t> todo;
@@ -407,20 +423,9 @@ bool radix_sort_impl(Ctx& ctx, K* keys, K* keys_alt, uint32_t* vals, uint32_t* v
     if (has_v && vals_iota) fill_iota(ctx, vals, n);
     return false;
   }
-  K* kin = keys;
-  K* kout = keys_alt;
-  uint32_t* vin = vals;
-  uint32_t* vout = vals_alt;
-  for (size_t t = 0; t < todo.size(); ++t) {
-    const uint32_t p = todo[t];
-    const PassArgs a{vin, vout, n, digits[p], bases + p * kRadix, sc + status_at[p], ticket + p};
-    if (!has_v) launch_pass<K, false, false>(ctx, items, kin, kout, a);
-    else if (t == 0 && vals_iota) launch_pass<K, true, true>(ctx, items, kin, kout, a);
-    else launch_pass<K, true, false>(ctx, items, kin, kout, a);
-    std::swap(kin, kout);
-    std::swap(vin, vout);
-  }
-  return kin == keys_alt;
+  const uint64_t* pb[kMaxPasses];
+  for (uint32_t p = 0; p < passes; ++p) pb[p] = bases + p * kRadix;
+  return run_passes(ctx, keys, keys_alt, vals, vals_alt, n, dl, pb, todo, ps, sc, vals_iota);
 }
 
 }  // namespace
@@ -435,16 +440,6 @@ void radix_plan(std::vector<RadixDigit>& digits, int begin, int end) {
 }
 
 bool radix_sort_u32(Ctx& ctx, uint32_t* keys, uint32_t* keys_alt, uint32_t* vals, uint32_t* vals_alt,
-                    uint64_t n, const std::vector<RadixDigit>& digits, bool vals_iota, bool host_skip) {
-  return radix_sort_impl<uint32_t>(ctx, keys, keys_alt, vals, vals_alt, n, digits, vals_iota, host_skip);
-}
-
-bool radix_sort_u64(Ctx& ctx, uint64_t* keys, uint64_t* keys_alt, uint32_t* vals, uint32_t* vals_alt,
-                    uint64_t n, const std::vector<RadixDigit>& digits, bool vals_iota, bool host_skip) {
-  return radix_sort_impl<uint64_t>(ctx, keys, keys_alt, vals, vals_alt, n, digits, vals_iota, host_skip);
-}
-
-bool radix_sort_u32(Ctx& ctx, uint32_t* keys, uint32_t* keys_alt, uint32_t* vals, uint32_t* vals_alt,
                     uint64_t n, int end_bit, bool vals_iota, bool host_skip) {
   std::vector<RadixDigit> digits;
   radix_plan(digits, 0, end_bit);
@@ -458,10 +453,17 @@ bool radix_sort_u64(Ctx& ctx, uint64_t* keys, uint64_t* keys_alt, uint32_t* vals
   return radix_sort_impl<uint64_t>(ctx, keys, keys_alt, vals, vals_alt, n, digits, vals_iota, host_skip);
 }
 
-bool radix_sort_u64_bits(Ctx& ctx, uint64_t* keys, uint64_t* keys_alt, uint64_t n, int begin_bit, int end_bit) {
-  std::vector<RadixDigit> digits;
-  radix_plan(digits, begin_bit, end_bit);
-  return radix_sort_impl<uint64_t>(ctx, keys, keys_alt, nullptr, nullptr, n, digits, false, true);
+bool radix_sort_u64_counted(Ctx& ctx, uint64_t* keys, uint64_t* keys_alt, uint64_t n,
+                            const std::vector<RadixDigit>& digits, const std::vector<const uint64_t*>& bases) {
+  if (n == 0 || digits.empty()) return false;
+  const DigitList dl = digit_list(digits);
+  const PassScratch ps(ctx, n, dl);
+  Scratch<char> scratch(ctx, ps.bytes);
+  VG_CUDA(cudaMemsetAsync(scratch.get(), 0, ps.bytes, ctx.stream));
+  std::vector<uint32_t> todo(dl.n);
+  for (uint32_t p = 0; p < dl.n; ++p) todo[p] = p;
+  return run_passes<uint64_t>(ctx, keys, keys_alt, nullptr, nullptr, n, dl, bases.data(), todo, ps, scratch.get(),
+                              false);
 }
 
 void fill_iota(Ctx& ctx, uint32_t* out, uint64_t n) {

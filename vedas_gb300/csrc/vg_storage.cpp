@@ -44,61 +44,41 @@ void build_index(Ctx& ctx, const uint32_t* s, const uint32_t* p, const uint32_t*
   ix.ctx = &ctx;
   ix.full = full;
   ix.n = n;
-  uint32_t mx[3];
-  column_max3(ctx, s, p, o, n, mx);
-  const uint32_t ms = mx[0], mp = mx[1], mo = mx[2];
-  ix.max_id = std::max(ms, std::max(mp, mo));
   auto put = [&](const char* name, const DevArray& a) { ix.dev[name] = a; };
-  {
-    // PSO by a full sort; POS from PSO's sorted keys by a sort of (p, o) only
-    PermOutputs pso, pos;
-    pso.want_col1 = pso.want_col2 = pso.want_l1 = pso.want_l2 = true;
-    pos.want_col1 = pos.want_col2 = pos.want_l2 = true;
-    const uint32_t m[3] = {mp, ms, mo};
-    build_permutation_pair(ctx, p, s, o, n, m, pso, pos);
-    put("p_idx_values", pso.l1_vals);
-    put("p_idx_offsets", pso.l1_offs);
-    put("ps_data", pso.col1);
-    put("pso_data", pso.col2);
-    put("ps_s_idx_values", pso.l2_vals);
-    put("ps_idx_offsets", pso.l2_offs);
-    put("po_data", pos.col1);
-    put("pos_data", pos.col2);
-    put("po_o_idx_values", pos.l2_vals);
-    put("po_idx_offsets", pos.l2_offs);
-  }
+  Permutations q;
+  q.pso.want_col1 = q.pso.want_col2 = q.pso.want_l1 = q.pso.want_l2 = true;
+  q.pos.want_col1 = q.pos.want_col2 = q.pos.want_l2 = true;
+  q.spo.want_col2 = q.spo.want_l2 = true;
+  q.sop.want_col2 = q.sop.want_l2 = true;
+  q.osp.want_col1 = q.osp.want_col2 = q.osp.want_l1 = true;
+  q.ops.want_col2 = q.ops.want_l2 = true;
+  ix.max_id = build_permutations(ctx, s, p, o, n, q, full);
+  put("p_idx_values", q.pso.l1_vals);
+  put("p_idx_offsets", q.pso.l1_offs);
+  put("ps_data", q.pso.col1);
+  put("pso_data", q.pso.col2);
+  put("ps_s_idx_values", q.pso.l2_vals);
+  put("ps_idx_offsets", q.pso.l2_offs);
+  put("po_data", q.pos.col1);
+  put("pos_data", q.pos.col2);
+  put("po_o_idx_values", q.pos.l2_vals);
+  put("po_idx_offsets", q.pos.l2_offs);
   if (full) {
     put("s_idx_values", DevArray());
     put("s_idx_offsets", DevArray());
-    PermOutputs spo;
-    spo.want_col2 = spo.want_l2 = true;
-    const uint32_t m1[3] = {ms, mp, mo};
-    build_permutation(ctx, s, p, o, n, m1, spo);
-    put("spo_data", spo.col2);
-    put("sp_p_idx_values", spo.l2_vals);
-    put("sp_idx_offsets", spo.l2_offs);
-    PermOutputs sop;
-    sop.want_col2 = sop.want_l2 = true;
-    const uint32_t m2[3] = {ms, mo, mp};
-    build_permutation(ctx, s, o, p, n, m2, sop);
-    put("sop_data", sop.col2);
-    put("so_o_idx_values", sop.l2_vals);
-    put("so_idx_offsets", sop.l2_offs);
-    PermOutputs os;
-    os.want_col1 = os.want_col2 = os.want_l1 = true;
-    const uint32_t m3[3] = {mo, ms, mp};
-    build_permutation(ctx, o, s, p, n, m3, os);
-    put("o_idx_values", os.l1_vals);
-    put("o_idx_offsets", os.l1_offs);
-    put("os_data", os.col1);
-    put("osp_data", os.col2);
-    PermOutputs ops;
-    ops.want_col2 = ops.want_l2 = true;
-    const uint32_t m4[3] = {mo, mp, ms};
-    build_permutation(ctx, o, p, s, n, m4, ops);
-    put("ops_data", ops.col2);
-    put("op_p_idx_values", ops.l2_vals);
-    put("op_idx_offsets", ops.l2_offs);
+    put("spo_data", q.spo.col2);
+    put("sp_p_idx_values", q.spo.l2_vals);
+    put("sp_idx_offsets", q.spo.l2_offs);
+    put("sop_data", q.sop.col2);
+    put("so_o_idx_values", q.sop.l2_vals);
+    put("so_idx_offsets", q.sop.l2_offs);
+    put("o_idx_values", q.osp.l1_vals);
+    put("o_idx_offsets", q.osp.l1_offs);
+    put("os_data", q.osp.col1);
+    put("osp_data", q.osp.col2);
+    put("ops_data", q.ops.col2);
+    put("op_p_idx_values", q.ops.l2_vals);
+    put("op_idx_offsets", q.ops.l2_offs);
   }
 }
 
