@@ -1,19 +1,20 @@
 // N-Triples ingest on the device.
 //
-// 1. newline positions: tiles of 4096 bytes, counts scanned with a decoupled
-//    look-back, positions written in order;
-// 2. one thread parses each line into term spans (subject, predicate,
-//    object, literal flag); valid lines are compacted in order by a second
-//    look-back scan, so triple t is the t-th statement of the file;
-// 3. per dictionary, every occurrence gets a 63-bit hash of its text; a
-//    stable radix sort by hash keeps equal hashes in order of appearance, so
-//    the first element of each run is the term's first occurrence;
-// 4. run heads are counted (look-back scan), every member is checked against
-//    its head byte by byte (a run holding different terms is a hash collision:
-//    that dictionary is then resolved exactly on the host), and the heads are
-//    sorted by first occurrence: rank r gets id base + r;
-// 5. ids are scattered back to the s, p, o columns, and the term of every id
-//    is read from the host copy of the text.
+// 1. newlines are counted (the count sizes everything else);
+// 2. blocks take 16 KiB pieces of the text into shared memory, find their
+//    lines, and one thread parses each line into its three terms and looks
+//    them up in one open-addressing table of terms: a slot is claimed by the
+//    place of a term's text, so terms are compared byte by byte and equal
+//    hashes need no further care.  Every slot keeps the lowest line its term
+//    occurs on;
+// 3. a scan over the lines counts statements and, per dictionary, the terms
+//    that occur first on each line: their ids, in order of first appearance;
+// 4. ids go to the s, p, o columns, and the place of every id's term to a list
+//    from which the host reads the terms in its own copy of the text.
+//
+// The table replaced a radix sort of 63-bit hashes per dictionary (31 passes),
+// run heads, a byte-by-byte check and a second sort into id order: 2.5 ms of
+// kernels for 1M statements (101 MB).
 #include "vg_ingest.h"
 
 #include <algorithm>
@@ -25,31 +26,50 @@
 
 #include "vg_pool.h"
 #include "vg_prims.cuh"
-#include "vg_sort.h"
 
 namespace vg {
 namespace {
 
 constexpr int kBlock = 256;
-constexpr int kNlBytes = 16;                      // bytes per thread
-constexpr uint64_t kNlTile = kBlock * kNlBytes;   // 4096
+constexpr uint32_t kPiece = kBlock * 64;       // bytes of text per block
+constexpr uint32_t kHalo = 1024;               // bytes after the piece, for the line that leaves it
+constexpr uint32_t kLineList = 2048;           // lines of a piece listed at a time
 constexpr int kRows = 8;
-constexpr uint64_t kTileRows = kBlock * kRows;
+constexpr uint64_t kTileLines = kBlock * kRows;
+constexpr uint32_t kProbeMax = 8192;           // a longer search gives up (the host then resolves the terms)
 
 std::atomic<int> g_hash_bits{63};
 
+// Where the terms of each line lie (only made for the host's exact path):
+// lengths are 0 where the line holds no statement.
 struct Spans {
-  uint64_t* s_off;
-  uint64_t* p_off;
-  uint64_t* o_off;
-  uint32_t* s_len;
-  uint32_t* p_len;
-  uint32_t* o_len;
+  uint64_t* off[3];   // subject, predicate, object
+  uint64_t* len[3];
   uint8_t* lit;
 };
 
+// A slot of the term table.  loc is the place of the term that claimed it:
+// (offset << len_bits | length) << 2 | dictionary (0 subjects and objects, 1
+// predicates, 2 literals), never 0.  first holds ~(lowest line), so that
+// zeroed memory is an empty table; id is set once ids are known.
+struct Slot {
+  unsigned long long loc;
+  uint32_t first;
+  uint32_t id;
+};
+static_assert(sizeof(Slot) == 16, "one 16-byte slot");
+constexpr uint32_t kNoSlot = 0xffffffffu;
+
+struct Flags {                   // device flags of the parse
+  unsigned long long bad_line;   // lowest malformed line, from 1 (~0: none)
+  uint32_t give_up;              // a term too long for loc, or a search past kProbeMax
+  uint32_t pad;
+};
+
 // ---------------------------------------------------------------------------
-// 1. newline positions (a counting pass sizes the position array)
+// 1. newlines
+constexpr uint32_t kNewlines = 0x0a0a0a0au;
+
 __global__ void newline_count_kernel(const uint8_t* __restrict__ text, uint64_t len,
                                      unsigned long long* __restrict__ count) {
   const uint64_t words = len / 16;
@@ -57,11 +77,8 @@ __global__ void newline_count_kernel(const uint8_t* __restrict__ text, uint64_t 
   uint32_t c = 0;
   for (uint64_t w = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; w < words; w += stride) {
     const uint4 v = reinterpret_cast<const uint4*>(text)[w];
-    const uint32_t x[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-      for (int k = 0; k < 4; ++k) c += ((x[q] >> (8 * k)) & 0xFFu) == '\n' ? 1u : 0u;
+    c += (__popc(__vcmpeq4(v.x, kNewlines)) + __popc(__vcmpeq4(v.y, kNewlines)) +
+          __popc(__vcmpeq4(v.z, kNewlines)) + __popc(__vcmpeq4(v.w, kNewlines))) >> 3;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0)
     for (uint64_t b = words * 16; b < len; ++b) c += text[b] == '\n' ? 1u : 0u;
@@ -69,66 +86,42 @@ __global__ void newline_count_kernel(const uint8_t* __restrict__ text, uint64_t 
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, static_cast<unsigned long long>(c));
 }
 
-__global__ void __launch_bounds__(kBlock) newline_kernel(const uint8_t* __restrict__ text, uint64_t len,
-                                                         uint64_t* __restrict__ nl, uint64_t* status,
-                                                         uint32_t* ticket, uint64_t* total, DeviceErrors* err) {
-  __shared__ uint32_t s_scan[kBlock / 32 + 1];
-  __shared__ uint64_t s_b;
-  __shared__ uint32_t s_tile;
-  if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
-  __syncthreads();
-  const uint64_t tile = s_tile;
-  const uint64_t b0 = tile * kNlTile + static_cast<uint64_t>(threadIdx.x) * kNlBytes;
-  uint32_t mask = 0;   // bit k: byte b0 + k is a newline
-  if (b0 + kNlBytes <= len) {
-    const uint4 v = *reinterpret_cast<const uint4*>(text + b0);
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if (((w[q] >> (8 * k)) & 0xFFu) == '\n') mask |= 1u << (4 * q + k);
-  } else {
-    for (int k = 0; k < kNlBytes && b0 + k < len; ++k)
-      if (text[b0 + k] == '\n') mask |= 1u << k;
-  }
-  uint32_t tot;
-  const uint32_t e = block_excl_scan<kBlock>(__popc(mask), tot, s_scan);
-  if (threadIdx.x < 32) {
-    const uint64_t p = warp_lookback(status, static_cast<uint32_t>(tile), tot, err);
-    if (threadIdx.x == 0) s_b = p;
-  }
-  __syncthreads();
-  uint64_t o = s_b + e;
-  while (mask) {
-    const int k = __ffs(mask) - 1;
-    nl[o++] = b0 + k;
-    mask &= mask - 1;
-  }
-  if (tile == gridDim.x - 1 && threadIdx.x == 0) *total = s_b + tot;
-}
 
 // ---------------------------------------------------------------------------
-// 2. line parser (N-Triples statements)
+// 2. lines, statements and terms
 __device__ __forceinline__ bool is_ws(uint8_t c) { return c == ' ' || c == '\t' || c == '\r'; }
 
-// Term at text[i]; returns its end (one past) or 0 on a malformed term.
-// kind: 0 any, 1 IRI only (predicate), 2 IRI or blank node (subject).
-__device__ uint64_t term_end(const uint8_t* t, uint64_t i, uint64_t end, int kind, bool& literal) {
+// nb (1..8) bytes at p + off as a little-endian word.  p is 8-byte aligned;
+// only the aligned words that hold those bytes are read.
+__device__ __forceinline__ uint64_t word_at(const uint8_t* p, uint64_t off, uint32_t nb) {
+  const uint64_t* q = reinterpret_cast<const uint64_t*>(p + (off & ~7ull));
+  const uint32_t in = static_cast<uint32_t>(off & 7);
+  uint64_t w = q[0] >> (8 * in);
+  if (in + nb > 8) w |= q[1] << (64 - 8 * in);
+  return nb < 8 ? w & ((1ull << (8 * nb)) - 1) : w;
+}
+
+// Term at t[i]; returns its end (one past) or 0 on a malformed term.
+// kind: 0 any, 1 IRI only (predicate), 2 IRI or blank node (subject).  I is
+// 32 bits wide for lines in shared memory.
+template <typename I>
+__device__ __forceinline__ I iri_end(const uint8_t* t, I i, I end) {
+  for (I j = i + 1; j < end; ++j) {
+    if (t[j] == '>') return j + 1;
+    if (t[j] == ' ' || t[j] == '\t') return 0;
+  }
+  return 0;
+}
+template <typename I>
+__device__ I term_end(const uint8_t* t, I i, I end, int kind, bool& literal) {
   literal = false;
   if (i >= end) return 0;
   const uint8_t c = t[i];
-  if (c == '<') {
-    for (uint64_t j = i + 1; j < end; ++j) {
-      if (t[j] == '>') return j + 1;
-      if (t[j] == ' ' || t[j] == '\t') return 0;
-    }
-    return 0;
-  }
+  if (c == '<') return iri_end<I>(t, i, end);
   if (kind == 1) return 0;
   if (c == '_') {
     if (i + 1 >= end || t[i + 1] != ':') return 0;
-    uint64_t j = i + 2;
+    I j = i + 2;
     while (j < end && !is_ws(t[j])) ++j;
     if (j == i + 2) return 0;
     // a label does not end with '.': "_:b1." before the statement's dot
@@ -136,7 +129,7 @@ __device__ uint64_t term_end(const uint8_t* t, uint64_t i, uint64_t end, int kin
     return j;
   }
   if (kind == 2 || c != '"') return 0;
-  uint64_t j = i + 1;
+  I j = i + 1;
   while (j < end) {
     if (t[j] == '\\') {
       j += 2;
@@ -149,103 +142,44 @@ __device__ uint64_t term_end(const uint8_t* t, uint64_t i, uint64_t end, int kin
   ++j;   // past the closing quote
   literal = true;
   if (j < end && t[j] == '@') {
-    uint64_t k = j + 1;
+    I k = j + 1;
     while (k < end && ((t[k] >= 'a' && t[k] <= 'z') || (t[k] >= 'A' && t[k] <= 'Z') ||
                        (t[k] >= '0' && t[k] <= '9') || t[k] == '-'))
       ++k;
     if (k == j + 1) return 0;
     return k;
   }
-  if (j + 1 < end && t[j] == '^' && t[j + 1] == '^') {
-    bool dummy;
-    const uint64_t k = term_end(t, j + 2, end, 1, dummy);
-    return k;
-  }
+  if (j + 1 < end && t[j] == '^' && t[j + 1] == '^')
+    return j + 2 < end && t[j + 2] == '<' ? iri_end<I>(t, j + 2, end) : 0;
   return j;
 }
 
-__global__ void __launch_bounds__(kBlock) parse_kernel(const uint8_t* __restrict__ text, uint64_t len,
-                                                       const uint64_t* __restrict__ nl, uint64_t nnl, uint64_t lines,
-                                                       Spans out, uint64_t* status, uint32_t* ticket,
-                                                       uint64_t* count, unsigned long long* bad_line,
-                                                       DeviceErrors* err) {
-  __shared__ uint32_t s_scan[kBlock / 32 + 1];
-  __shared__ uint64_t s_b;
-  __shared__ uint32_t s_tile;
-  if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
-  __syncthreads();
-  const uint64_t tile = s_tile;
-  const uint64_t line = tile * kBlock + threadIdx.x;
-  bool valid = false, lit = false;
-  uint64_t so = 0, se = 0, po = 0, pe = 0, oo = 0, oe = 0;
-  if (line < lines) {
-    const uint64_t b = line == 0 ? 0 : nl[line - 1] + 1;
-    const uint64_t e = line < nnl ? nl[line] : len;
-    uint64_t i = b;
-    while (i < e && is_ws(text[i])) ++i;
-    if (i < e && text[i] != '#') {
-      bool ok = true, l0 = false, l1 = false;
-      so = i;
-      se = term_end(text, i, e, 2, l0);
-      ok = se != 0;
-      if (ok) {
-        i = se;
-        const uint64_t ws0 = i;
-        while (i < e && is_ws(text[i])) ++i;
-        ok = i > ws0;
-      }
-      if (ok) {
-        po = i;
-        pe = term_end(text, i, e, 1, l1);
-        ok = pe != 0;
-      }
-      if (ok) {
-        i = pe;
-        const uint64_t ws0 = i;
-        while (i < e && is_ws(text[i])) ++i;
-        ok = i > ws0;
-      }
-      if (ok) {
-        oo = i;
-        oe = term_end(text, i, e, 0, lit);
-        ok = oe != 0;
-      }
-      if (ok) {
-        i = oe;
-        while (i < e && is_ws(text[i])) ++i;
-        ok = i < e && text[i] == '.';
-        ++i;
-        while (ok && i < e && is_ws(text[i])) ++i;
-        ok = ok && (i >= e || text[i] == '#');
-      }
-      if (ok) valid = true;
-      else atomicMin(bad_line, static_cast<unsigned long long>(line + 1));
-    }
+// The statement on t[b, e): 0 none (blank or comment), 1 well formed (its
+// terms at off, len), 2 malformed.
+template <typename I>
+__device__ int parse_line(const uint8_t* t, I b, I e, I (&off)[3], I (&len)[3], bool& lit) {
+  I i = b;
+  while (i < e && is_ws(t[i])) ++i;
+  if (i >= e || t[i] == '#') return 0;
+#pragma unroll 1
+  for (int k = 0; k < 3; ++k) {
+    off[k] = i;
+    const I end = term_end<I>(t, i, e, k == 0 ? 2 : (k == 1 ? 1 : 0), lit);
+    if (end == 0) return 2;
+    len[k] = end - i;
+    i = end;
+    const I ws = i;
+    while (i < e && is_ws(t[i])) ++i;
+    if (k < 2 && i == ws) return 2;
   }
-  uint32_t tot;
-  const uint32_t ex = block_excl_scan<kBlock>(valid ? 1u : 0u, tot, s_scan);
-  if (threadIdx.x < 32) {
-    const uint64_t p = warp_lookback(status, static_cast<uint32_t>(tile), tot, err);
-    if (threadIdx.x == 0) s_b = p;
-  }
-  __syncthreads();
-  if (valid) {
-    const uint64_t t = s_b + ex;
-    out.s_off[t] = so;
-    out.s_len[t] = static_cast<uint32_t>(se - so);
-    out.p_off[t] = po;
-    out.p_len[t] = static_cast<uint32_t>(pe - po);
-    out.o_off[t] = oo;
-    out.o_len[t] = static_cast<uint32_t>(oe - oo);
-    out.lit[t] = lit ? 1 : 0;
-  }
-  if (tile == gridDim.x - 1 && threadIdx.x == 0) *count = s_b + tot;
+  if (i >= e || t[i] != '.') return 2;
+  ++i;
+  while (i < e && is_ws(t[i])) ++i;
+  return i >= e || t[i] == '#' ? 1 : 2;
 }
 
-// ---------------------------------------------------------------------------
-// 3. hashing of the occurrences of one dictionary
 // A 64-bit multiply-xorshift mix over 8-byte words (this project's own; any
-// good mix works, equality is checked byte by byte afterwards).
+// good mix works, terms are compared byte by byte).
 __device__ __forceinline__ uint64_t mix64(uint64_t h) {
   h ^= h >> 31;
   h *= 0x7fb5d329728ea185ull;
@@ -255,184 +189,280 @@ __device__ __forceinline__ uint64_t mix64(uint64_t h) {
   return h;
 }
 
-__device__ uint64_t term_hash(const uint8_t* t, uint64_t off, uint32_t len, int bits) {
-  uint64_t h = 0x243f6a8885a308d3ull ^ len;
-  uint32_t i = 0;
-  for (; i + 8 <= len; i += 8) {
-    uint64_t w = 0;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) w |= static_cast<uint64_t>(t[off + i + k]) << (8 * k);
-    h = mix64(h ^ w);
-  }
-  uint64_t w = 0;
-  for (int k = 0; i + k < len; ++k) w |= static_cast<uint64_t>(t[off + i + k]) << (8 * k);
-  h = mix64(h ^ w ^ (static_cast<uint64_t>(len) << 56));
-  return bits >= 63 ? (h >> 1) : (h >> (64 - bits));
-}
+struct Table {
+  Slot* slots;
+  uint64_t cap;
+  uint32_t len_bits;
+  int hash_bits;
+};
 
-// kind 0: subject/object dictionary over 2n occurrences (2t subject, 2t+1
-// object); kind 1: predicates; kind 2: literal objects.  Non-members get the
-// key ~0 (sorted after every member).
-__global__ void hash_kernel(const uint8_t* __restrict__ text, Spans sp, uint64_t n, int kind, bool literal_dict,
-                            int bits, uint64_t* __restrict__ keys, uint32_t* __restrict__ vals,
-                            unsigned long long* members) {
-  const uint64_t m = kind == 0 ? 2 * n : n;
-  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  uint32_t mine = 0;
-  for (uint64_t k = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; k < m; k += stride) {
-    uint64_t off = 0;
-    uint32_t len = 0;
-    bool member = true;
-    if (kind == 0) {
-      const uint64_t t = k >> 1;
-      if (k & 1) {
-        member = !(literal_dict && sp.lit[t]);
-        off = sp.o_off[t];
-        len = sp.o_len[t];
-      } else {
-        off = sp.s_off[t];
-        len = sp.s_len[t];
+// The slot of the term at t + off (text offset at), claimed if it is new;
+// kNoSlot (and give_up set) when there is none to be had.
+__device__ uint32_t find_slot(const Table& tb, const uint8_t* text, const uint8_t* t, uint64_t off, uint64_t at,
+                              uint64_t len, uint32_t dict, uint32_t line, Flags* fl) {
+  if (len >> tb.len_bits) {
+    fl->give_up = 1;
+    return kNoSlot;
+  }
+  uint64_t h = 0x243f6a8885a308d3ull ^ (len << 2 | dict);
+  for (uint64_t i = 0; i < len; i += 8)
+    h = mix64(h ^ word_at(t, off + i, static_cast<uint32_t>(len - i < 8 ? len - i : 8)));
+  if (tb.hash_bits < 63) h &= ~((1ull << (64 - tb.hash_bits)) - 1);
+  const unsigned long long mine = ((at << tb.len_bits | len) << 2) | dict;
+  uint64_t i = __umul64hi(h, tb.cap);
+  for (uint32_t probe = 0; probe < kProbeMax; ++probe) {
+    Slot* s = &tb.slots[i];
+    unsigned long long loc = s->loc;
+    if (loc == 0) loc = atomicCAS(&s->loc, 0ull, mine);
+    bool same = loc == 0 || loc == mine;
+    if (!same && (loc & 3) == dict && ((loc >> 2) & ((1ull << tb.len_bits) - 1)) == len) {
+      const uint64_t other = loc >> (2 + tb.len_bits);
+      same = true;
+      for (uint64_t k = 0; same && k < len; k += 8) {
+        const uint32_t nb = static_cast<uint32_t>(len - k < 8 ? len - k : 8);
+        same = word_at(t, off + k, nb) == word_at(text, other + k, nb);
       }
-    } else if (kind == 1) {
-      off = sp.p_off[k];
-      len = sp.p_len[k];
-    } else {
-      member = sp.lit[k] != 0;
-      off = sp.o_off[k];
-      len = sp.o_len[k];
     }
-    keys[k] = member ? term_hash(text, off, len, bits) : ~0ull;
-    vals[k] = static_cast<uint32_t>(k);
-    mine += member ? 1u : 0u;
+    if (same) {
+      // most occurrences come after their term's first one: no atomic then
+      if (s->first < ~line) atomicMax(&s->first, ~line);
+      return static_cast<uint32_t>(i);
+    }
+    if (++i == tb.cap) i = 0;
+    if ((probe & 63) == 63 && *reinterpret_cast<volatile uint32_t*>(&fl->give_up)) return kNoSlot;
   }
-  if (mine) atomicAdd(members, static_cast<unsigned long long>(mine));
+  fl->give_up = 1;
+  return kNoSlot;
 }
 
-__device__ __forceinline__ void occ_span(const Spans& sp, int kind, uint32_t k, uint64_t& off, uint32_t& len) {
-  if (kind == 0) {
-    const uint32_t t = k >> 1;
-    if (k & 1) {
-      off = sp.o_off[t];
-      len = sp.o_len[t];
-    } else {
-      off = sp.s_off[t];
-      len = sp.s_len[t];
+// A block per piece of kPiece bytes, in ticket order; it owns the lines that
+// start after the piece's newlines (and the text's first line).  The piece
+// lies in shared memory: one thread per line reads its line byte by byte,
+// which from global memory costs a cache access per byte and lane (0.27 ms
+// for 101 MB, and again for the hashes).  slots: [3][lines], kNoSlot in the
+// subject's place where the line holds no statement.
+__global__ void __launch_bounds__(kBlock) parse_kernel(const uint8_t* __restrict__ text, uint64_t len, uint64_t lines,
+                                                       Table tb, uint32_t* __restrict__ slots, Spans sp,
+                                                       bool literal_dict, uint64_t* status, uint32_t* ticket,
+                                                       Flags* fl, DeviceErrors* err) {
+  __shared__ __align__(16) uint8_t s_text[kPiece + kHalo + 16];
+  __shared__ uint16_t s_start[kLineList + 1];   // first bytes of the listed lines (kPiece at most)
+  __shared__ uint32_t s_scan[kBlock / 32 + 1];
+  __shared__ uint64_t s_b;
+  __shared__ uint32_t s_tile;
+  const uint32_t tid = threadIdx.x;
+  if (tid == 0) s_tile = atomicAdd(ticket, 1u);
+  __syncthreads();
+  const uint64_t base = static_cast<uint64_t>(s_tile) * kPiece;
+  // the text is padded to whole 16-byte words
+  const uint32_t have = static_cast<uint32_t>(len - base < kPiece + kHalo ? len - base : kPiece + kHalo);
+  for (uint32_t w = tid; w < (have + 15) / 16; w += kBlock)
+    reinterpret_cast<uint4*>(s_text)[w] = reinterpret_cast<const uint4*>(text + base)[w];
+  __syncthreads();
+  // the thread's 64 bytes: bit k of nl, byte k is a newline
+  uint64_t nl = 0;
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    const uint32_t m = __vcmpeq4(reinterpret_cast<const uint32_t*>(s_text)[tid * 16 + q], kNewlines) & 0x08040201u;
+    nl |= static_cast<uint64_t>((m | m >> 8 | m >> 16 | m >> 24) & 15u) << (4 * q);
+  }
+  const uint32_t mine0 = tid * 64;
+  const uint32_t piece = have < kPiece ? have : kPiece;
+  if (mine0 >= piece) nl = 0;
+  else if (piece - mine0 < 64) nl &= (1ull << (piece - mine0)) - 1;
+  uint32_t total;
+  const uint32_t ahead = block_excl_scan<kBlock>(static_cast<uint32_t>(__popcll(nl)), total, s_scan);
+  if (tid < 32) {
+    const uint64_t p = warp_lookback(status, s_tile, total, err);
+    if (tid == 0) s_b = p;
+  }
+  __syncthreads();
+  // line k (from 0) of the piece starts after its newline k - 1; the text's
+  // first line counts as one more of piece 0
+  const uint32_t own0 = base == 0 ? 1u : 0u;
+  const uint64_t line0 = s_b + (base == 0 ? 0 : 1);   // number of the piece's line 0
+  const uint32_t n_lines = total + own0;
+  for (uint32_t from = 0; from < n_lines; from += kLineList) {
+    // list entries [from, from + kLineList] (one more: the end of the last)
+    __syncthreads();
+    if (own0 && from == 0 && tid == 0) s_start[0] = 0;
+    {
+      uint64_t m = nl;
+      uint32_t k = ahead + own0;
+      while (m) {
+        const uint32_t q = __ffsll(static_cast<long long>(m)) - 1;
+        if (k >= from && k <= from + kLineList) s_start[k - from] = static_cast<uint16_t>(mine0 + q + 1);
+        m &= m - 1;
+        ++k;
+      }
     }
-  } else if (kind == 1) {
-    off = sp.p_off[k];
-    len = sp.p_len[k];
-  } else {
-    off = sp.o_off[k];
-    len = sp.o_len[k];
+    __syncthreads();
+    for (uint32_t k = tid; k < kLineList && from + k < n_lines; k += kBlock) {
+      const uint64_t line = line0 + from + k;
+      const uint32_t b = s_start[k];
+      if (base + b >= len || line >= lines) continue;   // the text's last newline starts no line
+      uint64_t off[3] = {0, 0, 0}, tl[3] = {0, 0, 0};
+      bool lit = false, near = true;
+      int got;
+      uint32_t e = b;
+      if (from + k + 1 < n_lines) {
+        e = s_start[k + 1] - 1u;
+      } else {
+        e = piece > b ? piece : b;
+        while (e < have && s_text[e] != '\n') ++e;
+        near = e < have || base + have == len;   // the line ends within shared memory
+      }
+      const uint8_t* t = s_text;
+      if (near) {
+        uint32_t o4[3] = {0, 0, 0}, l4[3] = {0, 0, 0};
+        got = parse_line<uint32_t>(s_text, b, e, o4, l4, lit);
+        for (int q = 0; q < 3; ++q) {
+          off[q] = o4[q];
+          tl[q] = l4[q];
+        }
+      } else {
+        uint64_t eg = base + have;
+        while (eg < len && text[eg] != '\n') ++eg;
+        got = parse_line<uint64_t>(text, base + b, eg, off, tl, lit);
+        t = text;
+      }
+      if (got == 2) atomicMin(&fl->bad_line, static_cast<unsigned long long>(line + 1));
+      uint32_t sl[3] = {kNoSlot, kNoSlot, kNoSlot};
+      if (got == 1 && tb.slots) {
+        const uint64_t add = near ? base : 0;
+#pragma unroll 1
+        for (int q = 0; q < 3; ++q) {
+          const uint32_t dict = q == 1 ? 1u : (q == 2 && lit && literal_dict ? 2u : 0u);
+          sl[q] = find_slot(tb, text, t, off[q], off[q] + add, tl[q], dict, static_cast<uint32_t>(line), fl);
+        }
+      }
+      if (slots) {
+        slots[line] = sl[0];
+        slots[lines + line] = sl[1];
+        slots[2 * lines + line] = sl[2];
+      }
+      if (sp.lit) {
+        for (int q = 0; q < 3; ++q) {
+          sp.off[q][line] = off[q] + (near ? base : 0);
+          sp.len[q][line] = got == 1 ? tl[q] : 0;
+        }
+        sp.lit[line] = lit ? 1 : 0;
+      }
+    }
   }
 }
 
 // ---------------------------------------------------------------------------
-// 4. run heads: seg[i] = index of the run holding element i; head_pos[r] =
-// first element of run r.
-__global__ void __launch_bounds__(kBlock) heads_kernel(const uint64_t* __restrict__ keys, uint64_t m,
-                                                       uint32_t* __restrict__ seg, uint32_t* __restrict__ head_pos,
-                                                       uint64_t* status, uint32_t* ticket, uint64_t* total,
-                                                       DeviceErrors* err) {
+// 3. ids: per line, whether it holds a statement and which of its terms occur
+// on it first (a subject before an equal object), scanned over the lines.
+struct Counts {
+  uint64_t n[4];   // statements, terms of dictionaries 0, 1, 2
+};
+
+struct LineFirsts {
+  bool statement, s, p, o;
+  uint32_t o_dict;
+};
+__device__ __forceinline__ LineFirsts line_firsts(const uint32_t* __restrict__ slots, const Slot* __restrict__ table,
+                                                  uint64_t lines, uint64_t line, uint32_t (&sl)[3]) {
+  LineFirsts f{false, false, false, false, 0};
+  sl[0] = line < lines ? slots[line] : kNoSlot;
+  if (sl[0] == kNoSlot) return f;
+  sl[1] = slots[lines + line];
+  sl[2] = slots[2 * lines + line];
+  const uint32_t l = ~static_cast<uint32_t>(line);
+  const Slot o = table[sl[2]];
+  f.statement = true;
+  f.s = table[sl[0]].first == l;
+  f.p = table[sl[1]].first == l;
+  f.o = o.first == l && sl[2] != sl[0];
+  f.o_dict = static_cast<uint32_t>(o.loc & 3);
+  return f;
+}
+
+// base3: the first id of each dictionary.
+__global__ void __launch_bounds__(kBlock) ids_kernel(const uint32_t* __restrict__ slots, Slot* table, uint64_t lines,
+                                                     uint64_t tiles, uint3 base3, uint64_t* status, uint32_t* ticket,
+                                                     uint64_t* __restrict__ tile_first, Counts* counts,
+                                                     DeviceErrors* err) {
   __shared__ uint32_t s_scan[kBlock / 32 + 1];
-  __shared__ uint64_t s_b;
+  __shared__ uint64_t s_b[4];
   __shared__ uint32_t s_tile;
   if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
   __syncthreads();
-  const uint64_t tile = s_tile;
-  const uint64_t r0 = tile * kTileRows + static_cast<uint64_t>(threadIdx.x) * kRows;
-  uint32_t flags = 0;
-  uint64_t prev = (r0 > 0 && r0 - 1 < m) ? keys[r0 - 1] : 0;
+  const uint32_t tile = s_tile;
+  const uint64_t l0 = static_cast<uint64_t>(tile) * kTileLines + static_cast<uint64_t>(threadIdx.x) * kRows;
+  LineFirsts f[kRows];
+  uint32_t sl[kRows][3];
+  uint32_t c[4] = {0, 0, 0, 0};
 #pragma unroll
   for (int i = 0; i < kRows; ++i) {
-    const uint64_t r = r0 + i;
-    if (r < m) {
-      const uint64_t k = keys[r];
-      if (r == 0 || k != prev) flags |= 1u << i;
-      prev = k;
-    }
+    f[i] = line_firsts(slots, table, lines, l0 + i, sl[i]);
+    c[0] += f[i].statement;
+    c[1] += f[i].s + (f[i].o && f[i].o_dict == 0);
+    c[2] += f[i].p;
+    c[3] += f[i].o && f[i].o_dict == 2;
   }
-  uint32_t tot;
-  const uint32_t e = block_excl_scan<kBlock>(__popc(flags), tot, s_scan);
-  if (threadIdx.x < 32) {
-    const uint64_t p = warp_lookback(status, static_cast<uint32_t>(tile), tot, err);
-    if (threadIdx.x == 0) s_b = p;
+  uint32_t e[4], tot[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) e[q] = block_excl_scan<kBlock>(c[q], tot[q], s_scan);
+  const uint32_t warp = threadIdx.x >> 5;
+  if (warp < 4) {
+    const uint64_t p = warp_lookback(status + warp * tiles, tile, warp == 0 ? tot[0] : warp == 1 ? tot[1] : warp == 2 ? tot[2] : tot[3], err);
+    if ((threadIdx.x & 31) == 0) s_b[warp] = p;
   }
   __syncthreads();
-  uint64_t run = s_b + e;   // heads before this thread's rows
+  if (threadIdx.x == 0) {
+    tile_first[tile] = s_b[0];
+    if (tile == tiles - 1)
+      for (int q = 0; q < 4; ++q) counts->n[q] = s_b[q] + tot[q];
+  }
+  uint32_t id[3] = {base3.x + static_cast<uint32_t>(s_b[1] + e[1]), base3.y + static_cast<uint32_t>(s_b[2] + e[2]),
+                    base3.z + static_cast<uint32_t>(s_b[3] + e[3])};
 #pragma unroll
   for (int i = 0; i < kRows; ++i) {
-    const uint64_t r = r0 + i;
-    if (r >= m) break;
-    if (flags >> i & 1u) {
-      head_pos[run] = static_cast<uint32_t>(r);
-      ++run;
+    if (f[i].s) table[sl[i][0]].id = id[0]++;
+    if (f[i].o) {
+      if (f[i].o_dict == 0) table[sl[i][2]].id = id[0]++;
+      else table[sl[i][2]].id = id[2]++;
     }
-    seg[r] = static_cast<uint32_t>(run - 1);
-  }
-  if (tile == gridDim.x - 1 && threadIdx.x == 0) *total = s_b + tot;
-}
-
-// Every member's text equals its run head's text (else a hash collision).
-__global__ void verify_kernel(const uint8_t* __restrict__ text, Spans sp, int kind, const uint32_t* __restrict__ vals,
-                              const uint32_t* __restrict__ seg, const uint32_t* __restrict__ head_pos, uint64_t m,
-                              unsigned int* collision) {
-  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < m; i += stride) {
-    const uint32_t h = head_pos[seg[i]];
-    if (h == i) continue;
-    uint64_t a, b;
-    uint32_t la, lb;
-    occ_span(sp, kind, vals[i], a, la);
-    occ_span(sp, kind, vals[h], b, lb);
-    bool same = la == lb;
-    for (uint32_t k = 0; same && k < la; ++k) same = text[a + k] == text[b + k];
-    if (!same) atomicExch(collision, 1u);
+    if (f[i].p) table[sl[i][1]].id = id[1]++;
   }
 }
 
-// First occurrence of every run, to be sorted into id order.
-__global__ void first_pos_kernel(const uint32_t* __restrict__ vals, const uint32_t* __restrict__ head_pos,
-                                 uint64_t runs, uint32_t* __restrict__ fpos, uint32_t* __restrict__ rid) {
-  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  for (uint64_t r = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; r < runs; r += stride) {
-    fpos[r] = vals[head_pos[r]];
-    rid[r] = static_cast<uint32_t>(r);
-  }
-}
-
-__global__ void rank_kernel(const uint32_t* __restrict__ sorted_rid, uint64_t runs, uint32_t base,
-                            uint32_t* __restrict__ id_of_run) {
-  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  for (uint64_t r = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; r < runs; r += stride)
-    id_of_run[sorted_rid[r]] = base + static_cast<uint32_t>(r);
-}
-
-// 5. ids back to the columns
-__global__ void scatter_kernel(const uint32_t* __restrict__ vals, const uint32_t* __restrict__ seg,
-                               const uint32_t* __restrict__ id_of_run, uint64_t m, int kind, uint32_t* __restrict__ s,
-                               uint32_t* __restrict__ p, uint32_t* __restrict__ o) {
-  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < m; i += stride) {
-    const uint32_t k = vals[i];
-    const uint32_t id = id_of_run[seg[i]];
-    if (kind == 0) {
-      if (k & 1) o[k >> 1] = id;
-      else s[k >> 1] = id;
-    } else if (kind == 1) {
-      p[k] = id;
-    } else {
-      o[k] = id;
+// 4. ids to the columns, and the places of the terms in id order.
+struct TermList {
+  uint64_t* loc[3];   // per dictionary: offset << len_bits | length, by id - base
+};
+__global__ void __launch_bounds__(kBlock) columns_kernel(const uint32_t* __restrict__ slots,
+                                                         const Slot* __restrict__ table, uint64_t lines, uint3 base3,
+                                                         const uint64_t* __restrict__ tile_first,
+                                                         uint32_t* __restrict__ s, uint32_t* __restrict__ p,
+                                                         uint32_t* __restrict__ o, TermList terms) {
+  __shared__ uint32_t s_scan[kBlock / 32 + 1];
+  const uint64_t l0 = static_cast<uint64_t>(blockIdx.x) * kTileLines + static_cast<uint64_t>(threadIdx.x) * kRows;
+  uint32_t c = 0;
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) c += l0 + i < lines && slots[l0 + i] != kNoSlot;
+  uint32_t tot;
+  uint64_t t = tile_first[blockIdx.x] + block_excl_scan<kBlock>(c, tot, s_scan);
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) {
+    uint32_t sl[3];
+    const LineFirsts f = line_firsts(slots, table, lines, l0 + i, sl);
+    if (!f.statement) continue;
+    const Slot a = table[sl[0]], b = table[sl[1]], d = table[sl[2]];
+    s[t] = a.id;
+    p[t] = b.id;
+    o[t] = d.id;
+    ++t;
+    if (f.s) terms.loc[0][a.id - base3.x] = a.loc >> 2;
+    if (f.p) terms.loc[1][b.id - base3.y] = b.loc >> 2;
+    if (f.o) {
+      if (f.o_dict == 0) terms.loc[0][d.id - base3.x] = d.loc >> 2;
+      else terms.loc[2][d.id - base3.z] = d.loc >> 2;
     }
   }
-}
-
-// Spans of the terms in id order.
-__global__ void dict_spans_kernel(Spans sp, int kind, const uint32_t* __restrict__ fpos_sorted, uint64_t runs,
-                                  uint64_t* __restrict__ off, uint32_t* __restrict__ len) {
-  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  for (uint64_t r = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; r < runs; r += stride)
-    occ_span(sp, kind, fpos_sorted[r], off[r], len[r]);
 }
 
 unsigned grid(const Ctx& ctx, uint64_t units) {
@@ -442,140 +472,84 @@ unsigned grid(const Ctx& ctx, uint64_t units) {
   return static_cast<unsigned>(g < 1 ? 1 : g);
 }
 
-template <typename T>
-void download(Ctx& ctx, std::vector<T>& h, const T* d, uint64_t n) {
-  h.resize(n);
-  if (n) VG_CUDA(cudaMemcpyAsync(h.data(), d, n * sizeof(T), cudaMemcpyDeviceToHost, ctx.stream));
+// Runs parse_kernel; false when it gave up (nothing but the flags is of use).
+bool parse(Ctx& ctx, const uint8_t* dtext, uint64_t len, uint64_t lines, const Table& tb, uint32_t* slots,
+           const Spans& sp, bool literal_dict) {
+  const uint64_t tiles = div_up(len, static_cast<uint64_t>(kPiece));
+  Scratch<uint64_t> z(ctx, tiles + 1);   // look-back words, then the ticket
+  Scratch<Flags> flags(ctx, 1);
+  VG_CUDA(cudaMemsetAsync(z.get(), 0, (tiles + 1) * sizeof(uint64_t), ctx.stream));
+  VG_CUDA(cudaMemsetAsync(&flags.get()->bad_line, 0xFF, sizeof(unsigned long long), ctx.stream));
+  VG_CUDA(cudaMemsetAsync(&flags.get()->give_up, 0, 8, ctx.stream));
+  ctx.launch("ingest_parse", static_cast<double>(len) + 12.0 * lines, [&] {
+    parse_kernel<<<static_cast<unsigned>(tiles), kBlock, 0, ctx.stream>>>(
+        dtext, len, lines, tb, slots, sp, literal_dict, z.get(), reinterpret_cast<uint32_t*>(z.get() + tiles),
+        flags.get(), ctx.d_err);
+  });
+  VG_CUDA(cudaGetLastError());
+  VG_CUDA(cudaMemcpyAsync(ctx.h_small, flags.get(), sizeof(Flags), cudaMemcpyDeviceToHost, ctx.stream));
+  ctx.sync();
+  Flags h;
+  std::memcpy(&h, ctx.h_small, sizeof(h));
+  ctx.check_device_errors();
+  if (h.bad_line != ~0ull)
+    fail(VG_ERR_PARSE, "malformed N-Triples statement on line " + std::to_string(h.bad_line));
+  return h.give_up == 0;
 }
 
-// Exact first-appearance ids on the host for one dictionary (after a hash
-// collision): the statement handler's own rule, src/loader.cu:19-53.
-void resolve_exact(Ctx& ctx, const char* text, const Spans& sp, uint64_t n, int kind, bool literal_dict,
-                   uint32_t base, uint32_t* s, uint32_t* p, uint32_t* o, std::vector<std::string>& terms) {
-  std::vector<uint64_t> so, po, oo;
-  std::vector<uint32_t> sl, pl, ol;
-  std::vector<uint8_t> lit;
-  download(ctx, so, sp.s_off, n);
-  download(ctx, sl, sp.s_len, n);
-  download(ctx, po, sp.p_off, n);
-  download(ctx, pl, sp.p_len, n);
-  download(ctx, oo, sp.o_off, n);
-  download(ctx, ol, sp.o_len, n);
-  download(ctx, lit, sp.lit, n);
-  std::vector<uint32_t> hs, hp, ho;
-  download(ctx, hs, s, n);
-  download(ctx, hp, p, n);
-  download(ctx, ho, o, n);
+void check_ids(const uint64_t (&terms)[3], const uint32_t (&base)[3]) {
+  for (int k = 0; k < 3; ++k)
+    if (base[k] + terms[k] > 0xFFFFFFFFull) fail(VG_ERR_OVERFLOW, "dictionary ids exceed 32 bits");
+}
+
+// First-appearance ids on the host, for texts that the table cannot take (a
+// term too long for a slot's word, 2^32 lines or more, or a hash that fails
+// on the text): the statement handler's own rule, src/loader.cu:19-53.
+void ingest_on_host(Ctx& ctx, const char* text, uint64_t len, const uint8_t* dtext, uint64_t lines,
+                    bool literal_dict, Ingested& out) {
+  Scratch<uint64_t> so(ctx, 3 * lines), sl(ctx, 3 * lines);
+  Scratch<uint8_t> lit(ctx, lines);
+  Spans sp{};
+  for (int q = 0; q < 3; ++q) {
+    sp.off[q] = so.get() + q * lines;
+    sp.len[q] = sl.get() + q * lines;
+  }
+  sp.lit = lit.get();
+  parse(ctx, dtext, len, lines, Table{}, nullptr, sp, literal_dict);
+  std::vector<uint64_t> off(3 * lines), ln(3 * lines);
+  std::vector<uint8_t> hl(lines);
+  VG_CUDA(cudaMemcpyAsync(off.data(), so.get(), 3 * lines * sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx.stream));
+  VG_CUDA(cudaMemcpyAsync(ln.data(), sl.get(), 3 * lines * sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx.stream));
+  VG_CUDA(cudaMemcpyAsync(hl.data(), lit.get(), lines, cudaMemcpyDeviceToHost, ctx.stream));
   ctx.sync();
-  std::unordered_map<std::string_view, uint32_t> ids;
-  terms.clear();
-  auto id_of = [&](uint64_t off, uint32_t len) {
-    const std::string_view v(text + off, len);
-    auto it = ids.find(v);
-    if (it != ids.end()) return it->second;
-    const uint32_t id = base + static_cast<uint32_t>(terms.size());
-    ids.emplace(v, id);
-    terms.emplace_back(v);
-    return id;
-  };
-  for (uint64_t t = 0; t < n; ++t) {
-    if (kind == 0) {
-      hs[t] = id_of(so[t], sl[t]);
-      if (!(literal_dict && lit[t])) ho[t] = id_of(oo[t], ol[t]);
-    } else if (kind == 1) {
-      hp[t] = id_of(po[t], pl[t]);
-    } else if (lit[t]) {
-      ho[t] = id_of(oo[t], ol[t]);
+  std::vector<std::string>* terms[3] = {&out.dict.so, &out.dict.p, &out.dict.l};
+  const uint32_t base[3] = {1u, 1u, kLiteralStartId};
+  std::unordered_map<std::string_view, uint32_t> ids[3];
+  std::vector<uint32_t> col[3];
+  for (uint64_t i = 0; i < lines; ++i) {
+    if (ln[i] == 0) continue;
+    for (int q : {0, 2, 1}) {   // subject, object, predicate
+      const int k = q == 1 ? 1 : (q == 2 && literal_dict && hl[i] ? 2 : 0);
+      const std::string_view v(text + off[q * lines + i], ln[q * lines + i]);
+      auto it = ids[k].find(v);
+      if (it == ids[k].end()) {
+        it = ids[k].emplace(v, base[k] + static_cast<uint32_t>(terms[k]->size())).first;
+        terms[k]->emplace_back(v);
+      }
+      col[q].push_back(it->second);
     }
   }
-  if (n) {
-    VG_CUDA(cudaMemcpyAsync(s, hs.data(), n * 4, cudaMemcpyHostToDevice, ctx.stream));
-    VG_CUDA(cudaMemcpyAsync(p, hp.data(), n * 4, cudaMemcpyHostToDevice, ctx.stream));
-    VG_CUDA(cudaMemcpyAsync(o, ho.data(), n * 4, cudaMemcpyHostToDevice, ctx.stream));
+  out.n = col[0].size();
+  if (out.n > 0x7FFFFFFFull) fail(VG_ERR_OVERFLOW, "ingest is limited to 2^31 triples");
+  const uint64_t sizes[3] = {out.dict.so.size(), out.dict.p.size(), out.dict.l.size()};
+  check_ids(sizes, base);
+  uint32_t** dst[3] = {&out.s, &out.p, &out.o};
+  for (int q = 0; q < 3; ++q) {
+    *dst[q] = ctx.alloc<uint32_t>(out.n);
+    if (out.n)
+      VG_CUDA(cudaMemcpyAsync(*dst[q], col[q].data(), out.n * 4, cudaMemcpyHostToDevice, ctx.stream));
   }
   ctx.sync();
-}
-
-// One dictionary: hash, sort, runs, check, ids, scatter, terms.  Returns
-// false when a hash collision was found (nothing was written).
-bool encode_dict(Ctx& ctx, const char* host_text, const uint8_t* text, const Spans& sp, uint64_t n, int kind,
-                 bool literal_dict, uint32_t base, uint32_t* s, uint32_t* p, uint32_t* o,
-                 std::vector<std::string>& terms) {
-  const uint64_t m_all = kind == 0 ? 2 * n : n;
-  terms.clear();
-  if (m_all == 0) return true;
-  if (m_all > 0xFFFFFFFFull) fail(VG_ERR_OVERFLOW, "ingest is limited to 2^31 triples");
-  Scratch<uint64_t> keys(ctx, m_all), keys_alt(ctx, m_all);
-  Scratch<uint32_t> vals(ctx, m_all), vals_alt(ctx, m_all);
-  Scratch<unsigned long long> dm(ctx, 1);
-  VG_CUDA(cudaMemsetAsync(dm.get(), 0, sizeof(unsigned long long), ctx.stream));
-  ctx.launch("ingest_hash", 12.0 * m_all, [&] {
-    hash_kernel<<<grid(ctx, m_all), kBlock, 0, ctx.stream>>>(text, sp, n, kind, literal_dict, g_hash_bits.load(),
-                                                              keys.get(), vals.get(), dm.get());
-  });
-  VG_CUDA(cudaGetLastError());
-  const bool alt = radix_sort_u64(ctx, keys.get(), keys_alt.get(), vals.get(), vals_alt.get(), m_all, 64, false, true);
-  uint64_t* k = alt ? keys_alt.get() : keys.get();
-  uint32_t* v = alt ? vals_alt.get() : vals.get();
-  uint64_t m = 0;
-  VG_CUDA(cudaMemcpyAsync(&m, dm.get(), sizeof(m), cudaMemcpyDeviceToHost, ctx.stream));
-  ctx.sync();
-  if (m == 0) return true;
-  const uint64_t tiles = div_up(m, kTileRows);
-  Scratch<uint32_t> seg(ctx, m), head_pos(ctx, m), ticket(ctx, 1);
-  Scratch<uint64_t> status(ctx, tiles), runs_d(ctx, 1);
-  Scratch<unsigned int> coll(ctx, 1);
-  VG_CUDA(cudaMemsetAsync(status.get(), 0, tiles * sizeof(uint64_t), ctx.stream));
-  VG_CUDA(cudaMemsetAsync(ticket.get(), 0, sizeof(uint32_t), ctx.stream));
-  VG_CUDA(cudaMemsetAsync(coll.get(), 0, sizeof(unsigned int), ctx.stream));
-  ctx.launch("ingest_runs", 12.0 * m, [&] {
-    heads_kernel<<<static_cast<unsigned>(tiles), kBlock, 0, ctx.stream>>>(k, m, seg.get(), head_pos.get(),
-                                                                           status.get(), ticket.get(), runs_d.get(),
-                                                                           ctx.d_err);
-  });
-  VG_CUDA(cudaGetLastError());
-  ctx.launch("ingest_verify", 8.0 * m, [&] {
-    verify_kernel<<<grid(ctx, m), kBlock, 0, ctx.stream>>>(text, sp, kind, v, seg.get(), head_pos.get(), m,
-                                                            coll.get());
-  });
-  VG_CUDA(cudaGetLastError());
-  uint64_t runs = 0;
-  unsigned int collided = 0;
-  VG_CUDA(cudaMemcpyAsync(&runs, runs_d.get(), sizeof(runs), cudaMemcpyDeviceToHost, ctx.stream));
-  VG_CUDA(cudaMemcpyAsync(&collided, coll.get(), sizeof(collided), cudaMemcpyDeviceToHost, ctx.stream));
-  ctx.sync();
-  if (collided) return false;
-  if (static_cast<uint64_t>(base) + runs > 0xFFFFFFFFull) fail(VG_ERR_OVERFLOW, "dictionary ids exceed 32 bits");
-  Scratch<uint32_t> fpos(ctx, runs), fpos_alt(ctx, runs), rid(ctx, runs), rid_alt(ctx, runs), id_of_run(ctx, runs);
-  ctx.launch("ingest_ids", 8.0 * runs, [&] {
-    first_pos_kernel<<<grid(ctx, runs), kBlock, 0, ctx.stream>>>(v, head_pos.get(), runs, fpos.get(), rid.get());
-  });
-  VG_CUDA(cudaGetLastError());
-  const bool alt2 = radix_sort_u32(ctx, fpos.get(), fpos_alt.get(), rid.get(), rid_alt.get(), runs, 32, false, true);
-  const uint32_t* fs = alt2 ? fpos_alt.get() : fpos.get();
-  const uint32_t* rs = alt2 ? rid_alt.get() : rid.get();
-  ctx.launch("ingest_ids", 8.0 * runs, [&] {
-    rank_kernel<<<grid(ctx, runs), kBlock, 0, ctx.stream>>>(rs, runs, base, id_of_run.get());
-  });
-  VG_CUDA(cudaGetLastError());
-  ctx.launch("ingest_scatter", 12.0 * m, [&] {
-    scatter_kernel<<<grid(ctx, m), kBlock, 0, ctx.stream>>>(v, seg.get(), id_of_run.get(), m, kind, s, p, o);
-  });
-  VG_CUDA(cudaGetLastError());
-  Scratch<uint64_t> toff(ctx, runs);
-  Scratch<uint32_t> tlen(ctx, runs);
-  ctx.launch("ingest_terms", 12.0 * runs, [&] {
-    dict_spans_kernel<<<grid(ctx, runs), kBlock, 0, ctx.stream>>>(sp, kind, fs, runs, toff.get(), tlen.get());
-  });
-  VG_CUDA(cudaGetLastError());
-  std::vector<uint64_t> ho;
-  std::vector<uint32_t> hl;
-  download(ctx, ho, toff.get(), runs);
-  download(ctx, hl, tlen.get(), runs);
-  ctx.sync();
-  terms.resize(runs);
-  parallel_for(runs, [&](size_t r) { terms[r].assign(host_text + ho[r], hl[r]); });
-  return true;
 }
 
 }  // namespace
@@ -610,74 +584,88 @@ void ingest_ntriples(Ctx& ctx, const char* text, uint64_t len, bool literal_dict
   // the text, padded to whole 16-byte words
   Scratch<uint8_t> dtext(ctx, div_up(len, 16) * 16);
   VG_CUDA(cudaMemcpyAsync(dtext.get(), text, len, cudaMemcpyHostToDevice, ctx.stream));
-  // 1. newlines
-  const uint64_t ntiles = div_up(len, kNlTile);
-  if (ntiles > 0xFFFFFFFFull) fail(VG_ERR_OVERFLOW, "ingest text too long");
+  // 1. lines
+  if (div_up(len, static_cast<uint64_t>(kPiece)) > 0x7FFFFFFFull) fail(VG_ERR_OVERFLOW, "ingest text too long");
   Scratch<unsigned long long> ncount(ctx, 1);
   VG_CUDA(cudaMemsetAsync(ncount.get(), 0, sizeof(unsigned long long), ctx.stream));
   ctx.launch("ingest_newlines", static_cast<double>(len), [&] {
-    newline_count_kernel<<<grid(ctx, div_up(len, 16)), kBlock, 0, ctx.stream>>>(dtext.get(), len, ncount.get());
+    newline_count_kernel<<<grid(ctx, div_up(len, 64)), kBlock, 0, ctx.stream>>>(dtext.get(), len, ncount.get());
   });
   VG_CUDA(cudaGetLastError());
-  unsigned long long nl_count = 0;
-  VG_CUDA(cudaMemcpyAsync(&nl_count, ncount.get(), sizeof(nl_count), cudaMemcpyDeviceToHost, ctx.stream));
+  VG_CUDA(cudaMemcpyAsync(ctx.h_small, ncount.get(), sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx.stream));
   ctx.sync();
-  Scratch<uint64_t> nl(ctx, nl_count + 1), st1(ctx, ntiles), tot1(ctx, 1);
-  Scratch<uint32_t> tk1(ctx, 1);
-  VG_CUDA(cudaMemsetAsync(st1.get(), 0, ntiles * sizeof(uint64_t), ctx.stream));
-  VG_CUDA(cudaMemsetAsync(tk1.get(), 0, sizeof(uint32_t), ctx.stream));
-  ctx.launch("ingest_newlines", static_cast<double>(len), [&] {
-    newline_kernel<<<static_cast<unsigned>(ntiles), kBlock, 0, ctx.stream>>>(dtext.get(), len, nl.get(), st1.get(),
-                                                                            tk1.get(), tot1.get(), ctx.d_err);
-  });
-  VG_CUDA(cudaGetLastError());
-  uint64_t nnl = 0;
-  VG_CUDA(cudaMemcpyAsync(&nnl, tot1.get(), sizeof(nnl), cudaMemcpyDeviceToHost, ctx.stream));
-  ctx.sync();
-  const uint64_t lines = nnl + (text[len - 1] != '\n' ? 1 : 0);
-  // 2. statements
-  Scratch<uint64_t> s_off(ctx, lines), p_off(ctx, lines), o_off(ctx, lines);
-  Scratch<uint32_t> s_len(ctx, lines), p_len(ctx, lines), o_len(ctx, lines);
-  Scratch<uint8_t> lit(ctx, lines);
-  const Spans sp{s_off.get(), p_off.get(), o_off.get(), s_len.get(), p_len.get(), o_len.get(), lit.get()};
-  const uint64_t ptiles = div_up(lines, static_cast<uint64_t>(kBlock));
-  Scratch<uint64_t> st2(ctx, ptiles), cnt(ctx, 1);
-  Scratch<uint32_t> tk2(ctx, 1);
-  Scratch<unsigned long long> bad(ctx, 1);
-  VG_CUDA(cudaMemsetAsync(st2.get(), 0, ptiles * sizeof(uint64_t), ctx.stream));
-  VG_CUDA(cudaMemsetAsync(tk2.get(), 0, sizeof(uint32_t), ctx.stream));
-  VG_CUDA(cudaMemsetAsync(bad.get(), 0xFF, sizeof(unsigned long long), ctx.stream));
-  ctx.launch("ingest_parse", static_cast<double>(len) + 37.0 * lines, [&] {
-    parse_kernel<<<static_cast<unsigned>(ptiles), kBlock, 0, ctx.stream>>>(
-        dtext.get(), len, nl.get(), nnl, lines, sp, st2.get(), tk2.get(), cnt.get(), bad.get(), ctx.d_err);
-  });
-  VG_CUDA(cudaGetLastError());
-  uint64_t n = 0;
-  unsigned long long bad_line = 0;
-  VG_CUDA(cudaMemcpyAsync(&n, cnt.get(), sizeof(n), cudaMemcpyDeviceToHost, ctx.stream));
-  VG_CUDA(cudaMemcpyAsync(&bad_line, bad.get(), sizeof(bad_line), cudaMemcpyDeviceToHost, ctx.stream));
-  ctx.sync();
-  ctx.check_device_errors();
-  if (bad_line != ~0ull) fail(VG_ERR_PARSE, "malformed N-Triples statement on line " + std::to_string(bad_line));
-  if (n > 0x7FFFFFFFull) fail(VG_ERR_OVERFLOW, "ingest is limited to 2^31 triples");
-  out.n = n;
-  out.s = ctx.alloc<uint32_t>(n);
-  out.p = ctx.alloc<uint32_t>(n);
-  out.o = ctx.alloc<uint32_t>(n);
-  if (n == 0) return;
-  // 3-5. the dictionaries
-  struct Job {
-    int kind;
-    uint32_t base;
-    std::vector<std::string>* terms;
-  };
-  std::vector<Job> jobs = {{0, 1u, &out.dict.so}, {1, 1u, &out.dict.p}};
-  if (literal_dict) jobs.push_back({2, kLiteralStartId, &out.dict.l});
-  for (const Job& j : jobs) {
-    if (!encode_dict(ctx, text, dtext.get(), sp, n, j.kind, literal_dict, j.base, out.s, out.p, out.o, *j.terms)) {
-      ++out.collisions;
-      resolve_exact(ctx, text, sp, n, j.kind, literal_dict, j.base, out.s, out.p, out.o, *j.terms);
+  const uint64_t lines = ctx.h_small[0] + (text[len - 1] != '\n' ? 1 : 0);
+  // 2. statements and terms.  Three terms a line, four slots of the table for
+  // every three of them (2^32 slots at most).
+  bool done = false;
+  if (lines < 0xFFFFFFFFull) {
+    Table tb{};
+    int off_bits = 1;
+    while (len >> off_bits) ++off_bits;
+    tb.len_bits = static_cast<uint32_t>(62 - off_bits < off_bits ? 62 - off_bits : off_bits);
+    tb.cap = std::min<uint64_t>(4 * lines + 64, 0xFFFFFFFFull);
+    tb.hash_bits = g_hash_bits.load();
+    Scratch<Slot> table(ctx, tb.cap);
+    tb.slots = table.get();
+    VG_CUDA(cudaMemsetAsync(tb.slots, 0, tb.cap * sizeof(Slot), ctx.stream));
+    Scratch<uint32_t> slots(ctx, 3 * lines);
+    if (parse(ctx, dtext.get(), len, lines, tb, slots.get(), Spans{}, literal_dict)) {
+      // 3. ids
+      const uint32_t base[3] = {1u, 1u, kLiteralStartId};
+      const uint3 base3 = make_uint3(base[0], base[1], base[2]);
+      const uint64_t tiles = div_up(lines, kTileLines);
+      const size_t words = 4 * tiles + 5;   // look-back words, counts, ticket
+      Scratch<uint64_t> z(ctx, words), first(ctx, tiles);
+      VG_CUDA(cudaMemsetAsync(z.get(), 0, words * sizeof(uint64_t), ctx.stream));
+      auto* counts = reinterpret_cast<Counts*>(z.get() + 4 * tiles);
+      ctx.launch("ingest_ids", 12.0 * lines, [&] {
+        ids_kernel<<<static_cast<unsigned>(tiles), kBlock, 0, ctx.stream>>>(
+            slots.get(), tb.slots, lines, tiles, base3, z.get(), reinterpret_cast<uint32_t*>(counts + 1),
+            first.get(), counts, ctx.d_err);
+      });
+      VG_CUDA(cudaGetLastError());
+      VG_CUDA(cudaMemcpyAsync(ctx.h_small, counts, sizeof(Counts), cudaMemcpyDeviceToHost, ctx.stream));
+      ctx.sync();
+      Counts h;
+      std::memcpy(&h, ctx.h_small, sizeof(h));
+      ctx.check_device_errors();
+      if (h.n[0] > 0x7FFFFFFFull) fail(VG_ERR_OVERFLOW, "ingest is limited to 2^31 triples");
+      const uint64_t nterms[3] = {h.n[1], h.n[2], h.n[3]};
+      check_ids(nterms, base);
+      // 4. columns and terms
+      out.n = h.n[0];
+      out.s = ctx.alloc<uint32_t>(out.n);
+      out.p = ctx.alloc<uint32_t>(out.n);
+      out.o = ctx.alloc<uint32_t>(out.n);
+      if (out.n) {
+        const uint64_t all = nterms[0] + nterms[1] + nterms[2];
+        Scratch<uint64_t> dloc(ctx, all);
+        const TermList tl{{dloc.get(), dloc.get() + nterms[0], dloc.get() + nterms[0] + nterms[1]}};
+        ctx.launch("ingest_scatter", 24.0 * lines, [&] {
+          columns_kernel<<<static_cast<unsigned>(tiles), kBlock, 0, ctx.stream>>>(
+              slots.get(), tb.slots, lines, base3, first.get(), out.s, out.p, out.o, tl);
+        });
+        VG_CUDA(cudaGetLastError());
+        std::vector<uint64_t> loc(all);
+        VG_CUDA(cudaMemcpyAsync(loc.data(), dloc.get(), all * sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx.stream));
+        ctx.sync();
+        std::vector<std::string>* terms[3] = {&out.dict.so, &out.dict.p, &out.dict.l};
+        const uint64_t* at = loc.data();
+        for (int k = 0; k < 3; ++k) {
+          std::vector<std::string>& v = *terms[k];
+          v.resize(nterms[k]);
+          parallel_for(nterms[k], [&](size_t r) {
+            v[r].assign(text + (at[r] >> tb.len_bits), at[r] & ((1ull << tb.len_bits) - 1));
+          });
+          at += nterms[k];
+        }
+      }
+      done = true;
     }
+  }
+  if (!done) {
+    ++out.collisions;
+    ingest_on_host(ctx, text, len, dtext.get(), lines, literal_dict, out);
   }
   ctx.sync();
   ctx.check_device_errors();

@@ -47,7 +47,7 @@ struct Ingested {
   uint64_t n = 0;                                      // triples
   uint32_t *s = nullptr, *p = nullptr, *o = nullptr;   // device columns (context arena)
   Dict dict;
-  uint32_t collisions = 0;   // hash groups that held different terms (resolved exactly)
+  uint32_t collisions = 0;   // 1: the term table gave up and the host assigned the ids
 };
 
 // Parses `len` bytes of N-Triples text and assigns ids in order of first
@@ -68,8 +68,8 @@ std::string decode_rows(const Dict& d, const std::vector<const uint32_t*>& cols,
 void write_vdd(const Dict& d, const char* path);
 void read_vdd(const char* path, Dict& d);
 
-// Test hook: the number of hash bits used to group terms (63 by default);
-// fewer bits force collisions so that the exact resolution path runs.
+// Test hook: the number of hash bits that place terms in the table (63 by
+// default); fewer bits make long searches, one bit searches that give up.
 void set_ingest_hash_bits(int bits);
 
 }  // namespace vg
