@@ -102,8 +102,7 @@ __device__ __forceinline__ uint64_t word_at(const uint8_t* p, uint64_t off, uint
 }
 
 // Term at t[i]; returns its end (one past) or 0 on a malformed term.
-// kind: 0 any, 1 IRI only (predicate), 2 IRI or blank node (subject).  I is
-// 32 bits wide for lines in shared memory.
+// kind: 0 any, 1 IRI only (predicate), 2 IRI or blank node (subject).
 template <typename I>
 __device__ __forceinline__ I iri_end(const uint8_t* t, I i, I end) {
   for (I j = i + 1; j < end; ++j) {
@@ -235,21 +234,147 @@ __device__ uint32_t find_slot(const Table& tb, const uint8_t* text, const uint8_
   return kNoSlot;
 }
 
+// Byte classes of a piece as bitmaps, one 64-bit word per 64 bytes: a parser
+// that jumps from one byte of interest to the next reads a word or two where
+// it read every byte (0.47 ms for 101 MB).
+struct ByteMaps {
+  static constexpr uint32_t kWords = (kPiece + kHalo) / 64;
+  uint64_t iri_stop[kWords];   // '>', space, tab
+  uint64_t space[kWords];      // space, tab, carriage return
+  uint64_t quote[kWords];      // '"', backslash
+};
+
+// 0x80 in every byte of w that equals c.
+__device__ __forceinline__ uint32_t bytes_equal(uint32_t w, uint8_t c) {
+  const uint32_t x = w ^ (0x01010101u * c);
+  return ~(((x & 0x7f7f7f7fu) + 0x7f7f7f7fu) | x | 0x7f7f7f7fu);
+}
+// The four top bits of such a mask, lowest byte first.
+__device__ __forceinline__ uint64_t byte_bits(uint32_t m) {
+  return ((m >> 7) * 0x00204081u >> 21) & 15u;
+}
+
+// Classifies the 64 bytes at s_text + 64 * word (bytes from `have` on belong
+// to no class); returns their newlines.
+__device__ __forceinline__ uint64_t classify(const uint8_t* s_text, uint32_t word, uint32_t have, ByteMaps& bm) {
+  uint64_t stop = 0, space = 0, quote = 0, nl = 0;
+#pragma unroll 4
+  for (int q = 0; q < 16; ++q) {
+    const uint32_t w = reinterpret_cast<const uint32_t*>(s_text)[word * 16 + q];
+    const uint32_t blank = bytes_equal(w, ' ') | bytes_equal(w, '\t');
+    stop |= byte_bits(blank | bytes_equal(w, '>')) << (4 * q);
+    space |= byte_bits(blank | bytes_equal(w, '\r')) << (4 * q);
+    quote |= byte_bits(bytes_equal(w, '"') | bytes_equal(w, '\\')) << (4 * q);
+    nl |= byte_bits(bytes_equal(w, '\n')) << (4 * q);
+  }
+  const uint32_t first = word * 64;
+  const uint64_t in = first >= have ? 0 : have - first >= 64 ? ~0ull : (1ull << (have - first)) - 1;
+  bm.iri_stop[word] = stop & in;
+  bm.space[word] = space & in;
+  bm.quote[word] = quote & in;
+  return nl & in;
+}
+
+// First byte of [i, e) in the class (SET) or outside it; e when there is none.
+template <bool SET>
+__device__ __forceinline__ uint32_t next_byte(const uint64_t* map, uint32_t i, uint32_t e) {
+  if (i >= e) return e;
+  uint32_t w = i >> 6;
+  uint64_t m = (SET ? map[w] : ~map[w]) >> (i & 63);
+  uint32_t at = i;
+  while (m == 0) {
+    at = ++w * 64;
+    if (at >= e) return e;
+    m = SET ? map[w] : ~map[w];
+  }
+  at += __ffsll(static_cast<long long>(m)) - 1;
+  return at < e ? at : e;
+}
+
+// term_end and parse_line for a line within the piece, over its byte maps.
+__device__ __forceinline__ uint32_t mapped_term_end(const uint8_t* t, const ByteMaps& bm, uint32_t i, uint32_t end,
+                                                    int kind, bool& literal) {
+  literal = false;
+  if (i >= end) return 0;
+  const uint8_t c = t[i];
+  if (c == '<') {
+    const uint32_t j = next_byte<true>(bm.iri_stop, i + 1, end);
+    return j < end && t[j] == '>' ? j + 1 : 0;
+  }
+  if (kind == 1) return 0;
+  if (c == '_') {
+    if (i + 1 >= end || t[i + 1] != ':') return 0;
+    uint32_t j = next_byte<true>(bm.space, i + 2, end);
+    if (j == i + 2) return 0;
+    if (t[j - 1] == '.' && j - 1 > i + 2) --j;
+    return j;
+  }
+  if (kind == 2 || c != '"') return 0;
+  uint32_t j = i + 1;
+  while (true) {
+    j = next_byte<true>(bm.quote, j, end);
+    if (j >= end) return 0;
+    if (t[j] == '"') break;
+    j += 2;   // a backslash and what it escapes
+  }
+  ++j;
+  literal = true;
+  if (j < end && t[j] == '@') {
+    uint32_t k = j + 1;
+    while (k < end && ((t[k] >= 'a' && t[k] <= 'z') || (t[k] >= 'A' && t[k] <= 'Z') ||
+                       (t[k] >= '0' && t[k] <= '9') || t[k] == '-'))
+      ++k;
+    return k == j + 1 ? 0 : k;
+  }
+  if (j + 1 < end && t[j] == '^' && t[j + 1] == '^') {
+    if (j + 2 >= end || t[j + 2] != '<') return 0;
+    const uint32_t k = next_byte<true>(bm.iri_stop, j + 3, end);
+    return k < end && t[k] == '>' ? k + 1 : 0;
+  }
+  return j;
+}
+
+__device__ __forceinline__ int mapped_parse_line(const uint8_t* t, const ByteMaps& bm, uint32_t b, uint32_t e,
+                                                 uint32_t (&off)[3], uint32_t (&len)[3], bool& lit) {
+  uint32_t i = next_byte<false>(bm.space, b, e);
+  if (i >= e || t[i] == '#') return 0;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    off[k] = i;
+    const uint32_t end = mapped_term_end(t, bm, i, e, k == 0 ? 2 : (k == 1 ? 1 : 0), lit);
+    if (end == 0) return 2;
+    len[k] = end - i;
+    i = next_byte<false>(bm.space, end, e);
+    if (k < 2 && i == end) return 2;
+  }
+  if (i >= e || t[i] != '.') return 2;
+  i = next_byte<false>(bm.space, i + 1, e);
+  return i >= e || t[i] == '#' ? 1 : 2;
+}
+
 // A block per piece of kPiece bytes, in ticket order; it owns the lines that
 // start after the piece's newlines (and the text's first line).  The piece
-// lies in shared memory: one thread per line reads its line byte by byte,
-// which from global memory costs a cache access per byte and lane (0.27 ms
-// for 101 MB, and again for the hashes).  slots: [3][lines], kNoSlot in the
-// subject's place where the line holds no statement.
-__global__ void __launch_bounds__(kBlock) parse_kernel(const uint8_t* __restrict__ text, uint64_t len, uint64_t lines,
-                                                       Table tb, uint32_t* __restrict__ slots, Spans sp,
-                                                       bool literal_dict, uint64_t* status, uint32_t* ticket,
-                                                       Flags* fl, DeviceErrors* err) {
+// lies in shared memory (from global memory a byte at a time costs a cache
+// access per byte and lane).  Its lines are taken kBlock at a time: one
+// thread parses each, then the threads share their terms, three a line, out
+// among them for the table searches.  A line that ends more than kHalo bytes
+// after the piece is parsed and looked up by one thread from global memory.
+// slots: [3][lines], kNoSlot in the subject's place where the line holds no
+// statement.
+__global__ void __launch_bounds__(kBlock, 4) parse_kernel(const uint8_t* __restrict__ text, uint64_t len,
+                                                          uint64_t lines, Table tb, uint32_t* __restrict__ slots,
+                                                          Spans sp, bool literal_dict, uint64_t* status,
+                                                          uint32_t* ticket, Flags* fl, DeviceErrors* err) {
   __shared__ __align__(16) uint8_t s_text[kPiece + kHalo + 16];
+  __shared__ ByteMaps s_map;
   __shared__ uint16_t s_start[kLineList + 1];   // first bytes of the listed lines (kPiece at most)
+  __shared__ uint32_t s_term[3][kBlock];        // length << 16 | first byte (0: no term, or looked up already)
+  __shared__ uint8_t s_lit[kBlock];
   __shared__ uint32_t s_scan[kBlock / 32 + 1];
   __shared__ uint64_t s_b;
   __shared__ uint32_t s_tile;
+  static_assert(kPiece + kHalo < (1 << 16), "places and lengths in a piece fit 16 bits");
+  static_assert(kLineList % kBlock == 0, "listed lines are taken kBlock at a time");
   const uint32_t tid = threadIdx.x;
   if (tid == 0) s_tile = atomicAdd(ticket, 1u);
   __syncthreads();
@@ -259,17 +384,11 @@ __global__ void __launch_bounds__(kBlock) parse_kernel(const uint8_t* __restrict
   for (uint32_t w = tid; w < (have + 15) / 16; w += kBlock)
     reinterpret_cast<uint4*>(s_text)[w] = reinterpret_cast<const uint4*>(text + base)[w];
   __syncthreads();
-  // the thread's 64 bytes: bit k of nl, byte k is a newline
-  uint64_t nl = 0;
-#pragma unroll
-  for (int q = 0; q < 16; ++q) {
-    const uint32_t m = __vcmpeq4(reinterpret_cast<const uint32_t*>(s_text)[tid * 16 + q], kNewlines) & 0x08040201u;
-    nl |= static_cast<uint64_t>((m | m >> 8 | m >> 16 | m >> 24) & 15u) << (4 * q);
-  }
+  // newlines of the thread's 64 bytes, and of the bytes after the piece none
   const uint32_t mine0 = tid * 64;
+  const uint64_t nl = classify(s_text, tid, have, s_map);
+  if (tid < kHalo / 64) (void)classify(s_text, kBlock + tid, have, s_map);
   const uint32_t piece = have < kPiece ? have : kPiece;
-  if (mine0 >= piece) nl = 0;
-  else if (piece - mine0 < 64) nl &= (1ull << (piece - mine0)) - 1;
   uint32_t total;
   const uint32_t ahead = block_excl_scan<kBlock>(static_cast<uint32_t>(__popcll(nl)), total, s_scan);
   if (tid < 32) {
@@ -296,57 +415,67 @@ __global__ void __launch_bounds__(kBlock) parse_kernel(const uint8_t* __restrict
         ++k;
       }
     }
-    __syncthreads();
-    for (uint32_t k = tid; k < kLineList && from + k < n_lines; k += kBlock) {
+    for (uint32_t k0 = 0; k0 < kLineList && from + k0 < n_lines; k0 += kBlock) {
+      __syncthreads();   // the list is complete; the last round's terms are looked up
+      const uint32_t k = k0 + tid;
       const uint64_t line = line0 + from + k;
-      const uint32_t b = s_start[k];
-      if (base + b >= len || line >= lines) continue;   // the text's last newline starts no line
-      uint64_t off[3] = {0, 0, 0}, tl[3] = {0, 0, 0};
-      bool lit = false, near = true;
-      int got;
-      uint32_t e = b;
-      if (from + k + 1 < n_lines) {
-        e = s_start[k + 1] - 1u;
-      } else {
-        e = piece > b ? piece : b;
-        while (e < have && s_text[e] != '\n') ++e;
-        near = e < have || base + have == len;   // the line ends within shared memory
-      }
-      const uint8_t* t = s_text;
-      if (near) {
-        uint32_t o4[3] = {0, 0, 0}, l4[3] = {0, 0, 0};
-        got = parse_line<uint32_t>(s_text, b, e, o4, l4, lit);
-        for (int q = 0; q < 3; ++q) {
-          off[q] = o4[q];
-          tl[q] = l4[q];
+      const bool own = from + k < n_lines && base + s_start[k] < len && line < lines;
+      uint32_t o4[3] = {0, 0, 0}, l4[3] = {0, 0, 0};
+      bool lit = false;
+      int got = 0;
+      if (own) {   // (the text's last newline starts no line)
+        const uint32_t b = s_start[k];
+        uint32_t e;
+        bool near = true;
+        if (from + k + 1 < n_lines) {
+          e = s_start[k + 1] - 1u;
+        } else {
+          e = piece > b ? piece : b;
+          while (e < have && s_text[e] != '\n') ++e;
+          near = e < have || base + have == len;   // the line ends within shared memory
         }
-      } else {
-        uint64_t eg = base + have;
-        while (eg < len && text[eg] != '\n') ++eg;
-        got = parse_line<uint64_t>(text, base + b, eg, off, tl, lit);
-        t = text;
-      }
-      if (got == 2) atomicMin(&fl->bad_line, static_cast<unsigned long long>(line + 1));
-      uint32_t sl[3] = {kNoSlot, kNoSlot, kNoSlot};
-      if (got == 1 && tb.slots) {
-        const uint64_t add = near ? base : 0;
-#pragma unroll 1
-        for (int q = 0; q < 3; ++q) {
-          const uint32_t dict = q == 1 ? 1u : (q == 2 && lit && literal_dict ? 2u : 0u);
-          sl[q] = find_slot(tb, text, t, off[q], off[q] + add, tl[q], dict, static_cast<uint32_t>(line), fl);
+        if (near) {
+          got = mapped_parse_line(s_text, s_map, b, e, o4, l4, lit);
+          if (sp.lit)
+            for (int q = 0; q < 3; ++q) {
+              sp.off[q][line] = base + o4[q];
+              sp.len[q][line] = got == 1 ? l4[q] : 0;
+            }
+        } else {
+          uint64_t eg = base + have;
+          while (eg < len && text[eg] != '\n') ++eg;
+          uint64_t off[3] = {0, 0, 0}, tl[3] = {0, 0, 0};
+          got = parse_line<uint64_t>(text, base + b, eg, off, tl, lit);
+          if (got == 1 && slots)
+            for (int q = 0; q < 3; ++q) {
+              const uint32_t dict = q == 1 ? 1u : (q == 2 && lit && literal_dict ? 2u : 0u);
+              slots[q * lines + line] =
+                  find_slot(tb, text, text, off[q], off[q], tl[q], dict, static_cast<uint32_t>(line), fl);
+            }
+          if (sp.lit)
+            for (int q = 0; q < 3; ++q) {
+              sp.off[q][line] = off[q];
+              sp.len[q][line] = got == 1 ? tl[q] : 0;
+            }
         }
+        if (got == 2) atomicMin(&fl->bad_line, static_cast<unsigned long long>(line + 1));
+        if (got != 1 && slots) slots[line] = kNoSlot;
+        if (sp.lit) sp.lit[line] = lit ? 1 : 0;
       }
-      if (slots) {
-        slots[line] = sl[0];
-        slots[lines + line] = sl[1];
-        slots[2 * lines + line] = sl[2];
-      }
-      if (sp.lit) {
-        for (int q = 0; q < 3; ++q) {
-          sp.off[q][line] = off[q] + (near ? base : 0);
-          sp.len[q][line] = got == 1 ? tl[q] : 0;
-        }
-        sp.lit[line] = lit ? 1 : 0;
+#pragma unroll
+      for (int q = 0; q < 3; ++q) s_term[q][tid] = got == 1 ? (l4[q] << 16 | o4[q]) : 0u;
+      s_lit[tid] = lit ? 1 : 0;
+      __syncthreads();
+      if (!slots) continue;
+      const uint32_t here = n_lines - from - k0 < kBlock ? n_lines - from - k0 : kBlock;
+      for (uint32_t x = tid; x < 3 * here; x += kBlock) {
+        const uint32_t q = x / here, r = x - q * here, w = s_term[q][r];
+        if (w == 0) continue;
+        const uint64_t l = line0 + from + k0 + r;
+        const uint32_t off = w & 0xffffu;
+        const uint32_t dict = q == 1 ? 1u : (q == 2 && s_lit[r] && literal_dict ? 2u : 0u);
+        slots[q * lines + l] =
+            find_slot(tb, text, s_text, off, base + off, w >> 16, dict, static_cast<uint32_t>(l), fl);
       }
     }
   }
