@@ -696,8 +696,8 @@ uint64_t vg_dict_size(const vg_dict* d, int kind) {
 
 const char* vg_dict_term(const vg_dict* d, int kind, uint32_t id) {
   if (!d) return nullptr;
-  const std::string* t = d->d.term(kind, id);
-  return t ? t->c_str() : nullptr;
+  size_t at;
+  return d->d.has(kind, id, &at) ? d->d.terms(kind).c_str(at) : nullptr;
 }
 
 uint32_t vg_dict_lookup(vg_dict* d, int kind, const char* term) {

@@ -651,7 +651,7 @@ void ingest_on_host(Ctx& ctx, const char* text, uint64_t len, const uint8_t* dte
   VG_CUDA(cudaMemcpyAsync(ln.data(), sl.get(), 3 * lines * sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx.stream));
   VG_CUDA(cudaMemcpyAsync(hl.data(), lit.get(), lines, cudaMemcpyDeviceToHost, ctx.stream));
   ctx.sync();
-  std::vector<std::string>* terms[3] = {&out.dict.so, &out.dict.p, &out.dict.l};
+  TermTexts* terms[3] = {&out.dict.so, &out.dict.p, &out.dict.l};
   const uint32_t base[3] = {1u, 1u, kLiteralStartId};
   std::unordered_map<std::string_view, uint32_t> ids[3];
   std::vector<uint32_t> col[3];
@@ -663,7 +663,7 @@ void ingest_on_host(Ctx& ctx, const char* text, uint64_t len, const uint8_t* dte
       auto it = ids[k].find(v);
       if (it == ids[k].end()) {
         it = ids[k].emplace(v, base[k] + static_cast<uint32_t>(terms[k]->size())).first;
-        terms[k]->emplace_back(v);
+        terms[k]->push_back(v);
       }
       col[q].push_back(it->second);
     }
@@ -685,17 +685,52 @@ void ingest_on_host(Ctx& ctx, const char* text, uint64_t len, const uint8_t* dte
 
 void set_ingest_hash_bits(int bits) { g_hash_bits.store(bits < 1 ? 1 : (bits > 63 ? 63 : bits)); }
 
-const std::string* Dict::term(int kind, uint32_t id) const {
-  const std::vector<std::string>& v = kind == 0 ? so : (kind == 1 ? p : l);
+void TermTexts::push_back(std::string_view v) {
+  const size_t end = at_.back(), need = end + v.size() + 1;
+  if (need > cap_) {
+    const size_t cap = std::max<size_t>(2 * cap_, need + 64);
+    std::unique_ptr<char[]> grown(new char[cap]);
+    if (end) std::memcpy(grown.get(), text_.get(), end);
+    text_ = std::move(grown);
+    cap_ = cap;
+  }
+  std::memcpy(text_.get() + end, v.data(), v.size());
+  text_[end + v.size()] = 0;
+  at_.push_back(need);
+}
+
+void TermTexts::assign(const char* text, size_t count,
+                       const std::function<std::pair<uint64_t, uint64_t>(size_t)>& span) {
+  at_.resize(count + 1);
+  uint64_t end = 0;
+  for (size_t i = 0; i < count; ++i) {
+    at_[i] = end;
+    end += span(i).second + 1;
+  }
+  at_[count] = end;
+  text_.reset(new char[end ? end : 1]);
+  cap_ = end;
+  constexpr size_t kTerms = 1024;   // terms per item of the parallel loop
+  parallel_for((count + kTerms - 1) / kTerms, [&](size_t b) {
+    for (size_t i = b * kTerms; i < std::min(count, (b + 1) * kTerms); ++i) {
+      const auto s = span(i);
+      std::memcpy(text_.get() + at_[i], text + s.first, s.second);
+      text_[at_[i + 1] - 1] = 0;
+    }
+  });
+}
+
+bool Dict::has(int kind, uint32_t id, size_t* at) const {
   const uint32_t base = kind == 2 ? kLiteralStartId : 1u;
-  if (id < base || id - base >= v.size()) return nullptr;
-  return &v[id - base];
+  if (id < base || id - base >= terms(kind).size()) return false;
+  *at = id - base;
+  return true;
 }
 
 uint32_t Dict::lookup(int kind, const std::string& t) {
   if (kind < 0 || kind > 2) return 0;
   auto& rev = rev_[kind];
-  const std::vector<std::string>& v = kind == 0 ? so : (kind == 1 ? p : l);
+  const TermTexts& v = terms(kind);
   const uint32_t base = kind == 2 ? kLiteralStartId : 1u;
   if (rev.size() != v.size()) {
     rev.clear();
@@ -778,13 +813,11 @@ void ingest_ntriples(Ctx& ctx, const char* text, uint64_t len, bool literal_dict
         std::vector<uint64_t> loc(all);
         VG_CUDA(cudaMemcpyAsync(loc.data(), dloc.get(), all * sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx.stream));
         ctx.sync();
-        std::vector<std::string>* terms[3] = {&out.dict.so, &out.dict.p, &out.dict.l};
+        TermTexts* terms[3] = {&out.dict.so, &out.dict.p, &out.dict.l};
         const uint64_t* at = loc.data();
         for (int k = 0; k < 3; ++k) {
-          std::vector<std::string>& v = *terms[k];
-          v.resize(nterms[k]);
-          parallel_for(nterms[k], [&](size_t r) {
-            v[r].assign(text + (at[r] >> tb.len_bits), at[r] & ((1ull << tb.len_bits) - 1));
+          terms[k]->assign(text, nterms[k], [&](size_t r) {
+            return std::make_pair(at[r] >> tb.len_bits, at[r] & ((1ull << tb.len_bits) - 1));
           });
           at += nterms[k];
         }
@@ -801,11 +834,11 @@ void ingest_ntriples(Ctx& ctx, const char* text, uint64_t len, bool literal_dict
 }
 
 DictResolver::DictResolver(const Dict* d) {
-  const std::vector<std::string>* v[3] = {&d->so, &d->p, &d->l};
   for (int k = 0; k < 3; ++k) {
+    const TermTexts& v = d->terms(k);
     const uint32_t base = k == 2 ? kLiteralStartId : 1u;
-    rev_[k].reserve(v[k]->size());
-    for (size_t i = 0; i < v[k]->size(); ++i) rev_[k].emplace((*v[k])[i], base + static_cast<uint32_t>(i));
+    rev_[k].reserve(v.size());
+    for (size_t i = 0; i < v.size(); ++i) rev_[k].emplace(std::string(v[i]), base + static_cast<uint32_t>(i));
   }
 }
 
@@ -832,8 +865,9 @@ std::string decode_rows(const Dict& d, const std::vector<const uint32_t*>& cols,
       for (size_t c = 0; c < cols.size(); ++c) {
         if (c) o += '\t';
         const uint32_t id = cols[c][r];
-        const std::string* t = (d.literal_dict && id >= kLiteralStartId) ? d.term(2, id) : d.term(0, id);
-        if (t) o += *t;
+        const int kind = d.literal_dict && id >= kLiteralStartId ? 2 : 0;
+        size_t at;
+        if (d.has(kind, id, &at)) o += d.terms(kind)[at];
         else o += "?" + std::to_string(id);
       }
       o += '\n';
@@ -850,7 +884,7 @@ std::string decode_rows(const Dict& d, const std::vector<const uint32_t*>& cols,
 void write_vdd(const Dict& d, const char* path) {
   std::ofstream out(path);
   if (!out) fail(VG_ERR_INVALID, std::string("cannot write ") + path);
-  auto section = [&](const std::vector<std::string>& v, uint32_t base) {
+  auto section = [&](const TermTexts& v, uint32_t base) {
     out << v.size() << "\n";
     for (size_t i = 0; i < v.size(); ++i) out << (base + i) << " " << v[i] << "\n";
   };
@@ -864,7 +898,7 @@ void read_vdd(const char* path, Dict& d) {
   std::ifstream in(path);
   if (!in) fail(VG_ERR_INVALID, std::string("cannot open ") + path);
   d = Dict();
-  auto section = [&](std::vector<std::string>& v, uint32_t base) {
+  auto section = [&](TermTexts& v, uint32_t base) {
     std::string line;
     if (!std::getline(in, line)) fail(VG_ERR_INVALID, "truncated .vdd");
     const uint64_t count = std::stoull(line);
@@ -880,13 +914,12 @@ void read_vdd(const char* path, Dict& d) {
     std::sort(e.begin(), e.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
     for (size_t i = 0; i < e.size(); ++i)
       if (e[i].first != base + i) fail(VG_ERR_INVALID, ".vdd ids are not dense");
-    v.resize(e.size());
-    for (size_t i = 0; i < e.size(); ++i) v[i] = std::move(e[i].second);
+    for (size_t i = 0; i < e.size(); ++i) v.push_back(e[i].second);
   };
   section(d.so, 1u);
   section(d.p, 1u);
   section(d.l, kLiteralStartId);
-  d.literal_dict = !d.l.empty();
+  d.literal_dict = d.l.size() > 0;
 }
 
 }  // namespace vg
