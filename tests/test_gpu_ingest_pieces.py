@@ -106,3 +106,25 @@ def test_malformed_lines_are_numbered(ctx, bad):
     with pytest.raises(vg.VgError, match="line 2501") as e:
         vg.ingest_ntriples(ctx, "\n".join(lines).encode())
     assert e.value.status == 6
+
+
+def test_dictionary_texts_in_chunks(ctx):
+    """Dictionary texts of more than 64 MiB come to the host in several copies
+    (a term longer than that in one of its own)."""
+    import vedas_gb300 as vg
+
+    long = "k" * (70 << 20)
+    lines = [f"<s{i}> <p> <{'v' * 900}{i}> ." for i in range(40_000)] + [f"<{long}> <p> \"{long}\" .", "<z> <p> <s1> ."]
+    text = "\n".join(lines).encode()
+    ing = vg.ingest_ntriples(ctx, text, literal_dict=True)
+    n = 40_000
+    assert ing.dict.size("so") == 2 * n + 2 and ing.dict.size("l") == 1
+    for i in (0, 1, n // 2, n - 1):
+        assert ing.dict.term("so", 2 * i + 1) == f"<s{i}>"
+        assert ing.dict.term("so", 2 * i + 2) == f"<{'v' * 900}{i}>"
+    assert ing.dict.term("so", 2 * n + 1) == f"<{long}>" and ing.dict.term("so", 2 * n + 2) == "<z>"
+    assert ing.dict.term("l", 50_000_000) == f'"{long}"' and ing.dict.term("p", 1) == "<p>"
+    s, p, o = ing.columns()
+    assert np.array_equal(s, np.append(np.arange(n) * 2 + 1, [2 * n + 1, 2 * n + 2]))
+    assert np.array_equal(o, np.append(np.arange(n) * 2 + 2, [50_000_000, 3])) and (p == 1).all()
+    ing.free()

@@ -9,8 +9,8 @@
 //    occurs on;
 // 3. a scan over the lines counts statements and, per dictionary, the terms
 //    that occur first on each line: their ids, in order of first appearance;
-// 4. ids go to the s, p, o columns, and the place of every id's term to a list
-//    from which the host reads the terms in its own copy of the text.
+// 4. ids go to the s, p, o columns, and the text of every id's term, in id
+//    order, to the host.
 //
 // The table replaced a radix sort of 63-bit hashes per dictionary (31 passes),
 // run heads, a byte-by-byte check and a second sort into id order: 2.5 ms of
@@ -21,6 +21,7 @@
 #include <atomic>
 #include <cstring>
 #include <fstream>
+#include <optional>
 #include <sstream>
 #include <string_view>
 
@@ -485,7 +486,8 @@ __global__ void __launch_bounds__(kBlock, 4) parse_kernel(const uint8_t* __restr
 // 3. ids: per line, whether it holds a statement and which of its terms occur
 // on it first (a subject before an equal object), scanned over the lines.
 struct Counts {
-  uint64_t n[4];   // statements, terms of dictionaries 0, 1, 2
+  uint64_t n[4];                 // statements, terms of dictionaries 0, 1, 2
+  unsigned long long bytes[3];   // those terms' text, a NUL after each
 };
 
 struct LineFirsts {
@@ -511,7 +513,7 @@ __device__ __forceinline__ LineFirsts line_firsts(const uint32_t* __restrict__ s
 
 // base3: the first id of each dictionary.
 __global__ void __launch_bounds__(kBlock) ids_kernel(const uint32_t* __restrict__ slots, Slot* table, uint64_t lines,
-                                                     uint64_t tiles, uint3 base3, uint64_t* status, uint32_t* ticket,
+                                                     uint64_t tiles, uint32_t len_bits, uint3 base3, uint64_t* status, uint32_t* ticket,
                                                      uint64_t* __restrict__ tile_first, Counts* counts,
                                                      DeviceErrors* err) {
   __shared__ uint32_t s_scan[kBlock / 32 + 1];
@@ -546,16 +548,31 @@ __global__ void __launch_bounds__(kBlock) ids_kernel(const uint32_t* __restrict_
     if (tile == tiles - 1)
       for (int q = 0; q < 4; ++q) counts->n[q] = s_b[q] + tot[q];
   }
+  const uint64_t len_mask = (1ull << len_bits) - 1;
+  uint64_t bytes[3] = {0, 0, 0};
+  auto text_of = [&](uint32_t slot) { return (table[slot].loc >> 2 & len_mask) + 1; };
   uint32_t id[3] = {base3.x + static_cast<uint32_t>(s_b[1] + e[1]), base3.y + static_cast<uint32_t>(s_b[2] + e[2]),
                     base3.z + static_cast<uint32_t>(s_b[3] + e[3])};
 #pragma unroll
   for (int i = 0; i < kRows; ++i) {
-    if (f[i].s) table[sl[i][0]].id = id[0]++;
-    if (f[i].o) {
-      if (f[i].o_dict == 0) table[sl[i][2]].id = id[0]++;
-      else table[sl[i][2]].id = id[2]++;
+    if (f[i].s) {
+      table[sl[i][0]].id = id[0]++;
+      bytes[0] += text_of(sl[i][0]);
     }
-    if (f[i].p) table[sl[i][1]].id = id[1]++;
+    if (f[i].o) {
+      const int k = f[i].o_dict == 0 ? 0 : 2;
+      table[sl[i][2]].id = k == 0 ? id[0]++ : id[2]++;
+      (k == 0 ? bytes[0] : bytes[2]) += text_of(sl[i][2]);
+    }
+    if (f[i].p) {
+      table[sl[i][1]].id = id[1]++;
+      bytes[1] += text_of(sl[i][1]);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const uint64_t b = warp_sum64(bytes[k]);
+    if (lane_id() == 0 && b) atomicAdd(&counts->bytes[k], static_cast<unsigned long long>(b));
   }
 }
 
@@ -594,6 +611,51 @@ __global__ void __launch_bounds__(kBlock) columns_kernel(const uint32_t* __restr
   }
 }
 
+// The terms' places in one text of all of them (at[i]; at[terms] its length):
+// a scan of their lengths, a NUL after each.
+__global__ void __launch_bounds__(kBlock) term_places_kernel(const uint64_t* __restrict__ loc, uint64_t terms,
+                                                             uint32_t len_bits, uint64_t* __restrict__ at,
+                                                             uint64_t* status, uint32_t* ticket, DeviceErrors* err) {
+  __shared__ uint64_t s_scan[kBlock / 32 + 1];
+  __shared__ uint64_t s_b;
+  __shared__ uint32_t s_tile;
+  if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
+  __syncthreads();
+  const uint64_t r0 = static_cast<uint64_t>(s_tile) * kTileLines + static_cast<uint64_t>(threadIdx.x) * kRows;
+  const uint64_t mask = (1ull << len_bits) - 1;
+  uint64_t v[kRows], sum = 0;
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) {
+    v[i] = r0 + i < terms ? (loc[r0 + i] & mask) + 1 : 0;
+    sum += v[i];
+  }
+  uint64_t tot;
+  const uint64_t e = block_excl_scan64<kBlock>(sum, tot, s_scan);
+  uint64_t run = block_lookback(status, s_tile, tot, err, &s_b) + e;
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) {
+    if (r0 + i <= terms) at[r0 + i] = run;
+    run += v[i];
+  }
+}
+
+// The text of terms [i0, i1), one warp each, to out (term i0 at its start).
+// The host's own copy of the text is larger than its caches: collecting the
+// terms there took 0.8 ms for 22,000 of them.
+__global__ void __launch_bounds__(kBlock) term_texts_kernel(const uint8_t* __restrict__ text,
+                                                            const uint64_t* __restrict__ loc,
+                                                            const uint64_t* __restrict__ at, uint64_t i0, uint64_t i1,
+                                                            uint32_t len_bits, uint8_t* __restrict__ out) {
+  const uint64_t nw = static_cast<uint64_t>(gridDim.x) * (kBlock / 32);
+  const uint64_t start = at[i0];
+  for (uint64_t i = i0 + static_cast<uint64_t>(blockIdx.x) * (kBlock / 32) + (threadIdx.x >> 5); i < i1; i += nw) {
+    const uint64_t l = loc[i], len = l & ((1ull << len_bits) - 1);
+    const uint8_t* src = text + (l >> len_bits);
+    uint8_t* dst = out + (at[i] - start);
+    for (uint64_t k = lane_id(); k <= len; k += 32) dst[k] = k < len ? src[k] : 0;
+  }
+}
+
 unsigned grid(const Ctx& ctx, uint64_t units) {
   uint64_t g = div_up(units, static_cast<uint64_t>(kBlock));
   const uint64_t gmax = static_cast<uint64_t>(ctx.num_sms) * 16;
@@ -629,6 +691,121 @@ bool parse(Ctx& ctx, const uint8_t* dtext, uint64_t len, uint64_t lines, const T
 void check_ids(const uint64_t (&terms)[3], const uint32_t (&base)[3]) {
   for (int k = 0; k < 3; ++k)
     if (base[k] + terms[k] > 0xFFFFFFFFull) fail(VG_ERR_OVERFLOW, "dictionary ids exceed 32 bits");
+}
+
+// Steps 2 to 4: out.n and the columns, the counts, and the terms' places in id
+// order (none without statements); false when the table gave up.
+bool ids_and_columns(Ctx& ctx, const uint8_t* dtext, uint64_t len, uint64_t lines, uint32_t len_bits,
+                     bool literal_dict, Ingested& out, Counts& h, std::optional<Scratch<uint64_t>>& loc) {
+  Table tb{};
+  tb.len_bits = len_bits;
+  tb.cap = std::min<uint64_t>(4 * lines + 64, 0xFFFFFFFFull);
+  tb.hash_bits = g_hash_bits.load();
+  Scratch<Slot> table(ctx, tb.cap);
+  tb.slots = table.get();
+  VG_CUDA(cudaMemsetAsync(tb.slots, 0, tb.cap * sizeof(Slot), ctx.stream));
+  Scratch<uint32_t> slots(ctx, 3 * lines);
+  if (!parse(ctx, dtext, len, lines, tb, slots.get(), Spans{}, literal_dict)) return false;
+  // 3. ids
+  const uint32_t base[3] = {1u, 1u, kLiteralStartId};
+  const uint3 base3 = make_uint3(base[0], base[1], base[2]);
+  const uint64_t tiles = div_up(lines, kTileLines);
+  const size_t words = 4 * tiles + sizeof(Counts) / 8 + 1;   // look-back words, counts, ticket
+  Scratch<uint64_t> z(ctx, words), first(ctx, tiles);
+  VG_CUDA(cudaMemsetAsync(z.get(), 0, words * sizeof(uint64_t), ctx.stream));
+  auto* counts = reinterpret_cast<Counts*>(z.get() + 4 * tiles);
+  ctx.launch("ingest_ids", 12.0 * lines, [&] {
+    ids_kernel<<<static_cast<unsigned>(tiles), kBlock, 0, ctx.stream>>>(
+        slots.get(), tb.slots, lines, tiles, len_bits, base3, z.get(), reinterpret_cast<uint32_t*>(counts + 1),
+        first.get(), counts, ctx.d_err);
+  });
+  VG_CUDA(cudaGetLastError());
+  VG_CUDA(cudaMemcpyAsync(ctx.h_small, counts, sizeof(Counts), cudaMemcpyDeviceToHost, ctx.stream));
+  ctx.sync();
+  std::memcpy(&h, ctx.h_small, sizeof(h));
+  ctx.check_device_errors();
+  if (h.n[0] > 0x7FFFFFFFull) fail(VG_ERR_OVERFLOW, "ingest is limited to 2^31 triples");
+  const uint64_t nterms[3] = {h.n[1], h.n[2], h.n[3]};
+  check_ids(nterms, base);
+  // 4. columns
+  out.n = h.n[0];
+  out.s = ctx.alloc<uint32_t>(out.n);
+  out.p = ctx.alloc<uint32_t>(out.n);
+  out.o = ctx.alloc<uint32_t>(out.n);
+  if (out.n == 0) return true;
+  loc.emplace(ctx, nterms[0] + nterms[1] + nterms[2]);
+  uint64_t* l = loc->get();
+  const TermList tl{{l, l + nterms[0], l + nterms[0] + nterms[1]}};
+  ctx.launch("ingest_scatter", 24.0 * lines, [&] {
+    columns_kernel<<<static_cast<unsigned>(tiles), kBlock, 0, ctx.stream>>>(slots.get(), tb.slots, lines, base3,
+                                                                           first.get(), out.s, out.p, out.o, tl);
+  });
+  VG_CUDA(cudaGetLastError());
+  return true;
+}
+
+// The dictionaries' terms: places by a scan, texts collected on the device
+// (at most kTextChunk bytes at a time, or one term) and copied to the host.
+void term_texts(Ctx& ctx, const uint8_t* dtext, uint32_t len_bits, const uint64_t* loc, const Counts& h, Dict& dict) {
+  constexpr uint64_t kTextChunk = 64ull << 20;
+  const uint64_t all = h.n[1] + h.n[2] + h.n[3], bytes = h.bytes[0] + h.bytes[1] + h.bytes[2];
+  const uint64_t tiles = div_up(all + 1, kTileLines);
+  Scratch<uint64_t> at(ctx, all + 1), z(ctx, tiles + 1);   // z: look-back words, ticket
+  VG_CUDA(cudaMemsetAsync(z.get(), 0, (tiles + 1) * sizeof(uint64_t), ctx.stream));
+  ctx.launch("ingest_terms", 16.0 * all, [&] {
+    term_places_kernel<<<static_cast<unsigned>(tiles), kBlock, 0, ctx.stream>>>(
+        loc, all, len_bits, at.get(), z.get(), reinterpret_cast<uint32_t*>(z.get() + tiles), ctx.d_err);
+  });
+  VG_CUDA(cudaGetLastError());
+  auto collect = [&](uint64_t i0, uint64_t i1, uint8_t* out) {
+    ctx.launch("ingest_terms", static_cast<double>(bytes), [&] {
+      term_texts_kernel<<<grid(ctx, 32 * (i1 - i0)), kBlock, 0, ctx.stream>>>(dtext, loc, at.get(), i0, i1, len_bits,
+                                                                             out);
+    });
+    VG_CUDA(cudaGetLastError());
+  };
+  TermTexts* terms[3] = {&dict.so, &dict.p, &dict.l};
+  char* text[3];
+  uint64_t *host_at[3], first = 0;
+  for (int k = 0; k < 3; ++k) {
+    text[k] = terms[k]->fill(h.n[1 + k], h.bytes[k], &host_at[k]);
+    // the next dictionary's first place comes along as this one's end
+    VG_CUDA(cudaMemcpyAsync(host_at[k], at.get() + first, (h.n[1 + k] + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost,
+                            ctx.stream));
+    first += h.n[1 + k];
+  }
+  if (bytes <= kTextChunk) {
+    Scratch<uint8_t> buf(ctx, bytes);
+    if (all) collect(0, all, buf.get());
+    uint64_t off = 0;
+    for (int k = 0; k < 3; ++k) {
+      if (h.bytes[k])
+        VG_CUDA(cudaMemcpyAsync(text[k], buf.get() + off, h.bytes[k], cudaMemcpyDeviceToHost, ctx.stream));
+      off += h.bytes[k];
+    }
+    ctx.sync();
+  } else {
+    ctx.sync();
+    first = 0;
+    for (int k = 0; k < 3; ++k) {
+      const uint64_t n = h.n[1 + k], *a = host_at[k];
+      for (uint64_t i = 0; i < n;) {
+        uint64_t e = i + 1;   // the first term past the chunk
+        e = std::max<uint64_t>(e, std::upper_bound(a + i, a + n + 1, a[i] + kTextChunk) - a - 1);
+        Scratch<uint8_t> buf(ctx, a[e] - a[i]);
+        collect(first + i, first + e, buf.get());
+        VG_CUDA(cudaMemcpyAsync(text[k] + (a[i] - a[0]), buf.get(), a[e] - a[i], cudaMemcpyDeviceToHost, ctx.stream));
+        ctx.sync();
+        i = e;
+      }
+      first += n;
+    }
+  }
+  for (int k = 0; k < 3; ++k) {
+    const uint64_t a0 = host_at[k][0];
+    for (uint64_t i = 0; i <= h.n[1 + k]; ++i) host_at[k][i] -= a0;
+  }
+  ctx.check_device_errors();
 }
 
 // First-appearance ids on the host, for texts that the table cannot take (a
@@ -699,25 +876,12 @@ void TermTexts::push_back(std::string_view v) {
   at_.push_back(need);
 }
 
-void TermTexts::assign(const char* text, size_t count,
-                       const std::function<std::pair<uint64_t, uint64_t>(size_t)>& span) {
-  at_.resize(count + 1);
-  uint64_t end = 0;
-  for (size_t i = 0; i < count; ++i) {
-    at_[i] = end;
-    end += span(i).second + 1;
-  }
-  at_[count] = end;
-  text_.reset(new char[end ? end : 1]);
-  cap_ = end;
-  constexpr size_t kTerms = 1024;   // terms per item of the parallel loop
-  parallel_for((count + kTerms - 1) / kTerms, [&](size_t b) {
-    for (size_t i = b * kTerms; i < std::min(count, (b + 1) * kTerms); ++i) {
-      const auto s = span(i);
-      std::memcpy(text_.get() + at_[i], text + s.first, s.second);
-      text_[at_[i + 1] - 1] = 0;
-    }
-  });
+char* TermTexts::fill(size_t count, size_t bytes, uint64_t** at) {
+  text_.reset(new char[bytes ? bytes : 1]);
+  cap_ = bytes;
+  at_.assign(count + 1, 0);
+  *at = at_.data();
+  return text_.get();
 }
 
 bool Dict::has(int kind, uint32_t id, size_t* at) const {
@@ -763,67 +927,13 @@ void ingest_ntriples(Ctx& ctx, const char* text, uint64_t len, bool literal_dict
   // every three of them (2^32 slots at most).
   bool done = false;
   if (lines < 0xFFFFFFFFull) {
-    Table tb{};
     int off_bits = 1;
     while (len >> off_bits) ++off_bits;
-    tb.len_bits = static_cast<uint32_t>(62 - off_bits < off_bits ? 62 - off_bits : off_bits);
-    tb.cap = std::min<uint64_t>(4 * lines + 64, 0xFFFFFFFFull);
-    tb.hash_bits = g_hash_bits.load();
-    Scratch<Slot> table(ctx, tb.cap);
-    tb.slots = table.get();
-    VG_CUDA(cudaMemsetAsync(tb.slots, 0, tb.cap * sizeof(Slot), ctx.stream));
-    Scratch<uint32_t> slots(ctx, 3 * lines);
-    if (parse(ctx, dtext.get(), len, lines, tb, slots.get(), Spans{}, literal_dict)) {
-      // 3. ids
-      const uint32_t base[3] = {1u, 1u, kLiteralStartId};
-      const uint3 base3 = make_uint3(base[0], base[1], base[2]);
-      const uint64_t tiles = div_up(lines, kTileLines);
-      const size_t words = 4 * tiles + 5;   // look-back words, counts, ticket
-      Scratch<uint64_t> z(ctx, words), first(ctx, tiles);
-      VG_CUDA(cudaMemsetAsync(z.get(), 0, words * sizeof(uint64_t), ctx.stream));
-      auto* counts = reinterpret_cast<Counts*>(z.get() + 4 * tiles);
-      ctx.launch("ingest_ids", 12.0 * lines, [&] {
-        ids_kernel<<<static_cast<unsigned>(tiles), kBlock, 0, ctx.stream>>>(
-            slots.get(), tb.slots, lines, tiles, base3, z.get(), reinterpret_cast<uint32_t*>(counts + 1),
-            first.get(), counts, ctx.d_err);
-      });
-      VG_CUDA(cudaGetLastError());
-      VG_CUDA(cudaMemcpyAsync(ctx.h_small, counts, sizeof(Counts), cudaMemcpyDeviceToHost, ctx.stream));
-      ctx.sync();
-      Counts h;
-      std::memcpy(&h, ctx.h_small, sizeof(h));
-      ctx.check_device_errors();
-      if (h.n[0] > 0x7FFFFFFFull) fail(VG_ERR_OVERFLOW, "ingest is limited to 2^31 triples");
-      const uint64_t nterms[3] = {h.n[1], h.n[2], h.n[3]};
-      check_ids(nterms, base);
-      // 4. columns and terms
-      out.n = h.n[0];
-      out.s = ctx.alloc<uint32_t>(out.n);
-      out.p = ctx.alloc<uint32_t>(out.n);
-      out.o = ctx.alloc<uint32_t>(out.n);
-      if (out.n) {
-        const uint64_t all = nterms[0] + nterms[1] + nterms[2];
-        Scratch<uint64_t> dloc(ctx, all);
-        const TermList tl{{dloc.get(), dloc.get() + nterms[0], dloc.get() + nterms[0] + nterms[1]}};
-        ctx.launch("ingest_scatter", 24.0 * lines, [&] {
-          columns_kernel<<<static_cast<unsigned>(tiles), kBlock, 0, ctx.stream>>>(
-              slots.get(), tb.slots, lines, base3, first.get(), out.s, out.p, out.o, tl);
-        });
-        VG_CUDA(cudaGetLastError());
-        std::vector<uint64_t> loc(all);
-        VG_CUDA(cudaMemcpyAsync(loc.data(), dloc.get(), all * sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx.stream));
-        ctx.sync();
-        TermTexts* terms[3] = {&out.dict.so, &out.dict.p, &out.dict.l};
-        const uint64_t* at = loc.data();
-        for (int k = 0; k < 3; ++k) {
-          terms[k]->assign(text, nterms[k], [&](size_t r) {
-            return std::make_pair(at[r] >> tb.len_bits, at[r] & ((1ull << tb.len_bits) - 1));
-          });
-          at += nterms[k];
-        }
-      }
-      done = true;
-    }
+    const uint32_t len_bits = static_cast<uint32_t>(62 - off_bits < off_bits ? 62 - off_bits : off_bits);
+    std::optional<Scratch<uint64_t>> loc;   // the terms' places in the text, in id order
+    Counts h{};
+    done = ids_and_columns(ctx, dtext.get(), len, lines, len_bits, literal_dict, out, h, loc);
+    if (done && loc) term_texts(ctx, dtext.get(), len_bits, loc->get(), h, out.dict);
   }
   if (!done) {
     ++out.collisions;

@@ -3,12 +3,10 @@
 // src/loader.cu:19-93).
 #pragma once
 
-#include <functional>
 #include <memory>
 #include <string>
 #include <string_view>
 #include <unordered_map>
-#include <utility>
 #include <vector>
 
 #include "compat/vedas_compat.h"
@@ -30,9 +28,10 @@ class TermTexts {
   const char* c_str(size_t i) const { return text_.get() + at_[i]; }
   std::string_view operator[](size_t i) const { return {c_str(i), at_[i + 1] - at_[i] - 1}; }
   void push_back(std::string_view v);   // moves what c_str returned before
-  // `count` terms: term i is the part of `text` that span(i) = (offset,
-  // length) gives.
-  void assign(const char* text, size_t count, const std::function<std::pair<uint64_t, uint64_t>(size_t)>& span);
+  // Room for `count` terms of `bytes` bytes in all (their NULs included);
+  // returns where the text goes and sets *at to the count + 1 places of the
+  // terms in it, both to be filled by the caller.
+  char* fill(size_t count, size_t bytes, uint64_t** at);
 
  private:
   std::unique_ptr<char[]> text_;
