@@ -821,21 +821,9 @@ IR* JoinQueryJob::join(FullRelationIR* lir, FullRelationIR* rir) {
   if (w.sortL) w.lir->sortByFirstColumn();
   if (w.sortR) w.rir->sortByFirstColumn();
   vg::Rel joined;
-  vg::join(*ex->ctx, w.lir->rel(), w.rir->rel(), false, joined);
-  TYPEID fl[2] = {0, 0};
-  std::vector<TYPEID> c0;
-  if (joined.nrows > 0) {
-    VG_CUDA(cudaMemcpyAsync(&fl[0], joined.cols[0], 4, cudaMemcpyDeviceToHost, ex->ctx->stream));
-    VG_CUDA(cudaMemcpyAsync(&fl[1], joined.cols[0] + joined.nrows - 1, 4, cudaMemcpyDeviceToHost,
-                            ex->ctx->stream));
-    if (joined.nrows > 2 && joined.nrows < 100) {
-      c0.resize(joined.nrows);
-      VG_CUDA(cudaMemcpyAsync(c0.data(), joined.cols[0], joined.nrows * 4, cudaMemcpyDeviceToHost,
-                              ex->ctx->stream));
-    }
-    ex->ctx->sync();
-  }
-  finish(w, joined, fl[0], fl[1], &c0);
+  vg::JoinEnds ends;
+  vg::join(*ex->ctx, w.lir->rel(), w.rir->rel(), false, joined, &ends);
+  finish(w, joined, ends.first, ends.last, &ends.c0);
   return intermediateResult;
 }
 

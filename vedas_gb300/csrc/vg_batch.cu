@@ -341,80 +341,14 @@ __global__ void __launch_bounds__(kJcBlock, 4) bjoin_count_scan_kernel(
   const uint64_t i0 = (tile - bstart[j]) * static_cast<uint64_t>(kJcTile);
   uint32_t cnt[kJcKeys], lov[kJcKeys];
   jc_count_staged(g.lk, g.nl, g.rk, i0, lov, cnt, sm, err);
-  uint64_t sum = 0;
-#pragma unroll
-  for (int k = 0; k < kJcKeys; ++k) sum += cnt[k];
-  uint64_t tot;
-  const uint64_t e = block_excl_scan64<kJcBlock>(sum, tot, s_scan);   // every thread is past its search
-  const uint32_t tid = threadIdx.x;
-  const uint64_t first = i0 + static_cast<uint64_t>(tid) * kJcKeys;
-  const uint32_t tile_n = static_cast<uint32_t>(g.nl - i0 < kJcTile ? g.nl - i0 : kJcTile);
-  // a bulk copy that gave up may still land in the window: no staging there
-  const bool stage = !(sm.staged == 2 && sm.failed);
-  if (stage) {
-    // lower bounds and tile-relative offsets staged in the window while warp 0
-    // looks back; the tile's prefix is added when they are stored
-    uint32_t* s_lo = jc_stage_lo(sm);
-    uint64_t* s_off = jc_stage_off(sm);
-    uint64_t run = e;
-#pragma unroll
-    for (int k = 0; k < kJcKeys; ++k) {
-      const uint32_t q = tid * kJcKeys + k;
-      s_lo[q + q / 32] = lov[k];
-      s_off[q + q / 16] = run;
-      run += cnt[k];
-    }
-  }
-  if (threadIdx.x < 32) {
-    const uint64_t p = warp_lookback_seg(status, tile, bstart[j], tot, err);
-    if (threadIdx.x == 0) s_b = p;
-  }
-  __syncthreads();
-  const uint64_t base = s_b;
-  if (tile == bstart[j + 1] - 1 && tid == 0) totals[j] = base + tot;
-  if (!stage) {
-    uint64_t run = base + e;
-#pragma unroll
-    for (int k = 0; k < kJcKeys; ++k) {
-      if (first + k < g.nl) {
-        offs[g.row0 + first + k] = run;
-        lo[g.row0 + first + k] = lov[k];
-      }
-      run += cnt[k];
-    }
-    if (tid == 0) jc_drain_window(sm, err);
-    return;
-  }
-  const uint32_t* s_lo = jc_stage_lo(sm);
-  const uint64_t* s_off = jc_stage_off(sm);
-  uint32_t* lo_t = lo + g.row0 + i0;
-  uint64_t* off_t = offs + g.row0 + i0;
-  for (uint32_t q = tid; q < tile_n; q += kJcBlock) {
-    lo_t[q] = s_lo[q + q / 32];
-    off_t[q] = base + s_off[q + q / 16];
-  }
+  jc_finish_tile(g.nl, i0, lov, cnt, sm, s_scan, &s_b, tile, bstart[j], tile == bstart[j + 1] - 1, lo + g.row0,
+                 offs + g.row0, status, &totals[j], err);
 }
-
-struct JoinOut {
-  const uint64_t* offs;
-  const uint32_t* lo;
-  uint64_t nl, total;
-  const uint32_t* lc[VG_MAX_COLS];
-  const uint32_t* rc[VG_MAX_COLS];
-  uint32_t* oc[VG_MAX_COLS];
-  uint32_t nlc, nrc;
-};
 
 // Output rows [kb, kb + kTileRows) of one join per tile (the tile's join
 // from a per-tile table).  Blocks loop over tiles [blockIdx.x, T) with
 // stride gridDim.x; T is read from the device when ostart_end is given (a
-// device-side placement wrote it there).  Output row k comes from the left
-// row i with offs[i] <= k < offs[i + 1] and the right row lo[i] + (k -
-// offs[i]).  Two warps find the tile's left-row range at once; when it holds
-// at most kTileRows + 1 rows, its offsets and lower bounds are staged in
-// shared memory, and each thread walks its rows (k increasing, consecutive
-// threads on consecutive rows, so loads and stores coalesce) from the
-// previous one's left row.  Hub keys thus spread over many blocks.
+// device-side placement wrote it there), each written by jw_write_tile.
 //
 // Small outputs (at most Ctx::tune.write_small_rows rows of a join with at most kSmallJoin
 // left rows; most outputs of a wave) are written one join per warp first,
@@ -512,87 +446,7 @@ __global__ void __launch_bounds__(kBlock, 5) bjoin_write_kernel(const JoinOut* _
     __syncthreads();
     const uint64_t kb = (tile - tile0) * static_cast<uint64_t>(kTileRows);
     const uint64_t kend = (kb + kTileRows < s_o.total) ? kb + kTileRows : s_o.total;
-    const uint64_t ib = rg.x, ie = rg.y;
-    const uint64_t m = ie - ib;
-    const bool staged = m <= static_cast<uint64_t>(kStage);
-    if (staged)
-      for (uint32_t e = threadIdx.x; e < m; e += kBlock) {
-        s_off[e] = s_o.offs[ib + e];
-        s_lo[e] = s_o.lo[ib + e];
-      }
-    __syncthreads();
-    // 1. the left and right row of each of the thread's output rows
-    uint32_t li[kRows], ri[kRows];
-    if (staged) {
-      uint32_t p = 0;   // the current left row, relative to ib
-#pragma unroll
-      for (int it = 0; it < kRows; ++it) {
-        const uint64_t k = kb + static_cast<uint64_t>(it) * kBlock + threadIdx.x;
-        li[it] = ri[it] = 0;
-        if (k < kend) {
-          // last p with s_off[p] <= k, moving forward from the previous row's p
-          uint32_t step = 1;
-          while (p + step < m && s_off[p + step] <= k) {
-            p += step;
-            step <<= 1;
-          }
-          while (step > 1) {
-            step >>= 1;
-            if (p + step < m && s_off[p + step] <= k) p += step;
-          }
-          li[it] = static_cast<uint32_t>(ib + p);
-          ri[it] = static_cast<uint32_t>(s_lo[p] + (k - s_off[p]));
-        }
-      }
-    } else {
-      // a sparse tile (more than kStage left rows, most without matches): the
-      // left rows of kGroup of the thread's output rows at a time come from
-      // kGroup binary searches of the offsets advanced in lockstep, so each
-      // round has kGroup independent loads in flight
-      constexpr int kGroup = 4;
-#pragma unroll
-      for (int g0 = 0; g0 < kRows; g0 += kGroup) {
-        uint64_t lq[kGroup], kk[kGroup];
-#pragma unroll
-        for (int q = 0; q < kGroup; ++q) {
-          const uint64_t k = kb + static_cast<uint64_t>(g0 + q) * kBlock + threadIdx.x;
-          kk[q] = k < kend ? k : kend - 1;
-          lq[q] = ib;
-        }
-        uint64_t n = ie - ib;                     // last i in [ib, ie) with offs[i] <= k
-        while (n > 1) {
-          const uint64_t half = n >> 1;
-#pragma unroll
-          for (int q = 0; q < kGroup; ++q) lq[q] = (s_o.offs[lq[q] + half] <= kk[q]) ? lq[q] + half : lq[q];
-          n -= half;
-        }
-#pragma unroll
-        for (int q = 0; q < kGroup; ++q) {
-          li[g0 + q] = static_cast<uint32_t>(lq[q]);
-          ri[g0 + q] = static_cast<uint32_t>(s_o.lo[lq[q]] + (kk[q] - s_o.offs[lq[q]]));
-        }
-      }
-    }
-    // 2. column by column: each thread's kRows loads of a column are in
-    // flight together (read-only path), each store instruction writes
-    // consecutive rows, and one column's pointers are live at a time
-    const uint32_t nlc = s_o.nlc, ncols = s_o.nlc + s_o.nrc;
-    for (uint32_t c = 0; c < ncols; ++c) {
-      const bool left = c < nlc;
-      const uint32_t* src = left ? s_o.lc[c] : s_o.rc[c - nlc];
-      uint32_t* dst = s_o.oc[c];
-      uint32_t v[kRows];
-#pragma unroll
-      for (int it = 0; it < kRows; ++it) {
-        const uint64_t k = kb + static_cast<uint64_t>(it) * kBlock + threadIdx.x;
-        if (k < kend) v[it] = __ldg(src + (left ? li[it] : ri[it]));
-      }
-#pragma unroll
-      for (int it = 0; it < kRows; ++it) {
-        const uint64_t k = kb + static_cast<uint64_t>(it) * kBlock + threadIdx.x;
-        if (k < kend) dst[k] = v[it];
-      }
-    }
+    jw_write_tile<kRows>(s_o, kb, kend, rg.x, rg.y, s_off, s_lo);
   }
 }
 

@@ -312,13 +312,13 @@ vg_status vg_join(vg_ctx* ctx, const vg_ir* l, const vg_ir* r, vg_ir* out, uint3
     check_ir(l);
     check_ir(r);
     vg::Rel o;
-    vg::join(ctx->c, to_rel(l), to_rel(r), false, o);
+    vg::JoinEnds ends;
+    vg::join(ctx->c, to_rel(l), to_rel(r), false, o, &ends);
     from_rel(o, out);
     if (first_last && o.nrows > 0) {
-      VG_CUDA(cudaMemcpyAsync(&first_last[0], o.cols[0], 4, cudaMemcpyDeviceToHost, ctx->c.stream));
-      VG_CUDA(cudaMemcpyAsync(&first_last[1], o.cols[0] + o.nrows - 1, 4, cudaMemcpyDeviceToHost, ctx->c.stream));
+      first_last[0] = ends.first;
+      first_last[1] = ends.last;
     }
-    ctx->c.check_device_errors();
   });
 }
 
@@ -330,7 +330,6 @@ vg_status vg_join2(vg_ctx* ctx, const vg_ir* l, const vg_ir* r, vg_ir* out) {
     vg::Rel o;
     vg::join(ctx->c, to_rel(l), to_rel(r), true, o);
     from_rel(o, out);
-    ctx->c.check_device_errors();
   });
 }
 

@@ -22,15 +22,15 @@ struct JoinCountSmem {
 // Searches over the staged window, in 32-bit offsets from its first key
 // (s points at it in shared memory, n keys).  kUpper: first offset whose key
 // is above `key`; otherwise first offset whose key is not below it.
-template <bool kUpper>
-__device__ __forceinline__ bool smem_below(const uint32_t* s, uint32_t i, uint32_t key) {
-  const uint32_t a = s[i];
+template <bool kUpper, typename T>
+__device__ __forceinline__ bool smem_below(const T* s, uint32_t i, T key) {
+  const T a = s[i];
   return kUpper ? (a <= key) : (a < key);
 }
 
 // Binary search over [lo, n).
-template <bool kUpper>
-__device__ __forceinline__ uint32_t smem_search(const uint32_t* s, uint32_t lo, uint32_t n, uint32_t key) {
+template <bool kUpper, typename T>
+__device__ __forceinline__ uint32_t smem_search(const T* s, uint32_t lo, uint32_t n, T key) {
   uint32_t len = n - lo;
   while (len > 0) {
     const uint32_t half = len >> 1;
@@ -47,8 +47,8 @@ __device__ __forceinline__ uint32_t smem_search(const uint32_t* s, uint32_t lo, 
 // The same answer at or after `from`, galloping from there (steps 1, 2, 4,
 // ... then a binary search inside the last step): a thread's left keys are
 // consecutive, so the next bound is usually a few keys further on.
-template <bool kUpper>
-__device__ __forceinline__ uint32_t smem_gallop(const uint32_t* s, uint32_t from, uint32_t n, uint32_t key) {
+template <bool kUpper, typename T>
+__device__ __forceinline__ uint32_t smem_gallop(const T* s, uint32_t from, uint32_t n, T key) {
   if (from >= n || !smem_below<kUpper>(s, from, key)) return from;
   uint32_t lo = from, step = 1, hi = n;
   while (true) {
@@ -64,6 +64,22 @@ __device__ __forceinline__ uint32_t smem_gallop(const uint32_t* s, uint32_t from
   // below(lo) holds and the answer lies in (lo, hi]
   return smem_search<kUpper>(s, lo + 1, hi, key);
 }
+
+// The keys of a relation sorted by its first column, or (PairKeys) by its
+// first two, as 64-bit (column 0, column 1) words.
+struct OneKeys {
+  using T = uint32_t;
+  const uint32_t* c0;
+  __device__ __forceinline__ T operator()(uint64_t i) const { return __ldg(c0 + i); }
+};
+struct PairKeys {
+  using T = uint64_t;
+  const uint32_t* c0;
+  const uint32_t* c1;
+  __device__ __forceinline__ T operator()(uint64_t i) const {
+    return (static_cast<uint64_t>(__ldg(c0 + i)) << 32) | __ldg(c1 + i);
+  }
+};
 
 // First index in R[lo, hi) whose key is not below `key` (kUpper: above it),
 // found by one warp: each round 31 lanes probe evenly spaced keys and the
@@ -101,9 +117,9 @@ __device__ __forceinline__ uint64_t warp_bound(const T* __restrict__ R, uint64_t
 // keys of its range and the ballot of its comparisons narrows the range
 // 16-fold.  Every lane of the warp must call it with the same arguments;
 // every lane gets both bounds.
-template <bool kUpperA, bool kUpperB, typename T>
-__device__ __forceinline__ void warp_bound_pair(const T* __restrict__ R, uint64_t n, T ka, T kb, uint64_t& ra,
-                                                uint64_t& rb) {
+template <bool kUpperA, bool kUpperB, typename Keys, typename T>
+__device__ __forceinline__ void warp_bound_pair_of(const Keys& keys, uint64_t n, T ka, T kb, uint64_t& ra,
+                                                   uint64_t& rb) {
   const uint32_t lane = threadIdx.x & 31, sl = lane & 15;
   const bool second = lane >= 16;
   const bool upper = second ? kUpperB : kUpperA;
@@ -119,7 +135,7 @@ __device__ __forceinline__ void warp_bound_pair(const T* __restrict__ R, uint64_
       step = (hi - lo + 15) >> 4;
       const uint64_t p = lo + static_cast<uint64_t>(sl + 1) * step;
       if (sl < 15 && p < hi) {
-        const T a = __ldg(R + p);
+        const T a = keys(p);
         below = upper ? (a <= key) : (a < key);
       }
     }
@@ -133,12 +149,18 @@ __device__ __forceinline__ void warp_bound_pair(const T* __restrict__ R, uint64_
   }
   bool below = false;
   if (lo + sl < hi) {
-    const T a = __ldg(R + lo + sl);
+    const T a = keys(lo + sl);
     below = upper ? (a <= key) : (a < key);
   }
   const uint64_t res = lo + __popc(__ballot_sync(0xffffffffu, below) & half);
   ra = __shfl_sync(0xffffffffu, res, 0);
   rb = __shfl_sync(0xffffffffu, res, 16);
+}
+
+template <bool kUpperA, bool kUpperB, typename T>
+__device__ __forceinline__ void warp_bound_pair(const T* __restrict__ R, uint64_t n, T ka, T kb, uint64_t& ra,
+                                                uint64_t& rb) {
+  warp_bound_pair_of<kUpperA, kUpperB>([R](uint64_t i) { return __ldg(R + i); }, n, ka, kb, ra, rb);
 }
 
 // A tile's right-key window: the lower bound of klo and the upper bound of
@@ -148,43 +170,16 @@ __device__ __forceinline__ void warp_window(const uint32_t* __restrict__ R, uint
   warp_bound_pair<false, true, uint32_t>(R, nr, klo, khi, w0, w1);
 }
 
-// Lower and upper bounds of K keys in R[w0, w1) at once: branchless binary
-// searches advanced in lockstep, so each round has 2K independent loads in
-// flight instead of one dependent chain per key.
-template <int K>
-__device__ __forceinline__ void lockstep_bounds(const uint32_t* __restrict__ R, uint64_t w0, uint64_t w1,
-                                                const uint32_t (&key)[K], uint64_t (&lo)[K], uint64_t (&hi)[K]) {
-  if (w1 <= w0) {
-#pragma unroll
-    for (int j = 0; j < K; ++j) lo[j] = hi[j] = w0;
-    return;
-  }
-#pragma unroll
-  for (int j = 0; j < K; ++j) lo[j] = hi[j] = w0;
-  uint64_t n = w1 - w0;
-  while (n > 1) {
-    const uint64_t half = n >> 1;
-#pragma unroll
-    for (int j = 0; j < K; ++j) {
-      const uint32_t a = __ldg(R + lo[j] + half);
-      const uint32_t b = __ldg(R + hi[j] + half);
-      lo[j] = (a < key[j]) ? lo[j] + half : lo[j];
-      hi[j] = (b <= key[j]) ? hi[j] + half : hi[j];
-    }
-    n -= half;
-  }
-#pragma unroll
-  for (int j = 0; j < K; ++j) {
-    lo[j] += (__ldg(R + lo[j]) < key[j]) ? 1 : 0;
-    hi[j] += (__ldg(R + hi[j]) <= key[j]) ? 1 : 0;
-  }
-}
-
-// lockstep_bounds with 32-bit positions (every join side has fewer than 2^32
-// rows), which halves the registers the bounds hold.
-template <int K>
-__device__ __forceinline__ void lockstep_bounds32(const uint32_t* __restrict__ R, uint32_t w0, uint32_t w1,
-                                                  const uint32_t (&key)[K], uint32_t (&lo)[K], uint32_t (&hi)[K]) {
+// Lower and upper bounds of K keys in the right keys [w0, w1) at once:
+// branchless binary searches advanced in lockstep, so each round has 2K
+// independent loads in flight instead of one dependent chain per key.
+// Positions have 32 bits (every join side has fewer than 2^32 rows), which
+// halves the registers the bounds hold.
+template <int K, typename Keys>
+__device__ __forceinline__ void lockstep_bounds_of(const Keys& keys, uint32_t w0, uint32_t w1,
+                                                   const typename Keys::T (&key)[K], uint32_t (&lo)[K],
+                                                   uint32_t (&hi)[K]) {
+  using T = typename Keys::T;
 #pragma unroll
   for (int j = 0; j < K; ++j) lo[j] = hi[j] = w0;
   if (w1 <= w0) return;
@@ -193,8 +188,8 @@ __device__ __forceinline__ void lockstep_bounds32(const uint32_t* __restrict__ R
     const uint32_t half = n >> 1;
 #pragma unroll
     for (int j = 0; j < K; ++j) {
-      const uint32_t a = __ldg(R + lo[j] + half);
-      const uint32_t b = __ldg(R + hi[j] + half);
+      const T a = keys(static_cast<uint64_t>(lo[j]) + half);
+      const T b = keys(static_cast<uint64_t>(hi[j]) + half);
       lo[j] = (a < key[j]) ? lo[j] + half : lo[j];
       hi[j] = (b <= key[j]) ? hi[j] + half : hi[j];
     }
@@ -202,9 +197,15 @@ __device__ __forceinline__ void lockstep_bounds32(const uint32_t* __restrict__ R
   }
 #pragma unroll
   for (int j = 0; j < K; ++j) {
-    lo[j] += (__ldg(R + lo[j]) < key[j]) ? 1 : 0;
-    hi[j] += (__ldg(R + hi[j]) <= key[j]) ? 1 : 0;
+    lo[j] += (keys(lo[j]) < key[j]) ? 1 : 0;
+    hi[j] += (keys(hi[j]) <= key[j]) ? 1 : 0;
   }
+}
+
+template <int K>
+__device__ __forceinline__ void lockstep_bounds32(const uint32_t* __restrict__ R, uint32_t w0, uint32_t w1,
+                                                  const uint32_t (&key)[K], uint32_t (&lo)[K], uint32_t (&hi)[K]) {
+  lockstep_bounds_of<K>(OneKeys{R}, w0, w1, key, lo, hi);
 }
 
 // Thread 0 of the block: records the tile's right-key window [w0, w1) and
@@ -234,6 +235,38 @@ __device__ __forceinline__ void jc_issue_window(const uint32_t* __restrict__ R, 
       sm.staged = 2;
     } else {
       sm.staged = 1;
+    }
+  }
+}
+
+// The thread's keys (of left rows i0 + 8 * thread, up to i_end) in a staged
+// window of n right keys, whose first is right row w0: the first key is
+// searched in full, the others gallop from the previous key's upper bound;
+// equal keys reuse its bounds.
+template <typename T>
+__device__ __forceinline__ void jc_search_staged(const T* win, uint32_t n, uint64_t w0, uint64_t i0, uint64_t i_end,
+                                                 const T (&key)[kJcKeys], uint32_t (&lov)[kJcKeys],
+                                                 uint32_t (&cnt)[kJcKeys]) {
+  const uint64_t first = i0 + static_cast<uint64_t>(threadIdx.x) * kJcKeys;
+  uint32_t plo = 0, phi = 0;
+  T pkey = 0;
+#pragma unroll
+  for (int j = 0; j < kJcKeys; ++j) {
+    if (first + j < i_end) {
+      const T k = key[j];
+      uint32_t lo, hi;
+      if (j > 0 && k == pkey) {
+        lo = plo;
+        hi = phi;
+      } else {
+        lo = (j == 0) ? smem_search<false, T>(win, 0, n, k) : smem_gallop<false, T>(win, phi, n, k);
+        hi = smem_gallop<true, T>(win, lo, n, k);
+      }
+      lov[j] = static_cast<uint32_t>(w0 + lo);
+      cnt[j] = hi - lo;
+      plo = lo;
+      phi = hi;
+      pkey = k;
     }
   }
 }
@@ -305,31 +338,8 @@ __device__ __forceinline__ void jc_count_staged(const uint32_t* __restrict__ L, 
     }
     return;
   }
-  // staged window: the thread's first key is searched in full, the others
-  // gallop from the previous key's upper bound; equal keys reuse its bounds
   const uint32_t* win = sm.keys + (w0 - base);
-  const uint32_t n = static_cast<uint32_t>(w1 - w0);
-  uint32_t plo = 0, phi = 0, pkey = 0;
-#pragma unroll
-  for (int j = 0; j < kJcKeys; ++j) {
-    const uint64_t i = first + j;
-    if (i < i_end) {
-      const uint32_t k = key[j];
-      uint32_t lo, hi;
-      if (j > 0 && k == pkey) {
-        lo = plo;
-        hi = phi;
-      } else {
-        lo = (j == 0) ? smem_search<false>(win, 0, n, k) : smem_gallop<false>(win, phi, n, k);
-        hi = smem_gallop<true>(win, lo, n, k);
-      }
-      lov[j] = static_cast<uint32_t>(w0 + lo);
-      cnt[j] = hi - lo;
-      plo = lo;
-      phi = hi;
-      pkey = k;
-    }
-  }
+  jc_search_staged<uint32_t>(win, static_cast<uint32_t>(w1 - w0), w0, i0, i_end, key, lov, cnt);
 }
 
 // A tile's lower bounds and output offsets, staged in the window's shared
@@ -353,51 +363,218 @@ __device__ __forceinline__ void jc_drain_window(JoinCountSmem& sm, DeviceErrors*
   if (sm.staged == 2 && sm.failed) (void)mbar_wait_bounded(&sm.bar, 0, err);
 }
 
-// The tile's window: lower bound of its first key and upper bound of its
-// last key in R, found by one warp each (every lane of the warp calls it).
-__device__ __forceinline__ uint64_t jc_window_bound(const uint32_t* __restrict__ L, uint64_t nl,
-                                                    const uint32_t* __restrict__ R, uint64_t nr, uint64_t i0,
-                                                    bool upper) {
-  const uint64_t i_end = (i0 + kJcTile < nl) ? i0 + kJcTile : nl;
-  return upper ? warp_bound<true, uint32_t>(R, 0, nr, L[i_end - 1]) : warp_bound<false, uint32_t>(R, 0, nr, L[i0]);
+// Staging of a PairKeys window: as 64-bit words, by the block's threads.
+constexpr uint32_t kJcPairWindow = kJcWindow / 2;
+__device__ __forceinline__ void jc_issue_pair_window(uint64_t w0, uint64_t w1, JoinCountSmem& sm) {
+  sm.w0 = w0;
+  sm.w1 = w1;
+  sm.staged = (w1 > w0 && w1 - w0 <= kJcPairWindow) ? 1 : 0;
+  sm.failed = 0;
 }
 
-// jc_count_staged with the window found by the block itself: two warps
-// search R at once, then thread 0 stages the window.
-__device__ __forceinline__ void join_count_tile_regs(const uint32_t* __restrict__ L, uint64_t nl,
-                                                     const uint32_t* __restrict__ R, uint64_t nr, uint64_t i0,
-                                                     uint32_t* __restrict__ lo_out, uint32_t (&cnt)[kJcKeys],
-                                                     JoinCountSmem& sm, DeviceErrors* err) {
+// jc_count_staged for keys of two columns.
+__device__ __forceinline__ void jc_count_staged_pairs(const PairKeys& L, uint64_t nl, const PairKeys& R, uint64_t i0,
+                                                      uint32_t (&lov)[kJcKeys], uint32_t (&cnt)[kJcKeys],
+                                                      JoinCountSmem& sm) {
+#pragma unroll
+  for (int j = 0; j < kJcKeys; ++j) cnt[j] = lov[j] = 0;
   const uint32_t tid = threadIdx.x;
-  if (tid < 64) {
-    const uint64_t w = jc_window_bound(L, nl, R, nr, i0, tid >= 32);
-    if (tid == 0) sm.w0 = w;
-    if (tid == 32) sm.w1 = w;
+  const uint64_t i_end = (i0 + kJcTile < nl) ? i0 + kJcTile : nl;
+  const uint64_t w0 = sm.w0, w1 = sm.w1 > sm.w0 ? sm.w1 : sm.w0;
+  const uint64_t first = i0 + static_cast<uint64_t>(tid) * kJcKeys;
+  uint64_t key[kJcKeys];
+#pragma unroll
+  for (int j = 0; j < kJcKeys; ++j) {
+    const uint64_t i = first + j;
+    key[j] = L(i < i_end ? i : i_end - 1);
+  }
+  uint64_t* win = reinterpret_cast<uint64_t*>(sm.keys);
+  if (sm.staged)
+    for (uint64_t e = w0 + tid; e < w1; e += kJcBlock) win[e - w0] = R(e);
+  __syncthreads();
+  if (first >= i_end) return;   // counts stay zero
+  if (sm.staged) {
+    jc_search_staged<uint64_t>(win, static_cast<uint32_t>(w1 - w0), w0, i0, i_end, key, lov, cnt);
+    return;
+  }
+  uint32_t lo[kJcKeys], hi[kJcKeys];
+  lockstep_bounds_of<kJcKeys>(R, static_cast<uint32_t>(w0), static_cast<uint32_t>(w1), key, lo, hi);
+#pragma unroll
+  for (int j = 0; j < kJcKeys; ++j)
+    if (first + j < i_end) {
+      lov[j] = lo[j];
+      cnt[j] = hi[j] - lo[j];
+    }
+}
+
+// What follows a tile's count: a block scan and a look-back over the same
+// join's tiles [first_tile, tile) give every left row its output offset; the
+// join's last tile writes its total.  lo and offs are the join's own arrays
+// (left row i0 is the tile's first).  Every thread of the block calls it.
+__device__ __forceinline__ void jc_finish_tile(uint64_t nl, uint64_t i0, const uint32_t (&lov)[kJcKeys],
+                                               const uint32_t (&cnt)[kJcKeys], JoinCountSmem& sm, uint64_t* s_scan,
+                                               uint64_t* s_b, uint64_t tile, uint64_t first_tile, bool last_tile,
+                                               uint32_t* __restrict__ lo, uint64_t* __restrict__ offs,
+                                               uint64_t* status, uint64_t* total, DeviceErrors* err) {
+  uint64_t sum = 0;
+#pragma unroll
+  for (int k = 0; k < kJcKeys; ++k) sum += cnt[k];
+  uint64_t tot;
+  const uint64_t e = block_excl_scan64<kJcBlock>(sum, tot, s_scan);   // every thread is past its search
+  const uint32_t tid = threadIdx.x;
+  const uint64_t first = i0 + static_cast<uint64_t>(tid) * kJcKeys;
+  const uint32_t tile_n = static_cast<uint32_t>(nl - i0 < kJcTile ? nl - i0 : kJcTile);
+  // a bulk copy that gave up may still land in the window: no staging there
+  const bool stage = !(sm.staged == 2 && sm.failed);
+  if (stage) {
+    // lower bounds and tile-relative offsets staged in the window while warp 0
+    // looks back; the tile's prefix is added when they are stored
+    uint32_t* s_lo = jc_stage_lo(sm);
+    uint64_t* s_off = jc_stage_off(sm);
+    uint64_t run = e;
+#pragma unroll
+    for (int k = 0; k < kJcKeys; ++k) {
+      const uint32_t q = tid * kJcKeys + k;
+      s_lo[q + q / 32] = lov[k];
+      s_off[q + q / 16] = run;
+      run += cnt[k];
+    }
+  }
+  if (threadIdx.x < 32) {
+    const uint64_t p = warp_lookback_seg(status, tile, first_tile, tot, err);
+    if (threadIdx.x == 0) *s_b = p;
   }
   __syncthreads();
-  if (tid == 0) jc_issue_window(R, sm.w0, sm.w1, sm);
-  __syncthreads();
-  uint32_t lov[kJcKeys];
-  jc_count_staged(L, nl, R, i0, lov, cnt, sm, err);
-  const uint64_t first = i0 + static_cast<uint64_t>(tid) * kJcKeys;
+  const uint64_t base = *s_b;
+  if (last_tile && tid == 0) *total = base + tot;
+  if (!stage) {
+    uint64_t run = base + e;
 #pragma unroll
-  for (int j = 0; j < kJcKeys; ++j)
-    if (first + j < nl) lo_out[first + j] = lov[j];
+    for (int k = 0; k < kJcKeys; ++k) {
+      if (first + k < nl) {
+        offs[first + k] = run;
+        lo[first + k] = lov[k];
+      }
+      run += cnt[k];
+    }
+    if (tid == 0) jc_drain_window(sm, err);
+    return;
+  }
+  const uint32_t* s_lo = jc_stage_lo(sm);
+  const uint64_t* s_off = jc_stage_off(sm);
+  for (uint32_t q = tid; q < tile_n; q += kJcBlock) {
+    lo[i0 + q] = s_lo[q + q / 32];
+    offs[i0 + q] = base + s_off[q + q / 16];
+  }
 }
 
-// Lower bound and match count of every left key of the tile, to lo_out and
-// cnt_out.
-__device__ __forceinline__ void join_count_tile(const uint32_t* __restrict__ L, uint64_t nl,
-                                                const uint32_t* __restrict__ R, uint64_t nr, uint64_t i0,
-                                                uint32_t* __restrict__ lo_out, uint32_t* __restrict__ cnt_out,
-                                                JoinCountSmem& sm, DeviceErrors* err) {
-  uint32_t cnt[kJcKeys];
-  join_count_tile_regs(L, nl, R, nr, i0, lo_out, cnt, sm, err);
-  const uint64_t first = i0 + static_cast<uint64_t>(threadIdx.x) * kJcKeys;
-  const uint64_t i_end = (i0 + kJcTile < nl) ? i0 + kJcTile : nl;
+// A join to write: left rows' lower bounds and output offsets, source and
+// output columns (lc: the key columns and the other left ones, rc: the right
+// ones without the keys).
+struct JoinOut {
+  const uint64_t* offs;
+  const uint32_t* lo;
+  uint64_t nl, total;
+  const uint32_t* lc[VG_MAX_COLS];
+  const uint32_t* rc[VG_MAX_COLS];
+  uint32_t* oc[VG_MAX_COLS];
+  uint32_t nlc, nrc;
+};
+
+constexpr int kJwBlock = 256;
+
+// Output rows [kb, kend) (at most kJwBlock * ROWS) of a join, by one block.
+// Output row k comes from the left row i with offs[i] <= k < offs[i + 1] and
+// the right row lo[i] + (k - offs[i]); the rows come from left rows [ib, ie).
+// When those are at most STAGE = kJwBlock * ROWS + 1, their offsets and lower
+// bounds are staged in shared memory and each thread walks its rows (k
+// increasing, consecutive threads on consecutive rows, so loads and stores
+// coalesce) from the previous one's left row.  Hub keys thus spread over many
+// blocks.
+template <int ROWS>
+__device__ __forceinline__ void jw_write_tile(const JoinOut& o, uint64_t kb, uint64_t kend, uint64_t ib, uint64_t ie,
+                                              uint64_t* s_off, uint32_t* s_lo) {
+  constexpr int kStage = kJwBlock * ROWS + 1;
+  const uint64_t m = ie - ib;
+  const bool staged = m <= static_cast<uint64_t>(kStage);
+  if (staged)
+    for (uint32_t e = threadIdx.x; e < m; e += kJwBlock) {
+      s_off[e] = o.offs[ib + e];
+      s_lo[e] = o.lo[ib + e];
+    }
+  __syncthreads();
+  // 1. the left and right row of each of the thread's output rows
+  uint32_t li[ROWS], ri[ROWS];
+  if (staged) {
+    uint32_t p = 0;   // the current left row, relative to ib
 #pragma unroll
-  for (int j = 0; j < kJcKeys; ++j)
-    if (first + j < i_end) cnt_out[first + j] = cnt[j];
+    for (int it = 0; it < ROWS; ++it) {
+      const uint64_t k = kb + static_cast<uint64_t>(it) * kJwBlock + threadIdx.x;
+      li[it] = ri[it] = 0;
+      if (k < kend) {
+        // last p with s_off[p] <= k, moving forward from the previous row's p
+        uint32_t step = 1;
+        while (p + step < m && s_off[p + step] <= k) {
+          p += step;
+          step <<= 1;
+        }
+        while (step > 1) {
+          step >>= 1;
+          if (p + step < m && s_off[p + step] <= k) p += step;
+        }
+        li[it] = static_cast<uint32_t>(ib + p);
+        ri[it] = static_cast<uint32_t>(s_lo[p] + (k - s_off[p]));
+      }
+    }
+  } else {
+    // a sparse tile (more than kStage left rows, most without matches): the
+    // left rows of kGroup of the thread's output rows at a time come from
+    // kGroup binary searches of the offsets advanced in lockstep, so each
+    // round has kGroup independent loads in flight
+    constexpr int kGroup = ROWS < 4 ? ROWS : 4;
+#pragma unroll
+    for (int g0 = 0; g0 < ROWS; g0 += kGroup) {
+      uint64_t lq[kGroup], kk[kGroup];
+#pragma unroll
+      for (int q = 0; q < kGroup; ++q) {
+        const uint64_t k = kb + static_cast<uint64_t>(g0 + q) * kJwBlock + threadIdx.x;
+        kk[q] = k < kend ? k : kend - 1;
+        lq[q] = ib;
+      }
+      uint64_t n = ie - ib;                     // last i in [ib, ie) with offs[i] <= k
+      while (n > 1) {
+        const uint64_t half = n >> 1;
+#pragma unroll
+        for (int q = 0; q < kGroup; ++q) lq[q] = (o.offs[lq[q] + half] <= kk[q]) ? lq[q] + half : lq[q];
+        n -= half;
+      }
+#pragma unroll
+      for (int q = 0; q < kGroup; ++q) {
+        li[g0 + q] = static_cast<uint32_t>(lq[q]);
+        ri[g0 + q] = static_cast<uint32_t>(o.lo[lq[q]] + (kk[q] - o.offs[lq[q]]));
+      }
+    }
+  }
+  // 2. column by column: each thread's ROWS loads of a column are in flight
+  // together (read-only path), each store instruction writes consecutive
+  // rows, and one column's pointers are live at a time
+  const uint32_t nlc = o.nlc, ncols = o.nlc + o.nrc;
+  for (uint32_t c = 0; c < ncols; ++c) {
+    const bool left = c < nlc;
+    const uint32_t* src = left ? o.lc[c] : o.rc[c - nlc];
+    uint32_t* dst = o.oc[c];
+    uint32_t v[ROWS];
+#pragma unroll
+    for (int it = 0; it < ROWS; ++it) {
+      const uint64_t k = kb + static_cast<uint64_t>(it) * kJwBlock + threadIdx.x;
+      if (k < kend) v[it] = __ldg(src + (left ? li[it] : ri[it]));
+    }
+#pragma unroll
+    for (int it = 0; it < ROWS; ++it) {
+      const uint64_t k = kb + static_cast<uint64_t>(it) * kJwBlock + threadIdx.x;
+      if (k < kend) dst[k] = v[it];
+    }
+  }
 }
 
 }  // namespace vg

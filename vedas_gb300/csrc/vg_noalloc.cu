@@ -7,10 +7,10 @@
 // latency-critical serving threads that may only launch work.  Such a caller
 // cannot create a vg_ctx, whose arena is one cudaMalloc.
 //
-// The join's scratch (per-left-row lower bound, match count and output
+// The join's scratch (per-left-row lower bound and output
 // offset, plus the look-back status words) lives in one file-scope
 // __device__ array instead.  Its size is fixed: at most kMaxLeftRows left
-// rows (about 32 MiB of device memory, held by every GPU that loads this
+// rows (about 24 MiB of device memory, held by every GPU that loads this
 // library until the process exits).  Host code may not use the array's name
 // as a device address, so on the first call on each device, with that device
 // current, the entry point looks the address up with cudaGetSymbolAddress and
@@ -31,7 +31,6 @@ constexpr uint64_t kMaxTiles = kMaxLeftRows / kTileRows;
 
 struct NoAllocScratch {
   uint32_t lo[kMaxLeftRows];
-  uint32_t cnt[kMaxLeftRows];
   uint64_t offs[kMaxLeftRows];
   uint64_t status[kMaxTiles];
   uint64_t total;
@@ -96,7 +95,7 @@ extern "C" vg_status vg_join_noalloc(const uint32_t* const* l_cols, uint32_t l_n
     VG_CUDA(cudaMemsetAsync(&sc->total, 0, sizeof(uint64_t), s));
     VG_CUDA(cudaMemsetAsync(&sc->ticket, 0, sizeof(uint32_t), s));
     VG_CUDA(cudaMemsetAsync(&sc->err, 0, sizeof(vg::DeviceErrors), s));
-    const uint64_t t = vg::join_into(s, 0, l, r, out_cols, out_capacity, sc->lo, sc->cnt, sc->offs, sc->status,
+    const uint64_t t = vg::join_into(s, l, r, out_cols, out_capacity, sc->lo, sc->offs, sc->status,
                                      &sc->ticket, &sc->total, &sc->err);
     vg::DeviceErrors he{};
     VG_CUDA(cudaMemcpyAsync(&he, &sc->err, sizeof(he), cudaMemcpyDeviceToHost, s));

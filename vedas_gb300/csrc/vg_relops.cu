@@ -2,9 +2,9 @@
 // join (count -> scan -> load-balanced write), gathers and relation sorts.
 #include "vg_relops.h"
 
-#include <cstring>
-
 #include <algorithm>
+#include <cstring>
+#include <optional>
 
 #include "vg_join_tile.cuh"
 #include "vg_prims.cuh"
@@ -16,6 +16,7 @@ namespace {
 constexpr int kBlock = 256;
 constexpr int kRows = 8;
 constexpr int kTileRows = kBlock * kRows;
+constexpr uint64_t kGuessRows = 1u << 20;   // joins of at most so many left rows guess their output (join())
 
 unsigned grid_for(const Ctx& ctx, uint64_t n, int per_thread, int per_sm = 16) {
   uint64_t g = div_up(n, static_cast<uint64_t>(kBlock) * per_thread);
@@ -108,142 +109,180 @@ __global__ void __launch_bounds__(kBlock) unique_kernel(UniqueArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// Join.  Count: lower bound and match count of every left key in the right
-// keys, searching inside the right-key window of the block's left keys.
-// Scan: exclusive scan of counts to output offsets.  Write: every output row
-// finds its left row by an upper-bound search of the offsets (load-balanced
-// across heavy keys) and gathers its columns.
+// Join of two relations.  Count and scan: lower bound, match count and output
+// offset of every left key (vg_join_tile.cuh).  Write: every output row finds
+// its left row by the offsets (load-balanced across heavy keys) and copies
+// its columns.
 // ---------------------------------------------------------------------------
 template <bool TWO>
-struct KeyOf {
-  const uint32_t* c0;
-  const uint32_t* c1;
-  __device__ __forceinline__ uint64_t operator()(uint64_t i) const {
-    return TWO ? ((static_cast<uint64_t>(c0[i]) << 32) | c1[i]) : static_cast<uint64_t>(c0[i]);
-  }
+struct KeysOf {
+  using K = OneKeys;
+  static __host__ __device__ K of(const uint32_t* c0, const uint32_t*) { return K{c0}; }
+};
+template <>
+struct KeysOf<true> {
+  using K = PairKeys;
+  static __host__ __device__ K of(const uint32_t* c0, const uint32_t* c1) { return K{c0, c1}; }
 };
 
+// Every tile's right-key window, one warp per tile (both ends at once).
 template <bool TWO>
-__device__ uint64_t key_lower_bound(const KeyOf<TWO>& k, uint64_t lo, uint64_t hi, uint64_t key) {
-  while (lo < hi) {
-    uint64_t mid = (lo + hi) >> 1;
-    if (k(mid) < key) lo = mid + 1;
-    else hi = mid;
+__global__ void __launch_bounds__(kJcBlock) join_window_kernel(typename KeysOf<TWO>::K L, uint64_t nl,
+                                                               typename KeysOf<TWO>::K R, uint64_t nr,
+                                                               uint64_t tiles, uint2* __restrict__ win) {
+  const uint64_t nw = static_cast<uint64_t>(gridDim.x) * (kJcBlock / 32);
+  for (uint64_t t = static_cast<uint64_t>(blockIdx.x) * (kJcBlock / 32) + (threadIdx.x >> 5); t < tiles; t += nw) {
+    const uint64_t i0 = t * kJcTile, i1 = (i0 + kJcTile < nl ? i0 + kJcTile : nl) - 1;
+    uint64_t w0, w1;
+    warp_bound_pair_of<false, true>(R, nr, L(i0), L(i1), w0, w1);
+    if ((threadIdx.x & 31) == 0) win[t] = make_uint2(static_cast<uint32_t>(w0), static_cast<uint32_t>(w1));
   }
-  return lo;
-}
-template <bool TWO>
-__device__ uint64_t key_upper_bound(const KeyOf<TWO>& k, uint64_t lo, uint64_t hi, uint64_t key) {
-  while (lo < hi) {
-    uint64_t mid = (lo + hi) >> 1;
-    if (key < k(mid)) hi = mid;
-    else lo = mid + 1;
-  }
-  return lo;
 }
 
+// One block per 2048 left keys, in ticket order.  The window comes from
+// join_window_kernel where there are more tiles than the GPU runs at a time
+// (a block's own search is five rounds of global loads before its copy can
+// start), else warp 0 finds it.
 template <bool TWO>
-__global__ void __launch_bounds__(kBlock) join_count_kernel(KeyOf<TWO> L, uint64_t nl, KeyOf<TWO> R,
-                                                            uint64_t nr, uint32_t* __restrict__ lo_out,
-                                                            uint32_t* __restrict__ cnt_out) {
-  __shared__ uint64_t s_win[2];
-  const uint64_t i0 = static_cast<uint64_t>(blockIdx.x) * kBlock;
-  if (threadIdx.x == 0) {
-    const uint64_t i1 = (i0 + kBlock < nl ? i0 + kBlock : nl) - 1;
-    const uint64_t w0 = key_lower_bound(R, 0, nr, L(i0));
-    s_win[0] = w0;
-    s_win[1] = key_upper_bound(R, w0, nr, L(i1));
-  }
-  __syncthreads();
-  const uint64_t i = i0 + threadIdx.x;
-  if (i >= nl) return;
-  const uint64_t k = L(i);
-  const uint64_t lo = key_lower_bound(R, s_win[0], s_win[1], k);
-  const uint64_t hi = key_upper_bound(R, lo, s_win[1], k);
-  lo_out[i] = static_cast<uint32_t>(lo);
-  cnt_out[i] = static_cast<uint32_t>(hi - lo);
-}
-
-// One block per 2048 left keys; the right-key window is staged in shared
-// memory by a bulk copy (vg_join_tile.cuh).
-__global__ void __launch_bounds__(kJcBlock, 4) join_count_tiled_kernel(const uint32_t* __restrict__ L, uint64_t nl,
-                                                                    const uint32_t* __restrict__ R, uint64_t nr,
-                                                                    uint32_t* __restrict__ lo,
-                                                                    uint32_t* __restrict__ cnt, DeviceErrors* err) {
+__global__ void __launch_bounds__(kJcBlock, 4) join_count_scan_kernel(
+    typename KeysOf<TWO>::K L, uint64_t nl, typename KeysOf<TWO>::K R, uint64_t nr, const uint2* __restrict__ win,
+    uint32_t* __restrict__ lo, uint64_t* __restrict__ offs, uint64_t* status, uint32_t* ticket, uint64_t* total,
+    DeviceErrors* err) {
   __shared__ JoinCountSmem sm;
-  join_count_tile(L, nl, R, nr, static_cast<uint64_t>(blockIdx.x) * kJcTile, lo, cnt, sm, err);
-  if (threadIdx.x == 0) jc_drain_window(sm, err);
-}
-
-// Exclusive scan of uint32 counts into uint64 offsets (+ total).
-__global__ void __launch_bounds__(kBlock) scan_counts_kernel(const uint32_t* __restrict__ in,
-                                                             uint64_t* __restrict__ out, uint64_t n,
-                                                             uint64_t* status, uint32_t* ticket,
-                                                             uint64_t* total, uint64_t tiles,
-                                                             DeviceErrors* err) {
-  __shared__ uint64_t s_scan[kBlock / 32 + 1];
+  __shared__ uint64_t s_scan[kJcBlock / 32 + 1];
   __shared__ uint64_t s_b;
   __shared__ uint32_t s_tile;
-  if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
-  __syncthreads();
-  const uint32_t tile = s_tile;
-  const uint64_t r0 = static_cast<uint64_t>(tile) * kTileRows + threadIdx.x * kRows;
-  uint32_t v[kRows];
-  uint64_t sum = 0;
-#pragma unroll
-  for (int i = 0; i < kRows; ++i) {
-    v[i] = (r0 + i < n) ? in[r0 + i] : 0u;
-    sum += v[i];
+  if (threadIdx.x < 32) {
+    uint32_t t = 0;
+    if (threadIdx.x == 0) t = atomicAdd(ticket, 1u);
+    t = __shfl_sync(0xffffffffu, t, 0);
+    uint64_t w0, w1;
+    if (win) {
+      const uint2 w = win[t];
+      w0 = w.x;
+      w1 = w.y;
+    } else {
+      const uint64_t b = static_cast<uint64_t>(t) * kJcTile, e = (b + kJcTile < nl ? b + kJcTile : nl) - 1;
+      warp_bound_pair_of<false, true>(R, nr, L(b), L(e), w0, w1);
+    }
+    if (threadIdx.x == 0) {
+      s_tile = t;
+      if constexpr (TWO) jc_issue_pair_window(w0, w1, sm);
+      else jc_issue_window(R.c0, w0, w1, sm);
+    }
   }
-  uint64_t tot;
-  const uint64_t e = block_excl_scan64<kBlock>(sum, tot, s_scan);
-  const uint64_t g = block_lookback(status, tile, tot, err, &s_b);
-  if (tile == tiles - 1 && threadIdx.x == 0) *total = g + tot;
-  uint64_t run = g + e;
-#pragma unroll
-  for (int i = 0; i < kRows; ++i) {
-    if (r0 + i < n) out[r0 + i] = run;
-    run += v[i];
+  __syncthreads();
+  const uint64_t i0 = static_cast<uint64_t>(s_tile) * kJcTile;
+  uint32_t cnt[kJcKeys], lov[kJcKeys];
+  if constexpr (TWO) jc_count_staged_pairs(L, nl, R, i0, lov, cnt, sm);
+  else jc_count_staged(L.c0, nl, R.c0, i0, lov, cnt, sm, err);
+  jc_finish_tile(nl, i0, lov, cnt, sm, s_scan, &s_b, s_tile, 0, s_tile == gridDim.x - 1, lo, offs, status, total, err);
+}
+
+// What the host reads of a join (page-locked memory that the write kernel
+// stores to).
+constexpr uint32_t kTailKeys = 100;   // column 0 of smaller outputs is scanned for empty intervals
+struct JoinTail {
+  uint64_t total;
+  DeviceErrors err;
+  uint32_t first, last;        // of column 0, when rows were written
+  uint32_t c0[kTailKeys];      // column 0, when fewer rows than that were written
+};
+static_assert(sizeof(JoinTail) <= Ctx::kSmallWords * sizeof(uint64_t), "the tail fits the small staging buffer");
+
+// Left rows [x, y) of every output tile, one warp per tile.
+__global__ void __launch_bounds__(kJwBlock) join_ranges_kernel(const uint64_t* __restrict__ offs, uint64_t nl,
+                                                               uint64_t total, uint64_t tiles, uint32_t tile_rows,
+                                                               uint2* __restrict__ ranges) {
+  const uint64_t nw = static_cast<uint64_t>(gridDim.x) * (kJwBlock / 32);
+  for (uint64_t t = static_cast<uint64_t>(blockIdx.x) * (kJwBlock / 32) + (threadIdx.x >> 5); t < tiles; t += nw) {
+    const uint64_t kb = t * tile_rows, kend = kb + tile_rows < total ? kb + tile_rows : total;
+    uint64_t a, b;
+    warp_bound_pair<true, true, uint64_t>(offs, nl, kb, kend - 1, a, b);
+    if ((threadIdx.x & 31) == 0) ranges[t] = make_uint2(static_cast<uint32_t>(a - 1), static_cast<uint32_t>(b));
   }
 }
 
-struct JoinWriteArgs {
-  const uint64_t* offs;
-  const uint32_t* lo;
-  uint64_t nl, total;
-  const uint32_t* lc[VG_MAX_COLS];
-  const uint32_t* rc[VG_MAX_COLS];
-  uint32_t* oc[VG_MAX_COLS];
-  uint32_t nlc, nrc;
-};
+// The output rows, kJwBlock * ROWS per tile; a block loops over tiles.  The
+// row count comes from o.total or, when total_dev is given, from the device:
+// the outputs then hold `cap` rows and nothing is written when there are
+// more.  Nothing is written either after a wait that gave up (the offsets are
+// wrong).  Ranges come from join_ranges_kernel or are found by warp 0.
+template <int ROWS>
+__global__ void __launch_bounds__(kJwBlock, 5) join_write_kernel(JoinOut o, const uint64_t* total_dev, uint64_t cap,
+                                                                 const uint2* __restrict__ ranges,
+                                                                 const DeviceErrors* err, JoinTail* tail) {
+  constexpr uint32_t kTile = kJwBlock * ROWS;
+  __shared__ JoinOut s_o;
+  __shared__ uint64_t s_off[kTile + 1];
+  __shared__ uint32_t s_lo[kTile + 1];
+  __shared__ uint64_t s_range[2];
+  const uint64_t total = total_dev ? *total_dev : o.total;
+  const DeviceErrors e = *err;
+  if (tail && blockIdx.x == 0 && threadIdx.x == 0) {
+    tail->total = total;
+    tail->err = e;
+  }
+  if (e.timeout || total > cap) return;
+  if (threadIdx.x == 0) s_o = o;
+  const uint64_t tiles = (total + kTile - 1) / kTile;
+#pragma unroll 1
+  for (uint64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const uint64_t kb = tile * kTile, kend = kb + kTile < total ? kb + kTile : total;
+    __syncthreads();   // s_o is set; the previous tile's readers of the shared arrays are done
+    if (threadIdx.x < 32) {
+      uint64_t a, b;
+      if (ranges) {
+        const uint2 r = ranges[tile];
+        a = r.x;
+        b = r.y;
+      } else {
+        warp_bound_pair<true, true, uint64_t>(s_o.offs, s_o.nl, kb, kend - 1, a, b);
+        --a;
+      }
+      if (threadIdx.x == 0) {
+        s_range[0] = a;
+        s_range[1] = b;
+      }
+    }
+    __syncthreads();
+    jw_write_tile<ROWS>(s_o, kb, kend, s_range[0], s_range[1], s_off, s_lo);
+    if (tail) {   // each by the thread that wrote the row
+      const uint32_t* c0 = s_o.oc[0];
+      if (tile == 0 && threadIdx.x == 0) tail->first = c0[0];
+      if (tile == tiles - 1 && threadIdx.x == (total - 1 - kb) % kJwBlock) tail->last = c0[total - 1];
+      if (total < kTailKeys && threadIdx.x < total) tail->c0[threadIdx.x] = c0[threadIdx.x];
+    }
+  }
+}
 
-__global__ void __launch_bounds__(kBlock) join_write_kernel(JoinWriteArgs a) {
-  __shared__ uint64_t s_i[2];
-  const uint64_t kb = static_cast<uint64_t>(blockIdx.x) * kTileRows;
-  if (threadIdx.x == 0) {
-    const uint64_t klast = (kb + kTileRows < a.total ? kb + kTileRows : a.total) - 1;
-    const uint64_t f = upper_bound_dev(a.offs, 0, a.nl, kb) - 1;
-    s_i[0] = f;
-    s_i[1] = upper_bound_dev(a.offs, f, a.nl, klast);
-  }
-  __syncthreads();
-  const uint64_t ib = s_i[0], ie = s_i[1];
-#pragma unroll 2
-  for (int it = 0; it < kRows; ++it) {
-    const uint64_t k = kb + static_cast<uint64_t>(it) * kBlock + threadIdx.x;
-    if (k >= a.total) break;
-    const uint64_t i = upper_bound_dev(a.offs, ib, ie, k) - 1;
-    const uint64_t j = a.lo[i] + (k - a.offs[i]);
-    // every value of the row loaded (read-only path) before any is stored
-    uint32_t v[VG_MAX_COLS];
-    const int ncols = static_cast<int>(a.nlc + a.nrc);
-#pragma unroll
-    for (int c = 0; c < VG_MAX_COLS; ++c)
-      if (c < ncols) v[c] = c < static_cast<int>(a.nlc) ? __ldg(a.lc[c] + i) : __ldg(a.rc[c - a.nlc] + j);
-#pragma unroll
-    for (int c = 0; c < VG_MAX_COLS; ++c)
-      if (c < ncols) a.oc[c][k] = v[c];
-  }
+// Tiles from which the windows and ranges are found by kernels of their own.
+// (blocks of one join that run at a time: 4 or 5 per SM)
+bool many_tiles(int num_sms, uint64_t tiles) { return tiles > 4ull * static_cast<uint64_t>(num_sms); }
+
+template <bool TWO>
+void launch_count_scan(cudaStream_t stream, const Rel& l, const Rel& r, const uint2* win, uint32_t* lo,
+                       uint64_t* offs, uint64_t* status, uint32_t* ticket, uint64_t* total, DeviceErrors* err) {
+  const unsigned tiles = static_cast<unsigned>(div_up(l.nrows, kJcTile));
+  join_count_scan_kernel<TWO><<<tiles, kJcBlock, 0, stream>>>(
+      KeysOf<TWO>::of(l.cols[0], TWO ? l.cols[1] : nullptr), l.nrows,
+      KeysOf<TWO>::of(r.cols[0], TWO ? r.cols[1] : nullptr), r.nrows, win, lo, offs, status, ticket, total, err);
+  VG_CUDA(cudaGetLastError());
+}
+
+JoinOut join_out(const Rel& l, const Rel& r, uint32_t nk, const uint64_t* offs, const uint32_t* lo, uint64_t total,
+                 uint32_t* const* oc) {
+  JoinOut o{};
+  o.offs = offs;
+  o.lo = lo;
+  o.nl = l.nrows;
+  o.total = total;
+  for (uint32_t c = 0; c < l.ncols; ++c) o.lc[c] = l.cols[c];
+  for (uint32_t c = nk; c < r.ncols; ++c) o.rc[c - nk] = r.cols[c];
+  o.nlc = l.ncols;
+  o.nrc = r.ncols - nk;
+  for (uint32_t c = 0; c < o.nlc + o.nrc; ++c) o.oc[c] = oc[c];
+  return o;
 }
 
 struct GatherCols {
@@ -354,85 +393,136 @@ uint64_t unique_rows(Ctx& ctx, const uint32_t* const* in, uint32_t* const* out, 
   return kept;
 }
 
-void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out) {
+void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnds* ends) {
   const uint32_t nk = two_keys ? 2 : 1;
   if (l.ncols < nk || r.ncols < nk) fail(VG_ERR_INVALID, "join: missing key columns");
   const uint32_t ncols = l.ncols + r.ncols - nk;
   if (ncols > VG_MAX_COLS) fail(VG_ERR_UNSUPPORTED, "join output has more than 9 columns");
   if (l.nrows > 0xFFFFFFFFull || r.nrows > 0xFFFFFFFFull)
     fail(VG_ERR_OVERFLOW, "join inputs are limited to 2^32 rows");
+  if (ends) *ends = JoinEnds();
   if (l.nrows == 0 || r.nrows == 0) {
     out = rel_alloc(ctx, ncols, 0);
     return;
   }
-  Scratch<uint32_t> lo(ctx, l.nrows), cnt(ctx, l.nrows);
-  const unsigned cgrid = static_cast<unsigned>(div_up(l.nrows, kBlock));
-  const double cbytes = 4.0 * nk * (l.nrows + r.nrows);
-  if (two_keys) {
-    KeyOf<true> kl{l.cols[0], l.cols[1]}, kr{r.cols[0], r.cols[1]};
-    ctx.launch("join_count", cbytes, [&] {
-      join_count_kernel<true><<<cgrid, kBlock, 0, ctx.stream>>>(kl, l.nrows, kr, r.nrows, lo.get(), cnt.get());
+  const uint64_t tiles = div_up(l.nrows, kJcTile);
+  if (tiles > 0x7FFFFFFFull) fail(VG_ERR_OVERFLOW, "join: too many tiles");
+  Scratch<uint32_t> lo(ctx, l.nrows);
+  Scratch<uint64_t> offs(ctx, l.nrows), z(ctx, tiles + 2);   // z: look-back words, total, ticket
+  uint64_t* total = z.get() + tiles;
+  VG_CUDA(cudaMemsetAsync(z.get(), 0, (tiles + 2) * sizeof(uint64_t), ctx.stream));
+  std::optional<Scratch<uint2>> win;
+  if (many_tiles(ctx.num_sms, tiles)) {
+    win.emplace(ctx, tiles);
+    const unsigned wblocks =
+        static_cast<unsigned>(std::min<uint64_t>(div_up(tiles, kJcBlock / 32), static_cast<uint64_t>(ctx.num_sms) * 8));
+    ctx.launch("join_windows", 8.0 * tiles, [&] {
+      if (two_keys)
+        join_window_kernel<true><<<wblocks, kJcBlock, 0, ctx.stream>>>({l.cols[0], l.cols[1]}, l.nrows,
+                                                                       {r.cols[0], r.cols[1]}, r.nrows, tiles,
+                                                                       win->get());
+      else
+        join_window_kernel<false><<<wblocks, kJcBlock, 0, ctx.stream>>>({l.cols[0]}, l.nrows, {r.cols[0]}, r.nrows,
+                                                                        tiles, win->get());
     });
-  } else {
-    ctx.launch("join_count", cbytes, [&] {
-      join_count_tiled_kernel<<<static_cast<unsigned>(div_up(l.nrows, kJcTile)), kJcBlock, 0, ctx.stream>>>(
-          l.cols[0], l.nrows, r.cols[0], r.nrows, lo.get(), cnt.get(), ctx.d_err);
-    });
+    VG_CUDA(cudaGetLastError());
   }
-  VG_CUDA(cudaGetLastError());
-  const uint64_t tiles = div_up(l.nrows, kTileRows);
-  Scratch<uint64_t> offs(ctx, l.nrows), status(ctx, tiles), total(ctx, 1);
-  Scratch<uint32_t> ticket(ctx, 1);
-  VG_CUDA(cudaMemsetAsync(status.get(), 0, tiles * sizeof(uint64_t), ctx.stream));
-  VG_CUDA(cudaMemsetAsync(ticket.get(), 0, sizeof(uint32_t), ctx.stream));
-  ctx.launch("join_scan", 12.0 * l.nrows, [&] {
-    scan_counts_kernel<<<static_cast<unsigned>(tiles), kBlock, 0, ctx.stream>>>(
-        cnt.get(), offs.get(), l.nrows, status.get(), ticket.get(), total.get(), tiles, ctx.d_err);
+  ctx.launch("join_count_scan", 4.0 * nk * (l.nrows + r.nrows) + 12.0 * l.nrows, [&] {
+    const uint2* w = win ? win->get() : nullptr;
+    auto* ticket = reinterpret_cast<uint32_t*>(total + 1);
+    if (two_keys) launch_count_scan<true>(ctx.stream, l, r, w, lo.get(), offs.get(), z.get(), ticket, total, ctx.d_err);
+    else launch_count_scan<false>(ctx.stream, l, r, w, lo.get(), offs.get(), z.get(), ticket, total, ctx.d_err);
   });
-  VG_CUDA(cudaGetLastError());
+  auto* tail = reinterpret_cast<JoinTail*>(ctx.h_small);
+  auto finish = [&](uint64_t t) {
+    if (ends && t > 0) {
+      ends->first = tail->first;
+      ends->last = tail->last;
+      if (t < kTailKeys) ends->c0.assign(tail->c0, tail->c0 + t);
+    }
+  };
+  auto free_cols = [&](Rel& x) {
+    for (uint32_t c = 0; c < x.ncols; ++c)
+      if (x.cols[c]) ctx.free(x.cols[c]);
+    x = Rel();
+  };
+  // A small left side: room for twice its rows is taken at once and the write
+  // follows the count without the host in between (a round trip, copies and an
+  // allocation, took 25 of 120 us at 3,000 rows); larger outputs are written
+  // below.  Columns that do not fit the arena now are left to that path too.
+  if (l.nrows <= kGuessRows) {
+    const uint64_t cap = std::max<uint64_t>(1024, 2 * l.nrows);
+    Rel guess;
+    guess.ncols = ncols;
+    bool fits = true;
+    for (uint32_t c = 0; c < ncols && fits; ++c) {
+      guess.cols[c] = static_cast<uint32_t*>(ctx.arena.try_alloc(cap * sizeof(uint32_t)));
+      fits = guess.cols[c] != nullptr;
+    }
+    if (fits) {
+      constexpr int kRowsSmall = 2;
+      const JoinOut o = join_out(l, r, nk, offs.get(), lo.get(), 0, guess.cols);
+      const unsigned grid = static_cast<unsigned>(
+          std::min<uint64_t>(div_up(cap, kJwBlock * kRowsSmall), static_cast<uint64_t>(ctx.num_sms) * 5));
+      ctx.launch("join_write", 0.0, [&] {
+        join_write_kernel<kRowsSmall><<<grid, kJwBlock, 0, ctx.stream>>>(o, total, cap, nullptr, ctx.d_err, tail);
+      });
+      VG_CUDA(cudaGetLastError());
+      ctx.sync();
+      const uint64_t t = tail->total;
+      if (tail->err.timeout || tail->err.overflow || t > cap) {
+        free_cols(guess);
+        ctx.raise_device_errors(tail->err);
+      } else {
+        guess.nrows = t;
+        for (uint32_t c = 0; c < ncols; ++c)
+          ctx.arena.shrink(guess.cols[c], std::max<uint64_t>(t, 1) * sizeof(uint32_t));
+        out = guess;
+        ctx.add_bytes("join_write", 4.0 * t * (2.0 * ncols - 1));
+        finish(t);
+        return;
+      }
+    } else {
+      free_cols(guess);
+    }
+  }
   // the total and the error record come back together: a look-back that gave
   // up leaves the offsets wrong, and the write must then not run
-  VG_CUDA(cudaMemcpyAsync(ctx.h_small, total.get(), sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx.stream));
-  VG_CUDA(cudaMemcpyAsync(ctx.h_small + 1, ctx.d_err, sizeof(DeviceErrors), cudaMemcpyDeviceToHost, ctx.stream));
+  VG_CUDA(cudaMemcpyAsync(&tail->total, total, sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx.stream));
+  VG_CUDA(cudaMemcpyAsync(&tail->err, ctx.d_err, sizeof(DeviceErrors), cudaMemcpyDeviceToHost, ctx.stream));
   ctx.sync();
-  const uint64_t t = ctx.h_small[0];
-  {
-    DeviceErrors he;
-    std::memcpy(&he, ctx.h_small + 1, sizeof(he));
-    ctx.raise_device_errors(he);
-  }
+  const uint64_t t = tail->total;
+  ctx.raise_device_errors(tail->err);
   if (t > 0xFFFFFFFFull) fail(VG_ERR_OVERFLOW, "join output exceeds 2^32 rows");
   out = rel_alloc(ctx, ncols, t);
   if (t == 0) return;
-  JoinWriteArgs a{};
-  a.offs = offs.get();
-  a.lo = lo.get();
-  a.nl = l.nrows;
-  a.total = t;
-  for (uint32_t c = 0; c < l.ncols; ++c) a.lc[c] = l.cols[c];
-  for (uint32_t c = nk; c < r.ncols; ++c) a.rc[c - nk] = r.cols[c];
-  for (uint32_t c = 0; c < ncols; ++c) a.oc[c] = out.cols[c];
-  a.nlc = l.ncols;
-  a.nrc = r.ncols - nk;
+  const JoinOut o = join_out(l, r, nk, offs.get(), lo.get(), t, out.cols);
+  const uint64_t otiles = div_up(t, static_cast<uint64_t>(kTileRows));
+  std::optional<Scratch<uint2>> ranges;
+  if (many_tiles(ctx.num_sms, otiles)) {
+    ranges.emplace(ctx, otiles);
+    const unsigned rblocks = static_cast<unsigned>(
+        std::min<uint64_t>(div_up(otiles, kJwBlock / 32), static_cast<uint64_t>(ctx.num_sms) * 8));
+    ctx.launch("join_write_ranges", 8.0 * otiles, [&] {
+      join_ranges_kernel<<<rblocks, kJwBlock, 0, ctx.stream>>>(offs.get(), l.nrows, t, otiles, kTileRows,
+                                                               ranges->get());
+    });
+    VG_CUDA(cudaGetLastError());
+  }
   ctx.launch("join_write", 4.0 * t * (2.0 * ncols - 1), [&] {
-    join_write_kernel<<<static_cast<unsigned>(div_up(t, kTileRows)), kBlock, 0, ctx.stream>>>(a);
+    join_write_kernel<kRows><<<static_cast<unsigned>(otiles), kJwBlock, 0, ctx.stream>>>(
+        o, nullptr, t, ranges ? ranges->get() : nullptr, ctx.d_err, tail);
   });
   VG_CUDA(cudaGetLastError());
+  ctx.sync();
+  finish(t);
 }
 
-uint64_t join_into(cudaStream_t stream, int num_sms, const Rel& l, const Rel& r, uint32_t* const* out_cols,
-                   uint64_t capacity, uint32_t* lo, uint32_t* cnt, uint64_t* offs, uint64_t* status,
-                   uint32_t* ticket, uint64_t* total, DeviceErrors* err) {
-  (void)num_sms;
+uint64_t join_into(cudaStream_t stream, const Rel& l, const Rel& r, uint32_t* const* out_cols, uint64_t capacity,
+                   uint32_t* lo, uint64_t* offs, uint64_t* status, uint32_t* ticket, uint64_t* total,
+                   DeviceErrors* err) {
   if (l.nrows == 0 || r.nrows == 0) return 0;
-  const uint32_t ncols = l.ncols + r.ncols - 1;
-  join_count_tiled_kernel<<<static_cast<unsigned>(div_up(l.nrows, kJcTile)), kJcBlock, 0, stream>>>(
-      l.cols[0], l.nrows, r.cols[0], r.nrows, lo, cnt, err);
-  VG_CUDA(cudaGetLastError());
-  const uint64_t tiles = div_up(l.nrows, kTileRows);
-  scan_counts_kernel<<<static_cast<unsigned>(tiles), kBlock, 0, stream>>>(cnt, offs, l.nrows, status, ticket,
-                                                                         total, tiles, err);
-  VG_CUDA(cudaGetLastError());
+  launch_count_scan<false>(stream, l, r, nullptr, lo, offs, status, ticket, total, err);
   uint64_t t = 0;
   DeviceErrors he{};
   VG_CUDA(cudaMemcpyAsync(&t, total, sizeof(uint64_t), cudaMemcpyDeviceToHost, stream));
@@ -441,17 +531,9 @@ uint64_t join_into(cudaStream_t stream, int num_sms, const Rel& l, const Rel& r,
   // a look-back that gave up leaves the offsets wrong: no write then
   if (he.timeout) fail(VG_ERR_TIMEOUT, "join_into: a bounded device wait expired");
   if (t == 0 || t > capacity) return t;
-  JoinWriteArgs a{};
-  a.offs = offs;
-  a.lo = lo;
-  a.nl = l.nrows;
-  a.total = t;
-  for (uint32_t c = 0; c < l.ncols; ++c) a.lc[c] = l.cols[c];
-  for (uint32_t c = 1; c < r.ncols; ++c) a.rc[c - 1] = r.cols[c];
-  for (uint32_t c = 0; c < ncols; ++c) a.oc[c] = out_cols[c];
-  a.nlc = l.ncols;
-  a.nrc = r.ncols - 1;
-  join_write_kernel<<<static_cast<unsigned>(div_up(t, kTileRows)), kBlock, 0, stream>>>(a);
+  const JoinOut o = join_out(l, r, 1, offs, lo, t, out_cols);
+  join_write_kernel<kRows><<<static_cast<unsigned>(std::min<uint64_t>(div_up(t, kTileRows), 0x7FFFFFFFull)), kJwBlock,
+                             0, stream>>>(o, nullptr, t, nullptr, err, nullptr);
   VG_CUDA(cudaGetLastError());
   return t;
 }

@@ -40,18 +40,26 @@ void multi_copy(Ctx& ctx, const CopyPiece* pieces, int np);
 uint64_t unique_rows(Ctx& ctx, const uint32_t* const* in, uint32_t* const* out, uint32_t ncols,
                      uint64_t n);
 
+// First and last value of a join's column 0 (when it has rows), and all of it
+// when it has fewer than 100.
+struct JoinEnds {
+  uint32_t first = 0, last = 0;
+  std::vector<uint32_t> c0;
+};
+
 // Sorted inner join of l and r on column 0 (two_keys: on columns 0 and 1).
 // Output layout: key column(s), l's other columns, r's other columns; rows
-// ordered by (left row, right row).  Allocates `out` from the arena.
-void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out);
+// ordered by (left row, right row).  Allocates `out` from the arena; the
+// output is complete on return, and device errors are raised.
+void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnds* ends = nullptr);
 
 // The same join on a caller's stream with caller-provided scratch and output
-// columns (nothing is allocated): lo/cnt/offs hold l.nrows entries, status
+// columns (nothing is allocated): lo/offs hold l.nrows entries, status
 // div_up(l.nrows, 2048) words; status, ticket and err must be zero.  Returns
 // the result row count; the outputs are written only when it fits `capacity`.
-uint64_t join_into(cudaStream_t stream, int num_sms, const Rel& l, const Rel& r, uint32_t* const* out_cols,
-                   uint64_t capacity, uint32_t* lo, uint32_t* cnt, uint64_t* offs, uint64_t* status,
-                   uint32_t* ticket, uint64_t* total, DeviceErrors* err);
+uint64_t join_into(cudaStream_t stream, const Rel& l, const Rel& r, uint32_t* const* out_cols, uint64_t capacity,
+                   uint32_t* lo, uint64_t* offs, uint64_t* status, uint32_t* ticket, uint64_t* total,
+                   DeviceErrors* err);
 
 // out[c][i] = in[c][perm[i]] for every column.
 void gather_cols(Ctx& ctx, const uint32_t* const* in, uint32_t* const* out, uint32_t ncols,
