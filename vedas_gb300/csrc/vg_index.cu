@@ -398,19 +398,14 @@ class Permuter {
     DigitList dl{};
     for (const Sort& q : sorts_)
       for (const RadixDigit& d : q.digits) dl.d[dl.n++] = d;
-    const size_t hist_bytes = dl.n * kRadixValues * sizeof(uint64_t);
-    counts_.emplace(ctx, 2 * hist_bytes + 128);
-    char* sc = counts_->get();
-    auto* hist = reinterpret_cast<unsigned long long*>(sc + 128);
-    auto* bases = reinterpret_cast<uint64_t*>(sc + 128 + hist_bytes);
-    VG_CUDA(cudaMemsetAsync(sc, 0, 128 + hist_bytes, ctx.stream));
+    counts_.emplace(ctx, dl);
     uint32_t at = 0;
     for (Sort& q : sorts_)
-      for (size_t d = 0; d < q.digits.size(); ++d) q.bases.push_back(bases + kRadixValues * at++);
+      for (size_t d = 0; d < q.digits.size(); ++d) q.bases.push_back(counts_->bases(at++));
     keys_.emplace(ctx, n);
     ctx.launch("index_pack", 20.0 * n, [&] {
       pack_count_kernel<<<grid_for(ctx, n, 16, 8), kBlock, dl.n * kRadixValues * sizeof(uint32_t), ctx.stream>>>(
-          s, p, o, n, f_[S], f_[P], f_[O], keys_->get(), dl, hist, bases, reinterpret_cast<uint32_t*>(sc));
+          s, p, o, n, f_[S], f_[P], f_[O], keys_->get(), dl, counts_->hist(), counts_->bases(), counts_->done());
     });
     VG_CUDA(cudaGetLastError());
   }
@@ -502,7 +497,7 @@ class Permuter {
   uint32_t max_o_;
   Field f_[3];
   std::vector<Sort> sorts_;
-  std::optional<Scratch<char>> counts_;     // digit counts and bases of every sort
+  std::optional<RadixCounts> counts_;       // digit counts and bases of every sort
   std::optional<Scratch<uint64_t>> keys_;   // the packed keys in their present order
 
   void plan(const std::vector<Col>& cols, int begin, int end) {

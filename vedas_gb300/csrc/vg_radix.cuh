@@ -15,6 +15,23 @@ struct DigitList {
   RadixDigit d[kRadixMaxPasses];
 };
 
+// Device memory of the counts of a digit list: zeroed counts and block counter,
+// and the bases.
+struct RadixCounts {
+  Scratch<char> mem;
+  size_t bytes;
+  static constexpr size_t kHead = 128;
+  RadixCounts(Ctx& ctx, const DigitList& dl)
+      : mem(ctx, 2 * dl.n * kRadixValues * sizeof(uint64_t) + kHead), bytes(dl.n * kRadixValues * sizeof(uint64_t)) {
+    VG_CUDA(cudaMemsetAsync(mem.get(), 0, kHead + bytes, ctx.stream));
+  }
+  unsigned long long* hist() const { return reinterpret_cast<unsigned long long*>(mem.get() + kHead); }
+  uint64_t* bases(uint32_t digit = 0) const {
+    return reinterpret_cast<uint64_t*>(mem.get() + kHead + bytes) + static_cast<size_t>(digit) * kRadixValues;
+  }
+  uint32_t* done() const { return reinterpret_cast<uint32_t*>(mem.get()); }
+};
+
 // s: dl.n * kRadixValues words of shared memory.
 template <int BLOCK>
 __device__ __forceinline__ void digit_counts_init(const DigitList& dl, uint32_t* s) {

@@ -8,6 +8,7 @@
 
 #include "vg_join_tile.cuh"
 #include "vg_prims.cuh"
+#include "vg_radix.cuh"
 #include "vg_sort.h"
 
 namespace vg {
@@ -69,43 +70,72 @@ __global__ void __launch_bounds__(kBlock) multi_copy_kernel(CopyArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// Adjacent-unique compaction (thrust::unique over zipped columns).
+// Adjacent-unique compaction (thrust::unique over zipped columns): one kernel
+// finds the rows to drop, a second one moves the others if there are any to
+// drop (most results of a query have none).
 // ---------------------------------------------------------------------------
 struct UniqueArgs {
   const uint32_t* in[VG_MAX_COLS];
   uint32_t* out[VG_MAX_COLS];
   uint32_t ncols;
   uint64_t n;
-  uint64_t* status;
-  uint32_t* ticket;
-  uint64_t* count;
-  uint64_t tiles;
-  DeviceErrors* err;
+  uint8_t* keep;          // bit i of byte b: row 8 b + i stays
+};
+struct UniqueTotal {   // zeroed before the first kernel
+  unsigned long long dropped;
+  uint32_t done;       // finished blocks
+  uint32_t ticket;     // of the second kernel
 };
 
-// Adjacent-unique compaction: each thread flags its kRows rows (16-byte
-// loads of aligned columns), a block scan and a look-back place the tile's
-// kept rows, which are stored column by column through shared memory so
-// that every store is coalesced.
-__global__ void __launch_bounds__(kBlock) unique_kernel(UniqueArgs a) {
+// Each thread flags its 8 rows.  Columns are compared from the last to the
+// first, and only while some row still equals the one before it: in sorted
+// rows and in join outputs the last columns change fastest, so most of the
+// time one column is read (7.4e7 rows of 8 columns without repetitions took
+// 1.41 ms when all were read, and once more to be written elsewhere).
+__global__ void __launch_bounds__(kBlock) unique_flags_kernel(UniqueArgs a, UniqueTotal* tot, uint64_t* host_dropped) {
   static_assert(kRows == 8, "unique_diff_bits and compact_store take 8 rows per thread");
+  uint32_t drop = 0;
+  const uint64_t step = static_cast<uint64_t>(gridDim.x) * kBlock * kRows;
+#pragma unroll 2
+  for (uint64_t r0 = (static_cast<uint64_t>(blockIdx.x) * kBlock + threadIdx.x) * kRows; r0 < a.n; r0 += step) {
+    const uint32_t here = a.n - r0 < kRows ? static_cast<uint32_t>(a.n - r0) : kRows;
+    const uint32_t all = (1u << here) - 1u;
+    uint32_t diff = (r0 == 0) ? 1u : 0u;
+    diff |= unique_diff_bits(a.in[a.ncols - 1], a.n, r0);
+    for (int c = static_cast<int>(a.ncols) - 2; c >= 0 && (diff & all) != all; --c)
+      diff |= unique_diff_bits(a.in[c], a.n, r0);
+    diff &= all;
+    a.keep[r0 / 8] = static_cast<uint8_t>(diff);
+    drop += here - __popc(diff);
+  }
+  drop = __reduce_add_sync(0xffffffffu, drop);
+  if (lane_id() == 0 && drop) atomicAdd(&tot->dropped, static_cast<unsigned long long>(drop));
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0 && atomicAdd(&tot->done, 1u) == gridDim.x - 1) {
+    __threadfence();
+    *host_dropped = ld_status_u64(reinterpret_cast<const uint64_t*>(&tot->dropped));
+  }
+}
+
+// A look-back over the tiles' counts places each tile's rows, which are
+// stored column by column through shared memory so that every store is
+// coalesced.
+__global__ void __launch_bounds__(kBlock) unique_move_kernel(UniqueArgs a, UniqueTotal* tot, uint64_t* status,
+                                                             DeviceErrors* err) {
   __shared__ uint32_t s_scan[kBlock / 32 + 1];
   __shared__ uint64_t s_b;
   __shared__ uint32_t s_tile;
   __shared__ uint32_t s_keep[2 * kTileRows];   // compact_store: two columns at a time
-  if (threadIdx.x == 0) s_tile = atomicAdd(a.ticket, 1u);
+  if (threadIdx.x == 0) s_tile = atomicAdd(&tot->ticket, 1u);
   __syncthreads();
   const uint32_t tile = s_tile;
   const uint64_t r0 = static_cast<uint64_t>(tile) * kTileRows + threadIdx.x * kRows;
-  uint32_t diff = (r0 == 0) ? 1u : 0u;
-  for (uint32_t c = 0; c < a.ncols; ++c) diff |= unique_diff_bits(a.in[c], a.n, r0);
-  if (r0 >= a.n) diff = 0;
-  else if (a.n - r0 < kRows) diff &= (1u << (a.n - r0)) - 1u;
-  uint32_t tot;
-  const uint32_t e = block_excl_scan<kBlock>(__popc(diff), tot, s_scan);
-  const uint64_t g = block_lookback(a.status, tile, tot, a.err, &s_b);
-  if (tile == a.tiles - 1 && threadIdx.x == 0) *a.count = g + tot;
-  compact_store<kBlock>(a.in, a.out, a.ncols, a.n, r0, diff, e, tot, g, s_keep);
+  const uint32_t diff = r0 < a.n ? a.keep[r0 / 8] : 0u;
+  uint32_t kept;
+  const uint32_t e = block_excl_scan<kBlock>(__popc(diff), kept, s_scan);
+  const uint64_t g = block_lookback(status, tile, kept, err, &s_b);
+  compact_store<kBlock>(a.in, a.out, a.ncols, a.n, r0, diff, e, kept, g, s_keep);
 }
 
 // ---------------------------------------------------------------------------
@@ -285,24 +315,89 @@ JoinOut join_out(const Rel& l, const Rel& r, uint32_t nk, const uint64_t* offs, 
   return o;
 }
 
+// ---------------------------------------------------------------------------
+// Rows packed into one 64-bit key each (column 0 on top), for sorts over all
+// columns.
+// ---------------------------------------------------------------------------
+struct PackCols {
+  uint32_t* col[VG_MAX_COLS];
+  uint32_t shift[VG_MAX_COLS];   // the column's lowest key bit
+  uint64_t mask[VG_MAX_COLS];    // its values' bits (0: a column of zeros)
+  uint32_t ncols;
+};
+
+// max[c] = the largest value of column c (blocks take columns in turn).
+__global__ void __launch_bounds__(kBlock) column_maxima_kernel(PackCols a, uint64_t n, uint32_t* max_out) {
+  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * kBlock;
+  for (uint32_t c = 0; c < a.ncols; ++c) {
+    uint32_t m = 0;
+    const uint64_t t = static_cast<uint64_t>(blockIdx.x) * kBlock + threadIdx.x;
+    uint64_t nv = 0;
+    if ((reinterpret_cast<uintptr_t>(a.col[c]) & 15u) == 0) {
+      nv = n / 4;
+      const uint4* v = reinterpret_cast<const uint4*>(a.col[c]);
+#pragma unroll 2
+      for (uint64_t i = t; i < nv; i += stride) {
+        const uint4 x = __ldg(v + i);
+        m = max(m, max(max(x.x, x.y), max(x.z, x.w)));
+      }
+    }
+    for (uint64_t i = nv * 4 + t; i < n; i += stride) m = max(m, __ldg(a.col[c] + i));
+    m = __reduce_max_sync(0xffffffffu, m);
+    if (lane_id() == 0 && m) atomicMax(&max_out[c], m);
+  }
+}
+
+__global__ void __launch_bounds__(kBlock) pack_rows_kernel(PackCols a, uint64_t n, uint64_t* __restrict__ keys,
+                                                           DigitList dl, unsigned long long* __restrict__ hist,
+                                                           uint64_t* __restrict__ bases, uint32_t* done) {
+  extern __shared__ uint32_t sh[];   // [dl.n][kRadixValues]
+  digit_counts_init<kBlock>(dl, sh);
+  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * kBlock;
+  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * kBlock + threadIdx.x; i < n; i += stride) {
+    uint64_t k = 0;
+#pragma unroll
+    for (int c = 0; c < VG_MAX_COLS; ++c)
+      if (c < static_cast<int>(a.ncols) && a.mask[c]) k |= static_cast<uint64_t>(__ldg(a.col[c] + i)) << a.shift[c];
+    keys[i] = k;
+    digit_counts_add(dl, sh, k);
+  }
+  digit_counts_finish<kBlock>(dl, sh, hist, bases, done);
+}
+
+__global__ void __launch_bounds__(kBlock) unpack_rows_kernel(PackCols a, uint64_t n, const uint64_t* __restrict__ keys) {
+  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * kBlock;
+  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * kBlock + threadIdx.x; i < n; i += stride) {
+    const uint64_t k = keys[i];
+#pragma unroll
+    for (int c = 0; c < VG_MAX_COLS; ++c)
+      if (c < static_cast<int>(a.ncols)) a.col[c][i] = static_cast<uint32_t>((k >> a.shift[c]) & a.mask[c]);
+  }
+}
+
 struct GatherCols {
   const uint32_t* in[VG_MAX_COLS];
   uint32_t* out[VG_MAX_COLS];
   uint32_t ncols;
 };
 
+// Four rows per thread at a time, kBlock apart: their row numbers, then each
+// column's four reads are in flight together.
 __global__ void __launch_bounds__(kBlock) gather_kernel(const uint32_t* __restrict__ perm, uint64_t n,
                                                         GatherCols g) {
-  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * kBlock;
-  for (uint64_t r = static_cast<uint64_t>(blockIdx.x) * kBlock + threadIdx.x; r < n; r += stride) {
-    const uint32_t p = perm[r];
-    uint32_t v[VG_MAX_COLS];
+  constexpr int kIn = 4;
+  const uint64_t step = static_cast<uint64_t>(gridDim.x) * kBlock * kIn;
+  for (uint64_t r = static_cast<uint64_t>(blockIdx.x) * kBlock * kIn + threadIdx.x; r < n; r += step) {
+    uint32_t p[kIn], v[kIn];
 #pragma unroll
-    for (int c = 0; c < VG_MAX_COLS; ++c)
-      if (c < static_cast<int>(g.ncols)) v[c] = __ldg(g.in[c] + p);
+    for (int q = 0; q < kIn; ++q) p[q] = r + q * kBlock < n ? perm[r + q * kBlock] : 0u;
+    for (uint32_t c = 0; c < g.ncols; ++c) {
 #pragma unroll
-    for (int c = 0; c < VG_MAX_COLS; ++c)
-      if (c < static_cast<int>(g.ncols)) g.out[c][r] = v[c];
+      for (int q = 0; q < kIn; ++q) v[q] = __ldg(g.in[c] + p[q]);
+#pragma unroll
+      for (int q = 0; q < kIn; ++q)
+        if (r + q * kBlock < n) g.out[c][r + q * kBlock] = v[q];
+    }
   }
 }
 }  // namespace
@@ -362,35 +457,6 @@ void multi_copy(Ctx& ctx, const CopyPiece* pieces, int np) {
   ctx.launch("select_copy", bytes,
              [&] { multi_copy_kernel<<<grid_for(ctx, a.start[a.np], 2), kBlock, 0, ctx.stream>>>(a); });
   VG_CUDA(cudaGetLastError());
-}
-
-uint64_t unique_rows(Ctx& ctx, const uint32_t* const* in, uint32_t* const* out, uint32_t ncols,
-                     uint64_t n) {
-  if (n == 0) return 0;
-  UniqueArgs a{};
-  for (uint32_t c = 0; c < ncols; ++c) {
-    a.in[c] = in[c];
-    a.out[c] = out[c];
-  }
-  a.ncols = ncols;
-  a.n = n;
-  a.tiles = div_up(n, kTileRows);
-  Scratch<uint64_t> status(ctx, a.tiles), count(ctx, 1);
-  Scratch<uint32_t> ticket(ctx, 1);
-  VG_CUDA(cudaMemsetAsync(status.get(), 0, a.tiles * sizeof(uint64_t), ctx.stream));
-  VG_CUDA(cudaMemsetAsync(ticket.get(), 0, sizeof(uint32_t), ctx.stream));
-  a.status = status.get();
-  a.ticket = ticket.get();
-  a.count = count.get();
-  a.err = ctx.d_err;
-  ctx.launch("unique_compact", 4.0 * n * ncols,
-             [&] { unique_kernel<<<static_cast<unsigned>(a.tiles), kBlock, 0, ctx.stream>>>(a); });
-  VG_CUDA(cudaGetLastError());
-  VG_CUDA(cudaMemcpyAsync(ctx.h_small, count.get(), sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx.stream));
-  ctx.sync();
-  const uint64_t kept = ctx.h_small[0];
-  ctx.add_bytes("unique_compact", 4.0 * kept * ncols);
-  return kept;
 }
 
 void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnds* ends) {
@@ -552,58 +618,136 @@ void gather_cols(Ctx& ctx, const uint32_t* const* in, uint32_t* const* out, uint
   VG_CUDA(cudaGetLastError());
 }
 
+// Columns [first, r.ncols) of r in the order of perm.  Up to kTogether cells
+// go in one launch (as far as the new columns fit the arena); larger columns
+// go one by one, so that each one's random reads have the L2 cache to
+// themselves (three columns of 8M rows: 0.145 ms one by one, 0.181 together).
+static void permute_columns(Ctx& ctx, Rel& r, uint32_t first, const uint32_t* perm) {
+  constexpr uint64_t kTogether = 4u << 20;
+  const bool together = r.nrows * (r.ncols - first) <= kTogether;
+  for (uint32_t c = first; c < r.ncols;) {
+    const uint32_t *in[VG_MAX_COLS] = {r.cols[c]};
+    uint32_t* out[VG_MAX_COLS] = {ctx.alloc<uint32_t>(r.nrows)};
+    uint32_t k = 1;
+    for (; together && c + k < r.ncols; ++k) {
+      out[k] = static_cast<uint32_t*>(ctx.arena.try_alloc(r.nrows * sizeof(uint32_t)));
+      if (!out[k]) break;
+      in[k] = r.cols[c + k];
+    }
+    gather_cols(ctx, in, out, k, perm, r.nrows);
+    for (uint32_t q = 0; q < k; ++q) {
+      rel_drop_col(ctx, r, c + q);
+      r.cols[c + q] = out[q];
+    }
+    c += k;
+  }
+}
+
+// An owned copy of column c where it is a view.
+static void own_column(Ctx& ctx, Rel& r, uint32_t c) {
+  if (!(r.borrowed >> c & 1u)) return;
+  Rel one;
+  one.ncols = 1;
+  one.nrows = r.nrows;
+  one.cols[0] = r.cols[c];
+  one.borrowed = 1;
+  rel_own(ctx, one);
+  r.cols[c] = one.cols[0];
+  r.borrowed &= ~(1u << c);
+}
+
 void sort_by_first(Ctx& ctx, Rel& r) {
   const uint64_t n = r.nrows;
   if (n <= 1 || r.ncols == 0) return;
   if (n > 0xFFFFFFFFull) fail(VG_ERR_OVERFLOW, "relation sorts are limited to 2^32 rows");
-  if (r.borrowed & 1u) {
-    // the sort uses column 0 as its key buffer: take a copy of a view
-    Rel k0;
-    k0.ncols = 1;
-    k0.nrows = n;
-    k0.cols[0] = r.cols[0];
-    k0.borrowed = 1;
-    rel_own(ctx, k0);
-    r.cols[0] = k0.cols[0];
-    r.borrowed &= ~1u;
-  }
+  own_column(ctx, r, 0);   // the sort uses column 0 as its key buffer
   uint32_t* keys_alt = ctx.alloc<uint32_t>(n);
-  if (r.ncols == 1) {
-    const bool alt = radix_sort_u32(ctx, r.cols[0], keys_alt, nullptr, nullptr, n, 32, false);
-    if (alt) {
-      ctx.free(r.cols[0]);
-      r.cols[0] = keys_alt;
-    } else {
-      ctx.free(keys_alt);
+  if (r.ncols <= 2) {
+    // a second column travels with the keys as their values: no row numbers,
+    // no gather
+    uint32_t *vals = nullptr, *vals_alt = nullptr;
+    if (r.ncols == 2) {
+      own_column(ctx, r, 1);
+      vals = r.cols[1];
+      vals_alt = ctx.alloc<uint32_t>(n);
     }
+    const bool alt = radix_sort_u32(ctx, r.cols[0], keys_alt, vals, vals_alt, n, 32, false);
+    if (alt) {
+      std::swap(r.cols[0], keys_alt);
+      if (vals) std::swap(r.cols[1], vals_alt);
+    }
+    ctx.free(keys_alt);
+    if (vals) ctx.free(vals_alt);
     return;
   }
   uint32_t* vals = ctx.alloc<uint32_t>(n);
   uint32_t* vals_alt = ctx.alloc<uint32_t>(n);
   const bool alt = radix_sort_u32(ctx, r.cols[0], keys_alt, vals, vals_alt, n, 32, true);
   uint32_t* perm = alt ? vals_alt : vals;
-  if (alt) {
-    ctx.free(r.cols[0]);
-    r.cols[0] = keys_alt;
-  } else {
-    ctx.free(keys_alt);
-  }
+  if (alt) std::swap(r.cols[0], keys_alt);
+  ctx.free(keys_alt);
   ctx.free(alt ? vals : vals_alt);
-  for (uint32_t c = 1; c < r.ncols; ++c) {
-    uint32_t* nc = ctx.alloc<uint32_t>(n);
-    const uint32_t* in[1] = {r.cols[c]};
-    uint32_t* out[1] = {nc};
-    gather_cols(ctx, in, out, 1, perm, n);
-    rel_drop_col(ctx, r, c);
-    r.cols[c] = nc;
-  }
+  permute_columns(ctx, r, 1, perm);
   ctx.free(perm);
+}
+
+// Rows of at most 64 bits (each column as wide as its largest value): one
+// sort of packed keys, which hold the whole rows.  5M rows of three 19-bit
+// columns: 8 passes over 8-byte keys instead of 9 over keys and row numbers
+// and six gathers.
+static bool sort_packed_rows(Ctx& ctx, Rel& r) {
+  const uint64_t n = r.nrows;
+  PackCols a{};
+  a.ncols = r.ncols;
+  for (uint32_t c = 0; c < r.ncols; ++c) a.col[c] = r.cols[c];
+  Scratch<uint32_t> mx(ctx, VG_MAX_COLS);
+  VG_CUDA(cudaMemsetAsync(mx.get(), 0, VG_MAX_COLS * sizeof(uint32_t), ctx.stream));
+  ctx.launch("column_max", 4.0 * n * r.ncols,
+             [&] { column_maxima_kernel<<<grid_for(ctx, n, 8, 8), kBlock, 0, ctx.stream>>>(a, n, mx.get()); });
+  VG_CUDA(cudaGetLastError());
+  VG_CUDA(cudaMemcpyAsync(ctx.h_small, mx.get(), VG_MAX_COLS * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx.stream));
+  ctx.sync();
+  const uint32_t* hm = reinterpret_cast<const uint32_t*>(ctx.h_small);
+  uint32_t total = 0;
+  for (int c = static_cast<int>(r.ncols) - 1; c >= 0; --c) {
+    const uint32_t bits = hm[c] ? 32 - static_cast<uint32_t>(__builtin_clz(hm[c])) : 0;
+    a.shift[c] = bits ? total : 0;
+    a.mask[c] = (1ull << bits) - 1;
+    total += bits;
+  }
+  if (total > 64) return false;
+  if (total == 0) return true;   // equal rows throughout
+  std::vector<RadixDigit> digits;
+  radix_plan(digits, 0, static_cast<int>(total));
+  DigitList dl{};
+  dl.n = static_cast<uint32_t>(digits.size());
+  for (uint32_t d = 0; d < dl.n; ++d) dl.d[d] = digits[d];
+  const RadixCounts counts(ctx, dl);
+  Scratch<uint64_t> keys(ctx, n), alt(ctx, n);
+  ctx.launch("sort_pack", (8.0 + 4.0 * r.ncols) * n, [&] {
+    pack_rows_kernel<<<grid_for(ctx, n, 8, 8), kBlock, dl.n * kRadixValues * sizeof(uint32_t), ctx.stream>>>(
+        a, n, keys.get(), dl, counts.hist(), counts.bases(), counts.done());
+  });
+  VG_CUDA(cudaGetLastError());
+  std::vector<const uint64_t*> bases;
+  for (uint32_t d = 0; d < dl.n; ++d) bases.push_back(counts.bases(d));
+  if (radix_sort_u64_counted(ctx, keys.get(), alt.get(), n, digits, bases)) std::swap(keys.p, alt.p);
+  for (uint32_t c = 0; c < r.ncols; ++c) {
+    if (r.borrowed >> c & 1u) r.cols[c] = ctx.alloc<uint32_t>(n);   // (a view is not written)
+    a.col[c] = r.cols[c];
+  }
+  r.borrowed = 0;
+  ctx.launch("sort_unpack", (8.0 + 4.0 * r.ncols) * n,
+             [&] { unpack_rows_kernel<<<grid_for(ctx, n, 8), kBlock, 0, ctx.stream>>>(a, n, keys.get()); });
+  VG_CUDA(cudaGetLastError());
+  return true;
 }
 
 void sort_rows(Ctx& ctx, Rel& r) {
   const uint64_t n = r.nrows;
   if (n <= 1 || r.ncols <= 1) return;  // one column: a no-op in the reference
   if (n > 0xFFFFFFFFull) fail(VG_ERR_OVERFLOW, "relation sorts are limited to 2^32 rows");
+  if (sort_packed_rows(ctx, r)) return;
   uint32_t* perm = ctx.alloc<uint32_t>(n);
   uint32_t* perm_alt = ctx.alloc<uint32_t>(n);
   uint32_t* keys = ctx.alloc<uint32_t>(n);
@@ -617,14 +761,7 @@ void sort_rows(Ctx& ctx, Rel& r) {
     const bool alt = radix_sort_u32(ctx, keys, keys_alt, perm, perm_alt, n, 32, false);
     if (alt) std::swap(perm, perm_alt);
   }
-  for (uint32_t c = 0; c < r.ncols; ++c) {
-    uint32_t* nc = ctx.alloc<uint32_t>(n);
-    const uint32_t* in[1] = {r.cols[c]};
-    uint32_t* out[1] = {nc};
-    gather_cols(ctx, in, out, 1, perm, n);
-    rel_drop_col(ctx, r, c);
-    r.cols[c] = nc;
-  }
+  permute_columns(ctx, r, 0, perm);
   ctx.free(perm);
   ctx.free(perm_alt);
   ctx.free(keys);
@@ -633,12 +770,37 @@ void sort_rows(Ctx& ctx, Rel& r) {
 
 void unique_in_place(Ctx& ctx, Rel& r) {
   if (r.nrows <= 1 || r.ncols == 0) return;
-  Rel out = rel_alloc(ctx, r.ncols, r.nrows);
-  const uint64_t kept = unique_rows(ctx, r.cols, out.cols, r.ncols, r.nrows);
+  const uint64_t n = r.nrows;
+  UniqueArgs a{};
+  for (uint32_t c = 0; c < r.ncols; ++c) a.in[c] = r.cols[c];
+  a.ncols = r.ncols;
+  a.n = n;
+  const uint64_t tiles = div_up(n, kTileRows);
+  Scratch<uint8_t> keep(ctx, div_up(n, 8));
+  Scratch<UniqueTotal> tot(ctx, 1);
+  a.keep = keep.get();
+  VG_CUDA(cudaMemsetAsync(tot.get(), 0, sizeof(UniqueTotal), ctx.stream));
+  const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(tiles, static_cast<uint64_t>(ctx.num_sms) * 8));
+  // (what must be read: a column at least)
+  ctx.launch("unique_flags", 4.0 * n,
+             [&] { unique_flags_kernel<<<grid, kBlock, 0, ctx.stream>>>(a, tot.get(), ctx.h_small); });
+  VG_CUDA(cudaGetLastError());
+  ctx.sync();
+  const uint64_t dropped = ctx.h_small[0];
+  if (dropped == 0) return;
+  const uint64_t kept = n - dropped;
+  Rel out = rel_alloc(ctx, r.ncols, kept);
+  for (uint32_t c = 0; c < r.ncols; ++c) a.out[c] = out.cols[c];
+  Scratch<uint64_t> status(ctx, tiles);
+  VG_CUDA(cudaMemsetAsync(status.get(), 0, tiles * sizeof(uint64_t), ctx.stream));
+  ctx.launch("unique_compact", 4.0 * (n + kept) * r.ncols, [&] {
+    unique_move_kernel<<<static_cast<unsigned>(tiles), kBlock, 0, ctx.stream>>>(a, tot.get(), status.get(),
+                                                                                 ctx.d_err);
+  });
+  VG_CUDA(cudaGetLastError());
   rel_free(ctx, r);
-  for (uint32_t c = 0; c < out.ncols; ++c) ctx.arena.shrink(out.cols[c], kept * sizeof(uint32_t));
-  out.nrows = kept;
   r = out;
+  ctx.check_device_errors();
 }
 
 void download(Ctx& ctx, const uint32_t* dev, uint64_t n, uint32_t* host) {

@@ -35,11 +35,6 @@ struct CopyPiece {
 // All pieces in one launch (up to 16).
 void multi_copy(Ctx& ctx, const CopyPiece* pieces, int np);
 
-// Adjacent-unique compaction of the rows of `in` (ncols columns, n rows) into
-// `out`; returns the number of rows kept (synchronizes).
-uint64_t unique_rows(Ctx& ctx, const uint32_t* const* in, uint32_t* const* out, uint32_t ncols,
-                     uint64_t n);
-
 // First and last value of a join's column 0 (when it has rows), and all of it
 // when it has fewer than 100.
 struct JoinEnds {
@@ -69,7 +64,8 @@ void gather_cols(Ctx& ctx, const uint32_t* const* in, uint32_t* const* out, uint
 void sort_by_first(Ctx& ctx, Rel& r);
 // Lexicographic sort of the rows over all columns (in place).
 void sort_rows(Ctx& ctx, Rel& r);
-// Adjacent duplicate-row removal in place.
+// Adjacent duplicate-row removal (synchronizes).  A relation without any
+// keeps its columns; views stay views.
 void unique_in_place(Ctx& ctx, Rel& r);
 
 // Copies `n` values of a device column to the host (synchronizes).
