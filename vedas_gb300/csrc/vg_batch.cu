@@ -6,10 +6,12 @@
 
 #include <algorithm>
 #include <cstring>
+#include <optional>
 
 #include "vg_join_tile.cuh"
 #include "vg_pool.h"
 #include "vg_prims.cuh"
+#include "vg_radix.cuh"
 #include "vg_sort.h"
 
 namespace vg {
@@ -19,12 +21,58 @@ constexpr int kBlock = 256;
 constexpr int kRows = 8;
 constexpr int kTileRows = kBlock * kRows;
 
-template <typename T>
-T* upload(Ctx& ctx, const std::vector<T>& v) {
-  T* d = static_cast<T*>(ctx.arena.alloc((v.empty() ? 1 : v.size()) * sizeof(T)));
-  if (!v.empty()) ctx.upload_bytes(d, v.data(), v.size() * sizeof(T));
-  return d;
-}
+// The tables of one call (and words that start at zero) sent to the device in
+// one copy: a copy of its own for each of the half dozen tables of a call, and
+// a memset for each counter, cost the engines' threads more than the kernels
+// took (a stage of a 64-query batch spent 110 to 490 us on about 30 runtime
+// calls).  The device block is released, in stream order, with the object.
+class Tables {
+ public:
+  explicit Tables(Ctx& ctx) : ctx_(ctx) {}
+  Tables(const Tables&) = delete;
+  Tables& operator=(const Tables&) = delete;
+  ~Tables() {
+    ctx_.free(dev_);
+    ctx_.free(zero_);
+  }
+  template <typename T>
+  size_t add(const std::vector<T>& v) {
+    const size_t at = room(v.size() * sizeof(T));
+    if (!v.empty()) std::memcpy(blob_.data() + at, v.data(), v.size() * sizeof(T));
+    return at;
+  }
+  // Zeroed words; many of them (kInline bytes and more) get a block and a
+  // memset of their own, so only one call per object may ask for that.
+  template <typename T>
+  size_t zeros(size_t count) {
+    const size_t bytes = count * sizeof(T);
+    if (bytes < kInline) return room(bytes);
+    if (zero_) fail(VG_ERR_INVALID, "tables: one large zeroed block at most");
+    zero_ = ctx_.alloc<char>(bytes);
+    VG_CUDA(cudaMemsetAsync(zero_, 0, bytes, ctx_.stream));
+    return kZeroBlock;
+  }
+  void send() {
+    dev_ = ctx_.alloc<char>(blob_.size());
+    ctx_.upload_bytes(dev_, blob_.data(), blob_.size());
+  }
+  template <typename T>
+  T* at(size_t off) const {
+    return reinterpret_cast<T*>(off == kZeroBlock ? zero_ : dev_ + off);
+  }
+
+ private:
+  static constexpr size_t kInline = 32 << 10, kZeroBlock = SIZE_MAX;
+  size_t room(size_t bytes) {
+    const size_t at = (blob_.size() + 15) / 16 * 16;
+    blob_.resize(at + (bytes ? bytes : 1), 0);
+    return at;
+  }
+  Ctx& ctx_;
+  std::vector<char> blob_;
+  char* dev_ = nullptr;
+  char* zero_ = nullptr;
+};
 
 unsigned grid_cap(const Ctx& ctx, uint64_t units, int per_thread) {
   uint64_t g = div_up(units, static_cast<uint64_t>(kBlock) * per_thread);
@@ -101,13 +149,22 @@ __global__ void __launch_bounds__(kBlock) bcopy_kernel(const CopyPiece* __restri
 // scan and a segmented look-back over the segment's earlier tiles.
 constexpr uint32_t kSmallSeg = 32 * kRows;
 
+// Bits of the rows r0 .. r0 + 7 that stay.  Columns are compared from the last
+// to the first (the last change fastest in join outputs), only while some row
+// still equals the one before it.
+__device__ __forceinline__ uint32_t kept_rows(const SegRows& g, uint64_t r0) {
+  if (r0 >= g.n) return 0;
+  const uint32_t all = g.n - r0 < kRows ? (1u << (g.n - r0)) - 1u : (1u << kRows) - 1u;
+  uint32_t diff = r0 == 0 ? 1u : 0u;
+  for (int c = static_cast<int>(g.ncols) - 1; c >= 0 && (diff & all) != all; --c)
+    diff |= unique_diff_bits(g.in[c], g.n, r0);
+  return diff & all;
+}
+
 __device__ __forceinline__ void unique_small_segment(const SegRows& g, uint64_t* count) {
   const uint32_t lane = lane_id();
   const uint64_t n = g.n, r0 = static_cast<uint64_t>(lane) * kRows;
-  uint32_t diff = (r0 == 0 && n > 0) ? 1u : 0u;
-  for (uint32_t c = 0; c < g.ncols; ++c) diff |= unique_diff_bits(g.in[c], n, r0);
-  if (r0 >= n) diff = 0;
-  else if (n - r0 < kRows) diff &= (1u << (n - r0)) - 1u;
+  const uint32_t diff = kept_rows(g, r0);
   const uint32_t cnt = __popc(diff);
   const uint32_t incl = warp_incl_scan(cnt);
   uint64_t o = incl - cnt;
@@ -147,10 +204,7 @@ __global__ void __launch_bounds__(kBlock) bunique_kernel(const SegRows* __restri
   const uint64_t n = s_seg.n;
   const uint32_t ncols = s_seg.ncols;
   const uint64_t r0 = (tile - tstart[s]) * kTileRows + threadIdx.x * kRows;
-  uint32_t diff = (r0 == 0) ? 1u : 0u;
-  for (uint32_t c = 0; c < ncols; ++c) diff |= unique_diff_bits(s_seg.in[c], n, r0);
-  if (r0 >= n) diff = 0;
-  else if (n - r0 < kRows) diff &= (1u << (n - r0)) - 1u;
+  const uint32_t diff = kept_rows(s_seg, r0);
   uint32_t tot;
   const uint32_t e = block_excl_scan<kBlock>(__popc(diff), tot, s_scan);
   if (threadIdx.x < 32) {
@@ -193,12 +247,14 @@ __device__ __forceinline__ void chunk_segments(const uint32_t* __restrict__ chun
 }
 
 // (segment, key) composite sort keys: the segment sits above the key's
-// key_bits bits, so one sort orders rows by segment and, within it, by key.
-__global__ void __launch_bounds__(kBlock) composite_keys_kernel(const uint32_t* const* __restrict__ col0,
-                                                                const uint64_t* __restrict__ rstart, uint32_t S,
-                                                                const uint32_t* __restrict__ chunk_seg,
-                                                                uint64_t nchunks, uint32_t key_bits,
-                                                                uint64_t* __restrict__ keys) {
+// key_bits bits, so one sort orders rows by segment and, within it, by key;
+// and the digit counts of that sort.
+__global__ void __launch_bounds__(kBlock) composite_keys_kernel(
+    const uint32_t* const* __restrict__ col0, const uint64_t* __restrict__ rstart, uint32_t S,
+    const uint32_t* __restrict__ chunk_seg, uint64_t nchunks, uint32_t key_bits, uint64_t* __restrict__ keys,
+    DigitList dl, unsigned long long* __restrict__ hist, uint64_t* __restrict__ bases, uint32_t* done) {
+  extern __shared__ uint32_t sh[];   // [dl.n][kRadixValues]
+  digit_counts_init<kBlock>(dl, sh);
   const uint64_t total = rstart[S];
   for (uint64_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
     uint32_t k0, k1;
@@ -208,9 +264,66 @@ __global__ void __launch_bounds__(kBlock) composite_keys_kernel(const uint32_t* 
       const uint64_t r = c * kChunkRows + static_cast<uint64_t>(it) * kBlock + threadIdx.x;
       if (r < total) {
         const uint32_t s = seg_of_row(rstart, k0, k1, r);
-        keys[r] = (static_cast<uint64_t>(s) << key_bits) | __ldg(col0[s] + (r - rstart[s]));
+        const uint64_t k = (static_cast<uint64_t>(s) << key_bits) | __ldg(col0[s] + (r - rstart[s]));
+        keys[r] = k;
+        digit_counts_add(dl, sh, k);
       }
     }
+  }
+  digit_counts_finish<kBlock>(dl, sh, hist, bases, done);
+}
+
+// Stable sorts of small relations by column 0, each in one step: a row's place
+// is the number of rows that go before it.  Up to 32 rows take one warp (the
+// first warp_blocks blocks), up to kSortSmall one block.  Most re-sorts of a
+// wave have a few rows, and a composite sort of all of them took some 20
+// runtime calls and ten kernels.
+constexpr uint32_t kSortWarp = 32, kSortSmall = 1024;
+
+__global__ void __launch_bounds__(kBlock) sort_small_kernel(const SegRows* __restrict__ segs,
+                                                            const uint32_t* __restrict__ by_warp, uint32_t nwarp,
+                                                            const uint32_t* __restrict__ by_block,
+                                                            uint32_t warp_blocks) {
+  if (blockIdx.x < warp_blocks) {
+    const uint32_t w = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5), lane = lane_id();
+    if (w >= nwarp) return;
+    const SegRows& g = segs[by_warp[w]];
+    const uint32_t n = static_cast<uint32_t>(g.n);
+    const uint32_t k = lane < n ? g.in[0][lane] : 0u;
+    uint32_t at = 0;
+    for (uint32_t j = 0; j < n; ++j) {
+      const uint32_t x = __shfl_sync(0xffffffffu, k, j);
+      at += (x < k || (x == k && j < lane)) ? 1u : 0u;
+    }
+    if (lane < n)
+      for (uint32_t c = 0; c < g.ncols; ++c) g.out[c][at] = g.in[c][lane];
+    return;
+  }
+  constexpr int kEach = kSortSmall / kBlock;
+  __shared__ __align__(16) uint32_t s_key[kSortSmall];
+  const SegRows& g = segs[by_block[blockIdx.x - warp_blocks]];
+  const uint32_t n = static_cast<uint32_t>(g.n), tid = threadIdx.x;
+  const uint32_t* col0 = g.in[0];
+  uint32_t k[kEach], at[kEach];
+#pragma unroll
+  for (int q = 0; q < kEach; ++q) {
+    const uint32_t r = q * kBlock + tid;
+    k[q] = r < n ? col0[r] : 0u;
+    s_key[r] = k[q];
+    at[q] = 0;
+  }
+  __syncthreads();
+  for (uint32_t j = 0; j < n; ++j) {
+    const uint32_t x = s_key[j];
+#pragma unroll
+    for (int q = 0; q < kEach; ++q) at[q] += (x < k[q] || (x == k[q] && j < q * kBlock + tid)) ? 1u : 0u;
+  }
+  for (uint32_t c = 0; c < g.ncols; ++c) {
+    const uint32_t* in = g.in[c];
+    uint32_t* out = g.out[c];
+#pragma unroll
+    for (int q = 0; q < kEach; ++q)
+      if (q * kBlock + tid < n) out[at[q]] = in[q * kBlock + tid];
   }
 }
 
@@ -246,8 +359,8 @@ struct JoinSeg {
 // One block per tile of kJcTile left keys of one join, tiles taken in ticket
 // order (the tile's join from a per-tile table, one load instead of a search
 // of the join starts).  The tile's match counts stay in registers (the
-// right-key window, found beforehand by jc_window_kernel, is staged by a bulk
-// copy when it fits); their block scan
+// right-key window, found beforehand by jc_window_kernel where there are more
+// tiles than run at a time, is staged by a bulk copy when it fits); their block scan
 // and a segmented decoupled look-back over the join's earlier tiles give
 // every left key its output offset directly, and the join's last tile writes
 // its total.
@@ -325,14 +438,27 @@ __global__ void __launch_bounds__(kJcBlock, 4) bjoin_count_scan_kernel(
   __shared__ uint64_t s_scan[kJcBlock / 32 + 1];
   __shared__ uint64_t s_b;
   __shared__ uint32_t s_tile, s_j;
-  if (threadIdx.x == 0) {
-    // the window is known: its bulk copy starts before the block's first barrier
-    const uint32_t t = atomicAdd(ticket, 1u);
+  if (threadIdx.x < 32) {
+    // the window's bulk copy starts before the block's first barrier
+    uint32_t t = 0;
+    if (threadIdx.x == 0) t = atomicAdd(ticket, 1u);
+    t = __shfl_sync(0xffffffffu, t, 0);
     const uint32_t jj = tile_join[t];
-    const uint2 w = win[t];
-    s_tile = t;
-    s_j = jj;
-    jc_issue_window(js[jj].rk, w.x, w.y, sm);
+    uint64_t w0, w1;
+    if (win) {
+      const uint2 w = win[t];
+      w0 = w.x;
+      w1 = w.y;
+    } else {   // few tiles: found here
+      const uint64_t b = (t - bstart[jj]) * static_cast<uint64_t>(kJcTile);
+      const uint64_t e = (b + kJcTile < js[jj].nl ? b + kJcTile : js[jj].nl) - 1;
+      warp_window(js[jj].rk, js[jj].nr, js[jj].lk[b], js[jj].lk[e], w0, w1);
+    }
+    if (threadIdx.x == 0) {
+      s_tile = t;
+      s_j = jj;
+      jc_issue_window(js[jj].rk, w0, w1, sm);
+    }
   }
   __syncthreads();
   const uint64_t tile = s_tile;
@@ -357,8 +483,25 @@ __global__ void __launch_bounds__(kJcBlock, 4) bjoin_count_scan_kernel(
 // Their list (small, nsmall of them; nsmall_dev when on the device) holds no
 // tiles.
 
+// What the host reads of a wave's written joins (page-locked memory): column
+// 0's first and last value of join j at fl[2j], fl[2j + 1], and the whole
+// column 0 of an output with 2 < rows < kSmallC0Words at stage + slot[j] *
+// kSmallC0Words where slot[j] >= 0.  Each word is stored by the thread that
+// wrote the row.
+struct JoinEdges {
+  uint32_t* fl;
+  const int32_t* slot;   // nullable
+  uint32_t* stage;
+};
+
+__device__ __forceinline__ uint32_t* edge_stage(const JoinEdges& ed, uint32_t j, uint64_t total) {
+  if (!ed.slot || total <= 2 || total >= kSmallC0Words) return nullptr;
+  const int32_t s = ed.slot[j];
+  return s < 0 ? nullptr : ed.stage + static_cast<uint64_t>(s) * kSmallC0Words;
+}
+
 __device__ __forceinline__ void write_small_join(const JoinOut* __restrict__ src, JoinOut* jp, uint64_t* s_off,
-                                                 uint32_t* s_lo) {
+                                                 uint32_t* s_lo, uint32_t j, const JoinEdges& ed) {
   const uint32_t lane = lane_id();
   // the join's description in the warp's shared slot: the row loop reads its
   // column pointers from shared memory
@@ -377,6 +520,7 @@ __device__ __forceinline__ void write_small_join(const JoinOut* __restrict__ src
   }
   __syncwarp();
   const uint32_t nlc = jp->nlc, nrc = jp->nrc;
+  uint32_t* stage = edge_stage(ed, j, total);
   for (uint64_t k = lane; k < total; k += 32) {
     uint32_t a = 0, b = static_cast<uint32_t>(nl);   // last p with s_off[p] <= k
     while (b - a > 1) {
@@ -386,67 +530,108 @@ __device__ __forceinline__ void write_small_join(const JoinOut* __restrict__ src
     }
     const uint64_t jj = s_lo[a] + (k - s_off[a]);
     copy_join_row(jp->oc, jp->lc, nlc, jp->rc, nrc, a, jj, k);
+    const uint32_t key = jp->oc[0][k];
+    if (k == 0) ed.fl[2 * j] = key;
+    if (k == total - 1) ed.fl[2 * j + 1] = key;
+    if (stage) stage[k] = key;
   }
   __syncwarp();   // the slice is free for the warp's next join
 }
 
-// Every output tile's left rows [x, y): x the last row whose output starts
-// at or before the tile's first row, y the first row whose output starts
-// after its last (one warp per tile, both searches at once), so that the
-// writing blocks start staging at once.  T as for bjoin_write_kernel.
+// The join of an output tile: the last one whose tiles start at or before it
+// (every lane of the warp calls it).
+__device__ __forceinline__ uint32_t tile_join_of(const uint64_t* __restrict__ ostart, uint32_t J, uint64_t tile) {
+  return static_cast<uint32_t>(warp_bound<true, uint64_t>(ostart, 0, static_cast<uint64_t>(J) + 1, tile) - 1);
+}
+
+// Every output tile's left rows [x, y) and join z: x the last row whose output
+// starts at or before the tile's first row, y the first row whose output
+// starts after its last (one warp per tile, both searches at once), so that
+// the writing blocks start staging at once.  T as for bjoin_write_kernel.
 __global__ void __launch_bounds__(kBlock) jw_range_kernel(const JoinOut* __restrict__ jo,
-                                                          const uint64_t* __restrict__ ostart,
-                                                          const uint32_t* __restrict__ tile_join, uint64_t T_host,
-                                                          const uint64_t* ostart_end, uint2* __restrict__ ranges) {
+                                                          const uint64_t* __restrict__ ostart, uint32_t J,
+                                                          uint64_t T_host, const uint64_t* ostart_end,
+                                                          uint4* __restrict__ ranges) {
   const uint64_t T = ostart_end ? *ostart_end : T_host;
   const uint64_t nw = static_cast<uint64_t>(gridDim.x) * (kBlock / 32);
   for (uint64_t t = static_cast<uint64_t>(blockIdx.x) * (kBlock / 32) + (threadIdx.x >> 5); t < T; t += nw) {
-    const uint32_t jn = tile_join[t];
+    const uint32_t jn = tile_join_of(ostart, J, t);
     const uint64_t total = jo[jn].total, nl = jo[jn].nl;
     const uint64_t kb = (t - ostart[jn]) * static_cast<uint64_t>(kTileRows);
     const uint64_t kend = (kb + kTileRows < total) ? kb + kTileRows : total;
     uint64_t a, b;
     warp_bound_pair<true, true, uint64_t>(jo[jn].offs, nl, kb, kend - 1, a, b);
-    if ((threadIdx.x & 31) == 0) ranges[t] = make_uint2(static_cast<uint32_t>(a - 1), static_cast<uint32_t>(b));
+    if ((threadIdx.x & 31) == 0)
+      ranges[t] = make_uint4(static_cast<uint32_t>(a - 1), static_cast<uint32_t>(b), jn, 0u);
   }
 }
 
+// Ranges come from jw_range_kernel, or (null: few tiles are expected) warp 0
+// finds each tile's join and left rows.
 __global__ void __launch_bounds__(kBlock, 5) bjoin_write_kernel(const JoinOut* __restrict__ jo,
-                                                             const uint64_t* __restrict__ ostart,
-                                                             const uint32_t* __restrict__ tile_join,
-                                                             const uint2* __restrict__ ranges,
+                                                             const uint64_t* __restrict__ ostart, uint32_t J,
+                                                             const uint4* __restrict__ ranges,
                                                              uint64_t T_host, const uint64_t* ostart_end,
                                                              const uint32_t* __restrict__ small, uint32_t nsmall_host,
-                                                             const uint32_t* nsmall_dev) {
+                                                             const uint32_t* nsmall_dev, JoinEdges ed) {
   constexpr int kStage = kTileRows + 1;
+  static_assert(kBlock == kJwBlock, "jw_write_tile's block");
   static_assert(kStage >= (kBlock / 32) * kSmallJoin, "a warp's slice holds a small join's left rows");
   __shared__ JoinOut s_o;
   __shared__ JoinOut s_w[kBlock / 32];
   __shared__ uint64_t s_off[kStage];
   __shared__ uint32_t s_lo[kStage];
+  __shared__ uint32_t s_j;
+  __shared__ uint64_t s_range[2];
   {
     const uint32_t nsm = nsmall_dev ? *nsmall_dev : nsmall_host;
     const uint32_t warp = threadIdx.x >> 5, nwarps = kBlock / 32;
     for (uint64_t w = static_cast<uint64_t>(blockIdx.x) * nwarps + warp; w < nsm;
          w += static_cast<uint64_t>(gridDim.x) * nwarps)
-      write_small_join(&jo[small[w]], &s_w[warp], s_off + warp * kSmallJoin, s_lo + warp * kSmallJoin);
+      write_small_join(&jo[small[w]], &s_w[warp], s_off + warp * kSmallJoin, s_lo + warp * kSmallJoin, small[w], ed);
   }
   const uint64_t T = ostart_end ? *ostart_end : T_host;
 #pragma unroll 1
   for (uint64_t tile = blockIdx.x; tile < T; tile += gridDim.x) {
     __syncthreads();   // the previous tile's readers of the shared arrays are done
-    const uint32_t jn = tile_join[tile];
-    const uint2 rg = ranges[tile];
-    const uint64_t tile0 = ostart[jn];
+    if (threadIdx.x < 32) {
+      uint32_t j;
+      uint64_t a, b;
+      if (ranges) {
+        const uint4 rg = ranges[tile];
+        j = rg.z;
+        a = rg.x;
+        b = rg.y;
+      } else {
+        j = tile_join_of(ostart, J, tile);
+        const uint64_t kb = (tile - ostart[j]) * static_cast<uint64_t>(kTileRows), tot = jo[j].total;
+        warp_bound_pair<true, true, uint64_t>(jo[j].offs, jo[j].nl, kb, (kb + kTileRows < tot ? kb + kTileRows : tot) - 1,
+                                              a, b);
+        --a;
+      }
+      if (threadIdx.x == 0) {
+        s_j = j;
+        s_range[0] = a;
+        s_range[1] = b;
+      }
+    }
+    __syncthreads();
+    const uint32_t jn = s_j;
     {
       const uint32_t* src = reinterpret_cast<const uint32_t*>(&jo[jn]);
       uint32_t* dst = reinterpret_cast<uint32_t*>(&s_o);
       for (uint32_t w = threadIdx.x; w < sizeof(JoinOut) / 4; w += kBlock) dst[w] = src[w];
     }
     __syncthreads();
-    const uint64_t kb = (tile - tile0) * static_cast<uint64_t>(kTileRows);
-    const uint64_t kend = (kb + kTileRows < s_o.total) ? kb + kTileRows : s_o.total;
-    jw_write_tile<kRows>(s_o, kb, kend, rg.x, rg.y, s_off, s_lo);
+    const uint64_t total = s_o.total;
+    const uint64_t kb = (tile - ostart[jn]) * static_cast<uint64_t>(kTileRows);
+    const uint64_t kend = (kb + kTileRows < total) ? kb + kTileRows : total;
+    jw_write_tile<kRows>(s_o, kb, kend, s_range[0], s_range[1], s_off, s_lo);
+    const uint32_t* c0 = s_o.oc[0];
+    if (kb == 0 && threadIdx.x == 0) ed.fl[2 * jn] = c0[0];
+    if (kend == total && threadIdx.x == (total - 1 - kb) % kBlock) ed.fl[2 * jn + 1] = c0[total - 1];
+    uint32_t* stage = edge_stage(ed, jn, total);
+    if (stage && threadIdx.x < total) stage[threadIdx.x] = c0[threadIdx.x];
   }
 }
 
@@ -471,89 +656,61 @@ struct JoinPlace {
   uint32_t* small;       // joins whose outputs are written one per warp (written)
   uint32_t* nsmall;      // their number (written)
   uint32_t small_rows;   // outputs of at most this many rows are small
+  uint64_t* totals_host; // page-locked: every join's rows,
+  uint64_t* bump_host;   // the bump after the wave
+  DeviceErrors* err_host;   // and the error record after the count
+  const DeviceErrors* err;
 };
 
 __global__ void __launch_bounds__(kPlaceBlock) join_place_kernel(JoinOut* __restrict__ jo,
                                                                  const uint64_t* __restrict__ totals, uint32_t J,
                                                                  JoinPlace pl) {
   __shared__ uint64_t s_scan[kPlaceBlock / 32 + 1];
+  __shared__ unsigned long long s_fit;   // end of the placed outputs, after the bump
   const uint64_t bump0 = *pl.bump;
-  uint64_t carry_b = 0, carry_t = 0, carry_s = 0, fit_b = 0;
+  // a look-back that gave up leaves the totals and offsets wrong: nothing is
+  // written then, and the host raises the error
+  const DeviceErrors e = *pl.err;
+  if (threadIdx.x == 0) s_fit = 0;
+  uint64_t carry_b = 0, carry_t = 0, carry_s = 0;
   for (uint32_t c0 = 0; c0 < J; c0 += kPlaceBlock) {
     const uint32_t j = c0 + threadIdx.x;
-    const uint64_t t = j < J ? totals[j] : 0;
+    const uint64_t t = j < J && !e.timeout ? totals[j] : 0;
     const uint32_t ncols = j < J ? jo[j].nlc + jo[j].nrc : 0;
     const uint64_t stride = place_stride(t);
     const uint64_t bytes = t ? ncols * stride : 0;
-    uint64_t tot_b, tot_t, fb_sum;
+    uint64_t tot_b, tot_ts;
     const uint64_t eb = block_excl_scan64<kPlaceBlock>(bytes, tot_b, s_scan);
     const uint64_t off = bump0 + carry_b + eb;
     const bool fits = off + bytes <= pl.cap;
     const bool is_small = fits && t > 0 && t <= pl.small_rows && j < J && jo[j].nl <= kSmallJoin;
     const uint64_t tiles = (fits && t && !is_small) ? div_up(t, kTileRows) : 0;
-    const uint64_t et = block_excl_scan64<kPlaceBlock>(tiles, tot_t, s_scan);
-    (void)block_excl_scan64<kPlaceBlock>(fits ? bytes : 0, fb_sum, s_scan);
-    uint64_t tot_s;
-    const uint64_t es = block_excl_scan64<kPlaceBlock>(is_small ? 1 : 0, tot_s, s_scan);
+    // tiles above bit 11, small outputs (at most kPlaceBlock < 2^11) below
+    static_assert(kPlaceBlock < (1 << 11), "a chunk's small outputs fit 11 bits");
+    const uint64_t ets = block_excl_scan64<kPlaceBlock>((tiles << 11) | (is_small ? 1 : 0), tot_ts, s_scan);
     if (j < J) {
       JoinOut& o = jo[j];
+      pl.totals_host[j] = t;
       o.total = fits ? t : 0;
       for (uint32_t c = 0; c < VG_MAX_COLS; ++c)
         o.oc[c] = (fits && t && c < ncols) ? reinterpret_cast<uint32_t*>(pl.base + off + c * stride) : nullptr;
-      pl.ostart[j] = carry_t + et;
-      if (is_small) pl.small[carry_s + es] = j;
+      pl.ostart[j] = carry_t + (ets >> 11);
+      if (is_small) pl.small[carry_s + (ets & 2047)] = j;
+      // what fits is a prefix of the joins with rows: its end is their sum
+      if (fits) atomicMax(&s_fit, static_cast<unsigned long long>(carry_b + eb + bytes));
     }
     carry_b += tot_b;
-    carry_t += tot_t;
-    carry_s += tot_s;
-    fit_b += fb_sum;
+    carry_t += tot_ts >> 11;
+    carry_s += tot_ts & 2047;
   }
+  __syncthreads();
   if (threadIdx.x == 0) {
     pl.ostart[J] = carry_t;
     *pl.nsmall = static_cast<uint32_t>(carry_s);
-    *pl.bump = bump0 + fit_b;
+    *pl.bump = bump0 + s_fit;
+    *pl.bump_host = bump0 + s_fit;
+    *pl.err_host = e;
   }
-}
-
-// tile_join[ostart[j] .. ostart[j + 1]) = j.
-__global__ void tile_join_fill_kernel(const uint64_t* __restrict__ ostart, uint32_t J,
-                                      uint32_t* __restrict__ tile_join) {
-  for (uint32_t j = blockIdx.x; j < J; j += gridDim.x)
-    for (uint64_t t = ostart[j] + threadIdx.x; t < ostart[j + 1]; t += blockDim.x) tile_join[t] = j;
-}
-
-// After a placed write, one warp per join: lane 0 writes the output's first
-// and last key; when the join has a stage slot (its host-side completion
-// scans column 0 for empty intervals) and a small output (2 < rows <
-// kSmallC0Words), the warp copies that column 0 into the slot's
-// kSmallC0Words-word stage.
-__global__ void __launch_bounds__(kBlock) join_edges_kernel(const JoinOut* __restrict__ jo, uint32_t J,
-                                                            uint32_t* __restrict__ fl,
-                                                            const int32_t* __restrict__ slot,
-                                                            uint32_t* __restrict__ stage) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint64_t nw = static_cast<uint64_t>(gridDim.x) * (kBlock / 32);
-  for (uint64_t j = static_cast<uint64_t>(blockIdx.x) * (kBlock / 32) + (threadIdx.x >> 5); j < J; j += nw) {
-    const uint64_t t = jo[j].total;
-    if (t == 0) continue;
-    const uint32_t* c0 = jo[j].oc[0];
-    if (lane == 0) {
-      fl[2 * j] = c0[0];
-      fl[2 * j + 1] = c0[t - 1];
-    }
-    const int32_t sl = slot ? slot[j] : -1;
-    if (sl < 0 || t <= 2 || t >= kSmallC0Words) continue;
-    for (uint32_t i = lane; i < t; i += 32) stage[static_cast<uint64_t>(sl) * kSmallC0Words + i] = c0[i];
-  }
-}
-
-__global__ void first_last_kernel(const JoinOut* __restrict__ jo, uint32_t J, uint32_t* __restrict__ fl) {
-  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= J) return;
-  const JoinOut& o = jo[j];
-  if (o.total == 0) return;
-  fl[2 * j] = o.oc[0][0];
-  fl[2 * j + 1] = o.oc[0][o.total - 1];
 }
 
 struct Col0Req {
@@ -601,16 +758,14 @@ void batched_copy(Ctx& ctx, const std::vector<CopyPiece>& pieces) {
       tile_piece[t] = k;
     }
   }
-  CopyPiece* dp = upload(ctx, p);
-  uint64_t* dc = upload(ctx, cstart);
-  uint32_t* dtp = upload(ctx, tile_piece);
+  Tables tb(ctx);
+  const size_t op = tb.add(p), oc = tb.add(cstart), ot = tb.add(tile_piece);
+  tb.send();
   ctx.launch("select_copy", bytes, [&] {
-    bcopy_kernel<<<grid_cap(ctx, cstart.back(), kCopyPer), kBlock, 0, ctx.stream>>>(dp, dc, P, dtp, ntiles);
+    bcopy_kernel<<<grid_cap(ctx, cstart.back(), kCopyPer), kBlock, 0, ctx.stream>>>(
+        tb.at<CopyPiece>(op), tb.at<uint64_t>(oc), P, tb.at<uint32_t>(ot), ntiles);
   });
   VG_CUDA(cudaGetLastError());
-  ctx.free(dp);
-  ctx.free(dc);
-  ctx.free(dtp);
 }
 
 void batched_unique_enqueue(Ctx& ctx, const std::vector<SegRows>& segs, uint64_t* counts_host) {
@@ -624,36 +779,26 @@ void batched_unique_enqueue(Ctx& ctx, const std::vector<SegRows>& segs, uint64_t
     if (is_small) small.push_back(s);
     tstart[s + 1] = tstart[s] + (is_small ? 0 : div_up(segs[s].n, kTileRows));
     bytes += 4.0 * segs[s].n * segs[s].ncols;
+    counts_host[s] = 0;   // the kernel stores the others' counts
   }
   const uint64_t tiles = tstart[S];
   const uint32_t nsmall = static_cast<uint32_t>(small.size());
   const uint32_t small_blocks = static_cast<uint32_t>(div_up(nsmall, kBlock / 32));
-  if (tiles == 0 && nsmall == 0) {
-    for (uint32_t s = 0; s < S; ++s) counts_host[s] = 0;
-    return;
-  }
+  if (tiles == 0 && nsmall == 0) return;
   std::vector<uint32_t> tile_seg(tiles);
   for (uint32_t s = 0; s < S; ++s)
     for (uint64_t t = tstart[s]; t < tstart[s + 1]; ++t) tile_seg[t] = s;
-  SegRows* ds = upload(ctx, segs);
-  uint64_t* dt = upload(ctx, tstart);
-  uint32_t* dts = upload(ctx, tile_seg);
-  uint32_t* dsm = upload(ctx, small);
-  Scratch<uint64_t> status(ctx, tiles), dcount(ctx, S);
-  Scratch<uint32_t> ticket(ctx, 1);
-  VG_CUDA(cudaMemsetAsync(status.get(), 0, tiles * sizeof(uint64_t), ctx.stream));
-  VG_CUDA(cudaMemsetAsync(dcount.get(), 0, S * sizeof(uint64_t), ctx.stream));
-  VG_CUDA(cudaMemsetAsync(ticket.get(), 0, sizeof(uint32_t), ctx.stream));
+  Tables tb(ctx);
+  const size_t og = tb.add(segs), ot = tb.add(tstart), os = tb.add(tile_seg), om = tb.add(small);
+  const size_t oz = tb.zeros<uint64_t>(tiles + 1);   // look-back words, then the ticket
+  tb.send();
+  uint64_t* status = tb.at<uint64_t>(oz);
   ctx.launch("unique_compact", bytes, [&] {
     bunique_kernel<<<static_cast<unsigned>(small_blocks + tiles), kBlock, 0, ctx.stream>>>(
-        ds, dt, dts, dsm, nsmall, small_blocks, status.get(), ticket.get(), dcount.get(), ctx.d_err);
+        tb.at<SegRows>(og), tb.at<uint64_t>(ot), tb.at<uint32_t>(os), tb.at<uint32_t>(om), nsmall, small_blocks,
+        status, reinterpret_cast<uint32_t*>(status + tiles), counts_host, ctx.d_err);
   });
   VG_CUDA(cudaGetLastError());
-  VG_CUDA(cudaMemcpyAsync(counts_host, dcount.get(), S * sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx.stream));
-  ctx.free(ds);
-  ctx.free(dt);
-  ctx.free(dts);
-  ctx.free(dsm);
 }
 
 void note_unique_writes(Ctx& ctx, const std::vector<SegRows>& segs, const uint64_t* counts) {
@@ -662,35 +807,69 @@ void note_unique_writes(Ctx& ctx, const std::vector<SegRows>& segs, const uint64
   ctx.add_bytes("unique_compact", wb);
 }
 
-std::vector<uint64_t> batched_unique(Ctx& ctx, const std::vector<SegRows>& segs) {
-  std::vector<uint64_t> counts(segs.size(), 0);
-  if (segs.empty()) return counts;
-  PinnedWords h(ctx);
-  batched_unique_enqueue(ctx, segs, h.reserve(segs.size()));
-  ctx.sync();
-  std::copy(h.data(), h.data() + segs.size(), counts.begin());
-  note_unique_writes(ctx, segs, counts.data());
-  return counts;
+namespace {
+
+// The relations' rows with newly allocated output columns.
+std::vector<SegRows> sort_segments(Ctx& ctx, const std::vector<Rel*>& rels) {
+  std::vector<SegRows> segs(rels.size());
+  parallel_for(rels.size(), [&](size_t s) {
+    segs[s].ncols = rels[s]->ncols;
+    segs[s].n = rels[s]->nrows;
+    for (uint32_t c = 0; c < rels[s]->ncols; ++c) {
+      segs[s].in[c] = rels[s]->cols[c];
+      segs[s].out[c] = ctx.alloc<uint32_t>(rels[s]->nrows);
+    }
+  });
+  return segs;
 }
 
+void take_sorted(Ctx& ctx, const std::vector<Rel*>& rels, const std::vector<SegRows>& segs) {
+  parallel_for(rels.size(), [&](size_t s) {
+    for (uint32_t c = 0; c < rels[s]->ncols; ++c) {
+      rel_drop_col(ctx, *rels[s], c);
+      rels[s]->cols[c] = segs[s].out[c];
+    }
+  });
+}
+
+// Relations of at most kSortSmall rows: one launch.
+void sort_small(Ctx& ctx, const std::vector<Rel*>& rels) {
+  const uint32_t S = static_cast<uint32_t>(rels.size());
+  if (S == 0) return;
+  const std::vector<SegRows> segs = sort_segments(ctx, rels);
+  std::vector<uint32_t> by_warp, by_block;
+  double bytes = 0;
+  for (uint32_t s = 0; s < S; ++s) {
+    (segs[s].n <= kSortWarp ? by_warp : by_block).push_back(s);
+    bytes += 8.0 * segs[s].n * segs[s].ncols;
+  }
+  Tables tb(ctx);
+  const size_t og = tb.add(segs), ow = tb.add(by_warp), ob = tb.add(by_block);
+  tb.send();
+  const uint32_t warp_blocks = static_cast<uint32_t>(div_up(by_warp.size(), kBlock / 32));
+  ctx.launch("sort_small", bytes, [&] {
+    sort_small_kernel<<<warp_blocks + static_cast<unsigned>(by_block.size()), kBlock, 0, ctx.stream>>>(
+        tb.at<SegRows>(og), tb.at<uint32_t>(ow), static_cast<uint32_t>(by_warp.size()), tb.at<uint32_t>(ob),
+        warp_blocks);
+  });
+  VG_CUDA(cudaGetLastError());
+  take_sorted(ctx, rels, segs);
+}
+
+}  // namespace
+
 void batched_sort_by_first(Ctx& ctx, const std::vector<Rel*>& rels_in, int key_bits) {
-  std::vector<Rel*> rels;
+  std::vector<Rel*> rels, small;
   for (Rel* r : rels_in)
-    if (r->nrows > 1 && r->ncols > 0) rels.push_back(r);
+    if (r->nrows > 1 && r->ncols > 0) (r->nrows <= kSortSmall ? small : rels).push_back(r);
+  sort_small(ctx, small);
   const uint32_t S = static_cast<uint32_t>(rels.size());
   if (S == 0) return;
   std::vector<uint64_t> rstart(S + 1, 0);
-  std::vector<const uint32_t*> col0(S);
-  for (uint32_t s = 0; s < S; ++s) {
-    rstart[s + 1] = rstart[s] + rels[s]->nrows;
-    col0[s] = rels[s]->cols[0];
-  }
+  for (uint32_t s = 0; s < S; ++s) rstart[s + 1] = rstart[s] + rels[s]->nrows;
   const uint64_t N = rstart[S];
   if (N > 0xFFFFFFFFull) fail(VG_ERR_OVERFLOW, "batched sort is limited to 2^32 rows");
-  const bool known = key_bits > 0 && key_bits <= 32;
-  const int kb = known ? key_bits : 32;
-  uint64_t* drs = upload(ctx, rstart);
-  const uint32_t** dc0 = upload(ctx, col0);
+  const int kb = key_bits > 0 && key_bits <= 32 ? key_bits : 32;
   // each chunk's first segment
   const uint64_t nchunks = div_up(N, static_cast<uint64_t>(kChunkRows));
   std::vector<uint32_t> chunk_seg(nchunks);
@@ -702,64 +881,73 @@ void batched_sort_by_first(Ctx& ctx, const std::vector<Rel*>& rels_in, int key_b
       chunk_seg[c] = sg;
     }
   }
-  uint32_t* dcs = upload(ctx, chunk_seg);
   const unsigned cgrid = static_cast<unsigned>(std::min<uint64_t>(nchunks, static_cast<uint64_t>(ctx.num_sms) * 8));
-  uint64_t* keys = ctx.alloc<uint64_t>(N);
-  uint64_t* keys_alt = ctx.alloc<uint64_t>(N);
-  uint32_t* vals = ctx.alloc<uint32_t>(N);
-  uint32_t* vals_alt = ctx.alloc<uint32_t>(N);
-  ctx.launch("sort_keys", 12.0 * N, [&] {
-    composite_keys_kernel<<<cgrid, kBlock, 0, ctx.stream>>>(dc0, drs, S, dcs, nchunks, static_cast<uint32_t>(kb),
-                                                            keys);
-  });
-  VG_CUDA(cudaGetLastError());
-  // with the key width known the passes are fixed and nothing waits on the device
-  const bool alt = radix_sort_u64(ctx, keys, keys_alt, vals, vals_alt, N, kb + bits_for_segments(S), true, !known);
-  uint32_t* perm = alt ? vals_alt : vals;
-  ctx.free(keys);
-  ctx.free(keys_alt);
-  std::vector<SegRows> segs(S);
+  Scratch<uint32_t> vals(ctx, N), vals_alt(ctx, N);
+  std::vector<RadixDigit> digits;
+  radix_plan(digits, 0, kb + bits_for_segments(S));
+  DigitList dl{};
+  dl.n = static_cast<uint32_t>(digits.size());
+  for (uint32_t d = 0; d < dl.n; ++d) dl.d[d] = digits[d];
+  std::vector<const uint32_t*> col0(S);
+  for (uint32_t s = 0; s < S; ++s) col0[s] = rels[s]->cols[0];
+  Tables tb(ctx);
+  const size_t okey = tb.add(col0), orow = tb.add(rstart), oc = tb.add(chunk_seg);
+  tb.send();
+  bool alt;
+  {
+    Scratch<uint64_t> keys(ctx, N), keys_alt(ctx, N);
+    const RadixCounts counts(ctx, dl);
+    ctx.launch("sort_keys", 12.0 * N, [&] {
+      composite_keys_kernel<<<cgrid, kBlock, dl.n * kRadixValues * sizeof(uint32_t), ctx.stream>>>(
+          tb.at<const uint32_t*>(okey), tb.at<uint64_t>(orow), S, tb.at<uint32_t>(oc), nchunks,
+          static_cast<uint32_t>(kb), keys.get(), dl, counts.hist(), counts.bases(), counts.done());
+    });
+    VG_CUDA(cudaGetLastError());
+    // the passes are fixed by the key width and nothing waits on the device
+    std::vector<const uint64_t*> bases;
+    for (uint32_t d = 0; d < dl.n; ++d) bases.push_back(counts.bases(d));
+    alt = radix_sort_u64_counted(ctx, keys.get(), keys_alt.get(), vals.get(), vals_alt.get(), N, digits, bases, true);
+  }
+  const uint32_t* perm = alt ? vals_alt.get() : vals.get();
+  const std::vector<SegRows> segs = sort_segments(ctx, rels);
   double bytes = 4.0 * N;
   for (uint32_t s = 0; s < S; ++s) bytes += 8.0 * rels[s]->nrows * rels[s]->ncols;
-  parallel_for(S, [&](size_t s) {
-    segs[s].ncols = rels[s]->ncols;
-    segs[s].n = rels[s]->nrows;
-    for (uint32_t c = 0; c < rels[s]->ncols; ++c) {
-      segs[s].in[c] = rels[s]->cols[c];
-      segs[s].out[c] = ctx.alloc<uint32_t>(rels[s]->nrows);
-    }
-  });
-  SegRows* dsg = upload(ctx, segs);
+  Tables tg(ctx);
+  const size_t og = tg.add(segs);
+  tg.send();
   ctx.launch("gather", bytes, [&] {
-    seg_gather_kernel<<<cgrid, kBlock, 0, ctx.stream>>>(dsg, drs, S, dcs, nchunks, perm);
+    seg_gather_kernel<<<cgrid, kBlock, 0, ctx.stream>>>(tg.at<SegRows>(og), tb.at<uint64_t>(orow), S,
+                                                        tb.at<uint32_t>(oc), nchunks, perm);
   });
   VG_CUDA(cudaGetLastError());
-  parallel_for(S, [&](size_t s) {
-    for (uint32_t c = 0; c < rels[s]->ncols; ++c) {
-      rel_drop_col(ctx, *rels[s], c);
-      rels[s]->cols[c] = segs[s].out[c];
-    }
-  });
-  ctx.free(vals);
-  ctx.free(vals_alt);
-  ctx.free(dsg);
-  ctx.free(drs);
-  ctx.free(dcs);
-  ctx.free(const_cast<uint32_t**>(dc0));
+  take_sorted(ctx, rels, segs);
 }
 
-void batched_join_count(Ctx& ctx, const std::vector<const Rel*>& l, const std::vector<const Rel*>& r, JoinBatch& jb,
-                        uint64_t* totals_host) {
+namespace {
+
+// Tiles of all joins of a wave above which the windows (and, by the left
+// rows, the output tiles' ranges) get kernels of their own: below, the blocks
+// all run at once and find their own in about the time of a launch.
+uint64_t window_tiles(const Ctx& ctx) { return 2ull * static_cast<uint64_t>(ctx.num_sms); }
+
+// The tables of a wave's join count (and what follows it in the same stage).
+struct CountTables {
+  size_t js, bstart, tile_join, small, zero;
+  uint32_t nsmall = 0, small_blocks = 0;
+  uint64_t T = 0, rows = 0;
+  double bytes = 0;
+};
+
+CountTables count_tables(Ctx& ctx, Tables& tb, const std::vector<const Rel*>& l, const std::vector<const Rel*>& r,
+                         JoinBatch& jb) {
+  CountTables ct;
   const uint32_t J = static_cast<uint32_t>(l.size());
   jb = JoinBatch();
   jb.J = J;
   jb.l = l;
   jb.r = r;
-  if (J == 0) return;
   std::vector<JoinSeg> js(J);
   std::vector<uint64_t> bstart(J + 1, 0);
-  uint64_t rows = 0;
-  double cbytes = 0;
   jb.row0.resize(J);
   std::vector<uint32_t> small;   // joins counted by one warp each
   for (uint32_t j = 0; j < J; ++j) {
@@ -767,55 +955,79 @@ void batched_join_count(Ctx& ctx, const std::vector<const Rel*>& l, const std::v
     if (l[j]->nrows > 0xFFFFFFFFull || r[j]->nrows > 0xFFFFFFFFull)
       fail(VG_ERR_OVERFLOW, "join inputs are limited to 2^32 rows");
     if (l[j]->ncols + r[j]->ncols - 1 > VG_MAX_COLS) fail(VG_ERR_UNSUPPORTED, "join output has more than 9 columns");
-    js[j] = {l[j]->cols[0], r[j]->cols[0], l[j]->nrows, r[j]->nrows, rows};
-    jb.row0[j] = rows;
-    rows += l[j]->nrows;
+    js[j] = {l[j]->cols[0], r[j]->cols[0], l[j]->nrows, r[j]->nrows, ct.rows};
+    jb.row0[j] = ct.rows;
+    ct.rows += l[j]->nrows;
     const bool is_small = l[j]->nrows <= std::min<uint32_t>(kSmallJoin, ctx.tune.join_small_rows);
     if (is_small) small.push_back(j);
     bstart[j + 1] = bstart[j] + (is_small ? 0 : div_up(l[j]->nrows, kJcTile));
-    cbytes += 4.0 * (l[j]->nrows + r[j]->nrows);
+    ct.bytes += 4.0 * (l[j]->nrows + r[j]->nrows);
   }
-  const uint32_t nsmall = static_cast<uint32_t>(small.size());
-  const uint32_t small_blocks = static_cast<uint32_t>(div_up(nsmall, kJcBlock / 32));
-  const uint64_t T = bstart[J];
-  if (T > 0x7FFFFFFFull) fail(VG_ERR_OVERFLOW, "batched join count: too many tiles");
-  std::vector<uint32_t> tile_join(T);
+  ct.T = bstart[J];
+  if (ct.T > 0x7FFFFFFFull) fail(VG_ERR_OVERFLOW, "batched join count: too many tiles");
+  ct.nsmall = static_cast<uint32_t>(small.size());
+  ct.small_blocks = static_cast<uint32_t>(div_up(ct.nsmall, kJcBlock / 32));
+  std::vector<uint32_t> tile_join(ct.T);
   for (uint32_t j = 0; j < J; ++j)
     for (uint64_t t = bstart[j]; t < bstart[j + 1]; ++t) tile_join[t] = j;
-  JoinSeg* djs = upload(ctx, js);
-  uint64_t* dbs = upload(ctx, bstart);
-  uint32_t* dtj = upload(ctx, tile_join);
-  uint32_t* dsm = upload(ctx, small);
-  jb.lo = ctx.alloc<uint32_t>(rows);
-  jb.offs = ctx.alloc<uint64_t>(rows);
-  uint64_t* status = ctx.alloc<uint64_t>(T);
-  uint64_t* totals = ctx.alloc<uint64_t>(J);
-  uint32_t* ticket = ctx.alloc<uint32_t>(1);
-  uint2* dwin = ctx.alloc<uint2>(T ? T : 1);
-  VG_CUDA(cudaMemsetAsync(status, 0, T * sizeof(uint64_t), ctx.stream));
-  VG_CUDA(cudaMemsetAsync(ticket, 0, sizeof(uint32_t), ctx.stream));
-  if (T) {
-    const uint64_t wblocks = std::min<uint64_t>(div_up(T, kJcBlock / 32), static_cast<uint64_t>(ctx.num_sms) * 8);
-    ctx.launch("join_windows", 8.0 * T, [&] {
-      jc_window_kernel<<<static_cast<unsigned>(wblocks), kJcBlock, 0, ctx.stream>>>(djs, dbs, dtj, T, dwin);
+  ct.js = tb.add(js);
+  ct.bstart = tb.add(bstart);
+  ct.tile_join = tb.add(tile_join);
+  ct.small = tb.add(small);
+  ct.zero = tb.zeros<uint64_t>(ct.T + 1);   // look-back words, then the ticket
+  return ct;
+}
+
+// Enqueues the count of the joins (tables sent): jb.lo, jb.offs and
+// jb.d_totals, which must hold J words.
+void launch_count(Ctx& ctx, const Tables& tb, const CountTables& ct, JoinBatch& jb) {
+  std::optional<Scratch<uint2>> win;
+  if (ct.T > window_tiles(ctx)) {
+    win.emplace(ctx, ct.T);
+    const uint64_t wblocks = std::min<uint64_t>(div_up(ct.T, kJcBlock / 32), static_cast<uint64_t>(ctx.num_sms) * 8);
+    ctx.launch("join_windows", 8.0 * ct.T, [&] {
+      jc_window_kernel<<<static_cast<unsigned>(wblocks), kJcBlock, 0, ctx.stream>>>(
+          tb.at<JoinSeg>(ct.js), tb.at<uint64_t>(ct.bstart), tb.at<uint32_t>(ct.tile_join), ct.T, win->get());
     });
     VG_CUDA(cudaGetLastError());
   }
-  ctx.launch("join_count_scan", cbytes + 12.0 * rows, [&] {
-    bjoin_count_scan_kernel<<<static_cast<unsigned>(small_blocks + T), kJcBlock, 0, ctx.stream>>>(
-        djs, dbs, dtj, dwin, dsm, nsmall, small_blocks, jb.lo, jb.offs, status, ticket, totals, ctx.d_err);
+  uint64_t* status = tb.at<uint64_t>(ct.zero);
+  ctx.launch("join_count_scan", ct.bytes + 12.0 * ct.rows, [&] {
+    bjoin_count_scan_kernel<<<static_cast<unsigned>(ct.small_blocks + ct.T), kJcBlock, 0, ctx.stream>>>(
+        tb.at<JoinSeg>(ct.js), tb.at<uint64_t>(ct.bstart), tb.at<uint32_t>(ct.tile_join), win ? win->get() : nullptr,
+        tb.at<uint32_t>(ct.small), ct.nsmall, ct.small_blocks, jb.lo, jb.offs, status,
+        reinterpret_cast<uint32_t*>(status + ct.T), jb.d_totals, ctx.d_err);
   });
   VG_CUDA(cudaGetLastError());
-  VG_CUDA(cudaMemcpyAsync(totals_host, totals, J * sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx.stream));
-  jb.d_totals = totals;   // for a device-side placement; released with lo and offs
-  // the stream orders every later use of these blocks after the kernel above
-  ctx.free(status);
-  ctx.free(ticket);
-  ctx.free(dwin);
-  ctx.free(djs);
-  ctx.free(dbs);
-  ctx.free(dtj);
-  ctx.free(dsm);
+}
+
+// Output descriptions without the output columns.
+void describe_join(const JoinBatch& jb, size_t j, JoinOut& o) {
+  const Rel* l = jb.l[j];
+  const Rel* r = jb.r[j];
+  std::memset(&o, 0, sizeof(o));
+  o.offs = jb.offs + jb.row0[j];
+  o.lo = jb.lo + jb.row0[j];
+  o.nl = l->nrows;
+  for (uint32_t c = 0; c < l->ncols; ++c) o.lc[c] = l->cols[c];
+  for (uint32_t c = 1; c < r->ncols; ++c) o.rc[c - 1] = r->cols[c];
+  o.nlc = l->ncols;
+  o.nrc = r->ncols - 1;
+}
+
+}  // namespace
+
+void batched_join_count(Ctx& ctx, const std::vector<const Rel*>& l, const std::vector<const Rel*>& r, JoinBatch& jb,
+                        uint64_t* totals_host) {
+  Tables tb(ctx);
+  const CountTables ct = count_tables(ctx, tb, l, r, jb);
+  if (jb.J == 0) return;
+  tb.send();
+  jb.lo = ctx.alloc<uint32_t>(ct.rows);
+  jb.offs = ctx.alloc<uint64_t>(ct.rows);
+  jb.d_totals = ctx.alloc<uint64_t>(jb.J);
+  launch_count(ctx, tb, ct, jb);
+  VG_CUDA(cudaMemcpyAsync(totals_host, jb.d_totals, jb.J * sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx.stream));
 }
 
 void batched_join_write(Ctx& ctx, JoinBatch& jb, const uint64_t* totals, std::vector<Rel>& out,
@@ -834,67 +1046,43 @@ void batched_join_write(Ctx& ctx, JoinBatch& jb, const uint64_t* totals, std::ve
     if (is_small) small.push_back(j);
     ostart[j + 1] = ostart[j] + (is_small ? 0 : div_up(rows(j), kTileRows));
     wbytes += 4.0 * rows(j) * (2.0 * (jb.l[j]->ncols + jb.r[j]->ncols - 1) - 1);
+    first_last_host[2 * j] = first_last_host[2 * j + 1] = 0;   // the kernel stores the others'
   }
   const uint32_t nsmall = static_cast<uint32_t>(small.size());
-  const uint64_t small_blocks = div_up(nsmall, kBlock / 32);
+  const uint64_t T = ostart[J], small_blocks = div_up(nsmall, kBlock / 32);
   // the outputs of a wave's joins are allocated and described on the host pool
   parallel_for(J, [&](size_t j) {
-    JoinOut& o = jo[j];
-    std::memset(&o, 0, sizeof(o));
+    std::memset(&jo[j], 0, sizeof(jo[j]));
     if (skip && skip[j]) return;                // written already: out[j] stays as it is
-    const Rel* l = jb.l[j];
-    const Rel* r = jb.r[j];
-    const uint32_t ncols = l->ncols + r->ncols - 1;
+    const uint32_t ncols = jb.l[j]->ncols + jb.r[j]->ncols - 1;
     out[j] = rel_alloc(ctx, ncols, totals[j]);
-    o.offs = jb.offs + jb.row0[j];
-    o.lo = jb.lo + jb.row0[j];
-    o.nl = l->nrows;
-    o.total = totals[j];
-    for (uint32_t c = 0; c < l->ncols; ++c) o.lc[c] = l->cols[c];
-    for (uint32_t c = 1; c < r->ncols; ++c) o.rc[c - 1] = r->cols[c];
-    for (uint32_t c = 0; c < ncols; ++c) o.oc[c] = out[j].cols[c];
-    o.nlc = l->ncols;
-    o.nrc = r->ncols - 1;
+    describe_join(jb, j, jo[j]);
+    jo[j].total = totals[j];
+    for (uint32_t c = 0; c < ncols; ++c) jo[j].oc[c] = out[j].cols[c];
   });
-  JoinOut* djo = upload(ctx, jo);
-  uint32_t* dfl = ctx.alloc<uint32_t>(2 * J);
-  VG_CUDA(cudaMemsetAsync(dfl, 0, 2 * J * sizeof(uint32_t), ctx.stream));
-  if (ostart[J] > 0 || nsmall > 0) {
-    if (ostart[J] > 0x7FFFFFFFull) fail(VG_ERR_OVERFLOW, "batched join write: too many tiles");
-    std::vector<uint32_t> tile_join(ostart[J]);
-    for (uint32_t j = 0; j < J; ++j)
-      for (uint64_t t = ostart[j]; t < ostart[j + 1]; ++t) tile_join[t] = j;
-    uint64_t* dos = upload(ctx, ostart);
-    uint32_t* dtj = upload(ctx, tile_join);
-    uint32_t* dsm = upload(ctx, small);
-    uint2* drg = ctx.alloc<uint2>(ostart[J] ? ostart[J] : 1);
-    if (ostart[J]) {
-      const uint64_t rblocks =
-          std::min<uint64_t>(div_up(ostart[J], kBlock / 32), static_cast<uint64_t>(ctx.num_sms) * 8);
-      ctx.launch("join_write_ranges", 8.0 * ostart[J], [&] {
-        jw_range_kernel<<<static_cast<unsigned>(rblocks), kBlock, 0, ctx.stream>>>(djo, dos, dtj, ostart[J], nullptr,
-                                                                                   drg);
+  if (T > 0 || nsmall > 0) {
+    if (T > 0x7FFFFFFFull) fail(VG_ERR_OVERFLOW, "batched join write: too many tiles");
+    Tables tb(ctx);
+    const size_t oj = tb.add(jo), os = tb.add(ostart), om = tb.add(small);
+    tb.send();
+    std::optional<Scratch<uint4>> ranges;
+    if (T > window_tiles(ctx)) {
+      ranges.emplace(ctx, T);
+      const uint64_t rblocks = std::min<uint64_t>(div_up(T, kBlock / 32), static_cast<uint64_t>(ctx.num_sms) * 8);
+      ctx.launch("join_write_ranges", 8.0 * T, [&] {
+        jw_range_kernel<<<static_cast<unsigned>(rblocks), kBlock, 0, ctx.stream>>>(
+            tb.at<JoinOut>(oj), tb.at<uint64_t>(os), J, T, nullptr, ranges->get());
       });
       VG_CUDA(cudaGetLastError());
     }
-    const unsigned grid = static_cast<unsigned>(std::max<uint64_t>(ostart[J], small_blocks));
+    const unsigned grid = static_cast<unsigned>(std::max<uint64_t>(T, small_blocks));
     ctx.launch("join_write", wbytes, [&] {
-      bjoin_write_kernel<<<grid, kBlock, 0, ctx.stream>>>(djo, dos, dtj, drg, ostart[J], nullptr, dsm, nsmall,
-                                                          nullptr);
+      bjoin_write_kernel<<<grid, kBlock, 0, ctx.stream>>>(
+          tb.at<JoinOut>(oj), tb.at<uint64_t>(os), J, ranges ? ranges->get() : nullptr, T, nullptr,
+          tb.at<uint32_t>(om), nsmall, nullptr, JoinEdges{first_last_host, nullptr, nullptr});
     });
     VG_CUDA(cudaGetLastError());
-    ctx.free(drg);
-    ctx.free(dos);
-    ctx.free(dtj);
-    ctx.free(dsm);
   }
-  ctx.launch("join_first_last", 8.0 * J, [&] {
-    first_last_kernel<<<static_cast<unsigned>(div_up(J, 128)), 128, 0, ctx.stream>>>(djo, J, dfl);
-  });
-  VG_CUDA(cudaGetLastError());
-  VG_CUDA(cudaMemcpyAsync(first_last_host, dfl, 2 * J * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx.stream));
-  ctx.free(dfl);
-  ctx.free(djo);
   jb.release(ctx);
 }
 
@@ -926,77 +1114,48 @@ uint64_t place_outputs_on_host(const JoinBatch& jb, const uint64_t* totals, cons
   return bump + fit;
 }
 
-void batched_join_place_write(Ctx& ctx, JoinBatch& jb, const Arena::Region* region, uint64_t* d_bump,
-                              const std::vector<int32_t>& c0_slot, uint32_t nslots, uint32_t* first_last_host,
-                              uint32_t* c0_host, uint64_t* bump_host) {
+void batched_join_placed(Ctx& ctx, const std::vector<const Rel*>& l, const std::vector<const Rel*>& r, JoinBatch& jb,
+                         const Arena::Region* region, uint64_t* d_bump, const std::vector<int32_t>& c0_slot,
+                         uint32_t nslots, const PlacedHost& host) {
+  Tables tb(ctx);
+  const CountTables ct = count_tables(ctx, tb, l, r, jb);
   const uint32_t J = jb.J;
   if (J == 0) return;
+  jb.lo = ctx.alloc<uint32_t>(ct.rows);
+  jb.offs = ctx.alloc<uint64_t>(ct.rows);
+  jb.d_totals = ctx.alloc<uint64_t>(J);
   std::vector<JoinOut> jo(J);
-  parallel_for(J, [&](size_t j) {
-    const Rel* l = jb.l[j];
-    const Rel* r = jb.r[j];
-    JoinOut& o = jo[j];
-    std::memset(&o, 0, sizeof(o));
-    o.offs = jb.offs + jb.row0[j];
-    o.lo = jb.lo + jb.row0[j];
-    o.nl = l->nrows;
-    for (uint32_t c = 0; c < l->ncols; ++c) o.lc[c] = l->cols[c];
-    for (uint32_t c = 1; c < r->ncols; ++c) o.rc[c - 1] = r->cols[c];
-    o.nlc = l->ncols;
-    o.nrc = r->ncols - 1;
-  });
-  JoinOut* djo = upload(ctx, jo);
-  int32_t* dslot = upload(ctx, c0_slot);
-  uint64_t* dos = ctx.alloc<uint64_t>(J + 1);
-  uint32_t* dsm = ctx.alloc<uint32_t>(J + 1);   // small list, then its length
-  // every placed output tile covers kTileRows rows of at least one 4-byte column
-  const uint64_t tile_cap = region->bytes / (4ull * kTileRows) + J + 1;
-  uint32_t* dtj = ctx.alloc<uint32_t>(tile_cap);
-  uint32_t* dfl = ctx.alloc<uint32_t>(2 * J);
-  uint32_t* dstage = ctx.alloc<uint32_t>(static_cast<uint64_t>(nslots ? nslots : 1) * kSmallC0Words);
-  VG_CUDA(cudaMemsetAsync(dfl, 0, 2 * J * sizeof(uint32_t), ctx.stream));
-  JoinPlace pl{region->begin, region->bytes, d_bump, dos, dsm, dsm + J, ctx.tune.write_small_rows};
+  parallel_for(J, [&](size_t j) { describe_join(jb, j, jo[j]); });
+  const size_t oj = tb.add(jo), oslot = tb.add(c0_slot);
+  tb.send();
+  launch_count(ctx, tb, ct, jb);
+  Scratch<uint64_t> ostart(ctx, J + 1);
+  Scratch<uint32_t> small(ctx, J + 1);   // small list, then its length
+  JoinOut* djo = tb.at<JoinOut>(oj);
+  const JoinPlace pl{region->begin, region->bytes, d_bump,        ostart.get(),   small.get(), small.get() + J,
+                     ctx.tune.write_small_rows,    host.totals, host.bump, host.err, ctx.d_err};
   ctx.launch("join_place", 16.0 * J, [&] {
     join_place_kernel<<<1, kPlaceBlock, 0, ctx.stream>>>(djo, jb.d_totals, J, pl);
   });
   VG_CUDA(cudaGetLastError());
-  const unsigned jgrid = static_cast<unsigned>(std::min<uint64_t>(J, static_cast<uint64_t>(ctx.num_sms) * 8));
-  ctx.launch("join_tile_map", 0.0, [&] { tile_join_fill_kernel<<<jgrid, 128, 0, ctx.stream>>>(dos, J, dtj); });
-  VG_CUDA(cudaGetLastError());
   // the tile count is on the device: fixed grids loop over the tiles (the
   // algorithmic bytes are added when the host reads the totals)
-  uint2* drg = ctx.alloc<uint2>(tile_cap);
-  ctx.launch("join_write_ranges", 0.0, [&] {
-    jw_range_kernel<<<static_cast<unsigned>(ctx.num_sms) * 8, kBlock, 0, ctx.stream>>>(djo, dos, dtj, 0, dos + J,
-                                                                                       drg);
-  });
-  VG_CUDA(cudaGetLastError());
-  ctx.launch("join_write", 0.0, [&] {
-    bjoin_write_kernel<<<static_cast<unsigned>(ctx.num_sms) * ctx.tune.write_blocks_per_sm, kBlock, 0,
-                         ctx.stream>>>(djo, dos, dtj, drg, 0, dos + J, dsm, 0, dsm + J);
-  });
-  VG_CUDA(cudaGetLastError());
-  {
-    const uint64_t eblocks = std::min<uint64_t>(div_up(J, kBlock / 32), static_cast<uint64_t>(ctx.num_sms) * 8);
-    ctx.launch("join_first_last", 8.0 * J + 8.0 * nslots * kSmallC0Words, [&] {
-      join_edges_kernel<<<static_cast<unsigned>(eblocks), kBlock, 0, ctx.stream>>>(djo, J, dfl,
-                                                                                   nslots ? dslot : nullptr, dstage);
+  std::optional<Scratch<uint4>> ranges;
+  if (ct.rows > kTileRows * window_tiles(ctx)) {
+    // every placed output tile covers kTileRows rows of at least one 4-byte column
+    ranges.emplace(ctx, region->bytes / (4ull * kTileRows) + J + 1);
+    ctx.launch("join_write_ranges", 0.0, [&] {
+      jw_range_kernel<<<static_cast<unsigned>(ctx.num_sms) * 8, kBlock, 0, ctx.stream>>>(
+          djo, ostart.get(), J, 0, ostart.get() + J, ranges->get());
     });
     VG_CUDA(cudaGetLastError());
   }
-  if (nslots)
-    VG_CUDA(cudaMemcpyAsync(c0_host, dstage, static_cast<size_t>(nslots) * kSmallC0Words * sizeof(uint32_t),
-                            cudaMemcpyDeviceToHost, ctx.stream));
-  VG_CUDA(cudaMemcpyAsync(first_last_host, dfl, 2 * J * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx.stream));
-  VG_CUDA(cudaMemcpyAsync(bump_host, d_bump, sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx.stream));
-  ctx.free(djo);
-  ctx.free(dslot);
-  ctx.free(dos);
-  ctx.free(dsm);
-  ctx.free(dtj);
-  ctx.free(drg);
-  ctx.free(dfl);
-  ctx.free(dstage);
+  ctx.launch("join_write", 0.0, [&] {
+    bjoin_write_kernel<<<static_cast<unsigned>(ctx.num_sms) * ctx.tune.write_blocks_per_sm, kBlock, 0, ctx.stream>>>(
+        djo, ostart.get(), J, ranges ? ranges->get() : nullptr, 0, ostart.get() + J, small.get(), 0, small.get() + J,
+        JoinEdges{host.first_last, nslots ? tb.at<int32_t>(oslot) : nullptr, host.c0});
+  });
+  VG_CUDA(cudaGetLastError());
 }
 
 void JoinBatch::release(Ctx& ctx) {
@@ -1006,34 +1165,6 @@ void JoinBatch::release(Ctx& ctx) {
   lo = nullptr;
   offs = nullptr;
   d_totals = nullptr;
-}
-
-void batched_join(Ctx& ctx, const std::vector<const Rel*>& l, const std::vector<const Rel*>& r,
-                  std::vector<Rel>& out, std::vector<uint32_t>& first_last) {
-  const uint32_t J = static_cast<uint32_t>(l.size());
-  out.assign(J, Rel());
-  first_last.assign(2 * J, 0);
-  if (J == 0) return;
-  PinnedWords tot(ctx), fl(ctx);
-  JoinBatch jb;
-  uint64_t* ht = tot.reserve(J + 1);
-  batched_join_count(ctx, l, r, jb, ht);
-  // the error record comes back with the totals: a look-back that gave up
-  // leaves the offsets wrong, and the write must then not run
-  VG_CUDA(cudaMemcpyAsync(ht + J, ctx.d_err, sizeof(DeviceErrors), cudaMemcpyDeviceToHost, ctx.stream));
-  ctx.sync();
-  {
-    DeviceErrors he;
-    std::memcpy(&he, ht + J, sizeof(he));
-    if (he.timeout) {
-      jb.release(ctx);
-      ctx.raise_device_errors(he);
-    }
-  }
-  batched_join_write(ctx, jb, tot.data(), out, reinterpret_cast<uint32_t*>(fl.reserve(J)));
-  ctx.sync();
-  const uint32_t* f = reinterpret_cast<const uint32_t*>(fl.data());
-  std::copy(f, f + 2 * J, first_last.begin());
 }
 
 uint64_t col0_words(const std::vector<const Rel*>& rels) {
@@ -1052,31 +1183,13 @@ void batched_col0_enqueue(Ctx& ctx, const std::vector<const Rel*>& rels, uint32_
     total += rels[q]->nrows;
   }
   if (total == 0) return;
-  Col0Req* drq = upload(ctx, rq);
-  uint32_t* buf = ctx.alloc<uint32_t>(total);
+  Tables tb(ctx);
+  const size_t orq = tb.add(rq);
+  tb.send();
   ctx.launch("col0_stage", 8.0 * total, [&] {
-    col0_kernel<<<R < 1024 ? R : 1024, 128, 0, ctx.stream>>>(drq, R, buf);
+    col0_kernel<<<R < 1024 ? R : 1024, 128, 0, ctx.stream>>>(tb.at<Col0Req>(orq), R, host);
   });
   VG_CUDA(cudaGetLastError());
-  VG_CUDA(cudaMemcpyAsync(host, buf, total * 4, cudaMemcpyDeviceToHost, ctx.stream));
-  ctx.free(buf);
-  ctx.free(drq);
-}
-
-void batched_col0(Ctx& ctx, const std::vector<const Rel*>& rels, std::vector<std::vector<uint32_t>>& out) {
-  const uint32_t R = static_cast<uint32_t>(rels.size());
-  out.assign(R, {});
-  const uint64_t total = col0_words(rels);
-  if (R == 0 || total == 0) return;
-  PinnedWords h(ctx);
-  uint32_t* p = reinterpret_cast<uint32_t*>(h.reserve((total + 1) / 2));
-  batched_col0_enqueue(ctx, rels, p);
-  ctx.sync();
-  uint64_t off = 0;
-  for (uint32_t q = 0; q < R; ++q) {
-    out[q].assign(p + off, p + off + rels[q]->nrows);
-    off += rels[q]->nrows;
-  }
 }
 
 PinnedWords::~PinnedWords() { ctx_.give_pinned(p_, cap_); }

@@ -1,10 +1,10 @@
 // Batched (multi-query) versions of the relation kernels: every call takes
 // the work of many queries and issues a fixed, small number of launches.
 //
-// The *_enqueue / *_count / *_write forms only enqueue work on the context
-// stream; the values they hand back land in page-locked host memory that is
-// valid once the stream has passed that point (the caller records an event).
-// The plain forms wait for their results.
+// They only enqueue work on the context stream.  The values they hand back
+// are stored by the kernels into page-locked host memory (the *_host
+// arguments), valid once the stream has passed that point (the caller records
+// an event).
 #pragma once
 
 #include <vector>
@@ -49,20 +49,18 @@ void batched_unique_enqueue(Ctx& ctx, const std::vector<SegRows>& segs, uint64_t
 // Adds the compaction's written bytes to the kernel statistics once the
 // counts are known.
 void note_unique_writes(Ctx& ctx, const std::vector<SegRows>& segs, const uint64_t* counts);
-std::vector<uint64_t> batched_unique(Ctx& ctx, const std::vector<SegRows>& segs);
 
-// Stable sort of every relation by its column 0: one onesweep sort over
-// (segment, key) composite keys, then one gather.  Columns are replaced.
-// key_bits (1..32) bounds every key (keys < 2^key_bits): the passes are then
-// fixed and nothing waits on the device; 0 reads the digit histogram on the
-// host to skip passes.
+// Stable sort of every relation by its column 0: those of up to 1024 rows by
+// one launch, the others by one radix sort over (segment, key) composite keys
+// and one gather.  Columns are replaced.  key_bits (1..32) bounds every key
+// (keys < 2^key_bits); 0: 32 bits.
 void batched_sort_by_first(Ctx& ctx, const std::vector<Rel*>& rels, int key_bits);
 
 // Inner joins on column 0 (l[j] with r[j], both sorted by column 0 and
 // non-empty), in two halves.  batched_join_count enqueues the per-key match
 // counts and their scan and copies each join's output size to
 // totals_host[j]; batched_join_write, given those sizes, allocates the
-// outputs from the arena, enqueues the output write, and copies column 0's
+// outputs from the arena, enqueues the output write, and stores column 0's
 // first and last value of out[j] to first_last_host[2j], [2j+1] (zero for an
 // empty output).  The relations must stay alive and unchanged in between.
 struct JoinBatch {
@@ -84,30 +82,31 @@ void batched_join_write(Ctx& ctx, JoinBatch& jb, const uint64_t* totals, std::ve
 
 constexpr uint32_t kSmallC0Words = 100;   // staged column-0 words per small join output
 
-// The join write without a host round trip after the count: the outputs are
-// placed on the device in `region` (its bump pointer at d_bump, whose value
-// after the wave is copied to *bump_host), written, and their first/last
-// values copied to first_last_host and, for the joins with c0_slot[j] >= 0
-// and 2 < rows < kSmallC0Words, column 0 to c0_host + slot * kSmallC0Words.
-// Outputs that do not fit stay unplaced.  jb's device arrays stay alive:
+// Count and write without a host round trip in between: the outputs are placed
+// on the device in `region` (its bump pointer at d_bump) and written.  Outputs
+// that do not fit stay unplaced.  jb's device arrays stay alive:
 // place_outputs_on_host then tells which joins were placed (the same
 // arithmetic on the copied totals), and the caller writes the others with
 // batched_join_write(..., skip = placed), or releases jb.
-void batched_join_place_write(Ctx& ctx, JoinBatch& jb, const Arena::Region* region, uint64_t* d_bump,
-                              const std::vector<int32_t>& c0_slot, uint32_t nslots, uint32_t* first_last_host,
-                              uint32_t* c0_host, uint64_t* bump_host);
+struct PlacedHost {       // page-locked
+  uint64_t* totals;       // every join's output rows
+  uint64_t* bump;         // the region's bump pointer after the wave
+  DeviceErrors* err;      // the error record after the count; nothing is placed when it holds a timeout
+  uint32_t* first_last;   // of the placed outputs with rows
+  uint32_t* c0;           // for joins with c0_slot[j] >= 0 and 2 < rows < kSmallC0Words: column 0 at slot * kSmallC0Words
+};
+void batched_join_placed(Ctx& ctx, const std::vector<const Rel*>& l, const std::vector<const Rel*>& r, JoinBatch& jb,
+                         const Arena::Region* region, uint64_t* d_bump, const std::vector<int32_t>& c0_slot,
+                         uint32_t nslots, const PlacedHost& host);
 // Returns the region's bump after the wave; out[j] is the placed output of
 // join j (placed[j] = 1) and `blocks` the number of its columns in the region.
 uint64_t place_outputs_on_host(const JoinBatch& jb, const uint64_t* totals, const Arena::Region* region,
                                uint64_t bump, std::vector<Rel>& out, std::vector<uint8_t>& placed,
                                int64_t& blocks);
-void batched_join(Ctx& ctx, const std::vector<const Rel*>& l, const std::vector<const Rel*>& r,
-                  std::vector<Rel>& out, std::vector<uint32_t>& first_last);
 
-// Column 0 of each relation copied to the host, back to back (one launch,
-// one copy): col0_words(rels) uint32 words.
+// Column 0 of each relation stored to the host, back to back (one launch):
+// col0_words(rels) uint32 words.
 uint64_t col0_words(const std::vector<const Rel*>& rels);
 void batched_col0_enqueue(Ctx& ctx, const std::vector<const Rel*>& rels, uint32_t* host);
-void batched_col0(Ctx& ctx, const std::vector<const Rel*>& rels, std::vector<std::vector<uint32_t>>& out);
 
 }  // namespace vg

@@ -713,15 +713,18 @@ void WaveEngine::stage_a(std::vector<PlannedQuery*>& completed) {
   tr.h_copy = since(tp);
   tp = Clock::now();
   if (!jl.empty()) {
-    batched_join_count(ctx_, jl, jr, jb_, ha + off_tot_);
     // the device error record comes back with the totals: a look-back that
-    // gave up leaves the offsets wrong, and stage B must then not write
-    VG_CUDA(cudaMemcpyAsync(ha + off_err_, ctx_.d_err, sizeof(DeviceErrors), cudaMemcpyDeviceToHost,
-                            ctx_.stream));
-    if (placed_wave_)
-      batched_join_place_write(ctx_, jb_, region_, d_bump_, c0_slot_, nslots,
-                               reinterpret_cast<uint32_t*>(ha + off_fla_), reinterpret_cast<uint32_t*>(ha + off_c0a_),
-                               ha + off_bump_);
+    // gave up leaves the offsets wrong, and nothing must then be written
+    auto* err_host = reinterpret_cast<DeviceErrors*>(ha + off_err_);
+    if (placed_wave_) {
+      batched_join_placed(ctx_, jl, jr, jb_, region_, d_bump_, c0_slot_, nslots,
+                          PlacedHost{ha + off_tot_, ha + off_bump_, err_host,
+                                     reinterpret_cast<uint32_t*>(ha + off_fla_),
+                                     reinterpret_cast<uint32_t*>(ha + off_c0a_)});
+    } else {
+      batched_join_count(ctx_, jl, jr, jb_, ha + off_tot_);
+      VG_CUDA(cudaMemcpyAsync(err_host, ctx_.d_err, sizeof(DeviceErrors), cudaMemcpyDeviceToHost, ctx_.stream));
+    }
     any = true;
   }
   tr.h_join = since(tp);

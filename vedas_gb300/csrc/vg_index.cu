@@ -428,7 +428,7 @@ class Permuter {
     if (!take(cols))
       for (Col c : cols) take({c});
     Scratch<uint64_t> alt(ctx_, n_);
-    if (radix_sort_u64_counted(ctx_, keys_->get(), alt.get(), n_, digits, bases)) std::swap(keys_->p, alt.p);
+    if (radix_sort_u64_counted(ctx_, keys_->get(), alt.get(), nullptr, nullptr, n_, digits, bases)) std::swap(keys_->p, alt.p);
   }
 
   // The requested outputs of the keys as (c0, c1, c2); groups: the keys are

@@ -731,7 +731,7 @@ static bool sort_packed_rows(Ctx& ctx, Rel& r) {
   VG_CUDA(cudaGetLastError());
   std::vector<const uint64_t*> bases;
   for (uint32_t d = 0; d < dl.n; ++d) bases.push_back(counts.bases(d));
-  if (radix_sort_u64_counted(ctx, keys.get(), alt.get(), n, digits, bases)) std::swap(keys.p, alt.p);
+  if (radix_sort_u64_counted(ctx, keys.get(), alt.get(), nullptr, nullptr, n, digits, bases)) std::swap(keys.p, alt.p);
   for (uint32_t c = 0; c < r.ncols; ++c) {
     if (r.borrowed >> c & 1u) r.cols[c] = ctx.alloc<uint32_t>(n);   // (a view is not written)
     a.col[c] = r.cols[c];

@@ -453,17 +453,23 @@ bool radix_sort_u64(Ctx& ctx, uint64_t* keys, uint64_t* keys_alt, uint32_t* vals
   return radix_sort_impl<uint64_t>(ctx, keys, keys_alt, vals, vals_alt, n, digits, vals_iota, host_skip);
 }
 
-bool radix_sort_u64_counted(Ctx& ctx, uint64_t* keys, uint64_t* keys_alt, uint64_t n,
-                            const std::vector<RadixDigit>& digits, const std::vector<const uint64_t*>& bases) {
-  if (n == 0 || digits.empty()) return false;
+bool radix_sort_u64_counted(Ctx& ctx, uint64_t* keys, uint64_t* keys_alt, uint32_t* vals, uint32_t* vals_alt,
+                            uint64_t n, const std::vector<RadixDigit>& digits,
+                            const std::vector<const uint64_t*>& bases, bool vals_iota) {
+  if (n == 0) return false;
+  if (n > 0xFFFFFFFFull && vals) fail(VG_ERR_OVERFLOW, "radix sort values are 32-bit row ids");
+  if (digits.empty()) {
+    if (vals && vals_iota) fill_iota(ctx, vals, n);
+    return false;
+  }
   const DigitList dl = digit_list(digits);
   const PassScratch ps(ctx, n, dl);
   Scratch<char> scratch(ctx, ps.bytes);
   VG_CUDA(cudaMemsetAsync(scratch.get(), 0, ps.bytes, ctx.stream));
   std::vector<uint32_t> todo(dl.n);
   for (uint32_t p = 0; p < dl.n; ++p) todo[p] = p;
-  return run_passes<uint64_t>(ctx, keys, keys_alt, nullptr, nullptr, n, dl, bases.data(), todo, ps, scratch.get(),
-                              false);
+  return run_passes<uint64_t>(ctx, keys, keys_alt, vals, vals_alt, n, dl, bases.data(), todo, ps, scratch.get(),
+                              vals_iota);
 }
 
 void fill_iota(Ctx& ctx, uint32_t* out, uint64_t n) {

@@ -28,12 +28,13 @@ bool radix_sort_u32(Ctx& ctx, uint32_t* keys, uint32_t* keys_alt, uint32_t* vals
                     uint64_t n, int end_bit, bool vals_iota, bool host_skip = true);
 bool radix_sort_u64(Ctx& ctx, uint64_t* keys, uint64_t* keys_alt, uint32_t* vals, uint32_t* vals_alt,
                     uint64_t n, int end_bit, bool vals_iota, bool host_skip = true);
-// Keys only, by the given digits in order (what lies outside them travels
-// with the key and does not count: equal digits keep their input order), with
-// the bases of each digit's 256 values already on the device.  Counts do not
-// depend on the keys' order, so one count serves several sorts.
-bool radix_sort_u64_counted(Ctx& ctx, uint64_t* keys, uint64_t* keys_alt, uint64_t n,
-                            const std::vector<RadixDigit>& digits, const std::vector<const uint64_t*>& bases);
+// By the given digits in order (what lies outside them travels with the key
+// and does not count: equal digits keep their input order), with the bases of
+// each digit's 256 values already on the device.  Counts do not depend on the
+// keys' order, so one count serves several sorts.
+bool radix_sort_u64_counted(Ctx& ctx, uint64_t* keys, uint64_t* keys_alt, uint32_t* vals, uint32_t* vals_alt,
+                            uint64_t n, const std::vector<RadixDigit>& digits,
+                            const std::vector<const uint64_t*>& bases, bool vals_iota = false);
 void fill_iota(Ctx& ctx, uint32_t* out, uint64_t n);
 
 }  // namespace vg
