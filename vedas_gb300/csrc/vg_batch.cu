@@ -500,7 +500,7 @@ __device__ __forceinline__ uint32_t* edge_stage(const JoinEdges& ed, uint32_t j,
   return s < 0 ? nullptr : ed.stage + static_cast<uint64_t>(s) * kSmallC0Words;
 }
 
-__device__ __forceinline__ void write_small_join(const JoinOut* __restrict__ src, JoinOut* jp, uint64_t* s_off,
+__device__ __forceinline__ void write_small_join(const JoinOut* __restrict__ src, JoinOut* jp, uint32_t* s_off,
                                                  uint32_t* s_lo, uint32_t j, const JoinEdges& ed) {
   const uint32_t lane = lane_id();
   // the join's description in the warp's shared slot: the row loop reads its
@@ -515,7 +515,7 @@ __device__ __forceinline__ void write_small_join(const JoinOut* __restrict__ src
   const uint64_t* offs = jp->offs;
   const uint32_t* lov = jp->lo;
   for (uint32_t e = lane; e < nl; e += 32) {
-    s_off[e] = offs[e];
+    s_off[e] = static_cast<uint32_t>(offs[e]);   // (a small output's rows)
     s_lo[e] = lov[e];
   }
   __syncwarp();
@@ -574,13 +574,11 @@ __global__ void __launch_bounds__(kBlock, 5) bjoin_write_kernel(const JoinOut* _
                                                              uint64_t T_host, const uint64_t* ostart_end,
                                                              const uint32_t* __restrict__ small, uint32_t nsmall_host,
                                                              const uint32_t* nsmall_dev, JoinEdges ed) {
-  constexpr int kStage = kTileRows + 1;
   static_assert(kBlock == kJwBlock, "jw_write_tile's block");
-  static_assert(kStage >= (kBlock / 32) * kSmallJoin, "a warp's slice holds a small join's left rows");
+  static_assert(JwStage<kRows>::kMost >= (kBlock / 32) * kSmallJoin, "a warp's slice holds a small join's left rows");
   __shared__ JoinOut s_o;
   __shared__ JoinOut s_w[kBlock / 32];
-  __shared__ uint64_t s_off[kStage];
-  __shared__ uint32_t s_lo[kStage];
+  __shared__ JwStage<kRows> s_stage;
   __shared__ uint32_t s_j;
   __shared__ uint64_t s_range[2];
   {
@@ -588,7 +586,8 @@ __global__ void __launch_bounds__(kBlock, 5) bjoin_write_kernel(const JoinOut* _
     const uint32_t warp = threadIdx.x >> 5, nwarps = kBlock / 32;
     for (uint64_t w = static_cast<uint64_t>(blockIdx.x) * nwarps + warp; w < nsm;
          w += static_cast<uint64_t>(gridDim.x) * nwarps)
-      write_small_join(&jo[small[w]], &s_w[warp], s_off + warp * kSmallJoin, s_lo + warp * kSmallJoin, small[w], ed);
+      write_small_join(&jo[small[w]], &s_w[warp], s_stage.off + warp * kSmallJoin, s_stage.lo + warp * kSmallJoin,
+                       small[w], ed);
   }
   const uint64_t T = ostart_end ? *ostart_end : T_host;
 #pragma unroll 1
@@ -626,7 +625,7 @@ __global__ void __launch_bounds__(kBlock, 5) bjoin_write_kernel(const JoinOut* _
     const uint64_t total = s_o.total;
     const uint64_t kb = (tile - ostart[jn]) * static_cast<uint64_t>(kTileRows);
     const uint64_t kend = (kb + kTileRows < total) ? kb + kTileRows : total;
-    jw_write_tile<kRows>(s_o, kb, kend, s_range[0], s_range[1], s_off, s_lo);
+    jw_write_tile<kRows>(s_o, kb, kend, s_range[0], s_range[1], s_stage);
     const uint32_t* c0 = s_o.oc[0];
     if (kb == 0 && threadIdx.x == 0) ed.fl[2 * jn] = c0[0];
     if (kend == total && threadIdx.x == (total - 1 - kb) % kBlock) ed.fl[2 * jn + 1] = c0[total - 1];

@@ -239,34 +239,55 @@ __device__ __forceinline__ void jc_issue_window(const uint32_t* __restrict__ R, 
   }
 }
 
-// The thread's keys (of left rows i0 + 8 * thread, up to i_end) in a staged
-// window of n right keys, whose first is right row w0: the first key is
-// searched in full, the others gallop from the previous key's upper bound;
-// equal keys reuse its bounds.
+// The thread's keys (of left rows i0 + 8 * thread, up to i_end; ascending, the
+// last repeated past the end) in a staged window of n right keys, whose first
+// is right row w0.  The lower bounds of the first and last key are searched in
+// lockstep over the window (a number of steps that the block shares), the
+// others in lockstep between those two (as many steps as the warp's widest
+// range takes; every lane of the warp calls this): no lane waits for another's loop, where galloping from key to
+// key left 18 of 32 lanes active.  The upper bound of a key that matches
+// gallops from its lower bound; equal keys share both.
 template <typename T>
 __device__ __forceinline__ void jc_search_staged(const T* win, uint32_t n, uint64_t w0, uint64_t i0, uint64_t i_end,
                                                  const T (&key)[kJcKeys], uint32_t (&lov)[kJcKeys],
                                                  uint32_t (&cnt)[kJcKeys]) {
   const uint64_t first = i0 + static_cast<uint64_t>(threadIdx.x) * kJcKeys;
-  uint32_t plo = 0, phi = 0;
-  T pkey = 0;
+  uint32_t lo[kJcKeys];
+  {
+    uint32_t a = 0, b = 0, len = n;
+    while (len > 1) {
+      const uint32_t half = len >> 1;
+      a = win[a + half - 1] < key[0] ? a + half : a;
+      b = win[b + half - 1] < key[kJcKeys - 1] ? b + half : b;
+      len -= half;
+    }
+    if (n) {
+      a += win[a] < key[0] ? 1 : 0;
+      b += win[b] < key[kJcKeys - 1] ? 1 : 0;
+    }
+    lo[0] = a;
+    lo[kJcKeys - 1] = b;
+  }
+  // positions in [a, b]: b - a right keys to compare with (none where keys do
+  // not ascend, so that nothing outside the window is ever read)
+  uint32_t len = lo[kJcKeys - 1] > lo[0] ? lo[kJcKeys - 1] - lo[0] : 0u;
+#pragma unroll
+  for (int j = 1; j < kJcKeys - 1; ++j) lo[j] = lo[0];
+  for (uint32_t most = __reduce_max_sync(0xffffffffu, len); most > 0; most >>= 1) {
+    const uint32_t half = (len + 1) >> 1;
+#pragma unroll
+    for (int j = 1; j < kJcKeys - 1; ++j)
+      if (half) lo[j] = win[lo[j] + half - 1] < key[j] ? lo[j] + half : lo[j];
+    len -= half;
+  }
+  uint32_t phi = 0;
 #pragma unroll
   for (int j = 0; j < kJcKeys; ++j) {
     if (first + j < i_end) {
-      const T k = key[j];
-      uint32_t lo, hi;
-      if (j > 0 && k == pkey) {
-        lo = plo;
-        hi = phi;
-      } else {
-        lo = (j == 0) ? smem_search<false, T>(win, 0, n, k) : smem_gallop<false, T>(win, phi, n, k);
-        hi = smem_gallop<true, T>(win, lo, n, k);
-      }
-      lov[j] = static_cast<uint32_t>(w0 + lo);
-      cnt[j] = hi - lo;
-      plo = lo;
+      const uint32_t hi = (j > 0 && key[j] == key[j - 1]) ? phi : smem_gallop<true, T>(win, lo[j], n, key[j]);
+      lov[j] = static_cast<uint32_t>(w0 + lo[j]);
+      cnt[j] = hi - lo[j];
       phi = hi;
-      pkey = k;
     }
   }
 }
@@ -300,7 +321,7 @@ __device__ __forceinline__ void jc_count_staged(const uint32_t* __restrict__ L, 
     const uint4 b = *reinterpret_cast<const uint4*>(L + first + 4);
     key[0] = a.x, key[1] = a.y, key[2] = a.z, key[3] = a.w;
     key[4] = b.x, key[5] = b.y, key[6] = b.z, key[7] = b.w;
-  } else if (first < i_end) {
+  } else {
 #pragma unroll
     for (int j = 0; j < kJcKeys; ++j) {
       const uint64_t i = first + j;
@@ -323,9 +344,8 @@ __device__ __forceinline__ void jc_count_staged(const uint32_t* __restrict__ L, 
   }
   __syncthreads();
   const bool use_smem = staged != 0 && sm.failed == 0;
-  if (first >= i_end) return;   // counts stay zero
-
   if (!use_smem) {
+    if (first >= i_end) return;   // counts stay zero
     uint32_t lo[kJcKeys], hi[kJcKeys];
     lockstep_bounds32<kJcKeys>(R, static_cast<uint32_t>(w0), static_cast<uint32_t>(w1), key, lo, hi);
 #pragma unroll
@@ -392,11 +412,11 @@ __device__ __forceinline__ void jc_count_staged_pairs(const PairKeys& L, uint64_
   if (sm.staged)
     for (uint64_t e = w0 + tid; e < w1; e += kJcBlock) win[e - w0] = R(e);
   __syncthreads();
-  if (first >= i_end) return;   // counts stay zero
   if (sm.staged) {
     jc_search_staged<uint64_t>(win, static_cast<uint32_t>(w1 - w0), w0, i0, i_end, key, lov, cnt);
     return;
   }
+  if (first >= i_end) return;   // counts stay zero
   uint32_t lo[kJcKeys], hi[kJcKeys];
   lockstep_bounds_of<kJcKeys>(R, static_cast<uint32_t>(w0), static_cast<uint32_t>(w1), key, lo, hi);
 #pragma unroll
@@ -483,51 +503,62 @@ struct JoinOut {
 
 constexpr int kJwBlock = 256;
 
+// Left rows that a tile of kJwBlock * ROWS output rows stages: twice as many,
+// since rows without matches lie between the others (16M left rows with 13M
+// output rows had no tile staged when only as many fitted: 0.26 ms).
+template <int ROWS>
+struct JwStage {
+  static constexpr uint32_t kMost = 2 * kJwBlock * ROWS;
+  uint32_t off[kMost];   // first output row, from the tile's first (0 where it lies before)
+  uint32_t lo[kMost];    // the right row that output row off comes from
+};
+
 // Output rows [kb, kend) (at most kJwBlock * ROWS) of a join, by one block.
 // Output row k comes from the left row i with offs[i] <= k < offs[i + 1] and
 // the right row lo[i] + (k - offs[i]); the rows come from left rows [ib, ie).
-// When those are at most STAGE = kJwBlock * ROWS + 1, their offsets and lower
-// bounds are staged in shared memory and each thread walks its rows (k
-// increasing, consecutive threads on consecutive rows, so loads and stores
-// coalesce) from the previous one's left row.  Hub keys thus spread over many
-// blocks.
+// When those fit the stage, their offsets and lower bounds lie in shared
+// memory and each thread walks its rows (k increasing, consecutive threads on
+// consecutive rows, so loads and stores coalesce) from the previous one's left
+// row.  Hub keys thus spread over many blocks.
 template <int ROWS>
 __device__ __forceinline__ void jw_write_tile(const JoinOut& o, uint64_t kb, uint64_t kend, uint64_t ib, uint64_t ie,
-                                              uint64_t* s_off, uint32_t* s_lo) {
-  constexpr int kStage = kJwBlock * ROWS + 1;
-  const uint64_t m = ie - ib;
-  const bool staged = m <= static_cast<uint64_t>(kStage);
-  if (staged)
-    for (uint32_t e = threadIdx.x; e < m; e += kJwBlock) {
-      s_off[e] = o.offs[ib + e];
-      s_lo[e] = o.lo[ib + e];
-    }
+                                              JwStage<ROWS>& st) {
+  const uint64_t m64 = ie - ib;
+  const bool staged = m64 <= JwStage<ROWS>::kMost;
+  const uint32_t m = static_cast<uint32_t>(staged ? m64 : 0);
+  for (uint32_t e = threadIdx.x; e < m; e += kJwBlock) {
+    const uint64_t f = o.offs[ib + e];
+    const uint32_t r = o.lo[ib + e];
+    st.off[e] = f > kb ? static_cast<uint32_t>(f - kb) : 0u;
+    st.lo[e] = f > kb ? r : r + static_cast<uint32_t>(kb - f);
+  }
   __syncthreads();
   // 1. the left and right row of each of the thread's output rows
   uint32_t li[ROWS], ri[ROWS];
   if (staged) {
+    const uint32_t rows = static_cast<uint32_t>(kend - kb);
     uint32_t p = 0;   // the current left row, relative to ib
 #pragma unroll
     for (int it = 0; it < ROWS; ++it) {
-      const uint64_t k = kb + static_cast<uint64_t>(it) * kJwBlock + threadIdx.x;
+      const uint32_t k = it * kJwBlock + threadIdx.x;
       li[it] = ri[it] = 0;
-      if (k < kend) {
-        // last p with s_off[p] <= k, moving forward from the previous row's p
+      if (k < rows) {
+        // last p with off[p] <= k, moving forward from the previous row's p
         uint32_t step = 1;
-        while (p + step < m && s_off[p + step] <= k) {
+        while (p + step < m && st.off[p + step] <= k) {
           p += step;
           step <<= 1;
         }
         while (step > 1) {
           step >>= 1;
-          if (p + step < m && s_off[p + step] <= k) p += step;
+          if (p + step < m && st.off[p + step] <= k) p += step;
         }
-        li[it] = static_cast<uint32_t>(ib + p);
-        ri[it] = static_cast<uint32_t>(s_lo[p] + (k - s_off[p]));
+        li[it] = static_cast<uint32_t>(ib) + p;
+        ri[it] = st.lo[p] + (k - st.off[p]);
       }
     }
   } else {
-    // a sparse tile (more than kStage left rows, most without matches): the
+    // a sparse tile (more left rows than the stage holds, most without matches): the
     // left rows of kGroup of the thread's output rows at a time come from
     // kGroup binary searches of the offsets advanced in lockstep, so each
     // round has kGroup independent loads in flight

@@ -244,8 +244,7 @@ __global__ void __launch_bounds__(kJwBlock, 5) join_write_kernel(JoinOut o, cons
                                                                  const DeviceErrors* err, JoinTail* tail) {
   constexpr uint32_t kTile = kJwBlock * ROWS;
   __shared__ JoinOut s_o;
-  __shared__ uint64_t s_off[kTile + 1];
-  __shared__ uint32_t s_lo[kTile + 1];
+  __shared__ JwStage<ROWS> s_stage;
   __shared__ uint64_t s_range[2];
   const uint64_t total = total_dev ? *total_dev : o.total;
   const DeviceErrors e = *err;
@@ -276,7 +275,7 @@ __global__ void __launch_bounds__(kJwBlock, 5) join_write_kernel(JoinOut o, cons
       }
     }
     __syncthreads();
-    jw_write_tile<ROWS>(s_o, kb, kend, s_range[0], s_range[1], s_off, s_lo);
+    jw_write_tile<ROWS>(s_o, kb, kend, s_range[0], s_range[1], s_stage);
     if (tail) {   // each by the thread that wrote the row
       const uint32_t* c0 = s_o.oc[0];
       if (tile == 0 && threadIdx.x == 0) tail->first = c0[0];
