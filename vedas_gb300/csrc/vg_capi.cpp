@@ -613,16 +613,48 @@ vg_status vg_batch_download_all(const vg_batch* b, uint32_t* host) {
     const uint64_t words = vg_batch_result_words(b);
     if (words == 0) return;
     if (!host) vg::fail(VG_ERR_INVALID, "null host buffer");
+    // Parts of the results are packed on the context's stream and copied on the
+    // download stream, so that the host's tables and the packing of one part go
+    // on while another is copied (596 MB: 3.86 ms in one part, 3.1 the copy
+    // alone).  The first part is small: nothing overlaps it.
+    // One of at most kOnePart words goes in one step on the context's stream.
+    constexpr uint64_t kOnePart = 4ull << 20;
     vg::Scratch<uint32_t> stage(ctx, words);
+    const cudaStream_t dl = words > kOnePart ? ctx.dl_stream() : static_cast<cudaStream_t>(ctx.stream);
+    struct Event {
+      cudaEvent_t e = nullptr;
+      Event() { VG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming)); }
+      ~Event() { cudaEventDestroy(e); }
+    } packed;
     std::vector<vg::CopyPiece> pieces;
-    uint64_t off = 0;
-    for (const auto& q : b->r.queries)
-      for (uint32_t c = 0; c < q.rel.ncols; ++c) {
-        pieces.push_back({q.rel.cols[c], stage.get() + off, q.rel.nrows});
-        off += q.rel.nrows;
+    uint64_t off = 0, sent = 0;
+    uint64_t part = words > kOnePart ? words / 16 : words;
+    auto send = [&] {
+      vg::batched_copy(ctx, pieces);
+      pieces.clear();
+      if (dl != ctx.stream) {
+        VG_CUDA(cudaEventRecord(packed.e, ctx.stream));
+        VG_CUDA(cudaStreamWaitEvent(dl, packed.e, 0));
       }
-    vg::batched_copy(ctx, pieces);
-    VG_CUDA(cudaMemcpyAsync(host, stage.get(), words * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx.stream));
+      VG_CUDA(cudaMemcpyAsync(host + sent, stage.get() + sent, (off - sent) * sizeof(uint32_t),
+                              cudaMemcpyDeviceToHost, dl));
+      sent = off;
+      part = words / 4;
+    };
+    try {
+      for (const auto& q : b->r.queries) {
+        for (uint32_t c = 0; c < q.rel.ncols; ++c) {
+          pieces.push_back({q.rel.cols[c], stage.get() + off, q.rel.nrows});
+          off += q.rel.nrows;
+        }
+        if (off - sent >= part) send();
+      }
+      if (off > sent) send();
+    } catch (...) {
+      cudaStreamSynchronize(dl);   // copies out of the stage end before it is freed
+      throw;
+    }
+    VG_CUDA(cudaStreamSynchronize(dl));
     ctx.sync();
   });
 }
