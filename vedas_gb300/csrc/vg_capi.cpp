@@ -391,10 +391,14 @@ vg_status vg_query(vg_ctx* ctx, vg_index* ix, const char* sparql, vg_result** ou
     vedas::FullRelationIR* ir = sr.getResultIR();
     for (size_t c = 0; c < ir->getColumnNum(); ++c) res->headers.push_back(ir->getHeader(c));
     res->rel = ir->release();
-    vg::rel_own(ctx->c, res->rel);   // a result never refers to index memory
+    // a result never refers to index memory; everything before has been waited
+    // for and its errors raised (removeDuplicate)
+    if (res->rel.borrowed) {
+      vg::rel_own(ctx->c, res->rel);
+      ctx->c.sync();
+    }
     res->ctx = ctx;
     res->log = ex.exe_log;
-    ctx->c.check_device_errors();
   });
   if (st == VG_OK) *out = res.release();
   return st;

@@ -81,6 +81,10 @@ struct UniqueArgs {
   uint64_t n;
   uint8_t* keep;          // bit i of byte b: row 8 b + i stays
 };
+struct UniqueHost {    // page-locked
+  uint64_t dropped;
+  DeviceErrors err;    // what the work before left, so that no copy of its own is needed
+};
 struct UniqueTotal {   // zeroed before the first kernel
   unsigned long long dropped;
   uint32_t done;       // finished blocks
@@ -90,9 +94,11 @@ struct UniqueTotal {   // zeroed before the first kernel
 // Each thread flags its 8 rows.  Columns are compared from the last to the
 // first, and only while some row still equals the one before it: in sorted
 // rows and in join outputs the last columns change fastest, so most of the
-// time one column is read (7.4e7 rows of 8 columns without repetitions took
-// 1.41 ms when all were read, and once more to be written elsewhere).
-__global__ void __launch_bounds__(kBlock) unique_flags_kernel(UniqueArgs a, UniqueTotal* tot, uint64_t* host_dropped) {
+// time one or two columns are read (7.4e7 rows of 8 columns without
+// repetitions: 0.13 ms, and 1.41 ms when all were read, and once more to be
+// written elsewhere).
+__global__ void __launch_bounds__(kBlock) unique_flags_kernel(UniqueArgs a, UniqueTotal* tot,
+                                                              const DeviceErrors* err, UniqueHost* host) {
   static_assert(kRows == 8, "unique_diff_bits and compact_store take 8 rows per thread");
   uint32_t drop = 0;
   const uint64_t step = static_cast<uint64_t>(gridDim.x) * kBlock * kRows;
@@ -101,8 +107,7 @@ __global__ void __launch_bounds__(kBlock) unique_flags_kernel(UniqueArgs a, Uniq
     const uint32_t here = a.n - r0 < kRows ? static_cast<uint32_t>(a.n - r0) : kRows;
     const uint32_t all = (1u << here) - 1u;
     uint32_t diff = (r0 == 0) ? 1u : 0u;
-    diff |= unique_diff_bits(a.in[a.ncols - 1], a.n, r0);
-    for (int c = static_cast<int>(a.ncols) - 2; c >= 0 && (diff & all) != all; --c)
+    for (int c = static_cast<int>(a.ncols) - 1; c >= 0 && (diff & all) != all; --c)
       diff |= unique_diff_bits(a.in[c], a.n, r0);
     diff &= all;
     a.keep[r0 / 8] = static_cast<uint8_t>(diff);
@@ -114,7 +119,8 @@ __global__ void __launch_bounds__(kBlock) unique_flags_kernel(UniqueArgs a, Uniq
   __syncthreads();
   if (threadIdx.x == 0 && atomicAdd(&tot->done, 1u) == gridDim.x - 1) {
     __threadfence();
-    *host_dropped = ld_status_u64(reinterpret_cast<const uint64_t*>(&tot->dropped));
+    host->dropped = ld_status_u64(reinterpret_cast<const uint64_t*>(&tot->dropped));
+    host->err = *err;
   }
 }
 
@@ -768,7 +774,10 @@ void sort_rows(Ctx& ctx, Rel& r) {
 }
 
 void unique_in_place(Ctx& ctx, Rel& r) {
-  if (r.nrows <= 1 || r.ncols == 0) return;
+  if (r.nrows <= 1 || r.ncols == 0) {
+    ctx.check_device_errors();
+    return;
+  }
   const uint64_t n = r.nrows;
   UniqueArgs a{};
   for (uint32_t c = 0; c < r.ncols; ++c) a.in[c] = r.cols[c];
@@ -780,12 +789,14 @@ void unique_in_place(Ctx& ctx, Rel& r) {
   a.keep = keep.get();
   VG_CUDA(cudaMemsetAsync(tot.get(), 0, sizeof(UniqueTotal), ctx.stream));
   const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(tiles, static_cast<uint64_t>(ctx.num_sms) * 8));
+  auto* host = reinterpret_cast<UniqueHost*>(ctx.h_small);
   // (what must be read: a column at least)
   ctx.launch("unique_flags", 4.0 * n,
-             [&] { unique_flags_kernel<<<grid, kBlock, 0, ctx.stream>>>(a, tot.get(), ctx.h_small); });
+             [&] { unique_flags_kernel<<<grid, kBlock, 0, ctx.stream>>>(a, tot.get(), ctx.d_err, host); });
   VG_CUDA(cudaGetLastError());
   ctx.sync();
-  const uint64_t dropped = ctx.h_small[0];
+  ctx.raise_device_errors(host->err);
+  const uint64_t dropped = host->dropped;
   if (dropped == 0) return;
   const uint64_t kept = n - dropped;
   Rel out = rel_alloc(ctx, r.ncols, kept);

@@ -64,8 +64,8 @@ void gather_cols(Ctx& ctx, const uint32_t* const* in, uint32_t* const* out, uint
 void sort_by_first(Ctx& ctx, Rel& r);
 // Lexicographic sort of the rows over all columns (in place).
 void sort_rows(Ctx& ctx, Rel& r);
-// Adjacent duplicate-row removal (synchronizes).  A relation without any
-// keeps its columns; views stay views.
+// Adjacent duplicate-row removal (synchronizes and raises device errors).  A
+// relation without any keeps its columns; views stay views.
 void unique_in_place(Ctx& ctx, Rel& r);
 
 // Copies `n` values of a device column to the host (synchronizes).
