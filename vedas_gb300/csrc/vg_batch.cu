@@ -374,7 +374,7 @@ struct JoinSeg {
 constexpr uint32_t kSmallJoin = 32 * kJcKeys;
 
 __device__ __forceinline__ void count_small_join(const JoinSeg& g, uint32_t* __restrict__ lo,
-                                                 uint64_t* __restrict__ offs, uint64_t* total) {
+                                                 uint32_t* __restrict__ offs, uint64_t* total) {
   const uint32_t lane = lane_id();
   const uint64_t nl = g.nl;
   const uint64_t w0 = warp_bound<false, uint32_t>(g.rk, 0, g.nr, g.lk[0]);
@@ -395,7 +395,7 @@ __device__ __forceinline__ void count_small_join(const JoinSeg& g, uint32_t* __r
   for (int q = 0; q < kJcKeys; ++q)
     if (first + q < nl) {
       lo[g.row0 + first + q] = static_cast<uint32_t>(lb[q]);
-      offs[g.row0 + first + q] = run;
+      offs[g.row0 + first + q] = static_cast<uint32_t>(run);
       run += ub[q] - lb[q];
     }
   if (lane == 31) *total = incl;
@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(kJcBlock) jc_window_kernel(const JoinSeg* __re
 __global__ void __launch_bounds__(kJcBlock, 4) bjoin_count_scan_kernel(
     const JoinSeg* __restrict__ js, const uint64_t* __restrict__ bstart, const uint32_t* __restrict__ tile_join,
     const uint2* __restrict__ win, const uint32_t* __restrict__ small, uint32_t nsmall, uint32_t small_blocks,
-    uint32_t* __restrict__ lo, uint64_t* __restrict__ offs, uint64_t* status, uint32_t* ticket,
+    uint32_t* __restrict__ lo, uint32_t* __restrict__ offs, uint64_t* status, uint32_t* ticket,
     uint64_t* __restrict__ totals, DeviceErrors* err) {
   if (blockIdx.x < small_blocks) {   // block-uniform: this block only counts small joins
     const uint64_t sj = static_cast<uint64_t>(blockIdx.x) * (kJcBlock / 32) + (threadIdx.x >> 5);
@@ -512,10 +512,10 @@ __device__ __forceinline__ void write_small_join(const JoinOut* __restrict__ src
     __syncwarp();
   }
   const uint64_t total = jp->total, nl = jp->nl;
-  const uint64_t* offs = jp->offs;
+  const uint32_t* offs = jp->offs;
   const uint32_t* lov = jp->lo;
   for (uint32_t e = lane; e < nl; e += 32) {
-    s_off[e] = static_cast<uint32_t>(offs[e]);   // (a small output's rows)
+    s_off[e] = offs[e];
     s_lo[e] = lov[e];
   }
   __syncwarp();
@@ -560,7 +560,8 @@ __global__ void __launch_bounds__(kBlock) jw_range_kernel(const JoinOut* __restr
     const uint64_t kb = (t - ostart[jn]) * static_cast<uint64_t>(kTileRows);
     const uint64_t kend = (kb + kTileRows < total) ? kb + kTileRows : total;
     uint64_t a, b;
-    warp_bound_pair<true, true, uint64_t>(jo[jn].offs, nl, kb, kend - 1, a, b);
+    warp_bound_pair<true, true, uint32_t>(jo[jn].offs, nl, static_cast<uint32_t>(kb), static_cast<uint32_t>(kend - 1), a,
+                                          b);
     if ((threadIdx.x & 31) == 0)
       ranges[t] = make_uint4(static_cast<uint32_t>(a - 1), static_cast<uint32_t>(b), jn, 0u);
   }
@@ -604,8 +605,9 @@ __global__ void __launch_bounds__(kBlock, 5) bjoin_write_kernel(const JoinOut* _
       } else {
         j = tile_join_of(ostart, J, tile);
         const uint64_t kb = (tile - ostart[j]) * static_cast<uint64_t>(kTileRows), tot = jo[j].total;
-        warp_bound_pair<true, true, uint64_t>(jo[j].offs, jo[j].nl, kb, (kb + kTileRows < tot ? kb + kTileRows : tot) - 1,
-                                              a, b);
+        const uint64_t kend = kb + kTileRows < tot ? kb + kTileRows : tot;
+        warp_bound_pair<true, true, uint32_t>(jo[j].offs, jo[j].nl, static_cast<uint32_t>(kb),
+                                              static_cast<uint32_t>(kend - 1), a, b);
         --a;
       }
       if (threadIdx.x == 0) {
@@ -991,7 +993,7 @@ void launch_count(Ctx& ctx, const Tables& tb, const CountTables& ct, JoinBatch& 
     VG_CUDA(cudaGetLastError());
   }
   uint64_t* status = tb.at<uint64_t>(ct.zero);
-  ctx.launch("join_count_scan", ct.bytes + 12.0 * ct.rows, [&] {
+  ctx.launch("join_count_scan", ct.bytes + 8.0 * ct.rows, [&] {
     bjoin_count_scan_kernel<<<static_cast<unsigned>(ct.small_blocks + ct.T), kJcBlock, 0, ctx.stream>>>(
         tb.at<JoinSeg>(ct.js), tb.at<uint64_t>(ct.bstart), tb.at<uint32_t>(ct.tile_join), win ? win->get() : nullptr,
         tb.at<uint32_t>(ct.small), ct.nsmall, ct.small_blocks, jb.lo, jb.offs, status,
@@ -1023,7 +1025,7 @@ void batched_join_count(Ctx& ctx, const std::vector<const Rel*>& l, const std::v
   if (jb.J == 0) return;
   tb.send();
   jb.lo = ctx.alloc<uint32_t>(ct.rows);
-  jb.offs = ctx.alloc<uint64_t>(ct.rows);
+  jb.offs = ctx.alloc<uint32_t>(ct.rows);
   jb.d_totals = ctx.alloc<uint64_t>(jb.J);
   launch_count(ctx, tb, ct, jb);
   VG_CUDA(cudaMemcpyAsync(totals_host, jb.d_totals, jb.J * sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx.stream));
@@ -1121,7 +1123,7 @@ void batched_join_placed(Ctx& ctx, const std::vector<const Rel*>& l, const std::
   const uint32_t J = jb.J;
   if (J == 0) return;
   jb.lo = ctx.alloc<uint32_t>(ct.rows);
-  jb.offs = ctx.alloc<uint64_t>(ct.rows);
+  jb.offs = ctx.alloc<uint32_t>(ct.rows);
   jb.d_totals = ctx.alloc<uint64_t>(J);
   std::vector<JoinOut> jo(J);
   parallel_for(J, [&](size_t j) { describe_join(jb, j, jo[j]); });

@@ -68,7 +68,7 @@ struct JoinBatch {
   std::vector<const Rel*> l, r;
   std::vector<uint64_t> row0;   // offset of each join's left rows in lo/offs
   uint32_t* lo = nullptr;       // lower bound in r of every left key
-  uint64_t* offs = nullptr;     // exclusive scan of the match counts
+  uint32_t* offs = nullptr;     // exclusive scan of the match counts (of joins below 2^32 output rows)
   uint64_t* d_totals = nullptr; // every join's output rows, on the device
   // Frees lo, offs and d_totals (in stream order).
   void release(Ctx& ctx);

@@ -362,15 +362,21 @@ __device__ __forceinline__ void jc_count_staged(const uint32_t* __restrict__ L, 
   jc_search_staged<uint32_t>(win, static_cast<uint32_t>(w1 - w0), w0, i0, i_end, key, lov, cnt);
 }
 
-// A tile's lower bounds and output offsets, staged in the window's shared
-// memory after the search so that they leave in coalesced stores: element e
-// of the tile (thread e / 8's key e % 8) sits at e + e / 32 (lower bounds,
-// 32-bit) and at e + e / 16 of the 64-bit area (offsets), which keeps both
-// the per-thread writes and the row-order reads free of bank conflicts.
+// A tile's lower bounds and output offsets (from the tile's first), staged in
+// the window's shared memory after the search so that they leave in coalesced
+// stores: element e of the tile (thread e / 8's key e % 8) sits at e + e / 32
+// of the 32-bit lower bounds, and at e + e / 32 (32-bit) or e + e / 16 (64-bit)
+// of the offsets, which keeps both the per-thread writes and the row-order
+// reads free of bank conflicts.
 constexpr uint32_t kJcStageLoWords = kJcTile + kJcTile / 32;
 __device__ __forceinline__ uint32_t* jc_stage_lo(JoinCountSmem& sm) { return sm.keys; }
-__device__ __forceinline__ uint64_t* jc_stage_off(JoinCountSmem& sm) {
-  return reinterpret_cast<uint64_t*>(sm.keys + kJcStageLoWords);
+template <typename Off>
+__device__ __forceinline__ Off* jc_stage_off(JoinCountSmem& sm) {
+  return reinterpret_cast<Off*>(sm.keys + kJcStageLoWords);
+}
+template <typename Off>
+__device__ __forceinline__ uint32_t jc_stage_at(uint32_t e) {
+  return e + e / (sizeof(Off) == 8 ? 16 : 32);
 }
 static_assert(kJcStageLoWords % 2 == 0, "the 64-bit staging area starts 8-byte aligned");
 static_assert(kJcStageLoWords + 2 * (kJcTile + kJcTile / 16) <= kJcWindow, "staging fits in the window");
@@ -430,11 +436,14 @@ __device__ __forceinline__ void jc_count_staged_pairs(const PairKeys& L, uint64_
 // What follows a tile's count: a block scan and a look-back over the same
 // join's tiles [first_tile, tile) give every left row its output offset; the
 // join's last tile writes its total.  lo and offs are the join's own arrays
-// (left row i0 is the tile's first).  Every thread of the block calls it.
+// (left row i0 is the tile's first).  Off: 32 bits hold every offset of a join
+// that is written (one with 2^32 rows or more is refused, by its 64-bit total);
+// 64 bits for the join that takes any.  Every thread of the block calls it.
+template <typename Off>
 __device__ __forceinline__ void jc_finish_tile(uint64_t nl, uint64_t i0, const uint32_t (&lov)[kJcKeys],
                                                const uint32_t (&cnt)[kJcKeys], JoinCountSmem& sm, uint64_t* s_scan,
                                                uint64_t* s_b, uint64_t tile, uint64_t first_tile, bool last_tile,
-                                               uint32_t* __restrict__ lo, uint64_t* __restrict__ offs,
+                                               uint32_t* __restrict__ lo, Off* __restrict__ offs,
                                                uint64_t* status, uint64_t* total, DeviceErrors* err) {
   uint64_t sum = 0;
 #pragma unroll
@@ -450,13 +459,13 @@ __device__ __forceinline__ void jc_finish_tile(uint64_t nl, uint64_t i0, const u
     // lower bounds and tile-relative offsets staged in the window while warp 0
     // looks back; the tile's prefix is added when they are stored
     uint32_t* s_lo = jc_stage_lo(sm);
-    uint64_t* s_off = jc_stage_off(sm);
+    Off* s_off = jc_stage_off<Off>(sm);
     uint64_t run = e;
 #pragma unroll
     for (int k = 0; k < kJcKeys; ++k) {
       const uint32_t q = tid * kJcKeys + k;
       s_lo[q + q / 32] = lov[k];
-      s_off[q + q / 16] = run;
+      s_off[jc_stage_at<Off>(q)] = static_cast<Off>(run);
       run += cnt[k];
     }
   }
@@ -472,7 +481,7 @@ __device__ __forceinline__ void jc_finish_tile(uint64_t nl, uint64_t i0, const u
 #pragma unroll
     for (int k = 0; k < kJcKeys; ++k) {
       if (first + k < nl) {
-        offs[first + k] = run;
+        offs[first + k] = static_cast<Off>(run);
         lo[first + k] = lov[k];
       }
       run += cnt[k];
@@ -481,18 +490,20 @@ __device__ __forceinline__ void jc_finish_tile(uint64_t nl, uint64_t i0, const u
     return;
   }
   const uint32_t* s_lo = jc_stage_lo(sm);
-  const uint64_t* s_off = jc_stage_off(sm);
+  const Off* s_off = jc_stage_off<Off>(sm);
   for (uint32_t q = tid; q < tile_n; q += kJcBlock) {
     lo[i0 + q] = s_lo[q + q / 32];
-    offs[i0 + q] = base + s_off[q + q / 16];
+    offs[i0 + q] = static_cast<Off>(base) + s_off[jc_stage_at<Off>(q)];
   }
 }
 
 // A join to write: left rows' lower bounds and output offsets, source and
 // output columns (lc: the key columns and the other left ones, rc: the right
 // ones without the keys).
-struct JoinOut {
-  const uint64_t* offs;
+template <typename Off>
+struct JoinOutOf {
+  using Offset = Off;
+  const Off* offs;
   const uint32_t* lo;
   uint64_t nl, total;
   const uint32_t* lc[VG_MAX_COLS];
@@ -500,6 +511,7 @@ struct JoinOut {
   uint32_t* oc[VG_MAX_COLS];
   uint32_t nlc, nrc;
 };
+using JoinOut = JoinOutOf<uint32_t>;
 
 constexpr int kJwBlock = 256;
 
@@ -520,8 +532,8 @@ struct JwStage {
 // memory and each thread walks its rows (k increasing, consecutive threads on
 // consecutive rows, so loads and stores coalesce) from the previous one's left
 // row.  Hub keys thus spread over many blocks.
-template <int ROWS>
-__device__ __forceinline__ void jw_write_tile(const JoinOut& o, uint64_t kb, uint64_t kend, uint64_t ib, uint64_t ie,
+template <int ROWS, typename Off>
+__device__ __forceinline__ void jw_write_tile(const JoinOutOf<Off>& o, uint64_t kb, uint64_t kend, uint64_t ib, uint64_t ie,
                                               JwStage<ROWS>& st) {
   const uint64_t m64 = ie - ib;
   const bool staged = m64 <= JwStage<ROWS>::kMost;

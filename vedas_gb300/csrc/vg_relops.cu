@@ -179,10 +179,10 @@ __global__ void __launch_bounds__(kJcBlock) join_window_kernel(typename KeysOf<T
 // join_window_kernel where there are more tiles than the GPU runs at a time
 // (a block's own search is five rounds of global loads before its copy can
 // start), else warp 0 finds it.
-template <bool TWO>
+template <bool TWO, typename Off>
 __global__ void __launch_bounds__(kJcBlock, 4) join_count_scan_kernel(
     typename KeysOf<TWO>::K L, uint64_t nl, typename KeysOf<TWO>::K R, uint64_t nr, const uint2* __restrict__ win,
-    uint32_t* __restrict__ lo, uint64_t* __restrict__ offs, uint64_t* status, uint32_t* ticket, uint64_t* total,
+    uint32_t* __restrict__ lo, Off* __restrict__ offs, uint64_t* status, uint32_t* ticket, uint64_t* total,
     DeviceErrors* err) {
   __shared__ JoinCountSmem sm;
   __shared__ uint64_t s_scan[kJcBlock / 32 + 1];
@@ -227,14 +227,14 @@ struct JoinTail {
 static_assert(sizeof(JoinTail) <= Ctx::kSmallWords * sizeof(uint64_t), "the tail fits the small staging buffer");
 
 // Left rows [x, y) of every output tile, one warp per tile.
-__global__ void __launch_bounds__(kJwBlock) join_ranges_kernel(const uint64_t* __restrict__ offs, uint64_t nl,
+__global__ void __launch_bounds__(kJwBlock) join_ranges_kernel(const uint32_t* __restrict__ offs, uint64_t nl,
                                                                uint64_t total, uint64_t tiles, uint32_t tile_rows,
                                                                uint2* __restrict__ ranges) {
   const uint64_t nw = static_cast<uint64_t>(gridDim.x) * (kJwBlock / 32);
   for (uint64_t t = static_cast<uint64_t>(blockIdx.x) * (kJwBlock / 32) + (threadIdx.x >> 5); t < tiles; t += nw) {
     const uint64_t kb = t * tile_rows, kend = kb + tile_rows < total ? kb + tile_rows : total;
     uint64_t a, b;
-    warp_bound_pair<true, true, uint64_t>(offs, nl, kb, kend - 1, a, b);
+    warp_bound_pair<true, true, uint32_t>(offs, nl, static_cast<uint32_t>(kb), static_cast<uint32_t>(kend - 1), a, b);
     if ((threadIdx.x & 31) == 0) ranges[t] = make_uint2(static_cast<uint32_t>(a - 1), static_cast<uint32_t>(b));
   }
 }
@@ -244,12 +244,12 @@ __global__ void __launch_bounds__(kJwBlock) join_ranges_kernel(const uint64_t* _
 // the outputs then hold `cap` rows and nothing is written when there are
 // more.  Nothing is written either after a wait that gave up (the offsets are
 // wrong).  Ranges come from join_ranges_kernel or are found by warp 0.
-template <int ROWS>
-__global__ void __launch_bounds__(kJwBlock, 5) join_write_kernel(JoinOut o, const uint64_t* total_dev, uint64_t cap,
+template <int ROWS, typename Off>
+__global__ void __launch_bounds__(kJwBlock, 5) join_write_kernel(JoinOutOf<Off> o, const uint64_t* total_dev, uint64_t cap,
                                                                  const uint2* __restrict__ ranges,
                                                                  const DeviceErrors* err, JoinTail* tail) {
   constexpr uint32_t kTile = kJwBlock * ROWS;
-  __shared__ JoinOut s_o;
+  __shared__ JoinOutOf<Off> s_o;
   __shared__ JwStage<ROWS> s_stage;
   __shared__ uint64_t s_range[2];
   const uint64_t total = total_dev ? *total_dev : o.total;
@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(kJwBlock, 5) join_write_kernel(JoinOut o, cons
         a = r.x;
         b = r.y;
       } else {
-        warp_bound_pair<true, true, uint64_t>(s_o.offs, s_o.nl, kb, kend - 1, a, b);
+        warp_bound_pair<true, true, Off>(s_o.offs, s_o.nl, static_cast<Off>(kb), static_cast<Off>(kend - 1), a, b);
         --a;
       }
       if (threadIdx.x == 0) {
@@ -295,19 +295,20 @@ __global__ void __launch_bounds__(kJwBlock, 5) join_write_kernel(JoinOut o, cons
 // (blocks of one join that run at a time: 4 or 5 per SM)
 bool many_tiles(int num_sms, uint64_t tiles) { return tiles > 4ull * static_cast<uint64_t>(num_sms); }
 
-template <bool TWO>
+template <bool TWO, typename Off>
 void launch_count_scan(cudaStream_t stream, const Rel& l, const Rel& r, const uint2* win, uint32_t* lo,
-                       uint64_t* offs, uint64_t* status, uint32_t* ticket, uint64_t* total, DeviceErrors* err) {
+                       Off* offs, uint64_t* status, uint32_t* ticket, uint64_t* total, DeviceErrors* err) {
   const unsigned tiles = static_cast<unsigned>(div_up(l.nrows, kJcTile));
-  join_count_scan_kernel<TWO><<<tiles, kJcBlock, 0, stream>>>(
+  join_count_scan_kernel<TWO, Off><<<tiles, kJcBlock, 0, stream>>>(
       KeysOf<TWO>::of(l.cols[0], TWO ? l.cols[1] : nullptr), l.nrows,
       KeysOf<TWO>::of(r.cols[0], TWO ? r.cols[1] : nullptr), r.nrows, win, lo, offs, status, ticket, total, err);
   VG_CUDA(cudaGetLastError());
 }
 
-JoinOut join_out(const Rel& l, const Rel& r, uint32_t nk, const uint64_t* offs, const uint32_t* lo, uint64_t total,
-                 uint32_t* const* oc) {
-  JoinOut o{};
+template <typename Off>
+JoinOutOf<Off> join_out(const Rel& l, const Rel& r, uint32_t nk, const Off* offs, const uint32_t* lo, uint64_t total,
+                        uint32_t* const* oc) {
+  JoinOutOf<Off> o{};
   o.offs = offs;
   o.lo = lo;
   o.nl = l.nrows;
@@ -478,8 +479,8 @@ void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
   }
   const uint64_t tiles = div_up(l.nrows, kJcTile);
   if (tiles > 0x7FFFFFFFull) fail(VG_ERR_OVERFLOW, "join: too many tiles");
-  Scratch<uint32_t> lo(ctx, l.nrows);
-  Scratch<uint64_t> offs(ctx, l.nrows), z(ctx, tiles + 2);   // z: look-back words, total, ticket
+  Scratch<uint32_t> lo(ctx, l.nrows), offs(ctx, l.nrows);
+  Scratch<uint64_t> z(ctx, tiles + 2);   // look-back words, total, ticket
   uint64_t* total = z.get() + tiles;
   VG_CUDA(cudaMemsetAsync(z.get(), 0, (tiles + 2) * sizeof(uint64_t), ctx.stream));
   std::optional<Scratch<uint2>> win;
@@ -498,7 +499,7 @@ void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
     });
     VG_CUDA(cudaGetLastError());
   }
-  ctx.launch("join_count_scan", 4.0 * nk * (l.nrows + r.nrows) + 12.0 * l.nrows, [&] {
+  ctx.launch("join_count_scan", 4.0 * nk * (l.nrows + r.nrows) + 8.0 * l.nrows, [&] {
     const uint2* w = win ? win->get() : nullptr;
     auto* ticket = reinterpret_cast<uint32_t*>(total + 1);
     if (two_keys) launch_count_scan<true>(ctx.stream, l, r, w, lo.get(), offs.get(), z.get(), ticket, total, ctx.d_err);
@@ -536,7 +537,7 @@ void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
       const unsigned grid = static_cast<unsigned>(
           std::min<uint64_t>(div_up(cap, kJwBlock * kRowsSmall), static_cast<uint64_t>(ctx.num_sms) * 5));
       ctx.launch("join_write", 0.0, [&] {
-        join_write_kernel<kRowsSmall><<<grid, kJwBlock, 0, ctx.stream>>>(o, total, cap, nullptr, ctx.d_err, tail);
+        join_write_kernel<kRowsSmall, uint32_t><<<grid, kJwBlock, 0, ctx.stream>>>(o, total, cap, nullptr, ctx.d_err, tail);
       });
       VG_CUDA(cudaGetLastError());
       ctx.sync();
@@ -581,7 +582,7 @@ void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
     VG_CUDA(cudaGetLastError());
   }
   ctx.launch("join_write", 4.0 * t * (2.0 * ncols - 1), [&] {
-    join_write_kernel<kRows><<<static_cast<unsigned>(otiles), kJwBlock, 0, ctx.stream>>>(
+    join_write_kernel<kRows, uint32_t><<<static_cast<unsigned>(otiles), kJwBlock, 0, ctx.stream>>>(
         o, nullptr, t, ranges ? ranges->get() : nullptr, ctx.d_err, tail);
   });
   VG_CUDA(cudaGetLastError());
@@ -602,8 +603,8 @@ uint64_t join_into(cudaStream_t stream, const Rel& l, const Rel& r, uint32_t* co
   // a look-back that gave up leaves the offsets wrong: no write then
   if (he.timeout) fail(VG_ERR_TIMEOUT, "join_into: a bounded device wait expired");
   if (t == 0 || t > capacity) return t;
-  const JoinOut o = join_out(l, r, 1, offs, lo, t, out_cols);
-  join_write_kernel<kRows><<<static_cast<unsigned>(std::min<uint64_t>(div_up(t, kTileRows), 0x7FFFFFFFull)), kJwBlock,
+  const JoinOutOf<uint64_t> o = join_out(l, r, 1, offs, lo, t, out_cols);
+  join_write_kernel<kRows, uint64_t><<<static_cast<unsigned>(std::min<uint64_t>(div_up(t, kTileRows), 0x7FFFFFFFull)), kJwBlock,
                              0, stream>>>(o, nullptr, t, nullptr, err, nullptr);
   VG_CUDA(cudaGetLastError());
   return t;
