@@ -99,3 +99,23 @@ def test_swap_of_many_columns_in_a_full_arena():
         order = np.argsort(cols[0], kind="stable")
         for a, b in zip(rel.to_host(), cols):
             assert np.array_equal(a, b[order])
+
+
+@pytest.mark.parametrize("n", [3000, 2048 * 5 + 1, 300_007])
+@pytest.mark.parametrize("size", [1, 2, 63, 64, 65, 200, 5000])
+def test_rows_that_agree_in_their_top_bits(ctx, n, size):
+    """Wide rows in groups of `size` that differ in the last column only (the
+    first columns tell the groups apart), across tiles of 2048 rows."""
+    import vedas_gb300 as vg
+
+    rng = np.random.default_rng(n + size)
+    group = np.arange(n) // size
+    a = (rng.permutation(group.max() + 1) * 3)[group].astype(np.uint32)
+    cols = [a, np.full(n, 1 << 20, dtype=np.uint32), rng.integers(0, 1 << 22, size=n, dtype=np.uint32)]
+    order = rng.permutation(n)
+    cols = [c[order] for c in cols]
+    rel = vg.Relation.from_host(ctx, cols)
+    vg.sort_rows(ctx, rel)
+    for x, y in zip(rel.to_host(), lexsorted(cols)):
+        assert np.array_equal(x, y)
+    rel.free()

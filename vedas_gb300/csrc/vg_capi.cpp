@@ -83,6 +83,14 @@ void from_rel(const vg::Rel& r, vg_ir* ir) {
   for (uint32_t c = 0; c < r.ncols; ++c) ir->cols[c] = r.cols[c];
 }
 
+// The relation's columns back to the caller's, also when the call throws (it
+// may have replaced some of them).
+struct WriteBack {
+  vg::Rel& r;
+  vg_ir* ir;
+  ~WriteBack() { from_rel(r, ir); }
+};
+
 void check_ir(const vg_ir* ir) {
   if (!ir || ir->ncols == 0 || ir->ncols > VG_MAX_COLS) vg::fail(VG_ERR_INVALID, "bad relation");
 }
@@ -349,9 +357,8 @@ vg_status vg_sort_rows(vg_ctx* ctx, vg_ir* ir) {
   return guard([&] {
     check_ir(ir);
     vg::Rel r = to_rel(ir);
+    WriteBack back{r, ir};
     vg::sort_rows(ctx->c, r);
-    from_rel(r, ir);
-    ctx->c.check_device_errors();
   });
 }
 
@@ -360,8 +367,8 @@ vg_status vg_unique(vg_ctx* ctx, vg_ir* ir) {
   return guard([&] {
     check_ir(ir);
     vg::Rel r = to_rel(ir);
+    WriteBack back{r, ir};
     vg::unique_in_place(ctx->c, r);
-    from_rel(r, ir);
   });
 }
 

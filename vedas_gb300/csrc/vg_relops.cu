@@ -381,6 +381,88 @@ __global__ void __launch_bounds__(kBlock) unpack_rows_kernel(PackCols a, uint64_
   }
 }
 
+// What the host reads of a row sort (page-locked).
+struct RowsHost {
+  uint32_t big;        // a group of more than kRowGroup rows was left as it was
+  uint32_t pad;
+  DeviceErrors err;
+};
+struct RowsDone {      // zeroed before the launch
+  uint32_t big;
+  uint32_t done;
+};
+constexpr uint32_t kRowGroup = 64;
+
+// Keys in order of their top bits (equal under `top`) to rows in full order:
+// the rows of a group of equal top bits are ranked by whole keys, as the index
+// build ranks the objects of a subject and predicate.  The tile's keys, 64 on
+// either side and the group heads lie in shared memory; a row's place is the
+// number of rows of its group that go before it.
+__global__ void __launch_bounds__(kBlock) unpack_groups_kernel(PackCols a, uint64_t n, const uint64_t* __restrict__ keys,
+                                                               uint64_t top, RowsDone* st, const DeviceErrors* err,
+                                                               RowsHost* host) {
+  constexpr uint32_t kHalo = kRowGroup;
+  __shared__ uint64_t s_key[kTileRows + 2 * kHalo];
+  __shared__ uint32_t s_head[(kTileRows + 2 * kHalo) / 32];
+  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+  const uint64_t t0 = static_cast<uint64_t>(blockIdx.x) * kTileRows;
+  // every 32 rows of the tile and its halos: keys and heads (rows outside the
+  // relation count as heads)
+  for (uint32_t g = warp; g < (kTileRows + 2 * kHalo) / 32; g += kBlock / 32) {
+    const uint32_t x = g * 32 + lane;
+    const bool in = t0 + x >= kHalo && t0 + x - kHalo < n;
+    const uint64_t r = t0 + x - kHalo;
+    const uint64_t k = in ? keys[r] : 0ull;
+    uint64_t pv = __shfl_up_sync(0xffffffffu, k, 1);
+    if (lane == 0) pv = in && r > 0 ? keys[r - 1] : 0ull;
+    s_key[x] = k;
+    const uint32_t h = __ballot_sync(0xffffffffu, !in || r == 0 || ((k ^ pv) & top));
+    if (lane == 0) s_head[g] = h;
+  }
+  __syncthreads();
+  bool big = false;
+#pragma unroll 1
+  for (int i = 0; i < kRows; ++i) {
+    const uint32_t x = kHalo + warp * (32u * kRows) + i * 32u + lane, w = x >> 5;
+    const uint64_t r = t0 + x - kHalo;
+    if (r >= n) break;
+    const uint32_t upto = 0xffffffffu >> (31u - lane);   // bits 0..lane (x & 31 == lane)
+    // [b, e): the group, as far as it lies within 64 rows of this one
+    uint32_t b = 0, e = 0xffffffffu;
+    if (s_head[w] & upto) b = w * 32 + 31 - __clz(s_head[w] & upto);
+    else if (s_head[w - 1]) b = w * 32 - 1 - __clz(s_head[w - 1]);
+    else if (s_head[w - 2]) b = w * 32 - 33 - __clz(s_head[w - 2]);
+    if (s_head[w] & ~upto) e = w * 32 + __ffs(s_head[w] & ~upto) - 1;
+    else if (s_head[w + 1]) e = w * 32 + 31 + __ffs(s_head[w + 1]);
+    else if (s_head[w + 2]) e = w * 32 + 63 + __ffs(s_head[w + 2]);
+    const uint64_t mine = s_key[x];
+    uint32_t at = x;
+    // (b == 0 is not a found head: see the index build's kernel)
+    if (b != 0 && e != 0xffffffffu && e - b <= kRowGroup) {
+      at = b;
+      for (uint32_t j = b; j < e; ++j) {
+        const uint64_t v = s_key[j];
+        at += (v < mine || (v == mine && j < x)) ? 1u : 0u;
+      }
+    } else {
+      big = true;
+    }
+    const uint64_t to = t0 + at - kHalo;
+#pragma unroll
+    for (int c = 0; c < VG_MAX_COLS; ++c)
+      if (c < static_cast<int>(a.ncols)) a.col[c][to] = static_cast<uint32_t>((mine >> a.shift[c]) & a.mask[c]);
+  }
+  if (__syncthreads_or(big) && threadIdx.x == 0) atomicExch(&st->big, 1u);
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&st->done, 1u) == gridDim.x - 1) {
+      __threadfence();
+      host->big = atomicAdd(&st->big, 0u);
+      host->err = *err;
+    }
+  }
+}
+
 struct GatherCols {
   const uint32_t* in[VG_MAX_COLS];
   uint32_t* out[VG_MAX_COLS];
@@ -697,10 +779,14 @@ void sort_by_first(Ctx& ctx, Rel& r) {
   ctx.free(perm);
 }
 
-// Rows of at most 64 bits (each column as wide as its largest value): one
-// sort of packed keys, which hold the whole rows.  5M rows of three 19-bit
-// columns: 8 passes over 8-byte keys instead of 9 over keys and row numbers
-// and six gathers.
+// Rows of at most 64 bits (each column as wide as its largest value): a sort
+// of packed keys, which hold the whole rows.  Where the row count lets fewer
+// bits tell most rows apart (its own bits and 4 more), only that many top bits
+// are sorted by and the groups of rows that agree in them, a few each, are
+// ranked while the columns are unpacked; if some group has more than kRowGroup
+// rows, the keys are sorted by all bits after all.  5M rows of three 19-bit
+// columns: 4 passes over 8-byte keys instead of 9 over keys and row numbers
+// and six gathers.  Waits for the result and raises device errors.
 static bool sort_packed_rows(Ctx& ctx, Rel& r) {
   const uint64_t n = r.nrows;
   PackCols a{};
@@ -722,9 +808,15 @@ static bool sort_packed_rows(Ctx& ctx, Rel& r) {
     total += bits;
   }
   if (total > 64) return false;
-  if (total == 0) return true;   // equal rows throughout
+  if (total == 0) {   // equal rows throughout
+    ctx.check_device_errors();
+    return true;
+  }
+  // the top bits fill whole passes of seven bits
+  const uint32_t want = (64 - static_cast<uint32_t>(__builtin_clzll(n)) + 4 + 6) / 7 * 7;
+  const uint32_t low = want + 7 <= total ? total - want : 0;   // at least one pass saved
   std::vector<RadixDigit> digits;
-  radix_plan(digits, 0, static_cast<int>(total));
+  radix_plan(digits, static_cast<int>(low), static_cast<int>(total));
   DigitList dl{};
   dl.n = static_cast<uint32_t>(digits.size());
   for (uint32_t d = 0; d < dl.n; ++d) dl.d[d] = digits[d];
@@ -743,9 +835,26 @@ static bool sort_packed_rows(Ctx& ctx, Rel& r) {
     a.col[c] = r.cols[c];
   }
   r.borrowed = 0;
-  ctx.launch("sort_unpack", (8.0 + 4.0 * r.ncols) * n,
+  const double bytes = (8.0 + 4.0 * r.ncols) * n;
+  if (low) {
+    Scratch<RowsDone> st(ctx, 1);
+    VG_CUDA(cudaMemsetAsync(st.get(), 0, sizeof(RowsDone), ctx.stream));
+    auto* host = reinterpret_cast<RowsHost*>(ctx.h_small);
+    ctx.launch("sort_unpack", bytes, [&] {
+      unpack_groups_kernel<<<static_cast<unsigned>(div_up(n, kTileRows)), kBlock, 0, ctx.stream>>>(
+          a, n, keys.get(), ~0ull << low, st.get(), ctx.d_err, host);
+    });
+    VG_CUDA(cudaGetLastError());
+    ctx.sync();
+    ctx.raise_device_errors(host->err);
+    if (!host->big) return true;
+    if (radix_sort_u64(ctx, keys.get(), alt.get(), nullptr, nullptr, n, static_cast<int>(total), false))
+      std::swap(keys.p, alt.p);
+  }
+  ctx.launch("sort_unpack", bytes,
              [&] { unpack_rows_kernel<<<grid_for(ctx, n, 8), kBlock, 0, ctx.stream>>>(a, n, keys.get()); });
   VG_CUDA(cudaGetLastError());
+  ctx.check_device_errors();
   return true;
 }
 
@@ -772,6 +881,7 @@ void sort_rows(Ctx& ctx, Rel& r) {
   ctx.free(perm_alt);
   ctx.free(keys);
   ctx.free(keys_alt);
+  ctx.check_device_errors();
 }
 
 void unique_in_place(Ctx& ctx, Rel& r) {

@@ -62,7 +62,8 @@ void gather_cols(Ctx& ctx, const uint32_t* const* in, uint32_t* const* out, uint
 
 // Stable sort of the rows by column 0 (in place; columns are replaced).
 void sort_by_first(Ctx& ctx, Rel& r);
-// Lexicographic sort of the rows over all columns (in place).
+// Lexicographic sort of the rows over all columns (in place); waits for the
+// result and raises device errors.
 void sort_rows(Ctx& ctx, Rel& r);
 // Adjacent duplicate-row removal (synchronizes and raises device errors).  A
 // relation without any keeps its columns; views stay views.
