@@ -19,6 +19,7 @@
 #include "vg_index.h"
 
 #include <algorithm>
+#include <cstring>
 #include <optional>
 
 #include "vg_prims.cuh"
@@ -366,6 +367,13 @@ void column_max4(Ctx& ctx, const uint32_t* a, const uint32_t* b, const uint32_t*
   for (int i = 0; i < 4; ++i) out[i] = reinterpret_cast<const uint32_t*>(ctx.h_small)[i];
 }
 
+// Builds of at most kLateRows rows wait for the host once, when the largest
+// free block holds kLateBytes per row (the full index's outputs at full size
+// and two key buffers take 108, up to twice that in the arena's size classes):
+// 1.25 -> 1.18 ms for the full index of 3M triples.  With more rows a wait is a
+// small part.
+constexpr uint64_t kLateRows = 16u << 20, kLateBytes = 256;
+
 // The packed keys of one build and the sorts and unpackings over them.
 class Permuter {
  public:
@@ -373,7 +381,7 @@ class Permuter {
 
   Permuter(Ctx& ctx, const uint32_t* s, const uint32_t* p, const uint32_t* o, uint64_t n, const uint32_t mx[4],
            bool full)
-      : ctx_(ctx), n_(n), max_o_(mx[2]) {
+      : ctx_(ctx), n_(n), max_o_(mx[2]), late_(n <= kLateRows && ctx.arena.largest_free() >= kLateBytes * n) {
     // objects without the unused range below the literals
     const bool lits = mx[2] >= kLiteralStart;
     const uint32_t cut = lits ? kLiteralStart - mx[3] : 0;
@@ -465,25 +473,50 @@ class Permuter {
       else unpack_rle_kernel<false><<<static_cast<unsigned>(a.tiles), kBlock, 0, ctx.stream>>>(a);
     });
     VG_CUDA(cudaGetLastError());
-    VG_CUDA(cudaMemcpyAsync(ctx.h_small, z.get(), 3 * sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx.stream));
+    // counts and error record, read when the stream has got here
+    const size_t slot = pending_.size();
+    uint64_t* h = ctx.h_small + slot * kSlotWords;
+    VG_CUDA(cudaMemcpyAsync(h, z.get(), 3 * sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx.stream));
+    VG_CUDA(cudaMemcpyAsync(h + 3, ctx.d_err, sizeof(DeviceErrors), cudaMemcpyDeviceToHost, ctx.stream));
+    pending_.push_back({&out, a, groups});
+    if (!late_) finish();
+  }
+
+  // Waits for the unpackings enqueued so far and gives their outputs their
+  // sizes.
+  void finish() {
+    Ctx& ctx = ctx_;
+    const std::vector<Pending> all = std::move(pending_);
+    pending_.clear();
+    if (all.empty()) return;
     ctx.sync();
-    const uint64_t hc[3] = {ctx.h_small[0], ctx.h_small[1], ctx.h_small[2]};
-    ctx.check_device_errors();
-    out.col1 = DevArray(a.col1, a.col1 ? n : 0);
-    out.col2 = DevArray(a.col2, a.col2 ? n : 0);
-    if (a.l1_vals) {
-      ctx.arena.shrink(a.l1_vals, hc[0] * 4);
-      ctx.arena.shrink(a.l1_offs, hc[0] * 4);
-      out.l1_vals = DevArray(a.l1_vals, hc[0]);
-      out.l1_offs = DevArray(a.l1_offs, hc[0]);
+    uint64_t hc[kSlots][3];
+    for (size_t k = 0; k < all.size(); ++k) {
+      const uint64_t* h = ctx.h_small + k * kSlotWords;
+      std::copy(h, h + 3, hc[k]);
+      DeviceErrors he;
+      std::memcpy(&he, h + 3, sizeof(he));
+      ctx.raise_device_errors(he);
     }
-    if (a.l2_vals) {
-      ctx.arena.shrink(a.l2_vals, hc[1] * 4);
-      ctx.arena.shrink(a.l2_offs, hc[1] * 4);
-      out.l2_vals = DevArray(a.l2_vals, hc[1]);
-      out.l2_offs = DevArray(a.l2_offs, hc[1]);
+    for (size_t k = 0; k < all.size(); ++k) {
+      PermOutputs& out = *all[k].out;
+      const UnpackArgs& a = all[k].a;
+      out.col1 = DevArray(a.col1, a.col1 ? n_ : 0);
+      out.col2 = DevArray(a.col2, a.col2 ? n_ : 0);
+      if (a.l1_vals) {
+        ctx.arena.shrink(a.l1_vals, hc[k][0] * 4);
+        ctx.arena.shrink(a.l1_offs, hc[k][0] * 4);
+        out.l1_vals = DevArray(a.l1_vals, hc[k][0]);
+        out.l1_offs = DevArray(a.l1_offs, hc[k][0]);
+      }
+      if (a.l2_vals) {
+        ctx.arena.shrink(a.l2_vals, hc[k][1] * 4);
+        ctx.arena.shrink(a.l2_offs, hc[k][1] * 4);
+        out.l2_vals = DevArray(a.l2_vals, hc[k][1]);
+        out.l2_offs = DevArray(a.l2_offs, hc[k][1]);
+      }
+      if (all[k].groups && hc[k][2]) sort_big_groups(out);
     }
-    if (groups && hc[2]) sort_big_groups(out);
   }
 
  private:
@@ -492,9 +525,22 @@ class Permuter {
     std::vector<RadixDigit> digits;
     std::vector<const uint64_t*> bases;
   };
+  struct Pending {
+    PermOutputs* out;
+    UnpackArgs a;
+    bool groups;
+  };
+  static constexpr size_t kSlots = 6, kSlotWords = 4;   // unpackings, and the words the host reads of each
+  static_assert(sizeof(DeviceErrors) <= sizeof(uint64_t) && kSlots * kSlotWords <= Ctx::kSmallWords,
+                "the counts and error records fit the small staging buffer");
   Ctx& ctx_;
   uint64_t n_;
   uint32_t max_o_;
+  // Whether the host waits for all unpackings at the end only, so that no sort
+  // waits for it: the boundary arrays, made for as many runs as rows, then
+  // keep that size until the end.
+  bool late_;
+  std::vector<Pending> pending_;
   Field f_[3];
   std::vector<Sort> sorts_;
   std::optional<RadixCounts> counts_;       // digit counts and bases of every sort
@@ -578,6 +624,7 @@ uint32_t build_permutations(Ctx& ctx, const uint32_t* s, const uint32_t* p, cons
       keys.sort_by({C::S});
       keys.unpack(C::S, C::O, C::P, out.sop);
     }
+    keys.finish();
   }
   return std::max(mx[0], std::max(mx[1], mx[2]));
 }
