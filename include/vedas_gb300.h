@@ -171,7 +171,7 @@ vg_status vg_join(vg_ctx* ctx, const vg_ir* l, const vg_ir* r, vg_ir* out,
  * that may only launch work, cannot give the core an arena; this variant
  * keeps its scratch in a fixed file-scope device array instead, which caps
  * l_rows at 2,097,152 (larger inputs return VG_ERR_OVERFLOW) and costs about
- * 24 MiB on every GPU that loads the library, until the process exits.
+ * 27 MiB on every GPU that loads the library, until the process exits.
  * Columns are device pointers, column 0 of each side its sorted join key;
  * out_cols are l_ncols + r_ncols - 1 caller-allocated device buffers of
  * out_capacity rows.  *out_rows receives the result row count; when it

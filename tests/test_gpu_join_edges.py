@@ -121,3 +121,17 @@ def test_a_guess_that_does_not_fit_the_arena():
         assert out.nrows == rk.shape[0]
         for col in out.to_host():
             assert np.array_equal(col, rk)
+
+
+@pytest.mark.parametrize("gap", [0, 7, 8, 9, 2047, 2048, 4097, 32_760, 32_767, 32_768, 32_769, 32_784, 300_001])
+@pytest.mark.parametrize("nl", [400_000, (1 << 20) + 700_003])
+def test_left_rows_without_matches(ctx, nl, gap):
+    """Output tiles whose left rows lie far apart: runs of `gap` rows without
+    matches between rows with one or a few, and a hub at either end."""
+    lk = np.arange(nl, dtype=np.uint32)
+    at = np.arange(3, nl - 1, gap + 1, dtype=np.uint32)
+    times = np.ones(at.shape[0], dtype=np.int64)
+    times[::5] = 3
+    times[0] = times[-1] = 5000
+    rk = np.repeat(at, times)
+    check_one(ctx, [lk, lk ^ np.uint32(0x5555)], [rk, np.arange(rk.shape[0], dtype=np.uint32)])

@@ -353,28 +353,32 @@ struct JoinSeg {
   const uint32_t* lk;
   const uint32_t* rk;
   uint64_t nl, nr;
-  uint64_t row0;   // offset of this join's left rows in the lo/cnt/offs arrays
+  uint64_t row0;   // offset of this join's left rows in the count's arrays (whole groups)
 };
 
-// One block per tile of kJcTile left keys of one join, tiles taken in ticket
-// order (the tile's join from a per-tile table, one load instead of a search
-// of the join starts).  The tile's match counts stay in registers (the
+// A join's part of the wave's count arrays.
+__host__ __device__ __forceinline__ JoinCounts<uint32_t> join_counts(const JoinCounts<uint32_t>& all, uint64_t row0,
+                                                                     uint64_t tile0) {
+  return {all.lo + row0, all.offs + row0, all.start + row0 / kJcKeys, all.match + row0 / kJcKeys, all.base + tile0};
+}
+
+// One block per tile of kJcTile left keys of one join (the tile's join from a
+// per-tile table, one load instead of a search of the join starts).  The
 // right-key window, found beforehand by jc_window_kernel where there are more
-// tiles than run at a time, is staged by a bulk copy when it fits); their block scan
-// and a segmented decoupled look-back over the join's earlier tiles give
-// every left key its output offset directly, and the join's last tile writes
-// its total.
+// tiles than run at a time, is staged by a bulk copy when it fits; the tile's
+// match counts stay in registers, their block scan gives every left key its
+// output offset from the tile's first row, and the join's last tile to arrive
+// scans its tiles' totals (jc_finish_tile).
 //
 // Joins with at most kSmallJoin left rows (most joins of a wave have a few)
 // take one warp each instead: the first small_blocks blocks hold
 // kJcBlock / 32 such joins, one per warp.  The warp finds the join's window
 // of right keys with two 32-ary searches, each lane counts the matches of
 // its kJcKeys keys with lockstep searches in that window, and a warp scan
-// gives the offsets and the total (no shared memory, no look-back).
+// gives the offsets and the total (no shared memory).
 constexpr uint32_t kSmallJoin = 32 * kJcKeys;
 
-__device__ __forceinline__ void count_small_join(const JoinSeg& g, uint32_t* __restrict__ lo,
-                                                 uint32_t* __restrict__ offs, uint64_t* total) {
+__device__ __forceinline__ void count_small_join(const JoinSeg& g, const JoinCounts<uint32_t>& c, uint64_t* total) {
   const uint32_t lane = lane_id();
   const uint64_t nl = g.nl;
   const uint64_t w0 = warp_bound<false, uint32_t>(g.rk, 0, g.nr, g.lk[0]);
@@ -390,15 +394,23 @@ __device__ __forceinline__ void count_small_join(const JoinSeg& g, uint32_t* __r
   for (int q = 0; q < kJcKeys; ++q)
     if (first + q < nl) sum += ub[q] - lb[q];
   const uint64_t incl = warp_incl_scan64(sum);
-  uint64_t run = incl - sum;
+  if (first < nl) {
+    uint32_t run = static_cast<uint32_t>(incl - sum), match = 0;
+    c.start[lane] = run;
 #pragma unroll
-  for (int q = 0; q < kJcKeys; ++q)
-    if (first + q < nl) {
-      lo[g.row0 + first + q] = static_cast<uint32_t>(lb[q]);
-      offs[g.row0 + first + q] = static_cast<uint32_t>(run);
-      run += ub[q] - lb[q];
-    }
-  if (lane == 31) *total = incl;
+    for (int q = 0; q < kJcKeys; ++q)
+      if (first + q < nl) {
+        c.lo[first + q] = lb[q];
+        c.offs[first + q] = run;
+        run += ub[q] - lb[q];
+        match |= (ub[q] != lb[q] ? 1u : 0u) << q;
+      }
+    c.match[lane] = static_cast<uint8_t>(match);
+  }
+  if (lane == 31) {
+    *c.base = 0;
+    *total = incl;
+  }
 }
 
 // Every tile's right-key window [win.x, win.y) (one warp per tile, both ends
@@ -421,54 +433,42 @@ __global__ void __launch_bounds__(kJcBlock) jc_window_kernel(const JoinSeg* __re
   }
 }
 
-__global__ void __launch_bounds__(kJcBlock, 4) bjoin_count_scan_kernel(
+__global__ void __launch_bounds__(kJcBlock, 4) bjoin_count_kernel(
     const JoinSeg* __restrict__ js, const uint64_t* __restrict__ bstart, const uint32_t* __restrict__ tile_join,
     const uint2* __restrict__ win, const uint32_t* __restrict__ small, uint32_t nsmall, uint32_t small_blocks,
-    uint32_t* __restrict__ lo, uint32_t* __restrict__ offs, uint64_t* status, uint32_t* ticket,
-    uint64_t* __restrict__ totals, DeviceErrors* err) {
+    JoinCounts<uint32_t> all, uint32_t* done, uint64_t* __restrict__ totals, DeviceErrors* err) {
   if (blockIdx.x < small_blocks) {   // block-uniform: this block only counts small joins
     const uint64_t sj = static_cast<uint64_t>(blockIdx.x) * (kJcBlock / 32) + (threadIdx.x >> 5);
     if (sj < nsmall) {
       const uint32_t j = small[sj];
-      count_small_join(js[j], lo, offs, &totals[j]);
+      count_small_join(js[j], join_counts(all, js[j].row0, gridDim.x - small_blocks + sj), &totals[j]);
     }
     return;
   }
   __shared__ JoinCountSmem sm;
   __shared__ uint64_t s_scan[kJcBlock / 32 + 1];
-  __shared__ uint64_t s_b;
-  __shared__ uint32_t s_tile, s_j;
+  const uint32_t tile = blockIdx.x - small_blocks, j = tile_join[tile];
+  const JoinSeg g = js[j];
+  const uint32_t tile0 = static_cast<uint32_t>(bstart[j]), tiles = static_cast<uint32_t>(bstart[j + 1]) - tile0;
+  const uint64_t i0 = static_cast<uint64_t>(tile - tile0) * kJcTile, i1 = i0 + kJcTile < g.nl ? i0 + kJcTile : g.nl;
+  uint32_t key[kJcKeys];
+  jc_load_keys(g.lk, i0 + static_cast<uint64_t>(threadIdx.x) * kJcKeys, i1, key);
   if (threadIdx.x < 32) {
-    // the window's bulk copy starts before the block's first barrier
-    uint32_t t = 0;
-    if (threadIdx.x == 0) t = atomicAdd(ticket, 1u);
-    t = __shfl_sync(0xffffffffu, t, 0);
-    const uint32_t jj = tile_join[t];
     uint64_t w0, w1;
     if (win) {
-      const uint2 w = win[t];
+      const uint2 w = win[tile];
       w0 = w.x;
       w1 = w.y;
     } else {   // few tiles: found here
-      const uint64_t b = (t - bstart[jj]) * static_cast<uint64_t>(kJcTile);
-      const uint64_t e = (b + kJcTile < js[jj].nl ? b + kJcTile : js[jj].nl) - 1;
-      warp_window(js[jj].rk, js[jj].nr, js[jj].lk[b], js[jj].lk[e], w0, w1);
+      warp_window(g.rk, g.nr, g.lk[i0], g.lk[i1 - 1], w0, w1);
     }
-    if (threadIdx.x == 0) {
-      s_tile = t;
-      s_j = jj;
-      jc_issue_window(js[jj].rk, w0, w1, sm);
-    }
+    if (threadIdx.x == 0) jc_issue_window(g.rk, w0, w1, sm);
   }
   __syncthreads();
-  const uint64_t tile = s_tile;
-  const uint32_t j = s_j;
-  const JoinSeg g = js[j];
-  const uint64_t i0 = (tile - bstart[j]) * static_cast<uint64_t>(kJcTile);
   uint32_t cnt[kJcKeys], lov[kJcKeys];
-  jc_count_staged(g.lk, g.nl, g.rk, i0, lov, cnt, sm, err);
-  jc_finish_tile(g.nl, i0, lov, cnt, sm, s_scan, &s_b, tile, bstart[j], tile == bstart[j + 1] - 1, lo + g.row0,
-                 offs + g.row0, status, &totals[j], err);
+  jc_count_staged(key, g.nl, g.rk, i0, lov, cnt, sm, err);
+  jc_finish_tile(i0, lov, cnt, sm, s_scan, tile - tile0, tiles, g.nl, join_counts(all, g.row0, tile0), &done[j],
+                 &totals[j], err);
 }
 
 // Output rows [kb, kb + kTileRows) of one join per tile (the tile's join
@@ -512,11 +512,23 @@ __device__ __forceinline__ void write_small_join(const JoinOut* __restrict__ src
     __syncwarp();
   }
   const uint64_t total = jp->total, nl = jp->nl;
-  const uint32_t* offs = jp->offs;
-  const uint32_t* lov = jp->lo;
-  for (uint32_t e = lane; e < nl; e += 32) {
-    s_off[e] = offs[e];
-    s_lo[e] = lov[e];
+  // one tile (its base is 0), a group per lane; a row without matches gets the
+  // offset of the next one with
+  static_assert(kSmallJoin <= 32 * kJcKeys, "a group per lane");
+  const JoinCounts<uint32_t>& c = jp->cnt;
+  const uint32_t first = lane * kJcKeys;
+  uint32_t next = static_cast<uint32_t>(total);
+  const bool own = first < nl;
+  const uint32_t s = own ? c.start[lane] : static_cast<uint32_t>(total), match = own ? c.match[lane] : 0u;
+  const uint32_t after = __shfl_down_sync(0xffffffffu, s, 1);
+  if (lane < 31) next = after;
+#pragma unroll
+  for (int q = kJcKeys - 1; q >= 0; --q) {
+    if (match >> q & 1u) {
+      next = c.offs[first + q];
+      s_lo[first + q] = c.lo[first + q];
+    }
+    s_off[first + q] = next;
   }
   __syncwarp();
   const uint32_t nlc = jp->nlc, nrc = jp->nrc;
@@ -544,9 +556,9 @@ __device__ __forceinline__ uint32_t tile_join_of(const uint64_t* __restrict__ os
   return static_cast<uint32_t>(warp_bound<true, uint64_t>(ostart, 0, static_cast<uint64_t>(J) + 1, tile) - 1);
 }
 
-// Every output tile's left rows [x, y) and join z: x the last row whose output
-// starts at or before the tile's first row, y the first row whose output
-// starts after its last (one warp per tile, both searches at once), so that
+// Every output tile's groups [x, y) of left rows and join z: x the last group
+// whose output starts at or before the tile's first row, y the first one whose
+// output starts after its last (one warp per tile, both searches at once), so that
 // the writing blocks start staging at once.  T as for bjoin_write_kernel.
 __global__ void __launch_bounds__(kBlock) jw_range_kernel(const JoinOut* __restrict__ jo,
                                                           const uint64_t* __restrict__ ostart, uint32_t J,
@@ -556,12 +568,11 @@ __global__ void __launch_bounds__(kBlock) jw_range_kernel(const JoinOut* __restr
   const uint64_t nw = static_cast<uint64_t>(gridDim.x) * (kBlock / 32);
   for (uint64_t t = static_cast<uint64_t>(blockIdx.x) * (kBlock / 32) + (threadIdx.x >> 5); t < T; t += nw) {
     const uint32_t jn = tile_join_of(ostart, J, t);
-    const uint64_t total = jo[jn].total, nl = jo[jn].nl;
+    const uint64_t total = jo[jn].total, ng = jo[jn].ngroups();
     const uint64_t kb = (t - ostart[jn]) * static_cast<uint64_t>(kTileRows);
     const uint64_t kend = (kb + kTileRows < total) ? kb + kTileRows : total;
     uint64_t a, b;
-    warp_bound_pair<true, true, uint32_t>(jo[jn].offs, nl, static_cast<uint32_t>(kb), static_cast<uint32_t>(kend - 1), a,
-                                          b);
+    warp_bound_pair_of<true, true>(jo[jn].groups(), ng, static_cast<uint32_t>(kb), static_cast<uint32_t>(kend - 1), a, b);
     if ((threadIdx.x & 31) == 0)
       ranges[t] = make_uint4(static_cast<uint32_t>(a - 1), static_cast<uint32_t>(b), jn, 0u);
   }
@@ -576,7 +587,7 @@ __global__ void __launch_bounds__(kBlock, 5) bjoin_write_kernel(const JoinOut* _
                                                              const uint32_t* __restrict__ small, uint32_t nsmall_host,
                                                              const uint32_t* nsmall_dev, JoinEdges ed) {
   static_assert(kBlock == kJwBlock, "jw_write_tile's block");
-  static_assert(JwStage<kRows>::kMost >= (kBlock / 32) * kSmallJoin, "a warp's slice holds a small join's left rows");
+  static_assert(JwStage<kRows>::kTile >= (kBlock / 32) * kSmallJoin, "a warp's slice holds a small join's left rows");
   __shared__ JoinOut s_o;
   __shared__ JoinOut s_w[kBlock / 32];
   __shared__ JwStage<kRows> s_stage;
@@ -587,13 +598,14 @@ __global__ void __launch_bounds__(kBlock, 5) bjoin_write_kernel(const JoinOut* _
     const uint32_t warp = threadIdx.x >> 5, nwarps = kBlock / 32;
     for (uint64_t w = static_cast<uint64_t>(blockIdx.x) * nwarps + warp; w < nsm;
          w += static_cast<uint64_t>(gridDim.x) * nwarps)
-      write_small_join(&jo[small[w]], &s_w[warp], s_stage.off + warp * kSmallJoin, s_stage.lo + warp * kSmallJoin,
+      write_small_join(&jo[small[w]], &s_w[warp], s_stage.left + warp * kSmallJoin, s_stage.right + warp * kSmallJoin,
                        small[w], ed);
   }
   const uint64_t T = ostart_end ? *ostart_end : T_host;
 #pragma unroll 1
   for (uint64_t tile = blockIdx.x; tile < T; tile += gridDim.x) {
     __syncthreads();   // the previous tile's readers of the shared arrays are done
+    jw_clear(s_stage);
     if (threadIdx.x < 32) {
       uint32_t j;
       uint64_t a, b;
@@ -606,8 +618,8 @@ __global__ void __launch_bounds__(kBlock, 5) bjoin_write_kernel(const JoinOut* _
         j = tile_join_of(ostart, J, tile);
         const uint64_t kb = (tile - ostart[j]) * static_cast<uint64_t>(kTileRows), tot = jo[j].total;
         const uint64_t kend = kb + kTileRows < tot ? kb + kTileRows : tot;
-        warp_bound_pair<true, true, uint32_t>(jo[j].offs, jo[j].nl, static_cast<uint32_t>(kb),
-                                              static_cast<uint32_t>(kend - 1), a, b);
+        warp_bound_pair_of<true, true>(jo[j].groups(), jo[j].ngroups(), static_cast<uint32_t>(kb),
+                                       static_cast<uint32_t>(kend - 1), a, b);
         --a;
       }
       if (threadIdx.x == 0) {
@@ -669,8 +681,7 @@ __global__ void __launch_bounds__(kPlaceBlock) join_place_kernel(JoinOut* __rest
   __shared__ uint64_t s_scan[kPlaceBlock / 32 + 1];
   __shared__ unsigned long long s_fit;   // end of the placed outputs, after the bump
   const uint64_t bump0 = *pl.bump;
-  // a look-back that gave up leaves the totals and offsets wrong: nothing is
-  // written then, and the host raises the error
+  // after a wait that gave up nothing is written, and the host raises the error
   const DeviceErrors e = *pl.err;
   if (threadIdx.x == 0) s_fit = 0;
   uint64_t carry_b = 0, carry_t = 0, carry_s = 0;
@@ -933,7 +944,7 @@ uint64_t window_tiles(const Ctx& ctx) { return 2ull * static_cast<uint64_t>(ctx.
 
 // The tables of a wave's join count (and what follows it in the same stage).
 struct CountTables {
-  size_t js, bstart, tile_join, small, zero;
+  size_t js, bstart, tile_join, small, done;   // done: tiles counted, per join
   uint32_t nsmall = 0, small_blocks = 0;
   uint64_t T = 0, rows = 0;
   double bytes = 0;
@@ -950,6 +961,7 @@ CountTables count_tables(Ctx& ctx, Tables& tb, const std::vector<const Rel*>& l,
   std::vector<JoinSeg> js(J);
   std::vector<uint64_t> bstart(J + 1, 0);
   jb.row0.resize(J);
+  jb.base_at.resize(J);
   std::vector<uint32_t> small;   // joins counted by one warp each
   for (uint32_t j = 0; j < J; ++j) {
     if (l[j]->nrows == 0 || r[j]->nrows == 0) fail(VG_ERR_INVALID, "batched join of an empty relation");
@@ -958,7 +970,7 @@ CountTables count_tables(Ctx& ctx, Tables& tb, const std::vector<const Rel*>& l,
     if (l[j]->ncols + r[j]->ncols - 1 > VG_MAX_COLS) fail(VG_ERR_UNSUPPORTED, "join output has more than 9 columns");
     js[j] = {l[j]->cols[0], r[j]->cols[0], l[j]->nrows, r[j]->nrows, ct.rows};
     jb.row0[j] = ct.rows;
-    ct.rows += l[j]->nrows;
+    ct.rows += div_up(l[j]->nrows, kJcKeys) * kJcKeys;
     const bool is_small = l[j]->nrows <= std::min<uint32_t>(kSmallJoin, ctx.tune.join_small_rows);
     if (is_small) small.push_back(j);
     bstart[j + 1] = bstart[j] + (is_small ? 0 : div_up(l[j]->nrows, kJcTile));
@@ -968,6 +980,8 @@ CountTables count_tables(Ctx& ctx, Tables& tb, const std::vector<const Rel*>& l,
   if (ct.T > 0x7FFFFFFFull) fail(VG_ERR_OVERFLOW, "batched join count: too many tiles");
   ct.nsmall = static_cast<uint32_t>(small.size());
   ct.small_blocks = static_cast<uint32_t>(div_up(ct.nsmall, kJcBlock / 32));
+  for (uint32_t j = 0; j < J; ++j) jb.base_at[j] = bstart[j];
+  for (uint32_t s = 0; s < ct.nsmall; ++s) jb.base_at[small[s]] = ct.T + s;   // after the tiles'
   std::vector<uint32_t> tile_join(ct.T);
   for (uint32_t j = 0; j < J; ++j)
     for (uint64_t t = bstart[j]; t < bstart[j + 1]; ++t) tile_join[t] = j;
@@ -975,12 +989,22 @@ CountTables count_tables(Ctx& ctx, Tables& tb, const std::vector<const Rel*>& l,
   ct.bstart = tb.add(bstart);
   ct.tile_join = tb.add(tile_join);
   ct.small = tb.add(small);
-  ct.zero = tb.zeros<uint64_t>(ct.T + 1);   // look-back words, then the ticket
+  ct.done = tb.zeros<uint32_t>(J);
   return ct;
 }
 
-// Enqueues the count of the joins (tables sent): jb.lo, jb.offs and
-// jb.d_totals, which must hold J words.
+// Device arrays of a count: before the joins are described.
+void alloc_count(Ctx& ctx, const CountTables& ct, JoinBatch& jb) {
+  const uint64_t groups = ct.rows / kJcKeys;
+  jb.cnt.lo = ctx.alloc<uint32_t>(ct.rows);
+  jb.cnt.offs = ctx.alloc<uint32_t>(ct.rows);
+  jb.cnt.start = ctx.alloc<uint32_t>(div_up(groups, 4) * 4 + div_up(groups, 16) * 4);   // and the match bits
+  jb.cnt.match = reinterpret_cast<uint8_t*>(jb.cnt.start + div_up(groups, 4) * 4);
+  jb.d_totals = ctx.alloc<uint64_t>(jb.J + ct.T + ct.nsmall);
+  jb.cnt.base = jb.d_totals + jb.J;
+}
+
+// Enqueues the count of the joins (tables sent): jb.cnt and jb.d_totals.
 void launch_count(Ctx& ctx, const Tables& tb, const CountTables& ct, JoinBatch& jb) {
   std::optional<Scratch<uint2>> win;
   if (ct.T > window_tiles(ctx)) {
@@ -992,12 +1016,10 @@ void launch_count(Ctx& ctx, const Tables& tb, const CountTables& ct, JoinBatch& 
     });
     VG_CUDA(cudaGetLastError());
   }
-  uint64_t* status = tb.at<uint64_t>(ct.zero);
-  ctx.launch("join_count_scan", ct.bytes + 8.0 * ct.rows, [&] {
-    bjoin_count_scan_kernel<<<static_cast<unsigned>(ct.small_blocks + ct.T), kJcBlock, 0, ctx.stream>>>(
+  ctx.launch("join_count", ct.bytes + 8.0 * ct.rows, [&] {
+    bjoin_count_kernel<<<static_cast<unsigned>(ct.small_blocks + ct.T), kJcBlock, 0, ctx.stream>>>(
         tb.at<JoinSeg>(ct.js), tb.at<uint64_t>(ct.bstart), tb.at<uint32_t>(ct.tile_join), win ? win->get() : nullptr,
-        tb.at<uint32_t>(ct.small), ct.nsmall, ct.small_blocks, jb.lo, jb.offs, status,
-        reinterpret_cast<uint32_t*>(status + ct.T), jb.d_totals, ctx.d_err);
+        tb.at<uint32_t>(ct.small), ct.nsmall, ct.small_blocks, jb.cnt, tb.at<uint32_t>(ct.done), jb.d_totals, ctx.d_err);
   });
   VG_CUDA(cudaGetLastError());
 }
@@ -1007,8 +1029,7 @@ void describe_join(const JoinBatch& jb, size_t j, JoinOut& o) {
   const Rel* l = jb.l[j];
   const Rel* r = jb.r[j];
   std::memset(&o, 0, sizeof(o));
-  o.offs = jb.offs + jb.row0[j];
-  o.lo = jb.lo + jb.row0[j];
+  o.cnt = join_counts(jb.cnt, jb.row0[j], jb.base_at[j]);
   o.nl = l->nrows;
   for (uint32_t c = 0; c < l->ncols; ++c) o.lc[c] = l->cols[c];
   for (uint32_t c = 1; c < r->ncols; ++c) o.rc[c - 1] = r->cols[c];
@@ -1024,9 +1045,7 @@ void batched_join_count(Ctx& ctx, const std::vector<const Rel*>& l, const std::v
   const CountTables ct = count_tables(ctx, tb, l, r, jb);
   if (jb.J == 0) return;
   tb.send();
-  jb.lo = ctx.alloc<uint32_t>(ct.rows);
-  jb.offs = ctx.alloc<uint32_t>(ct.rows);
-  jb.d_totals = ctx.alloc<uint64_t>(jb.J);
+  alloc_count(ctx, ct, jb);
   launch_count(ctx, tb, ct, jb);
   VG_CUDA(cudaMemcpyAsync(totals_host, jb.d_totals, jb.J * sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx.stream));
 }
@@ -1122,9 +1141,7 @@ void batched_join_placed(Ctx& ctx, const std::vector<const Rel*>& l, const std::
   const CountTables ct = count_tables(ctx, tb, l, r, jb);
   const uint32_t J = jb.J;
   if (J == 0) return;
-  jb.lo = ctx.alloc<uint32_t>(ct.rows);
-  jb.offs = ctx.alloc<uint32_t>(ct.rows);
-  jb.d_totals = ctx.alloc<uint64_t>(J);
+  alloc_count(ctx, ct, jb);
   std::vector<JoinOut> jo(J);
   parallel_for(J, [&](size_t j) { describe_join(jb, j, jo[j]); });
   const size_t oj = tb.add(jo), oslot = tb.add(c0_slot);
@@ -1160,11 +1177,11 @@ void batched_join_placed(Ctx& ctx, const std::vector<const Rel*>& l, const std::
 }
 
 void JoinBatch::release(Ctx& ctx) {
-  ctx.free(lo);
-  ctx.free(offs);
-  ctx.free(d_totals);
-  lo = nullptr;
-  offs = nullptr;
+  ctx.free(cnt.lo);
+  ctx.free(cnt.offs);
+  ctx.free(cnt.start);   // and match
+  ctx.free(d_totals);    // and base
+  cnt = {};
   d_totals = nullptr;
 }
 

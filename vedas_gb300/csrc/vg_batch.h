@@ -66,11 +66,10 @@ void batched_sort_by_first(Ctx& ctx, const std::vector<Rel*>& rels, int key_bits
 struct JoinBatch {
   uint32_t J = 0;
   std::vector<const Rel*> l, r;
-  std::vector<uint64_t> row0;   // offset of each join's left rows in lo/offs
-  uint32_t* lo = nullptr;       // lower bound in r of every left key
-  uint32_t* offs = nullptr;     // exclusive scan of the match counts (of joins below 2^32 output rows)
+  std::vector<uint64_t> row0, base_at;   // offsets of each join's left rows and tiles in cnt's arrays
+  JoinCounts<uint32_t> cnt{};
   uint64_t* d_totals = nullptr; // every join's output rows, on the device
-  // Frees lo, offs and d_totals (in stream order).
+  // Frees the arrays (in stream order).
   void release(Ctx& ctx);
 };
 void batched_join_count(Ctx& ctx, const std::vector<const Rel*>& l, const std::vector<const Rel*>& r, JoinBatch& jb,

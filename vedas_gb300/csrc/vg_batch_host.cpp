@@ -444,7 +444,7 @@ WaveEngine::~WaveEngine() {
   {
     ThreadExecScope sc(exec());   // the stream is idle: frees go back at once
     for (auto& r : jouts_) rel_free(ctx_, r);
-    if (jb_.lo || jb_.offs || jb_.d_totals) jb_.release(ctx_);
+    if (jb_.cnt.lo || jb_.cnt.offs || jb_.cnt.start || jb_.d_totals) jb_.release(ctx_);
     if (d_bump_) ctx_.free(d_bump_);
   }
   ctx_.flush(defer_);   // the stream is idle: every held-back free is safe now

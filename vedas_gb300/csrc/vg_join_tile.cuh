@@ -3,11 +3,12 @@
 #pragma once
 
 #include "vg_prims.cuh"
+#include "vg_relops.h"
 
 namespace vg {
 
 constexpr int kJcBlock = 256;
-constexpr int kJcKeys = 8;                      // left keys per thread, consecutive
+constexpr int kJcKeys = kJoinGroup;             // left keys per thread, consecutive
 constexpr int kJcTile = kJcBlock * kJcKeys;     // 2048 left keys per block
 constexpr int kJcWindow = 11264;                // right keys staged per block (44 KiB)
 
@@ -243,10 +244,12 @@ __device__ __forceinline__ void jc_issue_window(const uint32_t* __restrict__ R, 
 // last repeated past the end) in a staged window of n right keys, whose first
 // is right row w0.  The lower bounds of the first and last key are searched in
 // lockstep over the window (a number of steps that the block shares), the
-// others in lockstep between those two (as many steps as the warp's widest
-// range takes; every lane of the warp calls this): no lane waits for another's loop, where galloping from key to
-// key left 18 of 32 lanes active.  The upper bound of a key that matches
-// gallops from its lower bound; equal keys share both.
+// others in lockstep between those two, and then the upper bounds of the keys
+// that match, each before the next key's lower bound (both as many steps as
+// the warp's widest range takes; every lane of the warp calls this): no lane
+// waits for another's loop, where galloping from key to key left 18 of 32
+// lanes active.  Equal keys share their bounds.  A key that the next thread
+// has too, and the warp's last, gallop to their upper bound.
 template <typename T>
 __device__ __forceinline__ void jc_search_staged(const T* win, uint32_t n, uint64_t w0, uint64_t i0, uint64_t i_end,
                                                  const T (&key)[kJcKeys], uint32_t (&lov)[kJcKeys],
@@ -280,16 +283,68 @@ __device__ __forceinline__ void jc_search_staged(const T* win, uint32_t n, uint6
       if (half) lo[j] = win[lo[j] + half - 1] < key[j] ? lo[j] + half : lo[j];
     len -= half;
   }
-  uint32_t phi = 0;
+  // upper bounds: range[j] right keys from lo[j] on may equal key j
+  uint32_t hi[kJcKeys], most = 0;
+#pragma unroll
+  for (int j = 0; j < kJcKeys; ++j) hi[j] = lo[j];
+  const T next_key = __shfl_down_sync(0xffffffffu, key[0], 1);
+  const uint32_t next_lo = __shfl_down_sync(0xffffffffu, lo[0], 1);
+  const bool last_own = lane_id() < 31 && next_key != key[kJcKeys - 1];
+  uint32_t match = 0;   // keys whose upper bound the lockstep finds
 #pragma unroll
   for (int j = 0; j < kJcKeys; ++j) {
-    if (first + j < i_end) {
-      const uint32_t hi = (j > 0 && key[j] == key[j - 1]) ? phi : smem_gallop<true, T>(win, lo[j], n, key[j]);
-      lov[j] = static_cast<uint32_t>(w0 + lo[j]);
-      cnt[j] = hi - lo[j];
-      phi = hi;
+    const uint32_t to = j + 1 < kJcKeys ? lo[j + 1] : next_lo;
+    const bool own = j + 1 < kJcKeys ? key[j + 1] != key[j] : last_own;
+    if (own && to > lo[j] && win[lo[j]] == key[j]) {
+      match |= 1u << j;
+      hi[j] = lo[j] + 1;
+      most = max(most, to - lo[j] - 1);
     }
   }
+  for (most = __reduce_max_sync(0xffffffffu, most); most > 0;) {
+    const uint32_t half = (most + 1) >> 1;
+#pragma unroll
+    for (int j = 0; j < kJcKeys; ++j) {
+      const uint32_t at = hi[j] + half - 1;
+      if ((match >> j & 1u) && at < n && win[at] <= key[j]) hi[j] += half;
+    }
+    most -= half;
+  }
+  if (!last_own) hi[kJcKeys - 1] = smem_gallop<true, T>(win, lo[kJcKeys - 1], n, key[kJcKeys - 1]);
+#pragma unroll
+  for (int j = kJcKeys - 2; j >= 0; --j)
+    if (key[j] == key[j + 1]) hi[j] = hi[j + 1];
+#pragma unroll
+  for (int j = 0; j < kJcKeys; ++j)
+    if (first + j < i_end) {
+      lov[j] = static_cast<uint32_t>(w0 + lo[j]);
+      cnt[j] = max(hi[j], lo[j]) - lo[j];   // (keys out of order match nothing rather than 2^32 rows)
+    }
+}
+
+// The thread's left keys: L[first, first + kJcKeys), the last of the tile
+// repeated past its end.
+__device__ __forceinline__ void jc_load_keys(const uint32_t* __restrict__ L, uint64_t first, uint64_t i_end,
+                                             uint32_t (&key)[kJcKeys]) {
+  static_assert(kJcKeys == 8, "the vector loads take 8 keys");
+  if (first + kJcKeys <= i_end && (reinterpret_cast<uintptr_t>(L + first) & 15u) == 0) {
+    const uint4 a = *reinterpret_cast<const uint4*>(L + first);
+    const uint4 b = *reinterpret_cast<const uint4*>(L + first + 4);
+    key[0] = a.x, key[1] = a.y, key[2] = a.z, key[3] = a.w;
+    key[4] = b.x, key[5] = b.y, key[6] = b.z, key[7] = b.w;
+  } else {
+#pragma unroll
+    for (int j = 0; j < kJcKeys; ++j) key[j] = L[first + j < i_end ? first + j : i_end - 1];
+  }
+}
+__device__ __forceinline__ void jc_load_keys(const PairKeys& L, uint64_t first, uint64_t i_end,
+                                             uint64_t (&key)[kJcKeys]) {
+#pragma unroll
+  for (int j = 0; j < kJcKeys; ++j) key[j] = L(first + j < i_end ? first + j : i_end - 1);
+}
+__device__ __forceinline__ void jc_load_keys(const OneKeys& L, uint64_t first, uint64_t i_end,
+                                             uint32_t (&key)[kJcKeys]) {
+  jc_load_keys(L.c0, first, i_end, key);
 }
 
 // Lower bound (in R) and match count of L[i0, min(i0 + kJcTile, nl)), given
@@ -297,10 +352,10 @@ __device__ __forceinline__ void jc_search_staged(const T* win, uint32_t n, uint6
 // in it.  A staged window is searched in shared memory; one that does not
 // fit (a heavy key, or a right side much longer than the left) is searched in
 // global memory with lockstep bounds instead.
-// The tile's counts stay in registers: thread t holds the counts of left
-// keys i0 + 8t .. i0 + 8t + 7 in cnt[] and their lower bounds in lov[] (zero
-// past the end).  Every thread of the block must call it.
-__device__ __forceinline__ void jc_count_staged(const uint32_t* __restrict__ L, uint64_t nl,
+// Thread t holds left keys i0 + 8t .. i0 + 8t + 7 in key[] (jc_load_keys, before
+// the barrier, so that their loads are in flight with the window's), and gets
+// their counts in cnt[] and lower bounds in lov[] (zero past the end).  Every thread of the block must call it.
+__device__ __forceinline__ void jc_count_staged(const uint32_t (&key)[kJcKeys], uint64_t nl,
                                                 const uint32_t* __restrict__ R, uint64_t i0,
                                                 uint32_t (&lov)[kJcKeys], uint32_t (&cnt)[kJcKeys],
                                                 JoinCountSmem& sm, DeviceErrors* err) {
@@ -312,23 +367,7 @@ __device__ __forceinline__ void jc_count_staged(const uint32_t* __restrict__ L, 
   const uint64_t w0 = sm.w0, w1 = sm.w1 > sm.w0 ? sm.w1 : sm.w0;
   const uint32_t staged = sm.staged;
   const uint64_t base = ((w0 + mis) & ~3ull) - mis;
-  // the thread's left keys are loaded while the window's bulk copy is in flight
   const uint64_t first = i0 + static_cast<uint64_t>(tid) * kJcKeys;
-  uint32_t key[kJcKeys];
-  if (first + kJcKeys <= i_end && (reinterpret_cast<uintptr_t>(L + first) & 15u) == 0) {
-    // two 16-byte loads (the thread's keys are consecutive)
-    const uint4 a = *reinterpret_cast<const uint4*>(L + first);
-    const uint4 b = *reinterpret_cast<const uint4*>(L + first + 4);
-    key[0] = a.x, key[1] = a.y, key[2] = a.z, key[3] = a.w;
-    key[4] = b.x, key[5] = b.y, key[6] = b.z, key[7] = b.w;
-  } else {
-#pragma unroll
-    for (int j = 0; j < kJcKeys; ++j) {
-      const uint64_t i = first + j;
-      key[j] = L[i < i_end ? i : i_end - 1];
-    }
-  }
-  static_assert(kJcKeys == 8, "the vector loads above take 8 keys");
   if (staged) {
     const uint64_t a0 = (staged == 2) ? ((w0 + mis + 3) & ~3ull) - mis : w1;
     const uint64_t a1 = (staged == 2) ? ((w1 + mis) & ~3ull) - mis : w1;
@@ -362,25 +401,6 @@ __device__ __forceinline__ void jc_count_staged(const uint32_t* __restrict__ L, 
   jc_search_staged<uint32_t>(win, static_cast<uint32_t>(w1 - w0), w0, i0, i_end, key, lov, cnt);
 }
 
-// A tile's lower bounds and output offsets (from the tile's first), staged in
-// the window's shared memory after the search so that they leave in coalesced
-// stores: element e of the tile (thread e / 8's key e % 8) sits at e + e / 32
-// of the 32-bit lower bounds, and at e + e / 32 (32-bit) or e + e / 16 (64-bit)
-// of the offsets, which keeps both the per-thread writes and the row-order
-// reads free of bank conflicts.
-constexpr uint32_t kJcStageLoWords = kJcTile + kJcTile / 32;
-__device__ __forceinline__ uint32_t* jc_stage_lo(JoinCountSmem& sm) { return sm.keys; }
-template <typename Off>
-__device__ __forceinline__ Off* jc_stage_off(JoinCountSmem& sm) {
-  return reinterpret_cast<Off*>(sm.keys + kJcStageLoWords);
-}
-template <typename Off>
-__device__ __forceinline__ uint32_t jc_stage_at(uint32_t e) {
-  return e + e / (sizeof(Off) == 8 ? 16 : 32);
-}
-static_assert(kJcStageLoWords % 2 == 0, "the 64-bit staging area starts 8-byte aligned");
-static_assert(kJcStageLoWords + 2 * (kJcTile + kJcTile / 16) <= kJcWindow, "staging fits in the window");
-
 // Called by one thread after the block's last use of the window: a bulk copy
 // whose wait gave up may still be in flight into this block's shared memory,
 // and must land before the block exits (bounded again; a copy that still has
@@ -399,8 +419,8 @@ __device__ __forceinline__ void jc_issue_pair_window(uint64_t w0, uint64_t w1, J
 }
 
 // jc_count_staged for keys of two columns.
-__device__ __forceinline__ void jc_count_staged_pairs(const PairKeys& L, uint64_t nl, const PairKeys& R, uint64_t i0,
-                                                      uint32_t (&lov)[kJcKeys], uint32_t (&cnt)[kJcKeys],
+__device__ __forceinline__ void jc_count_staged_pairs(const uint64_t (&key)[kJcKeys], uint64_t nl, const PairKeys& R,
+                                                      uint64_t i0, uint32_t (&lov)[kJcKeys], uint32_t (&cnt)[kJcKeys],
                                                       JoinCountSmem& sm) {
 #pragma unroll
   for (int j = 0; j < kJcKeys; ++j) cnt[j] = lov[j] = 0;
@@ -408,12 +428,6 @@ __device__ __forceinline__ void jc_count_staged_pairs(const PairKeys& L, uint64_
   const uint64_t i_end = (i0 + kJcTile < nl) ? i0 + kJcTile : nl;
   const uint64_t w0 = sm.w0, w1 = sm.w1 > sm.w0 ? sm.w1 : sm.w0;
   const uint64_t first = i0 + static_cast<uint64_t>(tid) * kJcKeys;
-  uint64_t key[kJcKeys];
-#pragma unroll
-  for (int j = 0; j < kJcKeys; ++j) {
-    const uint64_t i = first + j;
-    key[j] = L(i < i_end ? i : i_end - 1);
-  }
   uint64_t* win = reinterpret_cast<uint64_t*>(sm.keys);
   if (sm.staged)
     for (uint64_t e = w0 + tid; e < w1; e += kJcBlock) win[e - w0] = R(e);
@@ -433,169 +447,245 @@ __device__ __forceinline__ void jc_count_staged_pairs(const PairKeys& L, uint64_
     }
 }
 
-// What follows a tile's count: a block scan and a look-back over the same
-// join's tiles [first_tile, tile) give every left row its output offset; the
-// join's last tile writes its total.  lo and offs are the join's own arrays
-// (left row i0 is the tile's first).  Off: 32 bits hold every offset of a join
-// that is written (one with 2^32 rows or more is refused, by its 64-bit total);
-// 64 bits for the join that takes any.  Every thread of the block calls it.
+constexpr uint32_t kJcTileGroups = kJcTile / kJcKeys;
+
+// What follows a tile's count: a block scan gives every left row its output
+// offset from the tile's first, and base[tile] becomes the tile's first output
+// row: the join's last tile to arrive scans the tiles' totals and writes the
+// join's.  No tile waits for another (a look-back over the earlier tiles'
+// totals kept the block's warps at a barrier for 8.3 of 18 stall cycles an
+// instruction; 16M left rows took 163 us, 109 us without it).
+// c and done (zero at first) are the join's own; left row i0 is the tile's
+// first.  Every thread of the block calls it.
 template <typename Off>
-__device__ __forceinline__ void jc_finish_tile(uint64_t nl, uint64_t i0, const uint32_t (&lov)[kJcKeys],
-                                               const uint32_t (&cnt)[kJcKeys], JoinCountSmem& sm, uint64_t* s_scan,
-                                               uint64_t* s_b, uint64_t tile, uint64_t first_tile, bool last_tile,
-                                               uint32_t* __restrict__ lo, Off* __restrict__ offs,
-                                               uint64_t* status, uint64_t* total, DeviceErrors* err) {
+__device__ __forceinline__ void jc_finish_tile(uint64_t i0, const uint32_t (&lov)[kJcKeys], const uint32_t (&cnt)[kJcKeys],
+                                               JoinCountSmem& sm, uint64_t* s_scan, uint32_t tile, uint32_t tiles,
+                                               uint64_t nl, const JoinCounts<Off>& c, uint32_t* done, uint64_t* total,
+                                               DeviceErrors* err) {
+  __shared__ uint32_t s_last;
   uint64_t sum = 0;
 #pragma unroll
   for (int k = 0; k < kJcKeys; ++k) sum += cnt[k];
   uint64_t tot;
   const uint64_t e = block_excl_scan64<kJcBlock>(sum, tot, s_scan);   // every thread is past its search
   const uint32_t tid = threadIdx.x;
-  const uint64_t first = i0 + static_cast<uint64_t>(tid) * kJcKeys;
-  const uint32_t tile_n = static_cast<uint32_t>(nl - i0 < kJcTile ? nl - i0 : kJcTile);
-  // a bulk copy that gave up may still land in the window: no staging there
-  const bool stage = !(sm.staged == 2 && sm.failed);
-  if (stage) {
-    // lower bounds and tile-relative offsets staged in the window while warp 0
-    // looks back; the tile's prefix is added when they are stored
-    uint32_t* s_lo = jc_stage_lo(sm);
-    Off* s_off = jc_stage_off<Off>(sm);
-    uint64_t run = e;
-#pragma unroll
-    for (int k = 0; k < kJcKeys; ++k) {
-      const uint32_t q = tid * kJcKeys + k;
-      s_lo[q + q / 32] = lov[k];
-      s_off[jc_stage_at<Off>(q)] = static_cast<Off>(run);
-      run += cnt[k];
+  if (tid == 0) {
+    jc_drain_window(sm, err);
+    if (tiles == 1) {
+      c.base[0] = 0;
+      *total = tot;
+    } else {   // (before the thread's stores of rows, which the fence would wait for)
+      __stcg(reinterpret_cast<unsigned long long*>(c.base + tile), static_cast<unsigned long long>(tot));
+      __threadfence();
+      s_last = atomicAdd(done, 1u) == tiles - 1;
     }
   }
-  if (threadIdx.x < 32) {
-    const uint64_t p = warp_lookback_seg(status, tile, first_tile, tot, err);
-    if (threadIdx.x == 0) *s_b = p;
-  }
-  __syncthreads();
-  const uint64_t base = *s_b;
-  if (last_tile && tid == 0) *total = base + tot;
-  if (!stage) {
-    uint64_t run = base + e;
+  const uint64_t first = i0 + static_cast<uint64_t>(tid) * kJcKeys, group = first / kJcKeys;
+  if (first < nl) {
+    uint32_t match = 0;
 #pragma unroll
-    for (int k = 0; k < kJcKeys; ++k) {
-      if (first + k < nl) {
-        offs[first + k] = static_cast<Off>(run);
-        lo[first + k] = lov[k];
+    for (int k = 0; k < kJcKeys; ++k) match |= (cnt[k] ? 1u : 0u) << k;
+    c.start[group] = static_cast<Off>(e);
+    c.match[group] = static_cast<uint8_t>(match);
+    if (match) {
+      static_assert(kJcKeys == 8, "the vector stores take 8 rows");
+      uint4* lo4 = reinterpret_cast<uint4*>(c.lo + first);
+      lo4[0] = make_uint4(lov[0], lov[1], lov[2], lov[3]);
+      lo4[1] = make_uint4(lov[4], lov[5], lov[6], lov[7]);
+      union {
+        Off v[kJcKeys];
+        uint4 w[kJcKeys * sizeof(Off) / 16];
+      } o;
+      Off run = static_cast<Off>(e);
+#pragma unroll
+      for (int k = 0; k < kJcKeys; ++k) {
+        o.v[k] = run;
+        run += cnt[k];
       }
-      run += cnt[k];
+#pragma unroll
+      for (size_t k = 0; k < kJcKeys * sizeof(Off) / 16; ++k) reinterpret_cast<uint4*>(c.offs + first)[k] = o.w[k];
     }
-    if (tid == 0) jc_drain_window(sm, err);
-    return;
   }
-  const uint32_t* s_lo = jc_stage_lo(sm);
-  const Off* s_off = jc_stage_off<Off>(sm);
-  for (uint32_t q = tid; q < tile_n; q += kJcBlock) {
-    lo[i0 + q] = s_lo[q + q / 32];
-    offs[i0 + q] = static_cast<Off>(base) + s_off[jc_stage_at<Off>(q)];
+  if (tiles == 1) return;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  constexpr uint32_t kEach = 8;
+  uint64_t before = 0;
+  for (uint32_t t0 = 0; t0 < tiles; t0 += kJcBlock * kEach) {
+    uint64_t v[kEach], mine = 0, all;
+#pragma unroll
+    for (uint32_t k = 0; k < kEach; ++k) {
+      const uint32_t t = t0 + tid * kEach + k;
+      v[k] = t < tiles ? __ldcg(reinterpret_cast<const unsigned long long*>(c.base + t)) : 0ull;
+      mine += v[k];
+    }
+    uint64_t at = before + block_excl_scan64<kJcBlock>(mine, all, s_scan);
+#pragma unroll
+    for (uint32_t k = 0; k < kEach; ++k) {
+      const uint32_t t = t0 + tid * kEach + k;
+      if (t < tiles) c.base[t] = at;
+      at += v[k];
+    }
+    before += all;
   }
+  if (tid == 0) *total = before;
 }
 
-// A join to write: left rows' lower bounds and output offsets, source and
-// output columns (lc: the key columns and the other left ones, rc: the right
-// ones without the keys).
+// The groups' first output rows (ascending), for searches.
+template <typename Off>
+struct JoinGroups {
+  using T = Off;
+  const Off* start;
+  const uint64_t* base;
+  __device__ __forceinline__ T operator()(uint64_t g) const {
+    return static_cast<Off>(__ldg(base + g / kJcTileGroups)) + __ldg(start + g);
+  }
+};
+
+// A join to write: its count, source and output columns (lc: the key columns
+// and the other left ones, rc: the right ones without the keys).
 template <typename Off>
 struct JoinOutOf {
-  using Offset = Off;
-  const Off* offs;
-  const uint32_t* lo;
+  JoinCounts<Off> cnt;
   uint64_t nl, total;
   const uint32_t* lc[VG_MAX_COLS];
   const uint32_t* rc[VG_MAX_COLS];
   uint32_t* oc[VG_MAX_COLS];
   uint32_t nlc, nrc;
+
+  __host__ __device__ __forceinline__ JoinGroups<Off> groups() const { return {cnt.start, cnt.base}; }
+  __host__ __device__ __forceinline__ uint64_t ngroups() const { return (nl + kJcKeys - 1) / kJcKeys; }
 };
 using JoinOut = JoinOutOf<uint32_t>;
 
 constexpr int kJwBlock = 256;
 
-// Left rows that a tile of kJwBlock * ROWS output rows stages: twice as many,
-// since rows without matches lie between the others (16M left rows with 13M
-// output rows had no tile staged when only as many fitted: 0.26 ms).
+// A tile's output rows that start a left row's ("heads"): the left row plus 1
+// (0: not a head), and the right row that output row 0 of the tile would have
+// from that head on (so that row k's is right + k).  heads: a bit per row.
 template <int ROWS>
 struct JwStage {
-  static constexpr uint32_t kMost = 2 * kJwBlock * ROWS;
-  uint32_t off[kMost];   // first output row, from the tile's first (0 where it lies before)
-  uint32_t lo[kMost];    // the right row that output row off comes from
+  static constexpr uint32_t kTile = kJwBlock * ROWS;
+  alignas(16) uint32_t left[kTile];
+  uint32_t right[kTile];
+  uint32_t heads[kTile / 32];
 };
 
-// Output rows [kb, kend) (at most kJwBlock * ROWS) of a join, by one block.
-// Output row k comes from the left row i with offs[i] <= k < offs[i + 1] and
-// the right row lo[i] + (k - offs[i]); the rows come from left rows [ib, ie).
-// When those fit the stage, their offsets and lower bounds lie in shared
-// memory and each thread walks its rows (k increasing, consecutive threads on
-// consecutive rows, so loads and stores coalesce) from the previous one's left
-// row.  Hub keys thus spread over many blocks.
+// The block's threads clear a tile's heads; a barrier before jw_write_tile.
+template <int ROWS>
+__device__ __forceinline__ void jw_clear(JwStage<ROWS>& st) {
+  for (uint32_t k = threadIdx.x; k < st.kTile / 4; k += kJwBlock)
+    reinterpret_cast<uint4*>(st.left)[k] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// Marks the heads of a group's rows with matches among output rows [kb, kend).
 template <int ROWS, typename Off>
-__device__ __forceinline__ void jw_write_tile(const JoinOutOf<Off>& o, uint64_t kb, uint64_t kend, uint64_t ib, uint64_t ie,
-                                              JwStage<ROWS>& st) {
-  const uint64_t m64 = ie - ib;
-  const bool staged = m64 <= JwStage<ROWS>::kMost;
-  const uint32_t m = static_cast<uint32_t>(staged ? m64 : 0);
-  for (uint32_t e = threadIdx.x; e < m; e += kJwBlock) {
-    const uint64_t f = o.offs[ib + e];
-    const uint32_t r = o.lo[ib + e];
-    st.off[e] = f > kb ? static_cast<uint32_t>(f - kb) : 0u;
-    st.lo[e] = f > kb ? r : r + static_cast<uint32_t>(kb - f);
-  }
-  __syncthreads();
-  // 1. the left and right row of each of the thread's output rows
-  uint32_t li[ROWS], ri[ROWS];
-  if (staged) {
-    const uint32_t rows = static_cast<uint32_t>(kend - kb);
-    uint32_t p = 0;   // the current left row, relative to ib
+__device__ __forceinline__ void jw_mark_group(const JoinOutOf<Off>& o, uint64_t g, uint32_t match, uint64_t kb,
+                                              uint64_t kend, JwStage<ROWS>& st) {
+  union {
+    Off v[kJcKeys];
+    uint4 w[kJcKeys * sizeof(Off) / 16];
+  } f;
+  union {
+    uint32_t v[kJcKeys];
+    uint4 w[2];
+  } r;
+  const uint64_t first = g * kJcKeys;
 #pragma unroll
-    for (int it = 0; it < ROWS; ++it) {
-      const uint32_t k = it * kJwBlock + threadIdx.x;
-      li[it] = ri[it] = 0;
-      if (k < rows) {
-        // last p with off[p] <= k, moving forward from the previous row's p
-        uint32_t step = 1;
-        while (p + step < m && st.off[p + step] <= k) {
-          p += step;
-          step <<= 1;
+  for (size_t k = 0; k < kJcKeys * sizeof(Off) / 16; ++k) f.w[k] = __ldg(reinterpret_cast<const uint4*>(o.cnt.offs + first) + k);
+#pragma unroll
+  for (int k = 0; k < 2; ++k) r.w[k] = __ldg(reinterpret_cast<const uint4*>(o.cnt.lo + first) + k);
+  const uint64_t base = __ldg(o.cnt.base + g / kJcTileGroups);
+#pragma unroll
+  for (int q = 0; q < kJcKeys; ++q) {
+    const uint64_t at = base + f.v[q];
+    if ((match >> q & 1u) && at < kend) {
+      // of the rows that start at or before kb the last one, which covers it,
+      // is marked last
+      const uint32_t p = at > kb ? static_cast<uint32_t>(at - kb) : 0u;
+      st.left[p] = static_cast<uint32_t>(first) + q + 1;
+      st.right[p] = r.v[q] + static_cast<uint32_t>(kb - at);
+    }
+  }
+}
+
+// Output rows [kb, kend) (at most kJwBlock * ROWS) of a join, by one block;
+// they come from the groups [ga, gb) of left rows.  Each left row with matches
+// marks its first output row as a head; an output row's left row is the
+// nearest head at or before it (a bit mask, one ballot per warp and 32 rows,
+// and a maximum scan over the words): about 12 instructions a row, where
+// galloping each row from the thread's previous one took over 100 (13.4M rows
+// from 16M left rows: 199 -> 108 us; the six joins of a hub query, 770 us
+// from 968).  Left rows without matches cost a bit.  Consecutive threads write consecutive rows, so
+// loads and stores coalesce; hub keys spread over many blocks.
+template <int ROWS, typename Off>
+__device__ __forceinline__ void jw_write_tile(const JoinOutOf<Off>& o, uint64_t kb, uint64_t kend, uint64_t ga, uint64_t gb,
+                                              JwStage<ROWS>& st) {
+  constexpr uint32_t kTile = kJwBlock * ROWS;
+  uint32_t li[ROWS], ri[ROWS];   // 1. the left and right row of each of the thread's output rows
+  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+  {
+    // groups that take few passes: a thread each.  More than that: 16 groups'
+    // bits at a time (few are set: at most kTile rows have matches).
+    constexpr uint32_t kNear = 16 * kJwBlock;
+    const uint8_t* match = o.cnt.match;
+    if (gb - ga <= kNear) {
+      for (uint64_t g = ga + threadIdx.x; g < gb; g += kJwBlock) {
+        const uint32_t m = __ldg(match + g);
+        if (m) jw_mark_group(o, g, m, kb, kend, st);
+      }
+    } else {
+      const uint32_t skew = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(match + ga) & 15u);
+      const uint4* match4 = reinterpret_cast<const uint4*>(match + ga - skew);   // (its array is whole words of 16)
+      const uint64_t words = (gb - ga + skew + 15) / 16;
+      for (uint64_t w = threadIdx.x; w < words; w += kJwBlock) {
+        const uint4 x = __ldg(match4 + w);
+        if ((x.x | x.y | x.z | x.w) == 0) continue;
+        const uint32_t part[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll 1
+        for (uint32_t b = 0; b < 16; ++b) {
+          const uint32_t m = (part[b >> 2] >> (8 * (b & 3))) & 255u;
+          const uint64_t g = ga - skew + w * 16 + b;   // (before ga for the first word's first bytes)
+          if (m && w * 16 + b >= skew && g < gb) jw_mark_group(o, g, m, kb, kend, st);
         }
-        while (step > 1) {
-          step >>= 1;
-          if (p + step < m && st.off[p + step] <= k) p += step;
-        }
-        li[it] = static_cast<uint32_t>(ib) + p;
-        ri[it] = st.lo[p] + (k - st.off[p]);
       }
     }
-  } else {
-    // a sparse tile (more left rows than the stage holds, most without matches): the
-    // left rows of kGroup of the thread's output rows at a time come from
-    // kGroup binary searches of the offsets advanced in lockstep, so each
-    // round has kGroup independent loads in flight
-    constexpr int kGroup = ROWS < 4 ? ROWS : 4;
+    __syncthreads();
+    uint32_t heads[ROWS];
 #pragma unroll
-    for (int g0 = 0; g0 < ROWS; g0 += kGroup) {
-      uint64_t lq[kGroup], kk[kGroup];
+    for (int it = 0; it < ROWS; ++it) {
+      heads[it] = __ballot_sync(0xffffffffu, st.left[it * kJwBlock + threadIdx.x] != 0);
+      if (lane == 0) st.heads[it * (kJwBlock / 32) + warp] = heads[it];
+    }
+    __syncthreads();
+    // upto[g]: in lane l, the last head up to word 32 * g + l (row 0 is one)
+    constexpr uint32_t kWords = kTile / 32, kGroups = (kWords + 31) / 32;
+    uint32_t upto[kGroups];
 #pragma unroll
-      for (int q = 0; q < kGroup; ++q) {
-        const uint64_t k = kb + static_cast<uint64_t>(g0 + q) * kJwBlock + threadIdx.x;
-        kk[q] = k < kend ? k : kend - 1;
-        lq[q] = ib;
+    for (uint32_t g = 0; g < kGroups; ++g) {
+      const uint32_t w = g * 32 + lane, x = w < kWords ? st.heads[w] : 0u;
+      upto[g] = x ? w * 32 + 31 - __clz(x) : 0u;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, upto[g], d);
+        if (static_cast<int>(lane) >= d) upto[g] = max(upto[g], y);
       }
-      uint64_t n = ie - ib;                     // last i in [ib, ie) with offs[i] <= k
-      while (n > 1) {
-        const uint64_t half = n >> 1;
+      if (g) upto[g] = max(upto[g], __shfl_sync(0xffffffffu, upto[g - 1], 31));
+    }
 #pragma unroll
-        for (int q = 0; q < kGroup; ++q) lq[q] = (o.offs[lq[q] + half] <= kk[q]) ? lq[q] + half : lq[q];
-        n -= half;
-      }
+    for (int it = 0; it < ROWS; ++it) {
+      const uint32_t k = it * kJwBlock + threadIdx.x, w = it * (kJwBlock / 32) + warp;
+      uint32_t h = 0;
 #pragma unroll
-      for (int q = 0; q < kGroup; ++q) {
-        li[g0 + q] = static_cast<uint32_t>(lq[q]);
-        ri[g0 + q] = static_cast<uint32_t>(o.lo[lq[q]] + (kk[q] - o.offs[lq[q]]));
+      for (uint32_t g = 0; g < kGroups; ++g) {   // the last head before word w
+        const uint32_t y = __shfl_sync(0xffffffffu, upto[g], (w - 1) & 31);
+        if (w > g * 32) h = y;
       }
+      const uint32_t mine = heads[it] & (0xffffffffu >> (31 - lane));
+      if (mine) h = w * 32 + 31 - __clz(mine);
+      li[it] = st.left[h] - 1;
+      ri[it] = st.right[h] + k;
     }
   }
   // 2. column by column: each thread's ROWS loads of a column are in flight

@@ -7,10 +7,9 @@
 // latency-critical serving threads that may only launch work.  Such a caller
 // cannot create a vg_ctx, whose arena is one cudaMalloc.
 //
-// The join's scratch (per-left-row lower bound and output
-// offset, plus the look-back status words) lives in one file-scope
-// __device__ array instead.  Its size is fixed: at most kMaxLeftRows left
-// rows (about 24 MiB of device memory, held by every GPU that loads this
+// The join's scratch (a lower bound and an output offset per left row, and the
+// groups' and tiles' words) lives in one file-scope __device__ array instead.  Its size is fixed: at most kMaxLeftRows left
+// rows (about 27 MiB of device memory, held by every GPU that loads this
 // library until the process exits).  Host code may not use the array's name
 // as a device address, so on the first call on each device, with that device
 // current, the entry point looks the address up with cudaGetSymbolAddress and
@@ -26,15 +25,17 @@
 namespace {
 
 constexpr uint64_t kMaxLeftRows = 1ull << 21;     // 2,097,152 left rows
-constexpr uint64_t kTileRows = 2048;              // rows per scan tile (vg_relops.cu)
+constexpr uint64_t kTileRows = 2048;              // rows per count tile (vg_join_tile.cuh)
 constexpr uint64_t kMaxTiles = kMaxLeftRows / kTileRows;
 
 struct NoAllocScratch {
   uint32_t lo[kMaxLeftRows];
   uint64_t offs[kMaxLeftRows];
-  uint64_t status[kMaxTiles];
+  uint64_t start[kMaxLeftRows / vg::kJoinGroup];
+  uint8_t match[kMaxLeftRows / vg::kJoinGroup];
+  uint64_t base[kMaxTiles];
   uint64_t total;
-  uint32_t ticket;
+  uint32_t done;
   uint32_t pad;
   vg::DeviceErrors err;
 };
@@ -88,15 +89,14 @@ extern "C" vg_status vg_join_noalloc(const uint32_t* const* l_cols, uint32_t l_n
     r.nrows = r_rows;
     for (uint32_t c = 0; c < l_ncols; ++c) l.cols[c] = const_cast<uint32_t*>(l_cols[c]);
     for (uint32_t c = 0; c < r_ncols; ++c) r.cols[c] = const_cast<uint32_t*>(r_cols[c]);
-    // The previous call's contents are still there: zero what the look-back
-    // and the error record read before they are written.
-    const uint64_t tiles = (l_rows + kTileRows - 1) / kTileRows;
-    VG_CUDA(cudaMemsetAsync(sc->status, 0, (tiles ? tiles : 1) * sizeof(uint64_t), s));
+    // The previous call's contents are still there: zero what is read before
+    // it is written.
     VG_CUDA(cudaMemsetAsync(&sc->total, 0, sizeof(uint64_t), s));
-    VG_CUDA(cudaMemsetAsync(&sc->ticket, 0, sizeof(uint32_t), s));
+    VG_CUDA(cudaMemsetAsync(&sc->done, 0, sizeof(uint32_t), s));
     VG_CUDA(cudaMemsetAsync(&sc->err, 0, sizeof(vg::DeviceErrors), s));
-    const uint64_t t = vg::join_into(s, l, r, out_cols, out_capacity, sc->lo, sc->offs, sc->status,
-                                     &sc->ticket, &sc->total, &sc->err);
+    const uint64_t t = vg::join_into(s, l, r, out_cols, out_capacity,
+                                     {sc->lo, sc->offs, sc->start, sc->match, sc->base}, &sc->done, &sc->total,
+                                     &sc->err);
     vg::DeviceErrors he{};
     VG_CUDA(cudaMemcpyAsync(&he, &sc->err, sizeof(he), cudaMemcpyDeviceToHost, s));
     VG_CUDA(cudaStreamSynchronize(s));

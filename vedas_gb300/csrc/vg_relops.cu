@@ -175,44 +175,38 @@ __global__ void __launch_bounds__(kJcBlock) join_window_kernel(typename KeysOf<T
   }
 }
 
-// One block per 2048 left keys, in ticket order.  The window comes from
-// join_window_kernel where there are more tiles than the GPU runs at a time
-// (a block's own search is five rounds of global loads before its copy can
-// start), else warp 0 finds it.
+// One block per 2048 left keys.  The window comes from join_window_kernel where
+// there are more tiles than the GPU runs at a time (a block's own search is
+// five rounds of global loads before its copy can start), else warp 0 finds it.
 template <bool TWO, typename Off>
-__global__ void __launch_bounds__(kJcBlock, 4) join_count_scan_kernel(
+__global__ void __launch_bounds__(kJcBlock, 4) join_count_kernel(
     typename KeysOf<TWO>::K L, uint64_t nl, typename KeysOf<TWO>::K R, uint64_t nr, const uint2* __restrict__ win,
-    uint32_t* __restrict__ lo, Off* __restrict__ offs, uint64_t* status, uint32_t* ticket, uint64_t* total,
-    DeviceErrors* err) {
+    JoinCounts<Off> c, uint32_t* done, uint64_t* total, DeviceErrors* err) {
   __shared__ JoinCountSmem sm;
   __shared__ uint64_t s_scan[kJcBlock / 32 + 1];
-  __shared__ uint64_t s_b;
-  __shared__ uint32_t s_tile;
+  const uint32_t tile = blockIdx.x;
+  const uint64_t i0 = static_cast<uint64_t>(tile) * kJcTile, i1 = i0 + kJcTile < nl ? i0 + kJcTile : nl;
+  typename KeysOf<TWO>::K::T key[kJcKeys];
+  jc_load_keys(L, i0 + static_cast<uint64_t>(threadIdx.x) * kJcKeys, i1, key);
   if (threadIdx.x < 32) {
-    uint32_t t = 0;
-    if (threadIdx.x == 0) t = atomicAdd(ticket, 1u);
-    t = __shfl_sync(0xffffffffu, t, 0);
     uint64_t w0, w1;
     if (win) {
-      const uint2 w = win[t];
+      const uint2 w = win[tile];
       w0 = w.x;
       w1 = w.y;
     } else {
-      const uint64_t b = static_cast<uint64_t>(t) * kJcTile, e = (b + kJcTile < nl ? b + kJcTile : nl) - 1;
-      warp_bound_pair_of<false, true>(R, nr, L(b), L(e), w0, w1);
+      warp_bound_pair_of<false, true>(R, nr, L(i0), L(i1 - 1), w0, w1);
     }
     if (threadIdx.x == 0) {
-      s_tile = t;
       if constexpr (TWO) jc_issue_pair_window(w0, w1, sm);
       else jc_issue_window(R.c0, w0, w1, sm);
     }
   }
   __syncthreads();
-  const uint64_t i0 = static_cast<uint64_t>(s_tile) * kJcTile;
   uint32_t cnt[kJcKeys], lov[kJcKeys];
-  if constexpr (TWO) jc_count_staged_pairs(L, nl, R, i0, lov, cnt, sm);
-  else jc_count_staged(L.c0, nl, R.c0, i0, lov, cnt, sm, err);
-  jc_finish_tile(nl, i0, lov, cnt, sm, s_scan, &s_b, s_tile, 0, s_tile == gridDim.x - 1, lo, offs, status, total, err);
+  if constexpr (TWO) jc_count_staged_pairs(key, nl, R, i0, lov, cnt, sm);
+  else jc_count_staged(key, nl, R.c0, i0, lov, cnt, sm, err);
+  jc_finish_tile(i0, lov, cnt, sm, s_scan, tile, gridDim.x, nl, c, done, total, err);
 }
 
 // What the host reads of a join (page-locked memory that the write kernel
@@ -226,15 +220,15 @@ struct JoinTail {
 };
 static_assert(sizeof(JoinTail) <= Ctx::kSmallWords * sizeof(uint64_t), "the tail fits the small staging buffer");
 
-// Left rows [x, y) of every output tile, one warp per tile.
-__global__ void __launch_bounds__(kJwBlock) join_ranges_kernel(const uint32_t* __restrict__ offs, uint64_t nl,
+// Groups [x, y) of left rows of every output tile, one warp per tile.
+__global__ void __launch_bounds__(kJwBlock) join_ranges_kernel(JoinGroups<uint32_t> groups, uint64_t ng,
                                                                uint64_t total, uint64_t tiles, uint32_t tile_rows,
                                                                uint2* __restrict__ ranges) {
   const uint64_t nw = static_cast<uint64_t>(gridDim.x) * (kJwBlock / 32);
   for (uint64_t t = static_cast<uint64_t>(blockIdx.x) * (kJwBlock / 32) + (threadIdx.x >> 5); t < tiles; t += nw) {
     const uint64_t kb = t * tile_rows, kend = kb + tile_rows < total ? kb + tile_rows : total;
     uint64_t a, b;
-    warp_bound_pair<true, true, uint32_t>(offs, nl, static_cast<uint32_t>(kb), static_cast<uint32_t>(kend - 1), a, b);
+    warp_bound_pair_of<true, true>(groups, ng, static_cast<uint32_t>(kb), static_cast<uint32_t>(kend - 1), a, b);
     if ((threadIdx.x & 31) == 0) ranges[t] = make_uint2(static_cast<uint32_t>(a - 1), static_cast<uint32_t>(b));
   }
 }
@@ -265,6 +259,7 @@ __global__ void __launch_bounds__(kJwBlock, 5) join_write_kernel(JoinOutOf<Off> 
   for (uint64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const uint64_t kb = tile * kTile, kend = kb + kTile < total ? kb + kTile : total;
     __syncthreads();   // s_o is set; the previous tile's readers of the shared arrays are done
+    jw_clear(s_stage);
     if (threadIdx.x < 32) {
       uint64_t a, b;
       if (ranges) {
@@ -272,7 +267,7 @@ __global__ void __launch_bounds__(kJwBlock, 5) join_write_kernel(JoinOutOf<Off> 
         a = r.x;
         b = r.y;
       } else {
-        warp_bound_pair<true, true, Off>(s_o.offs, s_o.nl, static_cast<Off>(kb), static_cast<Off>(kend - 1), a, b);
+        warp_bound_pair_of<true, true>(s_o.groups(), s_o.ngroups(), static_cast<Off>(kb), static_cast<Off>(kend - 1), a, b);
         --a;
       }
       if (threadIdx.x == 0) {
@@ -296,21 +291,20 @@ __global__ void __launch_bounds__(kJwBlock, 5) join_write_kernel(JoinOutOf<Off> 
 bool many_tiles(int num_sms, uint64_t tiles) { return tiles > 4ull * static_cast<uint64_t>(num_sms); }
 
 template <bool TWO, typename Off>
-void launch_count_scan(cudaStream_t stream, const Rel& l, const Rel& r, const uint2* win, uint32_t* lo,
-                       Off* offs, uint64_t* status, uint32_t* ticket, uint64_t* total, DeviceErrors* err) {
+void launch_count(cudaStream_t stream, const Rel& l, const Rel& r, const uint2* win,
+                  const JoinCounts<Off>& c, uint32_t* done, uint64_t* total, DeviceErrors* err) {
   const unsigned tiles = static_cast<unsigned>(div_up(l.nrows, kJcTile));
-  join_count_scan_kernel<TWO, Off><<<tiles, kJcBlock, 0, stream>>>(
+  join_count_kernel<TWO, Off><<<tiles, kJcBlock, 0, stream>>>(
       KeysOf<TWO>::of(l.cols[0], TWO ? l.cols[1] : nullptr), l.nrows,
-      KeysOf<TWO>::of(r.cols[0], TWO ? r.cols[1] : nullptr), r.nrows, win, lo, offs, status, ticket, total, err);
+      KeysOf<TWO>::of(r.cols[0], TWO ? r.cols[1] : nullptr), r.nrows, win, c, done, total, err);
   VG_CUDA(cudaGetLastError());
 }
 
 template <typename Off>
-JoinOutOf<Off> join_out(const Rel& l, const Rel& r, uint32_t nk, const Off* offs, const uint32_t* lo, uint64_t total,
+JoinOutOf<Off> join_out(const Rel& l, const Rel& r, uint32_t nk, const JoinCounts<Off>& c, uint64_t total,
                         uint32_t* const* oc) {
   JoinOutOf<Off> o{};
-  o.offs = offs;
-  o.lo = lo;
+  o.cnt = c;
   o.nl = l.nrows;
   o.total = total;
   for (uint32_t c = 0; c < l.ncols; ++c) o.lc[c] = l.cols[c];
@@ -561,10 +555,13 @@ void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
   }
   const uint64_t tiles = div_up(l.nrows, kJcTile);
   if (tiles > 0x7FFFFFFFull) fail(VG_ERR_OVERFLOW, "join: too many tiles");
-  Scratch<uint32_t> lo(ctx, l.nrows), offs(ctx, l.nrows);
-  Scratch<uint64_t> z(ctx, tiles + 2);   // look-back words, total, ticket
+  const uint64_t ngroups = div_up(l.nrows, kJcKeys);
+  Scratch<uint32_t> lo(ctx, ngroups * kJcKeys), offs(ctx, ngroups * kJcKeys), start(ctx, ngroups);
+  Scratch<uint8_t> match(ctx, div_up(ngroups, 16) * 16);
+  Scratch<uint64_t> z(ctx, tiles + 2);   // first output row of every tile, total, tiles done
   uint64_t* total = z.get() + tiles;
-  VG_CUDA(cudaMemsetAsync(z.get(), 0, (tiles + 2) * sizeof(uint64_t), ctx.stream));
+  const JoinCounts<uint32_t> cnt{lo.get(), offs.get(), start.get(), match.get(), z.get()};
+  VG_CUDA(cudaMemsetAsync(total, 0, 2 * sizeof(uint64_t), ctx.stream));
   std::optional<Scratch<uint2>> win;
   if (many_tiles(ctx.num_sms, tiles)) {
     win.emplace(ctx, tiles);
@@ -581,11 +578,11 @@ void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
     });
     VG_CUDA(cudaGetLastError());
   }
-  ctx.launch("join_count_scan", 4.0 * nk * (l.nrows + r.nrows) + 8.0 * l.nrows, [&] {
+  ctx.launch("join_count", 4.0 * nk * (l.nrows + r.nrows) + 8.0 * l.nrows, [&] {
     const uint2* w = win ? win->get() : nullptr;
-    auto* ticket = reinterpret_cast<uint32_t*>(total + 1);
-    if (two_keys) launch_count_scan<true>(ctx.stream, l, r, w, lo.get(), offs.get(), z.get(), ticket, total, ctx.d_err);
-    else launch_count_scan<false>(ctx.stream, l, r, w, lo.get(), offs.get(), z.get(), ticket, total, ctx.d_err);
+    auto* done = reinterpret_cast<uint32_t*>(total + 1);
+    if (two_keys) launch_count<true>(ctx.stream, l, r, w, cnt, done, total, ctx.d_err);
+    else launch_count<false>(ctx.stream, l, r, w, cnt, done, total, ctx.d_err);
   });
   auto* tail = reinterpret_cast<JoinTail*>(ctx.h_small);
   auto finish = [&](uint64_t t) {
@@ -615,7 +612,7 @@ void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
     }
     if (fits) {
       constexpr int kRowsSmall = 2;
-      const JoinOut o = join_out(l, r, nk, offs.get(), lo.get(), 0, guess.cols);
+      const JoinOut o = join_out(l, r, nk, cnt, 0, guess.cols);
       const unsigned grid = static_cast<unsigned>(
           std::min<uint64_t>(div_up(cap, kJwBlock * kRowsSmall), static_cast<uint64_t>(ctx.num_sms) * 5));
       ctx.launch("join_write", 0.0, [&] {
@@ -640,8 +637,8 @@ void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
       free_cols(guess);
     }
   }
-  // the total and the error record come back together: a look-back that gave
-  // up leaves the offsets wrong, and the write must then not run
+  // the total and the error record come back together: after a wait that gave
+  // up the write must not run
   VG_CUDA(cudaMemcpyAsync(&tail->total, total, sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx.stream));
   VG_CUDA(cudaMemcpyAsync(&tail->err, ctx.d_err, sizeof(DeviceErrors), cudaMemcpyDeviceToHost, ctx.stream));
   ctx.sync();
@@ -650,7 +647,7 @@ void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
   if (t > 0xFFFFFFFFull) fail(VG_ERR_OVERFLOW, "join output exceeds 2^32 rows");
   out = rel_alloc(ctx, ncols, t);
   if (t == 0) return;
-  const JoinOut o = join_out(l, r, nk, offs.get(), lo.get(), t, out.cols);
+  const JoinOut o = join_out(l, r, nk, cnt, t, out.cols);
   const uint64_t otiles = div_up(t, static_cast<uint64_t>(kTileRows));
   std::optional<Scratch<uint2>> ranges;
   if (many_tiles(ctx.num_sms, otiles)) {
@@ -658,7 +655,7 @@ void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
     const unsigned rblocks = static_cast<unsigned>(
         std::min<uint64_t>(div_up(otiles, kJwBlock / 32), static_cast<uint64_t>(ctx.num_sms) * 8));
     ctx.launch("join_write_ranges", 8.0 * otiles, [&] {
-      join_ranges_kernel<<<rblocks, kJwBlock, 0, ctx.stream>>>(offs.get(), l.nrows, t, otiles, kTileRows,
+      join_ranges_kernel<<<rblocks, kJwBlock, 0, ctx.stream>>>(o.groups(), ngroups, t, otiles, kTileRows,
                                                                ranges->get());
     });
     VG_CUDA(cudaGetLastError());
@@ -673,19 +670,18 @@ void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
 }
 
 uint64_t join_into(cudaStream_t stream, const Rel& l, const Rel& r, uint32_t* const* out_cols, uint64_t capacity,
-                   uint32_t* lo, uint64_t* offs, uint64_t* status, uint32_t* ticket, uint64_t* total,
-                   DeviceErrors* err) {
+                   const JoinCounts<uint64_t>& c, uint32_t* done, uint64_t* total, DeviceErrors* err) {
   if (l.nrows == 0 || r.nrows == 0) return 0;
-  launch_count_scan<false>(stream, l, r, nullptr, lo, offs, status, ticket, total, err);
+  launch_count<false>(stream, l, r, nullptr, c, done, total, err);
   uint64_t t = 0;
   DeviceErrors he{};
   VG_CUDA(cudaMemcpyAsync(&t, total, sizeof(uint64_t), cudaMemcpyDeviceToHost, stream));
   VG_CUDA(cudaMemcpyAsync(&he, err, sizeof(he), cudaMemcpyDeviceToHost, stream));
   VG_CUDA(cudaStreamSynchronize(stream));
-  // a look-back that gave up leaves the offsets wrong: no write then
+  // no write after a wait that gave up
   if (he.timeout) fail(VG_ERR_TIMEOUT, "join_into: a bounded device wait expired");
   if (t == 0 || t > capacity) return t;
-  const JoinOutOf<uint64_t> o = join_out(l, r, 1, offs, lo, t, out_cols);
+  const JoinOutOf<uint64_t> o = join_out(l, r, 1, c, t, out_cols);
   join_write_kernel<kRows, uint64_t><<<static_cast<unsigned>(std::min<uint64_t>(div_up(t, kTileRows), 0x7FFFFFFFull)), kJwBlock,
                              0, stream>>>(o, nullptr, t, nullptr, err, nullptr);
   VG_CUDA(cudaGetLastError());

@@ -48,13 +48,32 @@ struct JoinEnds {
 // output is complete on return, and device errors are raised.
 void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnds* ends = nullptr);
 
-// The same join on a caller's stream with caller-provided scratch and output
-// columns (nothing is allocated): lo/offs hold l.nrows entries, status
-// div_up(l.nrows, 2048) words; status, ticket and err must be zero.  Returns
+// What a join's count leaves in device memory.  Left rows come in groups of
+// kJoinGroup (one thread's): match has a bit for each of a group's rows that has
+// matches, and only groups with one have their rows' lower bounds (lo) and
+// output offsets (offs) stored, a sector of 32 bytes each; start is the group's
+// first output row, for the searches.  offs and start count from the tile's
+// first output row, which is base[tile] (tiles of 2048 left rows).  The arrays
+// cover whole groups, match whole 16 of them; lo, offs and match start on 16
+// bytes.  (With an offset and a bound for every row instead, a wave of joins
+// of which few left rows match moved twice the bytes.)
+// Off: 32 bits hold every offset of a join that is written (one with 2^32 rows
+// or more is refused, by its 64-bit total); 64 bits for the join that takes any.
+constexpr int kJoinGroup = 8;
+template <typename Off>
+struct JoinCounts {
+  uint32_t* lo;
+  Off* offs;
+  Off* start;
+  uint8_t* match;
+  uint64_t* base;
+};
+
+// The same join on a caller's stream with caller-provided scratch (c) and
+// output columns (nothing is allocated); done and err must be zero.  Returns
 // the result row count; the outputs are written only when it fits `capacity`.
 uint64_t join_into(cudaStream_t stream, const Rel& l, const Rel& r, uint32_t* const* out_cols, uint64_t capacity,
-                   uint32_t* lo, uint64_t* offs, uint64_t* status, uint32_t* ticket, uint64_t* total,
-                   DeviceErrors* err);
+                   const JoinCounts<uint64_t>& c, uint32_t* done, uint64_t* total, DeviceErrors* err);
 
 // out[c][i] = in[c][perm[i]] for every column.
 void gather_cols(Ctx& ctx, const uint32_t* const* in, uint32_t* const* out, uint32_t ncols,
