@@ -47,11 +47,14 @@ __device__ __forceinline__ void digit_counts_add(const DigitList& dl, uint32_t* 
 
 // Every thread of every block calls it once, after its last key.  hist (zeroed
 // before the launch) receives the counts, bases[p][v] the first output row of
-// value v; done counts the blocks (zeroed).
+// value v; done counts the blocks (zeroed).  whole (nullable, page-locked): bit
+// p set where all n keys have one value of digit p.
 template <int BLOCK>
-__device__ __forceinline__ void digit_counts_finish(const DigitList& dl, const uint32_t* s, unsigned long long* hist,
-                                                    uint64_t* bases, uint32_t* done) {
+__device__ __forceinline__ void digit_counts_finish(const DigitList& dl, const uint32_t* s,
+                                                    unsigned long long* hist, uint64_t* bases, uint32_t* done,
+                                                    uint64_t n = 0, uint32_t* whole = nullptr) {
   static_assert(BLOCK == kRadixValues, "one thread per digit value");
+  static_assert(kRadixMaxPasses <= 32, "a bit per digit");
   __shared__ uint64_t s_scan[BLOCK / 32 + 1];
   __shared__ bool s_last;
   __syncthreads();
@@ -63,11 +66,14 @@ __device__ __forceinline__ void digit_counts_finish(const DigitList& dl, const u
   __syncthreads();
   if (!s_last) return;
   __threadfence();
+  uint32_t one = 0;
   for (uint32_t p = 0; p < dl.n; ++p) {
     const uint64_t c = ld_status_u64(reinterpret_cast<const uint64_t*>(&hist[p * kRadixValues + threadIdx.x]));
     uint64_t tot;
     bases[p * kRadixValues + threadIdx.x] = block_excl_scan64<BLOCK>(c, tot, s_scan);
+    if (whole && __syncthreads_or(c == n)) one |= 1u << p;
   }
+  if (whole && threadIdx.x == 0) *whole = one;
 }
 
 }  // namespace vg

@@ -24,7 +24,8 @@ constexpr int kMaxPasses = kRadixMaxPasses;
 template <typename K>
 __global__ void __launch_bounds__(kBlock) radix_hist_kernel(const K* __restrict__ keys, uint64_t n, DigitList dl,
                                                             unsigned long long* __restrict__ hist,
-                                                            uint64_t* __restrict__ bases, uint32_t* done) {
+                                                            uint64_t* __restrict__ bases, uint32_t* done,
+                                                            uint32_t* whole) {
   extern __shared__ uint32_t sh[];   // [dl.n][kRadix]
   digit_counts_init<kBlock>(dl, sh);
   constexpr uint32_t kVec = 16 / sizeof(K);
@@ -47,7 +48,7 @@ __global__ void __launch_bounds__(kBlock) radix_hist_kernel(const K* __restrict_
     }
   }
   for (uint64_t i = nv * kVec + t; i < n; i += stride) digit_counts_add(dl, sh, keys[i]);
-  digit_counts_finish<kBlock>(dl, sh, hist, bases, done);
+  digit_counts_finish<kBlock>(dl, sh, hist, bases, done, n, whole);
 }
 
 __global__ void iota_kernel(uint32_t* out, uint64_t n) {
@@ -401,21 +402,18 @@ bool radix_sort_impl(Ctx& ctx, K* keys, K* keys_alt, uint32_t* vals, uint32_t* v
   const uint64_t gmax = static_cast<uint64_t>(ctx.num_sms) * 8;
   if (grid > gmax) grid = gmax;
   if (grid < 1) grid = 1;
+  auto* whole = reinterpret_cast<uint32_t*>(ctx.h_small);
   ctx.launch("radix_histogram", static_cast<double>(n) * sizeof(K), [&] {
     radix_hist_kernel<K><<<static_cast<unsigned>(grid), kBlock, (passes ? passes : 1) * kRadix * sizeof(uint32_t),
-                           ctx.stream>>>(keys, n, dl, hist, bases, done);
+                           ctx.stream>>>(keys, n, dl, hist, bases, done, host_skip ? whole : nullptr);
   });
   VG_CUDA(cudaGetLastError());
   std::vector<uint32_t> todo;
   if (host_skip) {
-    std::vector<unsigned long long> h(passes * kRadix);
-    VG_CUDA(cudaMemcpyAsync(h.data(), hist, hist_bytes, cudaMemcpyDeviceToHost, ctx.stream));
+    // (the kernel stored the host's word: no copy, and nothing for a copy to be staged in)
     ctx.sync();
-    for (uint32_t p = 0; p < passes; ++p) {
-      bool trivial = false;
-      for (int d = 0; d < kRadix; ++d) trivial = trivial || h[p * kRadix + d] == n;
-      if (!trivial) todo.push_back(p);
-    }
+    for (uint32_t p = 0; p < passes; ++p)
+      if (!(*whole >> p & 1u)) todo.push_back(p);
   } else {
     for (uint32_t p = 0; p < passes; ++p) todo.push_back(p);
   }
