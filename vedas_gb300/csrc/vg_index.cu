@@ -259,34 +259,48 @@ __global__ void __launch_bounds__(kBlock) unpack_rle_kernel(UnpackArgs a) {
     if (!GROUPS && r < a.n && a.col2) a.col2[r] = a.f2.get(key[i]);
   }
   if (GROUPS) {
-#pragma unroll 1
+    // the last head before and the first after every 32 rows (the same for the
+    // whole warp): a row's group is then two bit scans of its own 32 heads,
+    // where a search of the words from each row's own took 45 of the kernel's
+    // some 200 instructions a row, on diverging paths
+    const uint32_t wb = kHalo / 32 + warp * kRows;
+    uint32_t heads[kRows], next[kRows];
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) heads[i] = s_head[wb + i];
+    uint32_t prev = 0;   // 0: none found (a group that starts there is too long for the rows it is asked for)
+    if (s_head[wb - 1]) prev = wb * 32 - 1 - __clz(s_head[wb - 1]);
+    else if (s_head[wb - 2]) prev = wb * 32 - 33 - __clz(s_head[wb - 2]);
+    uint32_t nx = 0xffffffffu;
+    if (s_head[wb + kRows]) nx = (wb + kRows) * 32 - 1 + __ffs(s_head[wb + kRows]);
+    else if (s_head[wb + kRows + 1]) nx = (wb + kRows) * 32 + 31 + __ffs(s_head[wb + kRows + 1]);
+#pragma unroll
+    for (int i = kRows - 1; i >= 0; --i) {
+      next[i] = nx;
+      if (heads[i]) nx = (wb + i) * 32 - 1 + __ffs(heads[i]);
+    }
+#pragma unroll
     for (int i = 0; i < kRows; ++i) {
-      const uint64_t r = t0 + warp * (32u * kRows) + i * 32u + lane;
-      if (r >= a.n) break;
-      const uint32_t x = kHalo + warp * (32u * kRows) + i * 32u + lane, w = x >> 5;
-      const uint32_t upto = 0xffffffffu >> (31u - lane);   // bits 0..lane (x & 31 == lane)
-      // [b, e): the group, as far as it lies within 64 rows of this one
-      uint32_t b = 0, e = 0xffffffffu;
-      if (s_head[w] & upto) b = w * 32 + 31 - __clz(s_head[w] & upto);
-      else if (s_head[w - 1]) b = w * 32 - 1 - __clz(s_head[w - 1]);
-      else if (s_head[w - 2]) b = w * 32 - 33 - __clz(s_head[w - 2]);
-      if (s_head[w] & ~upto) e = w * 32 + __ffs(s_head[w] & ~upto) - 1;
-      else if (s_head[w + 1]) e = w * 32 + 31 + __ffs(s_head[w + 1]);
-      else if (s_head[w + 2]) e = w * 32 + 63 + __ffs(s_head[w + 2]);
+      const uint32_t w0 = (wb + i) * 32, x = w0 + lane;
+      const uint32_t upto = 0xffffffffu >> (31u - lane);   // bits 0..lane
+      const uint32_t hb = heads[i] & upto, he = heads[i] & ~upto;
+      const uint32_t b = hb ? w0 + 31 - __clz(hb) : prev;   // [b, e): the group
+      const uint32_t e = he ? w0 - 1 + __ffs(he) : next[i];
+      if (heads[i]) prev = w0 + 31 - __clz(heads[i]);
       const uint32_t mine = s_k2[x];
-      uint32_t at = x;
-      // (b == 0 is not a found head: a group that starts there and holds this
-      // row, 64 rows on or more, is too long)
-      if (b != 0 && e != 0xffffffffu && e - b <= kGroupMax) {
-        at = b;
-        for (uint32_t j = b; j < e; ++j) {
-          const uint32_t v = s_k2[j];
-          at += (v < mine || (v == mine && j < x)) ? 1u : 0u;
+      if (t0 + x - kHalo < a.n) {
+        uint32_t at = x;
+        if (b != 0 && e != 0xffffffffu && e - b <= kGroupMax) {
+          at = b;
+#pragma unroll 4
+          for (uint32_t j = b; j < e; ++j) {
+            const uint32_t v = s_k2[j];
+            at += (v < mine || (v == mine && j < x)) ? 1u : 0u;
+          }
+        } else {
+          a.counts[2] = 1;
         }
-      } else {
-        a.counts[2] = 1;
+        if (a.col2) a.col2[t0 + at - kHalo] = mine >= a.f2.thr ? mine + a.f2.add : mine;
       }
-      if (a.col2) a.col2[t0 + at - kHalo] = mine >= a.f2.thr ? mine + a.f2.add : mine;
     }
   }
   __syncthreads();
