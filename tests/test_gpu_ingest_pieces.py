@@ -128,3 +128,46 @@ def test_dictionary_texts_in_chunks(ctx):
     assert np.array_equal(s, np.append(np.arange(n) * 2 + 1, [2 * n + 1, 2 * n + 2]))
     assert np.array_equal(o, np.append(np.arange(n) * 2 + 2, [50_000_000, 3])) and (p == 1).all()
     ing.free()
+
+
+PART = 16 << 20   # longer texts than two such parts are parsed as they arrive
+
+
+def fill(rng, size):
+    block = "\n".join(statements(rng, 2000)) + "\n"
+    return block * (size // len(block) + 1)
+
+
+@pytest.mark.parametrize("edge", [-1500, -1, 0, 700])
+def test_text_in_parts(ctx, edge):
+    """Lines of 3,000 bytes around the end of a part, one longer than a part,
+    blank lines, and no newline at the end."""
+    rng = np.random.default_rng(edge + 2000)
+    text = fill(rng, 2 * PART + PART // 2)
+    at = text.rindex("\n", 0, PART + edge - 1400) + 1
+    text = text[:at] + f'<q> <r> "{"w" * 3000}" .\n\n<q2> <r> "{"w" * 3000}" .\n' + text[at:2 * PART] + \
+        f'\n<far> <r> "{"z" * (PART + 100)}" .\n' + text[:100_000].rsplit("\n", 1)[0]
+    check(ctx, mend(text))
+
+
+def mend(text):
+    """The line that the cut at 2 * PART broke becomes a comment."""
+    cut = text.index("\n<far>")
+    b = text.rindex("\n", 0, cut) + 1
+    return text[:b] + "#" + text[b:]
+
+
+def test_more_lines_than_samples_promise(ctx):
+    """Long comments, where the samples fall, between runs of short lines."""
+    rng = np.random.default_rng(8)
+    short = "\n".join(statements(rng, 300)) + "\n" * 2000
+    check(ctx, ("#" + "x" * (1 << 20) + "\n" + short) * 34)
+
+
+def test_malformed_line_in_a_later_part(ctx):
+    import vedas_gb300 as vg
+
+    lines = ["<a> <b> <c> ."] * (3 * PART // 14)
+    lines[-7] = "<a> <b>"
+    with pytest.raises(vg.VgError, match=f"line {len(lines) - 6}"):
+        vg.ingest_ntriples(ctx, "\n".join(lines).encode())
