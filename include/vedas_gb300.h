@@ -68,7 +68,7 @@ vg_status vg_stats_get(vg_ctx* ctx, uint32_t i, const char** name, uint64_t* lau
 /* Launch parameters of the context's kernels (no reference counterpart: the
  * reference's tile and block sizes are ModernGPU's and Thrust's built-in
  * ones).  Choices change speed only, never results:
- *   sort_items           radix-sort keys per thread, 8 or 16 (tile 2048 / 4096)
+ *   sort_items           radix-sort keys per thread, 8, 12 or 16 (tiles of 256 times that)
  *   join_small_rows      joins with at most this many left rows are counted
  *                        one per warp (0..256)
  *   write_small_rows     join outputs with at most this many rows (of joins

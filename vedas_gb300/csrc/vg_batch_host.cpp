@@ -713,8 +713,8 @@ void WaveEngine::stage_a(std::vector<PlannedQuery*>& completed) {
   tr.h_copy = since(tp);
   tp = Clock::now();
   if (!jl.empty()) {
-    // the device error record comes back with the totals: a look-back that
-    // gave up leaves the offsets wrong, and nothing must then be written
+    // the device error record comes back with the totals: after a wait that
+    // gave up nothing must be written
     auto* err_host = reinterpret_cast<DeviceErrors*>(ha + off_err_);
     if (placed_wave_) {
       batched_join_placed(ctx_, jl, jr, jb_, region_, d_bump_, c0_slot_, nslots,

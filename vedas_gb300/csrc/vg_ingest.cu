@@ -1,6 +1,7 @@
 // N-Triples ingest on the device.
 //
-// 1. newlines are counted (the count sizes everything else);
+// 1. the lines' number, which sizes everything else: newlines are counted, or
+//    (long texts, parsed while they are copied) guessed from samples;
 // 2. blocks take 16 KiB pieces of the text into shared memory, find their
 //    lines, and one thread parses each line into its three terms and looks
 //    them up in one open-addressing table of terms: a slot is claimed by the

@@ -616,9 +616,9 @@ __device__ __forceinline__ void jw_mark_group(const JoinOutOf<Off>& o, uint64_t 
 // nearest head at or before it (a bit mask, one ballot per warp and 32 rows,
 // and a maximum scan over the words): about 12 instructions a row, where
 // galloping each row from the thread's previous one took over 100 (13.4M rows
-// from 16M left rows: 199 -> 108 us; the six joins of a hub query, 770 us
-// from 968).  Left rows without matches cost a bit.  Consecutive threads write consecutive rows, so
-// loads and stores coalesce; hub keys spread over many blocks.
+// from 16M left rows: 199 -> 108 us; the six joins of a hub query 968 -> 770).
+// Left rows without matches cost a bit.  Consecutive threads write consecutive
+// rows, so loads and stores coalesce; hub keys spread over many blocks.
 template <int ROWS, typename Off>
 __device__ __forceinline__ void jw_write_tile(const JoinOutOf<Off>& o, uint64_t kb, uint64_t kend, uint64_t ga, uint64_t gb,
                                               JwStage<ROWS>& st) {
