@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <functional>
 #include <optional>
 
 #include "vg_join_tile.cuh"
@@ -33,7 +34,7 @@ class Tables {
   Tables& operator=(const Tables&) = delete;
   ~Tables() {
     ctx_.free(dev_);
-    ctx_.free(zero_);
+    for (char* z : zero_) ctx_.free(z);
   }
   template <typename T>
   size_t add(const std::vector<T>& v) {
@@ -42,27 +43,28 @@ class Tables {
     return at;
   }
   // Zeroed words; many of them (kInline bytes and more) get a block and a
-  // memset of their own, so only one call per object may ask for that.
+  // memset of their own.
   template <typename T>
   size_t zeros(size_t count) {
     const size_t bytes = count * sizeof(T);
     if (bytes < kInline) return room(bytes);
-    if (zero_) fail(VG_ERR_INVALID, "tables: one large zeroed block at most");
-    zero_ = ctx_.alloc<char>(bytes);
-    VG_CUDA(cudaMemsetAsync(zero_, 0, bytes, ctx_.stream));
-    return kZeroBlock;
+    char* z = ctx_.alloc<char>(bytes);
+    zero_.push_back(z);
+    VG_CUDA(cudaMemsetAsync(z, 0, bytes, ctx_.stream));
+    return SIZE_MAX - (zero_.size() - 1);
   }
   void send() {
+    if (blob_.empty()) return;
     dev_ = ctx_.alloc<char>(blob_.size());
     ctx_.upload_bytes(dev_, blob_.data(), blob_.size());
   }
   template <typename T>
   T* at(size_t off) const {
-    return reinterpret_cast<T*>(off == kZeroBlock ? zero_ : dev_ + off);
+    return reinterpret_cast<T*>(off > blob_.size() ? zero_[SIZE_MAX - off] : dev_ + off);
   }
 
  private:
-  static constexpr size_t kInline = 32 << 10, kZeroBlock = SIZE_MAX;
+  static constexpr size_t kInline = 32 << 10;
   size_t room(size_t bytes) {
     const size_t at = (blob_.size() + 15) / 16 * 16;
     blob_.resize(at + (bytes ? bytes : 1), 0);
@@ -71,7 +73,7 @@ class Tables {
   Ctx& ctx_;
   std::vector<char> blob_;
   char* dev_ = nullptr;
-  char* zero_ = nullptr;
+  std::vector<char*> zero_;
 };
 
 unsigned grid_cap(const Ctx& ctx, uint64_t units, int per_thread) {
@@ -744,7 +746,40 @@ int bits_for_segments(uint32_t S) {
 
 }  // namespace
 
-void batched_copy(Ctx& ctx, const std::vector<CopyPiece>& pieces) {
+struct BatchStage::Impl {
+  Tables tb;
+  std::vector<std::function<void()>> launches;
+  explicit Impl(Ctx& ctx) : tb(ctx) {}
+};
+
+BatchStage::BatchStage(Ctx& ctx) : impl_(new Impl(ctx)) {}
+BatchStage::~BatchStage() = default;
+
+namespace {
+
+// Adds a call's tables to the stage's and leaves the launch that `add` returns
+// to BatchStage::run; without a stage, runs it.
+template <typename Add>
+void in_stage(Ctx& ctx, BatchStage* stage, Add add) {
+  if (stage) {
+    stage->impl().launches.push_back(add(stage->impl().tb));
+    return;
+  }
+  Tables tb(ctx);
+  const std::function<void()> launch = add(tb);
+  tb.send();
+  launch();
+}
+
+}  // namespace
+
+void BatchStage::run() {
+  impl_->tb.send();
+  for (auto& f : impl_->launches) f();
+  impl_->launches.clear();
+}
+
+void batched_copy(Ctx& ctx, const std::vector<CopyPiece>& pieces, BatchStage* stage) {
   std::vector<CopyPiece> p;
   std::vector<uint64_t> cstart(1, 0);
   double bytes = 0;
@@ -770,17 +805,20 @@ void batched_copy(Ctx& ctx, const std::vector<CopyPiece>& pieces) {
       tile_piece[t] = k;
     }
   }
-  Tables tb(ctx);
-  const size_t op = tb.add(p), oc = tb.add(cstart), ot = tb.add(tile_piece);
-  tb.send();
-  ctx.launch("select_copy", bytes, [&] {
-    bcopy_kernel<<<grid_cap(ctx, cstart.back(), kCopyPer), kBlock, 0, ctx.stream>>>(
-        tb.at<CopyPiece>(op), tb.at<uint64_t>(oc), P, tb.at<uint32_t>(ot), ntiles);
+  const unsigned grid = grid_cap(ctx, cstart.back(), kCopyPer);
+  in_stage(ctx, stage, [&](Tables& tb) -> std::function<void()> {
+    const size_t op = tb.add(p), oc = tb.add(cstart), ot = tb.add(tile_piece);
+    return [=, &ctx, &tb] {
+      ctx.launch("select_copy", bytes, [&] {
+        bcopy_kernel<<<grid, kBlock, 0, ctx.stream>>>(tb.at<CopyPiece>(op), tb.at<uint64_t>(oc), P,
+                                                      tb.at<uint32_t>(ot), ntiles);
+      });
+      VG_CUDA(cudaGetLastError());
+    };
   });
-  VG_CUDA(cudaGetLastError());
 }
 
-void batched_unique_enqueue(Ctx& ctx, const std::vector<SegRows>& segs, uint64_t* counts_host) {
+void batched_unique_enqueue(Ctx& ctx, const std::vector<SegRows>& segs, uint64_t* counts_host, BatchStage* stage) {
   const uint32_t S = static_cast<uint32_t>(segs.size());
   if (S == 0) return;
   std::vector<uint64_t> tstart(S + 1, 0);
@@ -800,17 +838,19 @@ void batched_unique_enqueue(Ctx& ctx, const std::vector<SegRows>& segs, uint64_t
   std::vector<uint32_t> tile_seg(tiles);
   for (uint32_t s = 0; s < S; ++s)
     for (uint64_t t = tstart[s]; t < tstart[s + 1]; ++t) tile_seg[t] = s;
-  Tables tb(ctx);
-  const size_t og = tb.add(segs), ot = tb.add(tstart), os = tb.add(tile_seg), om = tb.add(small);
-  const size_t oz = tb.zeros<uint64_t>(tiles + 1);   // look-back words, then the ticket
-  tb.send();
-  uint64_t* status = tb.at<uint64_t>(oz);
-  ctx.launch("unique_compact", bytes, [&] {
-    bunique_kernel<<<static_cast<unsigned>(small_blocks + tiles), kBlock, 0, ctx.stream>>>(
-        tb.at<SegRows>(og), tb.at<uint64_t>(ot), tb.at<uint32_t>(os), tb.at<uint32_t>(om), nsmall, small_blocks,
-        status, reinterpret_cast<uint32_t*>(status + tiles), counts_host, ctx.d_err);
+  in_stage(ctx, stage, [&](Tables& tb) -> std::function<void()> {
+    const size_t og = tb.add(segs), ot = tb.add(tstart), os = tb.add(tile_seg), om = tb.add(small);
+    const size_t oz = tb.zeros<uint64_t>(tiles + 1);   // look-back words, then the ticket
+    return [=, &ctx, &tb] {
+      uint64_t* status = tb.at<uint64_t>(oz);
+      ctx.launch("unique_compact", bytes, [&] {
+        bunique_kernel<<<static_cast<unsigned>(small_blocks + tiles), kBlock, 0, ctx.stream>>>(
+            tb.at<SegRows>(og), tb.at<uint64_t>(ot), tb.at<uint32_t>(os), tb.at<uint32_t>(om), nsmall, small_blocks,
+            status, reinterpret_cast<uint32_t*>(status + tiles), counts_host, ctx.d_err);
+      });
+      VG_CUDA(cudaGetLastError());
+    };
   });
-  VG_CUDA(cudaGetLastError());
 }
 
 void note_unique_writes(Ctx& ctx, const std::vector<SegRows>& segs, const uint64_t* counts) {
@@ -1134,22 +1174,15 @@ uint64_t place_outputs_on_host(const JoinBatch& jb, const uint64_t* totals, cons
   return bump + fit;
 }
 
-void batched_join_placed(Ctx& ctx, const std::vector<const Rel*>& l, const std::vector<const Rel*>& r, JoinBatch& jb,
-                         const Arena::Region* region, uint64_t* d_bump, const std::vector<int32_t>& c0_slot,
-                         uint32_t nslots, const PlacedHost& host) {
-  Tables tb(ctx);
-  const CountTables ct = count_tables(ctx, tb, l, r, jb);
+namespace {
+
+// The count, the placement and the write (tables sent).
+void launch_placed(Ctx& ctx, const Tables& tb, const CountTables& ct, JoinBatch& jb, JoinOut* djo,
+                   const Arena::Region* region, uint64_t* d_bump, const int32_t* c0_slot, const PlacedHost& host) {
   const uint32_t J = jb.J;
-  if (J == 0) return;
-  alloc_count(ctx, ct, jb);
-  std::vector<JoinOut> jo(J);
-  parallel_for(J, [&](size_t j) { describe_join(jb, j, jo[j]); });
-  const size_t oj = tb.add(jo), oslot = tb.add(c0_slot);
-  tb.send();
   launch_count(ctx, tb, ct, jb);
   Scratch<uint64_t> ostart(ctx, J + 1);
   Scratch<uint32_t> small(ctx, J + 1);   // small list, then its length
-  JoinOut* djo = tb.at<JoinOut>(oj);
   const JoinPlace pl{region->begin, region->bytes, d_bump,        ostart.get(),   small.get(), small.get() + J,
                      ctx.tune.write_small_rows,    host.totals, host.bump, host.err, ctx.d_err};
   ctx.launch("join_place", 16.0 * J, [&] {
@@ -1171,9 +1204,30 @@ void batched_join_placed(Ctx& ctx, const std::vector<const Rel*>& l, const std::
   ctx.launch("join_write", 0.0, [&] {
     bjoin_write_kernel<<<static_cast<unsigned>(ctx.num_sms) * ctx.tune.write_blocks_per_sm, kBlock, 0, ctx.stream>>>(
         djo, ostart.get(), J, ranges ? ranges->get() : nullptr, 0, ostart.get() + J, small.get(), 0, small.get() + J,
-        JoinEdges{host.first_last, nslots ? tb.at<int32_t>(oslot) : nullptr, host.c0});
+        JoinEdges{host.first_last, c0_slot, host.c0});
   });
   VG_CUDA(cudaGetLastError());
+}
+
+}  // namespace
+
+void batched_join_placed(Ctx& ctx, const std::vector<const Rel*>& l, const std::vector<const Rel*>& r, JoinBatch& jb,
+                         const Arena::Region* region, uint64_t* d_bump, const std::vector<int32_t>& c0_slot,
+                         uint32_t nslots, const PlacedHost& host, BatchStage* stage) {
+  if (l.empty()) {
+    jb = JoinBatch();
+    return;
+  }
+  in_stage(ctx, stage, [&](Tables& tb) -> std::function<void()> {
+    const CountTables ct = count_tables(ctx, tb, l, r, jb);
+    alloc_count(ctx, ct, jb);
+    std::vector<JoinOut> jo(jb.J);
+    parallel_for(jb.J, [&](size_t j) { describe_join(jb, j, jo[j]); });
+    const size_t oj = tb.add(jo), oslot = tb.add(c0_slot);
+    return [=, &ctx, &tb, &jb] {
+      launch_placed(ctx, tb, ct, jb, tb.at<JoinOut>(oj), region, d_bump, nslots ? tb.at<int32_t>(oslot) : nullptr, host);
+    };
+  });
 }
 
 void JoinBatch::release(Ctx& ctx) {
@@ -1191,7 +1245,7 @@ uint64_t col0_words(const std::vector<const Rel*>& rels) {
   return t;
 }
 
-void batched_col0_enqueue(Ctx& ctx, const std::vector<const Rel*>& rels, uint32_t* host) {
+void batched_col0_enqueue(Ctx& ctx, const std::vector<const Rel*>& rels, uint32_t* host, BatchStage* stage) {
   const uint32_t R = static_cast<uint32_t>(rels.size());
   if (R == 0) return;
   std::vector<Col0Req> rq(R);
@@ -1201,13 +1255,15 @@ void batched_col0_enqueue(Ctx& ctx, const std::vector<const Rel*>& rels, uint32_
     total += rels[q]->nrows;
   }
   if (total == 0) return;
-  Tables tb(ctx);
-  const size_t orq = tb.add(rq);
-  tb.send();
-  ctx.launch("col0_stage", 8.0 * total, [&] {
-    col0_kernel<<<R < 1024 ? R : 1024, 128, 0, ctx.stream>>>(tb.at<Col0Req>(orq), R, host);
+  in_stage(ctx, stage, [&](Tables& tb) -> std::function<void()> {
+    const size_t orq = tb.add(rq);
+    return [=, &ctx, &tb] {
+      ctx.launch("col0_stage", 8.0 * total, [&] {
+        col0_kernel<<<R < 1024 ? R : 1024, 128, 0, ctx.stream>>>(tb.at<Col0Req>(orq), R, host);
+      });
+      VG_CUDA(cudaGetLastError());
+    };
   });
-  VG_CUDA(cudaGetLastError());
 }
 
 PinnedWords::~PinnedWords() { ctx_.give_pinned(p_, cap_); }

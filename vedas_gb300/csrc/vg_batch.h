@@ -7,6 +7,7 @@
 // an event).
 #pragma once
 
+#include <memory>
 #include <vector>
 
 #include "vg_relops.h"
@@ -32,8 +33,25 @@ class PinnedWords {
   size_t cap_ = 0;   // bytes
 };
 
+// The calls of one pipeline stage whose tables go up in one copy: each call
+// given the stage adds its tables and leaves its launches to run(), in the
+// order of the calls.  What the calls were given must live until then.  (A
+// copy, its event and the ring's bookkeeping for each call: 24 of them in a
+// 64-query batch.)
+class BatchStage {
+ public:
+  explicit BatchStage(Ctx& ctx);
+  ~BatchStage();
+  void run();
+  struct Impl;
+  Impl& impl() { return *impl_; }
+
+ private:
+  std::unique_ptr<Impl> impl_;
+};
+
 // All pieces in one launch (any number of pieces).
-void batched_copy(Ctx& ctx, const std::vector<CopyPiece>& pieces);
+void batched_copy(Ctx& ctx, const std::vector<CopyPiece>& pieces, BatchStage* stage = nullptr);
 
 // One relation segment: ncols columns of n rows, read from `in`, written to `out`.
 struct SegRows {
@@ -45,7 +63,8 @@ struct SegRows {
 
 // Adjacent-unique compaction of every segment; each segment's kept row count
 // goes to counts_host[s].
-void batched_unique_enqueue(Ctx& ctx, const std::vector<SegRows>& segs, uint64_t* counts_host);
+void batched_unique_enqueue(Ctx& ctx, const std::vector<SegRows>& segs, uint64_t* counts_host,
+                            BatchStage* stage = nullptr);
 // Adds the compaction's written bytes to the kernel statistics once the
 // counts are known.
 void note_unique_writes(Ctx& ctx, const std::vector<SegRows>& segs, const uint64_t* counts);
@@ -96,7 +115,7 @@ struct PlacedHost {       // page-locked
 };
 void batched_join_placed(Ctx& ctx, const std::vector<const Rel*>& l, const std::vector<const Rel*>& r, JoinBatch& jb,
                          const Arena::Region* region, uint64_t* d_bump, const std::vector<int32_t>& c0_slot,
-                         uint32_t nslots, const PlacedHost& host);
+                         uint32_t nslots, const PlacedHost& host, BatchStage* stage = nullptr);
 // Returns the region's bump after the wave; out[j] is the placed output of
 // join j (placed[j] = 1) and `blocks` the number of its columns in the region.
 uint64_t place_outputs_on_host(const JoinBatch& jb, const uint64_t* totals, const Arena::Region* region,
@@ -106,6 +125,6 @@ uint64_t place_outputs_on_host(const JoinBatch& jb, const uint64_t* totals, cons
 // Column 0 of each relation stored to the host, back to back (one launch):
 // col0_words(rels) uint32 words.
 uint64_t col0_words(const std::vector<const Rel*>& rels);
-void batched_col0_enqueue(Ctx& ctx, const std::vector<const Rel*>& rels, uint32_t* host);
+void batched_col0_enqueue(Ctx& ctx, const std::vector<const Rel*>& rels, uint32_t* host, BatchStage* stage = nullptr);
 
 }  // namespace vg

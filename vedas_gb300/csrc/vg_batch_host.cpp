@@ -701,13 +701,14 @@ void WaveEngine::stage_a(std::vector<PlannedQuery*>& completed) {
     any = true;
   }
   tr.h_sort = since(tp);
+  BatchStage stage(ctx_);   // what follows the sorts (whose columns the joins' tables hold)
   if (!swap_rels.empty()) {
-    batched_col0_enqueue(ctx_, swap_rels, reinterpret_cast<uint32_t*>(ha + off_c0_));
+    batched_col0_enqueue(ctx_, swap_rels, reinterpret_cast<uint32_t*>(ha + off_c0_), &stage);
     any = true;
   }
   tp = Clock::now();
   if (!pieces.empty()) {
-    batched_copy(ctx_, pieces);
+    batched_copy(ctx_, pieces, &stage);
     any = true;
   }
   tr.h_copy = since(tp);
@@ -720,7 +721,8 @@ void WaveEngine::stage_a(std::vector<PlannedQuery*>& completed) {
       batched_join_placed(ctx_, jl, jr, jb_, region_, d_bump_, c0_slot_, nslots,
                           PlacedHost{ha + off_tot_, ha + off_bump_, err_host,
                                      reinterpret_cast<uint32_t*>(ha + off_fla_),
-                                     reinterpret_cast<uint32_t*>(ha + off_c0a_)});
+                                     reinterpret_cast<uint32_t*>(ha + off_c0a_)},
+                          &stage);
     } else {
       batched_join_count(ctx_, jl, jr, jb_, ha + off_tot_);
       VG_CUDA(cudaMemcpyAsync(err_host, ctx_.d_err, sizeof(DeviceErrors), cudaMemcpyDeviceToHost, ctx_.stream));
@@ -730,9 +732,10 @@ void WaveEngine::stage_a(std::vector<PlannedQuery*>& completed) {
   tr.h_join = since(tp);
   tp = Clock::now();
   if (!fin_seg_.empty()) {
-    batched_unique_enqueue(ctx_, fin_seg_, ha + off_fin_);
+    batched_unique_enqueue(ctx_, fin_seg_, ha + off_fin_, &stage);
     any = true;
   }
+  stage.run();
   tr.h_unique = since(tp);
   if (any) {
     VG_CUDA(cudaEventRecord(ev_a_, ctx_.stream));
