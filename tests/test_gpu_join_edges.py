@@ -135,3 +135,15 @@ def test_left_rows_without_matches(ctx, nl, gap):
     times[0] = times[-1] = 5000
     rk = np.repeat(at, times)
     check_one(ctx, [lk, lk ^ np.uint32(0x5555)], [rk, np.arange(rk.shape[0], dtype=np.uint32)])
+
+
+@pytest.mark.parametrize("nl,times", [(1 << 18, 2), (1 << 18, 3), ((1 << 18) + 1, 2), ((1 << 18) + 1, 7),
+                                      ((1 << 18) + 1, 8), ((1 << 18) + 1, 9), (1 << 20, 8)])
+def test_outputs_around_the_guess(ctx, nl, times):
+    """Every left row matches `times` rows: room is taken for 2 (up to 2^18
+    left rows) or 8 times the left rows; one more output row than that."""
+    lk = np.arange(nl, dtype=np.uint32)
+    rk = np.repeat(lk, times)
+    check_one(ctx, [lk], [rk, np.arange(rk.shape[0], dtype=np.uint32)])
+    rk = np.append(rk, rk[-1])
+    check_one(ctx, [lk, lk], [rk])

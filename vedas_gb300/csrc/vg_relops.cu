@@ -17,7 +17,8 @@ namespace {
 constexpr int kBlock = 256;
 constexpr int kRows = 8;
 constexpr int kTileRows = kBlock * kRows;
-constexpr uint64_t kGuessRows = 1u << 20;   // joins of at most so many left rows guess their output (join())
+constexpr uint64_t kGuessRows = 1u << 20;   // joins of at most so many left rows guess their output (join()),
+constexpr uint64_t kWideGuess = (1u << 18) + 1;   // and from so many on as eight times those
 
 unsigned grid_for(const Ctx& ctx, uint64_t n, int per_thread, int per_sm = 16) {
   uint64_t g = div_up(n, static_cast<uint64_t>(kBlock) * per_thread);
@@ -610,8 +611,14 @@ void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
   // follows the count without the host in between (a round trip, copies and an
   // allocation, took 25 of 120 us at 3,000 rows); larger outputs are written
   // below.  Columns that do not fit the arena now are left to that path too.
+  // From kWideGuess rows on, where the columns are large blocks of the arena,
+  // whose unused tails go back to it (smaller ones keep their size class), the
+  // room is for eight times the rows (if that leaves as much again), and the
+  // write takes tiles of 2048 rows for its 512: 1M left rows with 3.3M output
+  // rows 126 -> 91 us.
   if (l.nrows <= kGuessRows) {
-    const uint64_t cap = std::max<uint64_t>(1024, 2 * l.nrows);
+    const bool wide = l.nrows >= kWideGuess && ctx.arena.largest_free() >= 2 * ncols * 8 * l.nrows * sizeof(uint32_t);
+    const uint64_t cap = wide ? 8 * l.nrows : std::max<uint64_t>(1024, 2 * l.nrows);
     Rel guess;
     guess.ncols = ncols;
     bool fits = true;
@@ -622,10 +629,12 @@ void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
     if (fits) {
       constexpr int kRowsSmall = 2;
       const JoinOut o = join_out(l, r, nk, cnt, 0, guess.cols);
-      const unsigned grid = static_cast<unsigned>(
-          std::min<uint64_t>(div_up(cap, kJwBlock * kRowsSmall), static_cast<uint64_t>(ctx.num_sms) * 5));
+      auto kernel = wide ? join_write_kernel<kRows, uint32_t> : join_write_kernel<kRowsSmall, uint32_t>;
+      const uint64_t rows = static_cast<uint64_t>(kJwBlock) * (wide ? kRows : kRowsSmall);
+      const unsigned grid =
+          static_cast<unsigned>(std::min<uint64_t>(div_up(cap, rows), static_cast<uint64_t>(ctx.num_sms) * 5));
       ctx.launch("join_write", 0.0, [&] {
-        join_write_kernel<kRowsSmall, uint32_t><<<grid, kJwBlock, 0, ctx.stream>>>(o, total, cap, nullptr, ctx.d_err, tail);
+        kernel<<<grid, kJwBlock, 0, ctx.stream>>>(o, total, cap, nullptr, ctx.d_err, tail);
       });
       VG_CUDA(cudaGetLastError());
       ctx.sync();
