@@ -94,7 +94,8 @@ struct Status<true> {
 //    ballot per digit bit, the first of them takes their places off the
 //    warp's running counter (which starts at the warp's first place) with one
 //    shared atomic, four keys' atomics in flight.  Lanes and keys are taken in
-//    input order, so the sort is stable;
+//    input order, so the sort is stable: a warp barrier after each key's atomic
+//    keeps the next key's first lane, often another one, behind it;
 // 3. keys (and values) go to their places in shared memory and leave from
 //    there in digit order, mostly coalesced.
 // Keys past the end are all ones: the tile's highest digit, placed after every
@@ -197,6 +198,7 @@ __global__ void __launch_bounds__(kBlock, HAS_V && sizeof(K) == 8 && ITEMS > 8 ?
       const uint32_t d = static_cast<uint32_t>(key[g + q] >> shift) & mask;
       first[q] = 0;
       if ((peers[q] & lanemask_lt()) == 0) first[q] = atomicAdd(&wh[d], __popc(peers[q]));
+      __syncwarp();
     }
 #pragma unroll
     for (int q = 0; q < kGroup; ++q) {
