@@ -663,6 +663,13 @@ constexpr int kPlaceBlock = 1024;
 
 __host__ __device__ inline uint64_t place_stride(uint64_t rows) { return (rows * 4 + 255) / 256 * 256; }
 
+// Bytes of an output in a region of `cap` bytes.  More rows than a join may
+// write (its 32-bit offsets would wrap, and the write read outside the columns;
+// the host refuses the join) count as more than any region holds.
+__host__ __device__ inline uint64_t place_bytes(uint64_t rows, uint32_t ncols, uint64_t cap) {
+  return rows > kMaxJoinRows ? cap + 1 : rows ? ncols * place_stride(rows) : 0;
+}
+
 struct JoinPlace {
   char* base;            // the region
   uint64_t cap;          // its bytes
@@ -692,7 +699,7 @@ __global__ void __launch_bounds__(kPlaceBlock) join_place_kernel(JoinOut* __rest
     const uint64_t t = j < J && !e.timeout ? totals[j] : 0;
     const uint32_t ncols = j < J ? jo[j].nlc + jo[j].nrc : 0;
     const uint64_t stride = place_stride(t);
-    const uint64_t bytes = t ? ncols * stride : 0;
+    const uint64_t bytes = place_bytes(t, ncols, pl.cap);
     uint64_t tot_b, tot_ts;
     const uint64_t eb = block_excl_scan64<kPlaceBlock>(bytes, tot_b, s_scan);
     const uint64_t off = bump0 + carry_b + eb;
@@ -1101,7 +1108,7 @@ void batched_join_write(Ctx& ctx, JoinBatch& jb, const uint64_t* totals, std::ve
   auto rows = [&](uint32_t j) -> uint64_t { return (skip && skip[j]) ? 0 : totals[j]; };
   std::vector<uint32_t> small;   // outputs written one join per warp
   for (uint32_t j = 0; j < J; ++j) {
-    if (rows(j) > 0xFFFFFFFFull) fail(VG_ERR_OVERFLOW, "join output exceeds 2^32 rows");
+    if (rows(j) > kMaxJoinRows) fail(VG_ERR_OVERFLOW, "join output exceeds 2^32 rows");
     const bool is_small = rows(j) > 0 && rows(j) <= ctx.tune.write_small_rows && jb.l[j]->nrows <= kSmallJoin;
     if (is_small) small.push_back(j);
     ostart[j + 1] = ostart[j] + (is_small ? 0 : div_up(rows(j), kTileRows));
@@ -1158,7 +1165,7 @@ uint64_t place_outputs_on_host(const JoinBatch& jb, const uint64_t* totals, cons
     const uint64_t t = totals[j];
     const uint32_t ncols = jb.l[j]->ncols + jb.r[j]->ncols - 1;
     const uint64_t stride = place_stride(t);
-    const uint64_t bytes = t ? ncols * stride : 0;
+    const uint64_t bytes = place_bytes(t, ncols, region->bytes);
     const bool fits = off + bytes <= region->bytes;
     if (fits && t) {
       Rel& r = out[j];

@@ -836,7 +836,7 @@ void WaveEngine::stage_b(std::vector<PlannedQuery*>& completed) {
     bool fallback = false;
     double wbytes = 0;
     for (size_t m = 0; m < J; ++m) {
-      if (tot[m] > 0xFFFFFFFFull) fail(VG_ERR_OVERFLOW, "join output exceeds 2^32 rows");
+      if (tot[m] > kMaxJoinRows) fail(VG_ERR_OVERFLOW, "join output exceeds 2^32 rows");
       const uint32_t ncols = jb_.l[m]->ncols + jb_.r[m]->ncols - 1;
       if (placed_[m]) {
         wbytes += 4.0 * tot[m] * (2.0 * ncols - 1);

@@ -662,7 +662,7 @@ void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
   ctx.sync();
   const uint64_t t = tail->total;
   ctx.raise_device_errors(tail->err);
-  if (t > 0xFFFFFFFFull) fail(VG_ERR_OVERFLOW, "join output exceeds 2^32 rows");
+  if (t > kMaxJoinRows) fail(VG_ERR_OVERFLOW, "join output exceeds 2^32 rows");
   out = rel_alloc(ctx, ncols, t);
   if (t == 0) return;
   const JoinOut o = join_out(l, r, nk, cnt, t, out.cols);

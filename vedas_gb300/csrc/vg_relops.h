@@ -60,6 +60,7 @@ void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
 // Off: 32 bits hold every offset of a join that is written (one with 2^32 rows
 // or more is refused, by its 64-bit total); 64 bits for the join that takes any.
 constexpr int kJoinGroup = 8;
+constexpr uint64_t kMaxJoinRows = 0xFFFFFFFFull;   // of an output with 32-bit offsets
 template <typename Off>
 struct JoinCounts {
   uint32_t* lo;
