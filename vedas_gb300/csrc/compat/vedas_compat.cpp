@@ -822,7 +822,7 @@ IR* JoinQueryJob::join(FullRelationIR* lir, FullRelationIR* rir) {
   if (w.sortR) w.rir->sortByFirstColumn();
   vg::Rel joined;
   vg::JoinEnds ends;
-  vg::join(*ex->ctx, w.lir->rel(), w.rir->rel(), false, joined, &ends);
+  (void)vg::join(*ex->ctx, w.lir->rel(), w.rir->rel(), false, joined, &ends);
   finish(w, joined, ends.first, ends.last, &ends.c0);
   return intermediateResult;
 }

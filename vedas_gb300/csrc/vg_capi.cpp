@@ -321,7 +321,7 @@ vg_status vg_join(vg_ctx* ctx, const vg_ir* l, const vg_ir* r, vg_ir* out, uint3
     check_ir(r);
     vg::Rel o;
     vg::JoinEnds ends;
-    vg::join(ctx->c, to_rel(l), to_rel(r), false, o, &ends);
+    if (vg::join(ctx->c, to_rel(l), to_rel(r), false, o, &ends)) ctx->c.sync();
     from_rel(o, out);
     if (first_last && o.nrows > 0) {
       first_last[0] = ends.first;
@@ -336,7 +336,7 @@ vg_status vg_join2(vg_ctx* ctx, const vg_ir* l, const vg_ir* r, vg_ir* out) {
     check_ir(l);
     check_ir(r);
     vg::Rel o;
-    vg::join(ctx->c, to_rel(l), to_rel(r), true, o);
+    if (vg::join(ctx->c, to_rel(l), to_rel(r), true, o)) ctx->c.sync();
     from_rel(o, out);
   });
 }

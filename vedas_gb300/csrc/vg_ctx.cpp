@@ -143,6 +143,14 @@ void Arena::big_free(size_t off, size_t sz) {
   add_free(off, sz);
 }
 
+size_t Arena::block_bytes(size_t bytes) {
+  bytes = std::max<size_t>((bytes + kAlign - 1) / kAlign, 1) * kAlign;
+  if (bytes > kSmallMax) return bytes;
+  size_t block = kAlign;
+  while (block < bytes) block <<= 1;
+  return block;
+}
+
 void* Arena::try_alloc(size_t bytes) {
   if (!base_) return nullptr;
   bytes = (bytes + kAlign - 1) / kAlign * kAlign;
@@ -347,9 +355,7 @@ void Arena::shrink(void* p, size_t new_bytes) {
 
 size_t Arena::largest_free() const {
   std::lock_guard<std::mutex> lk(mu_);
-  size_t m = 0;
-  for (auto& kv : free_) m = kv.second > m ? kv.second : m;
-  return m;
+  return by_size_.empty() ? 0 : by_size_.rbegin()->first;
 }
 
 void Ctx::upload_bytes(void* dst, const void* src, size_t bytes) {

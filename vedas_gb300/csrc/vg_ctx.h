@@ -52,6 +52,8 @@ class Arena {
   // Returns the tail of a live large block beyond new_bytes to the free list
   // (small blocks keep their class).
   void shrink(void* p, size_t new_bytes);
+  // Bytes of the block that a request for `bytes` gets.
+  static size_t block_bytes(size_t bytes);
   size_t capacity() const { return cap_; }
   // Bytes in live blocks (small blocks count their class size).  Exact once
   // no other thread allocates or frees.

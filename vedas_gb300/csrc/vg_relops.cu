@@ -19,6 +19,7 @@ constexpr int kRows = 8;
 constexpr int kTileRows = kBlock * kRows;
 constexpr uint64_t kGuessRows = 1u << 20;   // joins of at most so many left rows guess their output (join()),
 constexpr uint64_t kWideGuess = (1u << 18) + 1;   // and from so many on as eight times those
+constexpr uint32_t kGuessRooms = 4;   // places of different sizes taken for such an output
 
 unsigned grid_for(const Ctx& ctx, uint64_t n, int per_thread, int per_sm = 16) {
   uint64_t g = div_up(n, static_cast<uint64_t>(kBlock) * per_thread);
@@ -234,13 +235,28 @@ __global__ void __launch_bounds__(kJwBlock) join_ranges_kernel(JoinGroups<uint32
   }
 }
 
+// Rooms taken for a join's output before its size is known, from the largest
+// to the smallest: the output goes to the smallest one that holds it.
+struct JoinRooms {
+  uint32_t n;
+  uint64_t rows[kGuessRooms];
+  uint32_t* cols[kGuessRooms][VG_MAX_COLS];
+  __host__ __device__ uint32_t of(uint64_t total) const {   // (total <= rows[0])
+    uint32_t k = 0;
+    while (k + 1 < n && total <= rows[k + 1]) ++k;
+    return k;
+  }
+};
+
 // The output rows, kJwBlock * ROWS per tile; a block loops over tiles.  The
 // row count comes from o.total or, when total_dev is given, from the device:
-// the outputs then hold `cap` rows and nothing is written when there are
-// more.  Nothing is written either after a wait that gave up (the offsets are
-// wrong).  Ranges come from join_ranges_kernel or are found by warp 0.
+// the rows then go to one of `rooms`, and nothing is written when there are
+// more than the first holds.  Nothing is written either after a wait that gave
+// up (the offsets are wrong).  Ranges come from join_ranges_kernel or are found
+// by warp 0.
 template <int ROWS, typename Off>
-__global__ void __launch_bounds__(kJwBlock, 5) join_write_kernel(JoinOutOf<Off> o, const uint64_t* total_dev, uint64_t cap,
+__global__ void __launch_bounds__(kJwBlock, 5) join_write_kernel(JoinOutOf<Off> o, const uint64_t* total_dev,
+                                                                 const __grid_constant__ JoinRooms rooms,
                                                                  const uint2* __restrict__ ranges,
                                                                  const DeviceErrors* err, JoinTail* tail) {
   constexpr uint32_t kTile = kJwBlock * ROWS;
@@ -253,8 +269,14 @@ __global__ void __launch_bounds__(kJwBlock, 5) join_write_kernel(JoinOutOf<Off> 
     tail->total = total;
     tail->err = e;
   }
-  if (e.timeout || total > cap) return;
-  if (threadIdx.x == 0) s_o = o;
+  if (e.timeout || (total_dev && total > rooms.rows[0])) return;
+  if (threadIdx.x == 0) {
+    s_o = o;
+    if (total_dev) {
+      const uint32_t k = rooms.of(total);
+      for (uint32_t c = 0; c < o.nlc + o.nrc; ++c) s_o.oc[c] = rooms.cols[k][c];
+    }
+  }
   const uint64_t tiles = (total + kTile - 1) / kTile;
 #pragma unroll 1
   for (uint64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
@@ -312,7 +334,7 @@ JoinOutOf<Off> join_out(const Rel& l, const Rel& r, uint32_t nk, const JoinCount
   for (uint32_t c = nk; c < r.ncols; ++c) o.rc[c - nk] = r.cols[c];
   o.nlc = l.ncols;
   o.nrc = r.ncols - nk;
-  for (uint32_t c = 0; c < o.nlc + o.nrc; ++c) o.oc[c] = oc[c];
+  for (uint32_t c = 0; oc && c < o.nlc + o.nrc; ++c) o.oc[c] = oc[c];
   return o;
 }
 
@@ -551,7 +573,35 @@ void multi_copy(Ctx& ctx, const CopyPiece* pieces, int np) {
   VG_CUDA(cudaGetLastError());
 }
 
-void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnds* ends) {
+// Gives columns that lie in blocks of `bytes` the blocks that their rows ask
+// for: a large block's tail goes back to the arena, and rows that belong in a
+// size class (another one) are moved there, unless there is no block to be had.
+// True when they are: the copy is then on the stream.
+static bool fit_columns(Ctx& ctx, Rel& r, size_t bytes) {
+  const size_t own = std::max<uint64_t>(r.nrows, 1) * sizeof(uint32_t), block = Arena::block_bytes(own);
+  if (block == bytes || block > Arena::kSmallMax) {
+    for (uint32_t c = 0; c < r.ncols; ++c) ctx.arena.shrink(r.cols[c], own);
+    return false;
+  }
+  Rel to;
+  to.nrows = r.nrows;
+  CopyPiece pieces[VG_MAX_COLS];
+  for (; to.ncols < r.ncols; ++to.ncols) {
+    auto* p = static_cast<uint32_t*>(ctx.arena.try_alloc(own));
+    if (!p) {
+      rel_free(ctx, to);
+      return false;
+    }
+    to.cols[to.ncols] = p;
+    pieces[to.ncols] = {r.cols[to.ncols], p, r.nrows};
+  }
+  multi_copy(ctx, pieces, static_cast<int>(r.ncols));
+  rel_free(ctx, r);
+  r = to;
+  return r.nrows > 0;
+}
+
+bool join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnds* ends) {
   const uint32_t nk = two_keys ? 2 : 1;
   if (l.ncols < nk || r.ncols < nk) fail(VG_ERR_INVALID, "join: missing key columns");
   const uint32_t ncols = l.ncols + r.ncols - nk;
@@ -561,7 +611,7 @@ void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
   if (ends) *ends = JoinEnds();
   if (l.nrows == 0 || r.nrows == 0) {
     out = rel_alloc(ctx, ncols, 0);
-    return;
+    return false;
   }
   const uint64_t tiles = div_up(l.nrows, kJcTile);
   if (tiles > 0x7FFFFFFFull) fail(VG_ERR_OVERFLOW, "join: too many tiles");
@@ -602,57 +652,70 @@ void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
       if (t < kTailKeys) ends->c0.assign(tail->c0, tail->c0 + t);
     }
   };
-  auto free_cols = [&](Rel& x) {
-    for (uint32_t c = 0; c < x.ncols; ++c)
-      if (x.cols[c]) ctx.free(x.cols[c]);
-    x = Rel();
-  };
-  // A small left side: room for twice its rows is taken at once and the write
+  // A small left side: room for its output is taken at once and the write
   // follows the count without the host in between (a round trip, copies and an
   // allocation, took 25 of 120 us at 3,000 rows); larger outputs are written
-  // below.  Columns that do not fit the arena now are left to that path too.
+  // below.  There are several rooms, for twice the left rows, as many and half
+  // of them, each a size class of the arena, of which the output fills the one
+  // that it would have been given: a result holds no more than its rows ask for.
   // From kWideGuess rows on, where the columns are large blocks of the arena,
-  // whose unused tails go back to it (smaller ones keep their size class), the
-  // room is for eight times the rows (if that leaves as much again), and the
-  // write takes tiles of 2048 rows for its 512: 1M left rows with 3.3M output
-  // rows 126 -> 91 us.
+  // whose unused tails go back to it, there is also a room for eight times the
+  // rows, and the write takes tiles of 2048 rows for its 512: 1M left rows with
+  // 3.3M output rows 126 -> 91 us.  Of the largest free block the rooms take a
+  // quarter at most (blocks of a size class are carved from it for good), the
+  // large ones leave as much again; where they would take more, the size is
+  // waited for.
   if (l.nrows <= kGuessRows) {
-    const bool wide = l.nrows >= kWideGuess && ctx.arena.largest_free() >= 2 * ncols * 8 * l.nrows * sizeof(uint32_t);
-    const uint64_t cap = wide ? 8 * l.nrows : std::max<uint64_t>(1024, 2 * l.nrows);
-    Rel guess;
-    guess.ncols = ncols;
-    bool fits = true;
-    for (uint32_t c = 0; c < ncols && fits; ++c) {
-      guess.cols[c] = static_cast<uint32_t*>(ctx.arena.try_alloc(cap * sizeof(uint32_t)));
-      fits = guess.cols[c] != nullptr;
+    const bool wide = l.nrows >= kWideGuess;
+    const uint64_t asked[kGuessRooms] = {wide ? 8 * l.nrows : 0, std::max<uint64_t>(1024, 2 * l.nrows), l.nrows,
+                                         (l.nrows + 1) / 2};
+    JoinRooms rooms{};
+    uint64_t free_bytes = 0;   // asked of the largest free block
+    for (uint64_t rows : asked) {
+      const uint64_t room = Arena::block_bytes(rows * sizeof(uint32_t)) / sizeof(uint32_t);
+      if (rows == 0 || (rooms.n && room >= rooms.rows[rooms.n - 1])) continue;
+      rooms.rows[rooms.n++] = room;
+      const uint64_t bytes = room * sizeof(uint32_t);
+      free_bytes += (bytes > Arena::kSmallMax ? 2 : 4) * ncols * bytes;
     }
+    auto free_room = [&](uint32_t k) {
+      for (uint32_t c = 0; c < ncols; ++c) ctx.free(rooms.cols[k][c]);
+    };
+    bool fits = free_bytes <= ctx.arena.largest_free();
+    for (uint32_t k = 0; k < rooms.n && fits; ++k)
+      for (uint32_t c = 0; c < ncols && fits; ++c) {
+        rooms.cols[k][c] = static_cast<uint32_t*>(ctx.arena.try_alloc(rooms.rows[k] * sizeof(uint32_t)));
+        fits = rooms.cols[k][c] != nullptr;
+      }
     if (fits) {
       constexpr int kRowsSmall = 2;
-      const JoinOut o = join_out(l, r, nk, cnt, 0, guess.cols);
+      const JoinOut o = join_out(l, r, nk, cnt, 0, nullptr);
       auto kernel = wide ? join_write_kernel<kRows, uint32_t> : join_write_kernel<kRowsSmall, uint32_t>;
       const uint64_t rows = static_cast<uint64_t>(kJwBlock) * (wide ? kRows : kRowsSmall);
       const unsigned grid =
-          static_cast<unsigned>(std::min<uint64_t>(div_up(cap, rows), static_cast<uint64_t>(ctx.num_sms) * 5));
+          static_cast<unsigned>(std::min<uint64_t>(div_up(rooms.rows[0], rows), static_cast<uint64_t>(ctx.num_sms) * 5));
       ctx.launch("join_write", 0.0, [&] {
-        kernel<<<grid, kJwBlock, 0, ctx.stream>>>(o, total, cap, nullptr, ctx.d_err, tail);
+        kernel<<<grid, kJwBlock, 0, ctx.stream>>>(o, total, rooms, nullptr, ctx.d_err, tail);
       });
       VG_CUDA(cudaGetLastError());
       ctx.sync();
       const uint64_t t = tail->total;
-      if (tail->err.timeout || tail->err.overflow || t > cap) {
-        free_cols(guess);
-        ctx.raise_device_errors(tail->err);
-      } else {
-        guess.nrows = t;
-        for (uint32_t c = 0; c < ncols; ++c)
-          ctx.arena.shrink(guess.cols[c], std::max<uint64_t>(t, 1) * sizeof(uint32_t));
-        out = guess;
-        ctx.add_bytes("join_write", 4.0 * t * (2.0 * ncols - 1));
+      if (!tail->err.timeout && !tail->err.overflow && t <= rooms.rows[0]) {
+        const uint32_t k = rooms.of(t);
+        for (uint32_t q = 0; q < rooms.n; ++q)
+          if (q != k) free_room(q);
         finish(t);
-        return;
+        ctx.add_bytes("join_write", 4.0 * t * (2.0 * ncols - 1));
+        out = Rel();
+        out.ncols = ncols;
+        out.nrows = t;
+        std::copy(rooms.cols[k], rooms.cols[k] + ncols, out.cols);
+        return fit_columns(ctx, out, rooms.rows[k] * sizeof(uint32_t));
       }
+      for (uint32_t q = 0; q < rooms.n; ++q) free_room(q);
+      ctx.raise_device_errors(tail->err);
     } else {
-      free_cols(guess);
+      for (uint32_t q = 0; q < rooms.n; ++q) free_room(q);
     }
   }
   // the total and the error record come back together: after a wait that gave
@@ -664,7 +727,7 @@ void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
   ctx.raise_device_errors(tail->err);
   if (t > kMaxJoinRows) fail(VG_ERR_OVERFLOW, "join output exceeds 2^32 rows");
   out = rel_alloc(ctx, ncols, t);
-  if (t == 0) return;
+  if (t == 0) return false;
   const JoinOut o = join_out(l, r, nk, cnt, t, out.cols);
   const uint64_t otiles = div_up(t, static_cast<uint64_t>(kTileRows));
   std::optional<Scratch<uint2>> ranges;
@@ -680,11 +743,12 @@ void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
   }
   ctx.launch("join_write", 4.0 * t * (2.0 * ncols - 1), [&] {
     join_write_kernel<kRows, uint32_t><<<static_cast<unsigned>(otiles), kJwBlock, 0, ctx.stream>>>(
-        o, nullptr, t, ranges ? ranges->get() : nullptr, ctx.d_err, tail);
+        o, nullptr, JoinRooms{}, ranges ? ranges->get() : nullptr, ctx.d_err, tail);
   });
   VG_CUDA(cudaGetLastError());
   ctx.sync();
   finish(t);
+  return false;
 }
 
 uint64_t join_into(cudaStream_t stream, const Rel& l, const Rel& r, uint32_t* const* out_cols, uint64_t capacity,
@@ -701,7 +765,7 @@ uint64_t join_into(cudaStream_t stream, const Rel& l, const Rel& r, uint32_t* co
   if (t == 0 || t > capacity) return t;
   const JoinOutOf<uint64_t> o = join_out(l, r, 1, c, t, out_cols);
   join_write_kernel<kRows, uint64_t><<<static_cast<unsigned>(std::min<uint64_t>(div_up(t, kTileRows), 0x7FFFFFFFull)), kJwBlock,
-                             0, stream>>>(o, nullptr, t, nullptr, err, nullptr);
+                             0, stream>>>(o, nullptr, JoinRooms{}, nullptr, err, nullptr);
   VG_CUDA(cudaGetLastError());
   return t;
 }

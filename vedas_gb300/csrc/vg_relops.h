@@ -44,9 +44,10 @@ struct JoinEnds {
 
 // Sorted inner join of l and r on column 0 (two_keys: on columns 0 and 1).
 // Output layout: key column(s), l's other columns, r's other columns; rows
-// ordered by (left row, right row).  Allocates `out` from the arena; the
-// output is complete on return, and device errors are raised.
-void join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnds* ends = nullptr);
+// ordered by (left row, right row).  Allocates `out` from the arena, no more
+// than its rows take; waits for the result and raises device errors.  True
+// when a copy of the output to blocks of its size is still on the stream.
+bool join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnds* ends = nullptr);
 
 // What a join's count leaves in device memory.  Left rows come in groups of
 // kJoinGroup (one thread's): match has a bit for each of a group's rows that has
