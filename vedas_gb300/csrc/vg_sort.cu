@@ -9,6 +9,8 @@
 // the variant without a host round trip, which runs every pass.
 #include "vg_sort.h"
 
+#include <algorithm>
+
 #include "vg_prims.cuh"
 #include "vg_radix.cuh"
 
@@ -334,20 +336,34 @@ int items_for(const Ctx& ctx, uint64_t n) {
 }
 
 // Tickets and look-back words of a list of passes, to be zeroed before them:
-// the tickets (and one more word for the caller), then each pass's words.
+// the tickets (and one more word for the caller), then the words of as many
+// passes as half a byte a key holds (1 MiB in small sorts, and what that
+// leaves of the arena's block): four passes of 7-bit digits in tiles of 4096
+// keys, two of 8-bit ones, half of that from 2^30 keys on.  Later passes use
+// them again, zeroed in between (one memset more, 2 us).  With the words of all
+// passes at once a sort of 64-bit keys over eight digits held two bytes a key.
 struct PassScratch {
-  static constexpr size_t kHead = 128;
+  static constexpr size_t kHead = 128, kLeast = 1u << 20;
   static_assert((kMaxPasses + 1) * sizeof(uint32_t) <= kHead, "tickets and the caller's word");
-  size_t bytes = kHead;
-  size_t at[kMaxPasses];
+  size_t bytes;       // to be zeroed
+  size_t set = 0;     // bytes of a pass's words
+  uint32_t sets = 1;  // passes whose words there are
   int items;
-  PassScratch(const Ctx& ctx, uint64_t n, const DigitList& dl) : items(items_for(ctx, n)) {
+  // more: bytes that the caller puts behind them in the same block
+  PassScratch(const Ctx& ctx, uint64_t n, const DigitList& dl, size_t more) : items(items_for(ctx, n)) {
     const uint64_t tiles = div_up(n, static_cast<uint64_t>(kBlock) * items);
     const size_t word = wide_status(n) ? sizeof(uint64_t) : sizeof(uint32_t);
-    for (uint32_t p = 0; p < dl.n; ++p) {
-      at[p] = bytes;
-      bytes += tiles * status_row(dl.d[p].bits) * word;
-    }
+    for (uint32_t p = 0; p < dl.n; ++p) set = std::max(set, tiles * status_row(dl.d[p].bits) * word);
+    size_t room = std::max<size_t>(div_up(n, uint64_t{4096}) * 2048, kLeast);
+    if (room <= Arena::kSmallMax) room = std::max(Arena::block_bytes(room), kHead + more) - kHead - more;
+    if (set) sets = static_cast<uint32_t>(std::clamp<size_t>(room / set, 1, dl.n));
+    bytes = kHead + sets * set;
+  }
+  // Where the words of the t-th pass lie, zeroed on the stream if they have
+  // been used before.
+  void* words(Ctx& ctx, char* zeroed, size_t t) const {
+    if (t && t % sets == 0) VG_CUDA(cudaMemsetAsync(zeroed + kHead, 0, sets * set, ctx.stream));
+    return zeroed + kHead + t % sets * set;
   }
 };
 
@@ -372,7 +388,7 @@ bool run_passes(Ctx& ctx, K* keys, K* keys_alt, uint32_t* vals, uint32_t* vals_a
   uint32_t* vout = vals_alt;
   for (size_t t = 0; t < todo.size(); ++t) {
     const uint32_t p = todo[t];
-    const PassArgs a{vin, vout, n, dl.d[p], bases[p], zeroed + ps.at[p], reinterpret_cast<uint32_t*>(zeroed) + p};
+    const PassArgs a{vin, vout, n, dl.d[p], bases[p], ps.words(ctx, zeroed, t), reinterpret_cast<uint32_t*>(zeroed) + p};
     if (!has_v) launch_pass<K, false, false>(ctx, ps.items, kin, kout, a);
     else if (t == 0 && vals_iota) launch_pass<K, true, true>(ctx, ps.items, kin, kout, a);
     else launch_pass<K, true, false>(ctx, ps.items, kin, kout, a);
@@ -390,10 +406,10 @@ bool radix_sort_impl(Ctx& ctx, K* keys, K* keys_alt, uint32_t* vals, uint32_t* v
   if (n > 0xFFFFFFFFull && has_v) fail(VG_ERR_OVERFLOW, "radix sort values are 32-bit row ids");
   const DigitList dl = digit_list(digits);
   const uint32_t passes = dl.n;
-  // counts, tickets and every pass's look-back words in one block, zeroed by
+  // counts, tickets and the passes' look-back words in one block, zeroed by
   // one memset; the bases behind them
-  const PassScratch ps(ctx, n, dl);
   const size_t hist_bytes = passes * kRadix * sizeof(uint64_t);
+  const PassScratch ps(ctx, n, dl, 2 * hist_bytes);
   Scratch<char> scratch(ctx, ps.bytes + 2 * hist_bytes);
   char* sc = scratch.get();
   auto* hist = reinterpret_cast<unsigned long long*>(sc + ps.bytes);
@@ -463,7 +479,7 @@ bool radix_sort_u64_counted(Ctx& ctx, uint64_t* keys, uint64_t* keys_alt, uint32
     return false;
   }
   const DigitList dl = digit_list(digits);
-  const PassScratch ps(ctx, n, dl);
+  const PassScratch ps(ctx, n, dl, 0);
   Scratch<char> scratch(ctx, ps.bytes);
   VG_CUDA(cudaMemsetAsync(scratch.get(), 0, ps.bytes, ctx.stream));
   std::vector<uint32_t> todo(dl.n);
