@@ -468,12 +468,16 @@ class Permuter {
     a.f2 = f_[c2];
     a.m1 = a.f0.bits_of();
     a.m2 = a.m1 | a.f1.bits_of();
-    a.col1 = out.want_col1 ? ctx.alloc<uint32_t>(n) : nullptr;
-    a.col2 = out.want_col2 ? ctx.alloc<uint32_t>(n) : nullptr;
-    a.l1_vals = out.want_l1 ? ctx.alloc<uint32_t>(n) : nullptr;
-    a.l1_offs = out.want_l1 ? ctx.alloc<uint32_t>(n) : nullptr;
-    a.l2_vals = out.want_l2 ? ctx.alloc<uint32_t>(n) : nullptr;
-    a.l2_offs = out.want_l2 ? ctx.alloc<uint32_t>(n) : nullptr;
+    auto room = [&](bool want, DevArray& d) {   // (the outputs': freed with them if the build fails)
+      if (want) d = DevArray(ctx.alloc<uint32_t>(n), n);
+      return d.ptr;
+    };
+    a.col1 = room(out.want_col1, out.col1);
+    a.col2 = room(out.want_col2, out.col2);
+    a.l1_vals = room(out.want_l1, out.l1_vals);
+    a.l1_offs = room(out.want_l1, out.l1_offs);
+    a.l2_vals = room(out.want_l2, out.l2_vals);
+    a.l2_offs = room(out.want_l2, out.l2_offs);
     a.tiles = div_up(n, kTileRows);
     // counts, ticket and both levels' look-back words, zeroed together
     Scratch<uint64_t> z(ctx, 4 + 2 * a.tiles);
@@ -517,19 +521,15 @@ class Permuter {
     for (size_t k = 0; k < all.size(); ++k) {
       PermOutputs& out = *all[k].out;
       const UnpackArgs& a = all[k].a;
-      out.col1 = DevArray(a.col1, a.col1 ? n_ : 0);
-      out.col2 = DevArray(a.col2, a.col2 ? n_ : 0);
       if (a.l1_vals) {
         ctx.arena.shrink(a.l1_vals, hc[k][0] * 4);
         ctx.arena.shrink(a.l1_offs, hc[k][0] * 4);
-        out.l1_vals = DevArray(a.l1_vals, hc[k][0]);
-        out.l1_offs = DevArray(a.l1_offs, hc[k][0]);
+        out.l1_vals.len = out.l1_offs.len = hc[k][0];
       }
       if (a.l2_vals) {
         ctx.arena.shrink(a.l2_vals, hc[k][1] * 4);
         ctx.arena.shrink(a.l2_offs, hc[k][1] * 4);
-        out.l2_vals = DevArray(a.l2_vals, hc[k][1]);
-        out.l2_offs = DevArray(a.l2_offs, hc[k][1]);
+        out.l2_vals.len = out.l2_offs.len = hc[k][1];
       }
       if (all[k].groups && hc[k][2]) sort_big_groups(out);
     }
@@ -620,7 +620,8 @@ uint32_t build_permutations(Ctx& ctx, const uint32_t* s, const uint32_t* p, cons
   column_max4(ctx, s, p, o, n, mx);
   if (bits_for(mx[0]) + bits_for(mx[1]) + bits_for(mx[2]) > 64)
     fail(VG_ERR_UNSUPPORTED, "triple ids need more than 64 key bits for the packed index sort");
-  if (n) {
+  if (n == 0) return 0;
+  try {
     using C = Permuter;
     Permuter keys(ctx, s, p, o, n, mx, full);
     keys.sort_by({C::S, C::P});
@@ -641,6 +642,13 @@ uint32_t build_permutations(Ctx& ctx, const uint32_t* s, const uint32_t* p, cons
       keys.unpack(C::S, C::O, C::P, out.sop);
     }
     keys.finish();
+  } catch (...) {
+    for (PermOutputs* q : {&out.pso, &out.pos, &out.spo, &out.sop, &out.osp, &out.ops})
+      for (DevArray* d : {&q->col1, &q->col2, &q->l1_vals, &q->l1_offs, &q->l2_vals, &q->l2_offs}) {
+        if (d->ptr) ctx.free(d->ptr);
+        d->clear();
+      }
+    throw;
   }
   return std::max(mx[0], std::max(mx[1], mx[2]));
 }

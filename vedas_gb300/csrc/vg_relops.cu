@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cstring>
 #include <optional>
+#include <utility>
 
 #include "vg_join_tile.cuh"
 #include "vg_prims.cuh"
@@ -519,9 +520,13 @@ __global__ void __launch_bounds__(kBlock) gather_kernel(const uint32_t* __restri
 Rel rel_alloc(Ctx& ctx, uint32_t ncols, uint64_t nrows) {
   if (ncols > VG_MAX_COLS) fail(VG_ERR_UNSUPPORTED, "more than 9 columns");
   Rel r;
-  r.ncols = ncols;
   r.nrows = nrows;
-  for (uint32_t c = 0; c < ncols; ++c) r.cols[c] = ctx.alloc<uint32_t>(nrows);
+  try {
+    for (; r.ncols < ncols; ++r.ncols) r.cols[r.ncols] = ctx.alloc<uint32_t>(nrows);
+  } catch (...) {
+    rel_free(ctx, r);
+    throw;
+  }
   return r;
 }
 
@@ -547,8 +552,8 @@ void rel_own(Ctx& ctx, Rel& r) {
     if (r.nrows)
       VG_CUDA(cudaMemcpyAsync(o, r.cols[c], r.nrows * sizeof(uint32_t), cudaMemcpyDeviceToDevice, ctx.stream));
     r.cols[c] = o;
+    r.borrowed &= ~(1u << c);
   }
-  r.borrowed = 0;
 }
 
 void multi_copy(Ctx& ctx, const CopyPiece* pieces, int np) {
@@ -726,13 +731,13 @@ bool join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
   const uint64_t t = tail->total;
   ctx.raise_device_errors(tail->err);
   if (t > kMaxJoinRows) fail(VG_ERR_OVERFLOW, "join output exceeds 2^32 rows");
-  out = rel_alloc(ctx, ncols, t);
-  if (t == 0) return false;
-  const JoinOut o = join_out(l, r, nk, cnt, t, out.cols);
   const uint64_t otiles = div_up(t, static_cast<uint64_t>(kTileRows));
   std::optional<Scratch<uint2>> ranges;
-  if (many_tiles(ctx.num_sms, otiles)) {
-    ranges.emplace(ctx, otiles);
+  if (many_tiles(ctx.num_sms, otiles)) ranges.emplace(ctx, otiles);
+  out = rel_alloc(ctx, ncols, t);   // (the last block that is asked for: nothing is lost where one is not to be had)
+  if (t == 0) return false;
+  const JoinOut o = join_out(l, r, nk, cnt, t, out.cols);
+  if (ranges) {
     const unsigned rblocks = static_cast<unsigned>(
         std::min<uint64_t>(div_up(otiles, kJwBlock / 32), static_cast<uint64_t>(ctx.num_sms) * 8));
     ctx.launch("join_write_ranges", 8.0 * otiles, [&] {
@@ -827,34 +832,31 @@ void sort_by_first(Ctx& ctx, Rel& r) {
   if (n <= 1 || r.ncols == 0) return;
   if (n > 0xFFFFFFFFull) fail(VG_ERR_OVERFLOW, "relation sorts are limited to 2^32 rows");
   own_column(ctx, r, 0);   // the sort uses column 0 as its key buffer
-  uint32_t* keys_alt = ctx.alloc<uint32_t>(n);
-  if (r.ncols <= 2) {
-    // a second column travels with the keys as their values: no row numbers,
-    // no gather
-    uint32_t *vals = nullptr, *vals_alt = nullptr;
-    if (r.ncols == 2) {
-      own_column(ctx, r, 1);
-      vals = r.cols[1];
-      vals_alt = ctx.alloc<uint32_t>(n);
-    }
-    const bool alt = radix_sort_u32(ctx, r.cols[0], keys_alt, vals, vals_alt, n, 32, false);
-    if (alt) {
-      std::swap(r.cols[0], keys_alt);
-      if (vals) std::swap(r.cols[1], vals_alt);
-    }
-    ctx.free(keys_alt);
-    if (vals) ctx.free(vals_alt);
+  if (r.ncols == 2) own_column(ctx, r, 1);
+  std::optional<Scratch<uint32_t>> keys_alt(std::in_place, ctx, n);
+  if (r.ncols == 1) {
+    if (radix_sort_u32(ctx, r.cols[0], keys_alt->get(), nullptr, nullptr, n, 32, false)) std::swap(r.cols[0], keys_alt->p);
     return;
   }
-  uint32_t* vals = ctx.alloc<uint32_t>(n);
-  uint32_t* vals_alt = ctx.alloc<uint32_t>(n);
-  const bool alt = radix_sort_u32(ctx, r.cols[0], keys_alt, vals, vals_alt, n, 32, true);
-  uint32_t* perm = alt ? vals_alt : vals;
-  if (alt) std::swap(r.cols[0], keys_alt);
-  ctx.free(keys_alt);
-  ctx.free(alt ? vals : vals_alt);
-  permute_columns(ctx, r, 1, perm);
-  ctx.free(perm);
+  std::optional<Scratch<uint32_t>> vals_alt(std::in_place, ctx, n);
+  if (r.ncols == 2) {
+    // a second column travels with the keys as their values: no row numbers,
+    // no gather
+    if (radix_sort_u32(ctx, r.cols[0], keys_alt->get(), r.cols[1], vals_alt->get(), n, 32, false)) {
+      std::swap(r.cols[0], keys_alt->p);
+      std::swap(r.cols[1], vals_alt->p);
+    }
+    return;
+  }
+  Scratch<uint32_t> vals(ctx, n);
+  const bool alt = radix_sort_u32(ctx, r.cols[0], keys_alt->get(), vals.get(), vals_alt->get(), n, 32, true);
+  if (alt) {
+    std::swap(r.cols[0], keys_alt->p);
+    std::swap(vals.p, vals_alt->p);
+  }
+  keys_alt.reset();   // room for the new columns
+  vals_alt.reset();
+  permute_columns(ctx, r, 1, vals.get());
 }
 
 // Rows of at most 64 bits (each column as wide as its largest value): a sort
@@ -908,14 +910,17 @@ static bool sort_packed_rows(Ctx& ctx, Rel& r) {
   std::vector<const uint64_t*> bases;
   for (uint32_t d = 0; d < dl.n; ++d) bases.push_back(counts.bases(d));
   if (radix_sort_u64_counted(ctx, keys.get(), alt.get(), nullptr, nullptr, n, digits, bases)) std::swap(keys.p, alt.p);
-  for (uint32_t c = 0; c < r.ncols; ++c) {
-    if (r.borrowed >> c & 1u) r.cols[c] = ctx.alloc<uint32_t>(n);   // (a view is not written)
+  std::vector<Scratch<uint32_t>> own;   // for the columns that are views, which are not written
+  for (uint32_t c = 0; c < r.ncols; ++c)
+    if (r.borrowed >> c & 1u) own.emplace_back(ctx, n);
+  Scratch<RowsDone> st(ctx, 1);
+  for (uint32_t c = 0, k = 0; c < r.ncols; ++c) {
+    if (r.borrowed >> c & 1u) r.cols[c] = std::exchange(own[k++].p, nullptr);
     a.col[c] = r.cols[c];
   }
   r.borrowed = 0;
   const double bytes = (8.0 + 4.0 * r.ncols) * n;
   if (low) {
-    Scratch<RowsDone> st(ctx, 1);
     VG_CUDA(cudaMemsetAsync(st.get(), 0, sizeof(RowsDone), ctx.stream));
     auto* host = reinterpret_cast<RowsHost*>(ctx.h_small);
     ctx.launch("sort_unpack", bytes, [&] {
@@ -941,24 +946,17 @@ void sort_rows(Ctx& ctx, Rel& r) {
   if (n <= 1 || r.ncols <= 1) return;  // one column: a no-op in the reference
   if (n > 0xFFFFFFFFull) fail(VG_ERR_OVERFLOW, "relation sorts are limited to 2^32 rows");
   if (sort_packed_rows(ctx, r)) return;
-  uint32_t* perm = ctx.alloc<uint32_t>(n);
-  uint32_t* perm_alt = ctx.alloc<uint32_t>(n);
-  uint32_t* keys = ctx.alloc<uint32_t>(n);
-  uint32_t* keys_alt = ctx.alloc<uint32_t>(n);
-  fill_iota(ctx, perm, n);
+  Scratch<uint32_t> perm(ctx, n), perm_alt(ctx, n), keys(ctx, n), keys_alt(ctx, n);
+  fill_iota(ctx, perm.get(), n);
   // LSD over columns: stable sorts from the last column to the first.
   for (int c = static_cast<int>(r.ncols) - 1; c >= 0; --c) {
     const uint32_t* in[1] = {r.cols[c]};
-    uint32_t* out[1] = {keys};
-    gather_cols(ctx, in, out, 1, perm, n);
-    const bool alt = radix_sort_u32(ctx, keys, keys_alt, perm, perm_alt, n, 32, false);
-    if (alt) std::swap(perm, perm_alt);
+    uint32_t* out[1] = {keys.get()};
+    gather_cols(ctx, in, out, 1, perm.get(), n);
+    if (radix_sort_u32(ctx, keys.get(), keys_alt.get(), perm.get(), perm_alt.get(), n, 32, false))
+      std::swap(perm.p, perm_alt.p);
   }
-  permute_columns(ctx, r, 0, perm);
-  ctx.free(perm);
-  ctx.free(perm_alt);
-  ctx.free(keys);
-  ctx.free(keys_alt);
+  permute_columns(ctx, r, 0, perm.get());
   ctx.check_device_errors();
 }
 
@@ -988,9 +986,9 @@ void unique_in_place(Ctx& ctx, Rel& r) {
   const uint64_t dropped = host->dropped;
   if (dropped == 0) return;
   const uint64_t kept = n - dropped;
+  Scratch<uint64_t> status(ctx, tiles);
   Rel out = rel_alloc(ctx, r.ncols, kept);
   for (uint32_t c = 0; c < r.ncols; ++c) a.out[c] = out.cols[c];
-  Scratch<uint64_t> status(ctx, tiles);
   VG_CUDA(cudaMemsetAsync(status.get(), 0, tiles * sizeof(uint64_t), ctx.stream));
   ctx.launch("unique_compact", 4.0 * (n + kept) * r.ncols, [&] {
     unique_move_kernel<<<static_cast<unsigned>(tiles), kBlock, 0, ctx.stream>>>(a, tot.get(), status.get(),
