@@ -610,6 +610,50 @@ __device__ __forceinline__ void jw_mark_group(const JoinOutOf<Off>& o, uint64_t 
   }
 }
 
+// The left and right row of each of the thread's output rows, to st.left and
+// st.right, for a tile whose groups lie far apart: every row's group is
+// searched for, all of the thread's rows in lockstep (the last group that
+// starts at or before a row has it: what follows starts after it).
+template <int ROWS, typename Off>
+__device__ __forceinline__ void jw_search_rows(const JoinOutOf<Off>& o, uint64_t kb, uint64_t kend, uint64_t ga, uint64_t gb,
+                                            JwStage<ROWS>& st) {
+  const JoinGroups<Off> starts = o.groups();
+  uint32_t lo[ROWS];
+#pragma unroll
+  for (int it = 0; it < ROWS; ++it) lo[it] = 0;
+  for (uint32_t n = static_cast<uint32_t>(gb - ga); n > 1;) {
+    const uint32_t half = n >> 1;
+#pragma unroll
+    for (int it = 0; it < ROWS; ++it) {
+      const Off k = static_cast<Off>(kb) + it * kJwBlock + threadIdx.x;
+      if (starts(ga + lo[it] + half) <= k) lo[it] += half;
+    }
+    n -= half;
+  }
+#pragma unroll
+  for (int it = 0; it < ROWS; ++it) st.left[it * kJwBlock + threadIdx.x] = lo[it];
+#pragma unroll 1
+  for (int it = 0; it < ROWS; ++it) {
+    const uint32_t p = it * kJwBlock + threadIdx.x;
+    if (kb + p >= kend) break;
+    const uint64_t g = ga + st.left[p], first = g * kJcKeys;
+    const uint32_t match = __ldg(o.cnt.match + g);
+    const Off k = static_cast<Off>(kb) + p, base = static_cast<Off>(__ldg(o.cnt.base + g / kJcTileGroups));
+    uint32_t q = 0;
+    Off at = 0;
+#pragma unroll
+    for (uint32_t x = 0; x < kJcKeys; ++x) {
+      const Off f = base + __ldg(o.cnt.offs + first + x);   // (not set where no row of the group matches)
+      if ((match >> x & 1u) && f <= k) {
+        q = x;
+        at = f;
+      }
+    }
+    st.left[p] = static_cast<uint32_t>(first) + q;
+    st.right[p] = __ldg(o.cnt.lo + first + q) + static_cast<uint32_t>(k - at);
+  }
+}
+
 // Output rows [kb, kend) (at most kJwBlock * ROWS) of a join, by one block;
 // they come from the groups [ga, gb) of left rows.  Each left row with matches
 // marks its first output row as a head; an output row's left row is the
@@ -617,39 +661,32 @@ __device__ __forceinline__ void jw_mark_group(const JoinOutOf<Off>& o, uint64_t 
 // and a maximum scan over the words): about 12 instructions a row, where
 // galloping each row from the thread's previous one took over 100 (13.4M rows
 // from 16M left rows: 199 -> 108 us; the six joins of a hub query 968 -> 770).
-// Left rows without matches cost a bit.  Consecutive threads write consecutive
-// rows, so loads and stores coalesce; hub keys spread over many blocks.
+// Left rows without matches cost a bit, up to kFar groups: passes over them
+// (about 1 us each of 256 groups) take longer than the searches of a tile's
+// rows (some 15 us whatever the range) from there on.  1,000 output rows of 1M
+// left ones took 135 us without the searches and 56 with them, 3,000 of 3M 239
+// and 80; with the line at 32 passes 30,000 of 1M take 68 us for 62, at 64 passes
+// 77.  Consecutive threads write consecutive rows, so loads and stores coalesce;
+// hub keys spread over many blocks.
 template <int ROWS, typename Off>
 __device__ __forceinline__ void jw_write_tile(const JoinOutOf<Off>& o, uint64_t kb, uint64_t kend, uint64_t ga, uint64_t gb,
                                               JwStage<ROWS>& st) {
   constexpr uint32_t kTile = kJwBlock * ROWS;
   uint32_t li[ROWS], ri[ROWS];   // 1. the left and right row of each of the thread's output rows
   const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-  {
-    // groups that take few passes: a thread each.  More than that: 16 groups'
-    // bits at a time (few are set: at most kTile rows have matches).
-    constexpr uint32_t kNear = 16 * kJwBlock;
+  constexpr uint32_t kFar = 16 * kJwBlock;
+  if (gb - ga > kFar) {
+    jw_search_rows<ROWS>(o, kb, kend, ga, gb, st);
+#pragma unroll
+    for (int it = 0; it < ROWS; ++it) {   // (each thread's own)
+      li[it] = st.left[it * kJwBlock + threadIdx.x];
+      ri[it] = st.right[it * kJwBlock + threadIdx.x];
+    }
+  } else {
     const uint8_t* match = o.cnt.match;
-    if (gb - ga <= kNear) {
-      for (uint64_t g = ga + threadIdx.x; g < gb; g += kJwBlock) {
-        const uint32_t m = __ldg(match + g);
-        if (m) jw_mark_group(o, g, m, kb, kend, st);
-      }
-    } else {
-      const uint32_t skew = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(match + ga) & 15u);
-      const uint4* match4 = reinterpret_cast<const uint4*>(match + ga - skew);   // (its array is whole words of 16)
-      const uint64_t words = (gb - ga + skew + 15) / 16;
-      for (uint64_t w = threadIdx.x; w < words; w += kJwBlock) {
-        const uint4 x = __ldg(match4 + w);
-        if ((x.x | x.y | x.z | x.w) == 0) continue;
-        const uint32_t part[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll 1
-        for (uint32_t b = 0; b < 16; ++b) {
-          const uint32_t m = (part[b >> 2] >> (8 * (b & 3))) & 255u;
-          const uint64_t g = ga - skew + w * 16 + b;   // (before ga for the first word's first bytes)
-          if (m && w * 16 + b >= skew && g < gb) jw_mark_group(o, g, m, kb, kend, st);
-        }
-      }
+    for (uint64_t g = ga + threadIdx.x; g < gb; g += kJwBlock) {
+      const uint32_t m = __ldg(match + g);
+      if (m) jw_mark_group(o, g, m, kb, kend, st);
     }
     __syncthreads();
     uint32_t heads[ROWS];
