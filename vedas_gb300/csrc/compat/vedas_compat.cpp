@@ -115,7 +115,8 @@ std::string FullRelationIR::getHeaders(const std::string& d) const {
 }
 
 void FullRelationIR::sort() { vg::sort_rows(*ctx_, r_); }
-void FullRelationIR::removeDuplicate() { vg::unique_in_place(*ctx_, r_); }
+// (joins of distinct triples repeat no rows unless a variable was projected away)
+void FullRelationIR::removeDuplicate() { vg::unique_in_place(*ctx_, r_, false); }
 void FullRelationIR::sortByFirstColumn() { vg::sort_by_first(*ctx_, r_); }
 
 void FullRelationIR::swapColumn(size_t i, size_t j) {  // src/FullRelationIR.cu:715-727

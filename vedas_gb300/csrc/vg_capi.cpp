@@ -368,7 +368,7 @@ vg_status vg_unique(vg_ctx* ctx, vg_ir* ir) {
     check_ir(ir);
     vg::Rel r = to_rel(ir);
     WriteBack back{r, ir};
-    vg::unique_in_place(ctx->c, r);
+    vg::unique_in_place(ctx->c, r, true);
   });
 }
 

@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <initializer_list>
 #include <optional>
 #include <utility>
 
@@ -20,7 +21,6 @@ constexpr int kRows = 8;
 constexpr int kTileRows = kBlock * kRows;
 constexpr uint64_t kGuessRows = 1u << 20;   // joins of at most so many left rows guess their output (join()),
 constexpr uint64_t kWideGuess = (1u << 18) + 1;   // and from so many on as eight times those
-constexpr uint32_t kGuessRooms = 4;   // places of different sizes taken for such an output
 
 unsigned grid_for(const Ctx& ctx, uint64_t n, int per_thread, int per_sm = 16) {
   uint64_t g = div_up(n, static_cast<uint64_t>(kBlock) * per_thread);
@@ -72,79 +72,192 @@ __global__ void __launch_bounds__(kBlock) multi_copy_kernel(CopyArgs a) {
   }
 }
 
+// Rooms taken for an output before its size is known, from the largest to the
+// smallest: the output goes to the smallest one that holds it.
+constexpr uint32_t kRooms = 4;
+struct Rooms {
+  uint32_t n;
+  uint64_t rows[kRooms];
+  uint32_t* cols[kRooms][VG_MAX_COLS];
+  __host__ __device__ uint32_t of(uint64_t total) const {   // (total <= rows[0])
+    uint32_t k = 0;
+    while (k + 1 < n && total <= rows[k + 1]) ++k;
+    return k;
+  }
+};
+
 // ---------------------------------------------------------------------------
 // Adjacent-unique compaction (thrust::unique over zipped columns): one kernel
 // finds the rows to drop, a second one moves the others if there are any to
-// drop (most results of a query have none).
+// drop (most results of a query have none).  Relations of one tile take one
+// launch (100 rows: 34 us with two, 16.5 so).  Where repetitions are expected, up
+// to kSoonRows, the second kernel is launched at once, and has nothing to do if
+// none are dropped: 10,000 rows, half of them dropped, 31 -> 24 us, none dropped
+// 16 -> 20.  Otherwise the first one is waited for in between.
 // ---------------------------------------------------------------------------
 struct UniqueArgs {
   const uint32_t* in[VG_MAX_COLS];
-  uint32_t* out[VG_MAX_COLS];
   uint32_t ncols;
   uint64_t n;
-  uint8_t* keep;          // bit i of byte b: row 8 b + i stays
+  uint32_t* keep;         // bit i of word w: row 32 w + i stays (whole tiles)
 };
+constexpr uint64_t kSoonRows = 1u << 19;
 struct UniqueHost {    // page-locked
   uint64_t dropped;
   DeviceErrors err;    // what the work before left, so that no copy of its own is needed
 };
-struct UniqueTotal {   // zeroed before the first kernel
+struct UniqueTotal {   // zeroed before the first kernel, with the tiles' counts that follow it
   unsigned long long dropped;
   uint32_t done;       // finished blocks
-  uint32_t ticket;     // of the second kernel
+  uint32_t pad;
 };
 
-// Each thread flags its 8 rows.  Columns are compared from the last to the
-// first, and only while some row still equals the one before it: in sorted
-// rows and in join outputs the last columns change fastest, so most of the
-// time one or two columns are read (7.4e7 rows of 8 columns without
-// repetitions: 0.13 ms, and 1.41 ms when all were read, and once more to be
-// written elsewhere).
-__global__ void __launch_bounds__(kBlock) unique_flags_kernel(UniqueArgs a, UniqueTotal* tot,
-                                                              const DeviceErrors* err, UniqueHost* host) {
+// Which of the rows r0 .. r0 + 7 (of those below n) differ from the one before.
+// Columns are compared from the last to the first, and only while some row
+// still equals the one before it: in sorted rows and in join outputs the last
+// columns change fastest, so most of the time one column is read (7.4e7 rows of
+// 8 columns without repetitions: 0.13 ms, and 1.41 ms when all were read, and
+// once more to be written elsewhere).  diff: the last column's.
+__device__ __forceinline__ uint32_t unique_kept(const UniqueArgs& a, uint64_t r0, uint32_t diff, uint32_t& here) {
   static_assert(kRows == 8, "unique_diff_bits and compact_store take 8 rows per thread");
+  here = r0 >= a.n ? 0u : a.n - r0 < kRows ? static_cast<uint32_t>(a.n - r0) : kRows;
+  const uint32_t all = (1u << here) - 1u;
+  if (r0 == 0) diff |= 1u;
+#pragma unroll 1
+  for (int c = static_cast<int>(a.ncols) - 2; c >= 0 && (diff & all) != all; --c)
+    diff |= unique_diff_bits(a.in[c], a.n, r0);
+  return diff & all;
+}
+
+// The flags, each tile's count of rows to drop, and (by the last block) every
+// tile's first output row, so that the move waits for nothing.
+__global__ void __launch_bounds__(kBlock, 6) unique_flags_kernel(const __grid_constant__ UniqueArgs a, UniqueTotal* tot, uint32_t* tile_drops,
+                                                              uint64_t* __restrict__ tile_first, uint32_t tiles,
+                                                              const DeviceErrors* err, UniqueHost* host) {
+  __shared__ uint64_t s_scan[kBlock / 32 + 1];
+  __shared__ uint64_t s_dropped;
   uint32_t drop = 0;
-  const uint64_t step = static_cast<uint64_t>(gridDim.x) * kBlock * kRows;
-#pragma unroll 2
-  for (uint64_t r0 = (static_cast<uint64_t>(blockIdx.x) * kBlock + threadIdx.x) * kRows; r0 < a.n; r0 += step) {
-    const uint32_t here = a.n - r0 < kRows ? static_cast<uint32_t>(a.n - r0) : kRows;
-    const uint32_t all = (1u << here) - 1u;
-    uint32_t diff = (r0 == 0) ? 1u : 0u;
-    for (int c = static_cast<int>(a.ncols) - 1; c >= 0 && (diff & all) != all; --c)
-      diff |= unique_diff_bits(a.in[c], a.n, r0);
-    diff &= all;
-    a.keep[r0 / 8] = static_cast<uint8_t>(diff);
-    drop += here - __popc(diff);
+  const uint32_t* last = a.in[a.ncols - 1];
+  constexpr int kIn = 2;   // tiles whose last columns are read together
+  for (uint32_t t0 = blockIdx.x; t0 < tiles; t0 += kIn * gridDim.x) {
+    uint32_t diff[kIn];
+#pragma unroll
+    for (int q = 0; q < kIn; ++q)
+      diff[q] = unique_diff_bits(last, a.n, static_cast<uint64_t>(t0 + q * gridDim.x) * kTileRows + threadIdx.x * kRows);
+#pragma unroll
+    for (int q = 0; q < kIn; ++q) {
+      const uint32_t tile = t0 + q * gridDim.x;
+      if (tile >= tiles) break;
+      const uint64_t r0 = static_cast<uint64_t>(tile) * kTileRows + threadIdx.x * kRows;
+      uint32_t here;
+      const uint32_t kept = unique_kept(a, r0, diff[q], here);
+      reinterpret_cast<uint8_t*>(a.keep)[r0 / 8] = static_cast<uint8_t>(kept);
+      const uint32_t d = here - __popc(kept);
+      if (__any_sync(0xffffffffu, d)) {
+        const uint32_t w = __reduce_add_sync(0xffffffffu, d);
+        if (lane_id() == 0) atomicAdd(&tile_drops[tile], w);
+        drop += w;
+      }
+    }
   }
-  drop = __reduce_add_sync(0xffffffffu, drop);
   if (lane_id() == 0 && drop) atomicAdd(&tot->dropped, static_cast<unsigned long long>(drop));
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0 && atomicAdd(&tot->done, 1u) == gridDim.x - 1) {
-    __threadfence();
-    host->dropped = ld_status_u64(reinterpret_cast<const uint64_t*>(&tot->dropped));
-    host->err = *err;
+  if (threadIdx.x == 0) {
+    s_dropped = 0;
+    if (atomicAdd(&tot->done, 1u) == gridDim.x - 1) {
+      __threadfence();
+      s_dropped = ld_status_u64(reinterpret_cast<const uint64_t*>(&tot->dropped));
+      host->dropped = s_dropped;
+      host->err = *err;
+    }
+  }
+  __syncthreads();
+  if (s_dropped == 0) return;   // (or not the last block)
+  constexpr uint32_t kEach = 4;
+  uint64_t before = 0;
+  for (uint32_t t0 = 0; t0 < tiles; t0 += kBlock * kEach) {
+    uint32_t v[kEach];
+    uint64_t mine = 0, all;
+#pragma unroll
+    for (uint32_t k = 0; k < kEach; ++k) {
+      const uint32_t t = t0 + threadIdx.x * kEach + k;
+      v[k] = t < tiles ? __ldcg(tile_drops + t) : 0u;
+      mine += v[k];
+    }
+    uint64_t at = before + block_excl_scan64<kBlock>(mine, all, s_scan);
+#pragma unroll
+    for (uint32_t k = 0; k < kEach; ++k) {
+      const uint32_t t = t0 + threadIdx.x * kEach + k;
+      if (t < tiles) tile_first[t] = static_cast<uint64_t>(t) * kTileRows - at;
+      at += v[k];
+    }
+    before += all;
   }
 }
 
-// A look-back over the tiles' counts places each tile's rows, which are
-// stored column by column through shared memory so that every store is
-// coalesced.
-__global__ void __launch_bounds__(kBlock) unique_move_kernel(UniqueArgs a, UniqueTotal* tot, uint64_t* status,
-                                                             DeviceErrors* err) {
+// A warp takes 256 rows of a tile, 32 consecutive ones at a time, whose bits
+// tell each lane where its row goes: loads and stores coalesce, and nothing is
+// staged or waited for.  A column is loaded, all of its rows, while the bits or
+// the column before it are on their way: 20M rows of 3 columns, 1% of them
+// repeated, take 76 us (6.3 TB/s), and 154 with each column's loads after its
+// row numbers and stores.
+__global__ void __launch_bounds__(kBlock, 5) unique_move_kernel(const __grid_constant__ UniqueArgs a,
+                                                                const UniqueTotal* __restrict__ tot,
+                                                                const uint64_t* __restrict__ tile_first,
+                                                                const __grid_constant__ Rooms rooms) {
+  constexpr uint32_t kWords = kTileRows / 32;
+  static_assert(kWords == 64 && kRows == 8, "two words of the tile per lane, eight per warp");
+  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+  const uint64_t tile = blockIdx.x, r0 = tile * kTileRows + warp * (32u * kRows) + lane;
+  const uint64_t dropped = __ldcg(&tot->dropped);
+  if (dropped == 0) return;
+  const uint32_t w0 = __ldg(a.keep + tile * kWords + lane), w1 = __ldg(a.keep + tile * kWords + 32 + lane);
+  const uint64_t to = __ldg(tile_first + tile);
+  uint32_t v[kRows], next[kRows];
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) v[i] = r0 + i * 32 < a.n ? __ldg(a.in[0] + r0 + i * 32) : 0u;
+  const uint32_t i0 = warp_incl_scan(__popc(w0)), i1 = warp_incl_scan(__popc(w1));
+  const uint32_t first_half = __shfl_sync(0xffffffffu, i0, 31);
+  const bool lower = warp < 4;
+  const uint32_t word = lower ? w0 : w1, before = lower ? i0 - __popc(w0) : first_half + i1 - __popc(w1);
+  uint32_t at[kRows];       // the row's place in the tile's output (all ones: dropped)
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) {
+    const uint32_t k = (warp * kRows + i) & 31u, m = __shfl_sync(0xffffffffu, word, k);
+    at[i] = __shfl_sync(0xffffffffu, before, k) + __popc(m & lanemask_lt());
+    if (!(m >> lane & 1u)) at[i] = 0xffffffffu;
+  }
+  uint32_t* const* cols = rooms.cols[rooms.of(a.n - dropped)];
+  for (uint32_t c = 0; c < a.ncols; ++c) {
+    if (c + 1 < a.ncols) {
+#pragma unroll
+      for (int i = 0; i < kRows; ++i) next[i] = at[i] != 0xffffffffu ? __ldg(a.in[c + 1] + r0 + i * 32) : 0u;
+    }
+    uint32_t* out = cols[c] + to;
+#pragma unroll
+    for (int i = 0; i < kRows; ++i)
+      if (at[i] != 0xffffffffu) out[at[i]] = v[i];
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) v[i] = next[i];
+  }
+}
+
+// A relation of one tile, by one block.
+__global__ void __launch_bounds__(kBlock) unique_tile_kernel(const __grid_constant__ UniqueArgs a, const __grid_constant__ Rooms rooms,
+                                                             const DeviceErrors* err, UniqueHost* host) {
   __shared__ uint32_t s_scan[kBlock / 32 + 1];
-  __shared__ uint64_t s_b;
-  __shared__ uint32_t s_tile;
-  __shared__ uint32_t s_keep[2 * kTileRows];   // compact_store: two columns at a time
-  if (threadIdx.x == 0) s_tile = atomicAdd(&tot->ticket, 1u);
-  __syncthreads();
-  const uint32_t tile = s_tile;
-  const uint64_t r0 = static_cast<uint64_t>(tile) * kTileRows + threadIdx.x * kRows;
-  const uint32_t diff = r0 < a.n ? a.keep[r0 / 8] : 0u;
-  uint32_t kept;
+  __shared__ uint32_t s_keep[2 * kTileRows];
+  const uint64_t r0 = static_cast<uint64_t>(threadIdx.x) * kRows;
+  uint32_t here, kept;
+  const uint32_t diff = unique_kept(a, r0, unique_diff_bits(a.in[a.ncols - 1], a.n, r0), here);
   const uint32_t e = block_excl_scan<kBlock>(__popc(diff), kept, s_scan);
-  const uint64_t g = block_lookback(status, tile, kept, err, &s_b);
-  compact_store<kBlock>(a.in, a.out, a.ncols, a.n, r0, diff, e, kept, g, s_keep);
+  if (threadIdx.x == 0) {
+    host->dropped = a.n - kept;
+    host->err = *err;
+  }
+  if (kept < a.n)
+    compact_store<kBlock>(a.in, rooms.cols[rooms.of(kept)], a.ncols, a.n, r0, diff, e, kept, 0, s_keep);
 }
 
 // ---------------------------------------------------------------------------
@@ -236,19 +349,6 @@ __global__ void __launch_bounds__(kJwBlock) join_ranges_kernel(JoinGroups<uint32
   }
 }
 
-// Rooms taken for a join's output before its size is known, from the largest
-// to the smallest: the output goes to the smallest one that holds it.
-struct JoinRooms {
-  uint32_t n;
-  uint64_t rows[kGuessRooms];
-  uint32_t* cols[kGuessRooms][VG_MAX_COLS];
-  __host__ __device__ uint32_t of(uint64_t total) const {   // (total <= rows[0])
-    uint32_t k = 0;
-    while (k + 1 < n && total <= rows[k + 1]) ++k;
-    return k;
-  }
-};
-
 // The output rows, kJwBlock * ROWS per tile; a block loops over tiles.  The
 // row count comes from o.total or, when total_dev is given, from the device:
 // the rows then go to one of `rooms`, and nothing is written when there are
@@ -257,7 +357,7 @@ struct JoinRooms {
 // by warp 0.
 template <int ROWS, typename Off>
 __global__ void __launch_bounds__(kJwBlock, 5) join_write_kernel(JoinOutOf<Off> o, const uint64_t* total_dev,
-                                                                 const __grid_constant__ JoinRooms rooms,
+                                                                 const __grid_constant__ Rooms rooms,
                                                                  const uint2* __restrict__ ranges,
                                                                  const DeviceErrors* err, JoinTail* tail) {
   constexpr uint32_t kTile = kJwBlock * ROWS;
@@ -578,6 +678,34 @@ void multi_copy(Ctx& ctx, const CopyPiece* pieces, int np) {
   VG_CUDA(cudaGetLastError());
 }
 
+// Rooms of `asked` rows (0: none) and more, as their blocks allow, in falling
+// order; none (false) where they would take more than a quarter of the largest
+// free block (blocks of a size class are carved from it for good), or large
+// ones would not leave as much again.
+static bool take_rooms(Ctx& ctx, uint32_t ncols, std::initializer_list<uint64_t> asked, Rooms& rooms) {
+  uint64_t free_bytes = 0;   // asked of the largest free block
+  rooms = Rooms{};
+  for (uint64_t rows : asked) {
+    const uint64_t bytes = Arena::block_bytes(rows * sizeof(uint32_t)), room = bytes / sizeof(uint32_t);
+    if (rows == 0 || (rooms.n && room >= rooms.rows[rooms.n - 1])) continue;
+    rooms.rows[rooms.n++] = room;
+    free_bytes += (bytes > Arena::kSmallMax ? 2 : 4) * ncols * bytes;
+  }
+  bool fits = free_bytes <= ctx.arena.largest_free();
+  for (uint32_t k = 0; k < rooms.n && fits; ++k)
+    for (uint32_t c = 0; c < ncols && fits; ++c) {
+      rooms.cols[k][c] = static_cast<uint32_t*>(ctx.arena.try_alloc(rooms.rows[k] * sizeof(uint32_t)));
+      fits = rooms.cols[k][c] != nullptr;
+    }
+  return fits;
+}
+
+// Gives the rooms back, but the one numbered `but`.
+static void free_rooms(Ctx& ctx, uint32_t ncols, const Rooms& rooms, uint32_t but = kRooms) {
+  for (uint32_t k = 0; k < rooms.n; ++k)
+    for (uint32_t c = 0; c < ncols && k != but; ++c) ctx.free(rooms.cols[k][c]);
+}
+
 // Gives columns that lie in blocks of `bytes` the blocks that their rows ask
 // for: a large block's tail goes back to the arena, and rows that belong in a
 // size class (another one) are moved there, unless there is no block to be had.
@@ -604,6 +732,18 @@ static bool fit_columns(Ctx& ctx, Rel& r, size_t bytes) {
   rel_free(ctx, r);
   r = to;
   return r.nrows > 0;
+}
+
+// The relation of `rows` rows that a kernel wrote to its room; the others go
+// back.  True when a copy to blocks of its size is on the stream.
+static bool keep_room(Ctx& ctx, uint32_t ncols, const Rooms& rooms, uint64_t rows, Rel& out) {
+  const uint32_t k = rooms.of(rows);
+  free_rooms(ctx, ncols, rooms, k);
+  out = Rel();
+  out.ncols = ncols;
+  out.nrows = rows;
+  std::copy(rooms.cols[k], rooms.cols[k] + ncols, out.cols);
+  return fit_columns(ctx, out, rooms.rows[k] * sizeof(uint32_t));
 }
 
 bool join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnds* ends) {
@@ -666,32 +806,13 @@ bool join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
   // From kWideGuess rows on, where the columns are large blocks of the arena,
   // whose unused tails go back to it, there is also a room for eight times the
   // rows, and the write takes tiles of 2048 rows for its 512: 1M left rows with
-  // 3.3M output rows 126 -> 91 us.  Of the largest free block the rooms take a
-  // quarter at most (blocks of a size class are carved from it for good), the
-  // large ones leave as much again; where they would take more, the size is
-  // waited for.
+  // 3.3M output rows 126 -> 91 us.  Where there is no room for the rooms, the
+  // size is waited for.
   if (l.nrows <= kGuessRows) {
     const bool wide = l.nrows >= kWideGuess;
-    const uint64_t asked[kGuessRooms] = {wide ? 8 * l.nrows : 0, std::max<uint64_t>(1024, 2 * l.nrows), l.nrows,
-                                         (l.nrows + 1) / 2};
-    JoinRooms rooms{};
-    uint64_t free_bytes = 0;   // asked of the largest free block
-    for (uint64_t rows : asked) {
-      const uint64_t room = Arena::block_bytes(rows * sizeof(uint32_t)) / sizeof(uint32_t);
-      if (rows == 0 || (rooms.n && room >= rooms.rows[rooms.n - 1])) continue;
-      rooms.rows[rooms.n++] = room;
-      const uint64_t bytes = room * sizeof(uint32_t);
-      free_bytes += (bytes > Arena::kSmallMax ? 2 : 4) * ncols * bytes;
-    }
-    auto free_room = [&](uint32_t k) {
-      for (uint32_t c = 0; c < ncols; ++c) ctx.free(rooms.cols[k][c]);
-    };
-    bool fits = free_bytes <= ctx.arena.largest_free();
-    for (uint32_t k = 0; k < rooms.n && fits; ++k)
-      for (uint32_t c = 0; c < ncols && fits; ++c) {
-        rooms.cols[k][c] = static_cast<uint32_t*>(ctx.arena.try_alloc(rooms.rows[k] * sizeof(uint32_t)));
-        fits = rooms.cols[k][c] != nullptr;
-      }
+    Rooms rooms;
+    const bool fits = take_rooms(ctx, ncols, {wide ? 8 * l.nrows : 0, std::max<uint64_t>(1024, 2 * l.nrows), l.nrows,
+                                              (l.nrows + 1) / 2}, rooms);
     if (fits) {
       constexpr int kRowsSmall = 2;
       const JoinOut o = join_out(l, r, nk, cnt, 0, nullptr);
@@ -706,21 +827,14 @@ bool join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
       ctx.sync();
       const uint64_t t = tail->total;
       if (!tail->err.timeout && !tail->err.overflow && t <= rooms.rows[0]) {
-        const uint32_t k = rooms.of(t);
-        for (uint32_t q = 0; q < rooms.n; ++q)
-          if (q != k) free_room(q);
         finish(t);
         ctx.add_bytes("join_write", 4.0 * t * (2.0 * ncols - 1));
-        out = Rel();
-        out.ncols = ncols;
-        out.nrows = t;
-        std::copy(rooms.cols[k], rooms.cols[k] + ncols, out.cols);
-        return fit_columns(ctx, out, rooms.rows[k] * sizeof(uint32_t));
+        return keep_room(ctx, ncols, rooms, t, out);
       }
-      for (uint32_t q = 0; q < rooms.n; ++q) free_room(q);
+      free_rooms(ctx, ncols, rooms);
       ctx.raise_device_errors(tail->err);
     } else {
-      for (uint32_t q = 0; q < rooms.n; ++q) free_room(q);
+      free_rooms(ctx, ncols, rooms);
     }
   }
   // the total and the error record come back together: after a wait that gave
@@ -748,7 +862,7 @@ bool join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
   }
   ctx.launch("join_write", 4.0 * t * (2.0 * ncols - 1), [&] {
     join_write_kernel<kRows, uint32_t><<<static_cast<unsigned>(otiles), kJwBlock, 0, ctx.stream>>>(
-        o, nullptr, JoinRooms{}, ranges ? ranges->get() : nullptr, ctx.d_err, tail);
+        o, nullptr, Rooms{}, ranges ? ranges->get() : nullptr, ctx.d_err, tail);
   });
   VG_CUDA(cudaGetLastError());
   ctx.sync();
@@ -770,7 +884,7 @@ uint64_t join_into(cudaStream_t stream, const Rel& l, const Rel& r, uint32_t* co
   if (t == 0 || t > capacity) return t;
   const JoinOutOf<uint64_t> o = join_out(l, r, 1, c, t, out_cols);
   join_write_kernel<kRows, uint64_t><<<static_cast<unsigned>(std::min<uint64_t>(div_up(t, kTileRows), 0x7FFFFFFFull)), kJwBlock,
-                             0, stream>>>(o, nullptr, JoinRooms{}, nullptr, err, nullptr);
+                             0, stream>>>(o, nullptr, Rooms{}, nullptr, err, nullptr);
   VG_CUDA(cudaGetLastError());
   return t;
 }
@@ -960,7 +1074,7 @@ void sort_rows(Ctx& ctx, Rel& r) {
   ctx.check_device_errors();
 }
 
-void unique_in_place(Ctx& ctx, Rel& r) {
+void unique_in_place(Ctx& ctx, Rel& r, bool repeats) {
   if (r.nrows <= 1 || r.ncols == 0) {
     ctx.check_device_errors();
     return;
@@ -970,34 +1084,80 @@ void unique_in_place(Ctx& ctx, Rel& r) {
   for (uint32_t c = 0; c < r.ncols; ++c) a.in[c] = r.cols[c];
   a.ncols = r.ncols;
   a.n = n;
-  const uint64_t tiles = div_up(n, kTileRows);
-  Scratch<uint8_t> keep(ctx, div_up(n, 8));
-  Scratch<UniqueTotal> tot(ctx, 1);
-  a.keep = keep.get();
-  VG_CUDA(cudaMemsetAsync(tot.get(), 0, sizeof(UniqueTotal), ctx.stream));
-  const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(tiles, static_cast<uint64_t>(ctx.num_sms) * 8));
   auto* host = reinterpret_cast<UniqueHost*>(ctx.h_small);
+  Rooms rooms{};
+  if (n <= kTileRows) {
+    if (take_rooms(ctx, r.ncols, {n, (n + 1) / 2, (n + 3) / 4}, rooms)) {
+      ctx.launch("unique_flags", 4.0 * n,
+                 [&] { unique_tile_kernel<<<1, kBlock, 0, ctx.stream>>>(a, rooms, ctx.d_err, host); });
+      VG_CUDA(cudaGetLastError());
+      ctx.sync();
+      const uint64_t dropped = host->dropped;
+      if (host->err.timeout || host->err.overflow || dropped == 0) {
+        free_rooms(ctx, r.ncols, rooms);
+        ctx.raise_device_errors(host->err);
+        return;
+      }
+      Rel out;
+      const bool copied = keep_room(ctx, r.ncols, rooms, n - dropped, out);
+      rel_free(ctx, r);
+      r = out;
+      if (copied) ctx.sync();
+      return;
+    }
+    free_rooms(ctx, r.ncols, rooms);
+  }
+  const uint64_t tiles = div_up(n, kTileRows);
+  if (tiles > 0x7FFFFFFFull) fail(VG_ERR_OVERFLOW, "unique: too many tiles");
+  Scratch<uint32_t> keep(ctx, tiles * (kTileRows / 32));
+  const size_t zeroed = sizeof(UniqueTotal) + tiles * sizeof(uint32_t);
+  Scratch<char> z(ctx, zeroed);
+  Scratch<uint64_t> first(ctx, tiles);
+  const bool soon = repeats && n <= kSoonRows && take_rooms(ctx, r.ncols, {n, (n + 1) / 2, (n + 3) / 4}, rooms);
+  if (!soon) {
+    free_rooms(ctx, r.ncols, rooms);
+    rooms = Rooms{};
+  }
+  a.keep = keep.get();
+  auto* tot = reinterpret_cast<UniqueTotal*>(z.get());
+  VG_CUDA(cudaMemsetAsync(tot, 0, zeroed, ctx.stream));
+  const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(tiles, static_cast<uint64_t>(ctx.num_sms) * 6));
+  auto move = [&](double bytes) {
+    ctx.launch("unique_compact", bytes, [&] {
+      unique_move_kernel<<<static_cast<unsigned>(tiles), kBlock, 0, ctx.stream>>>(a, tot, first.get(), rooms);
+    });
+    VG_CUDA(cudaGetLastError());
+  };
   // (what must be read: a column at least)
-  ctx.launch("unique_flags", 4.0 * n,
-             [&] { unique_flags_kernel<<<grid, kBlock, 0, ctx.stream>>>(a, tot.get(), ctx.d_err, host); });
-  VG_CUDA(cudaGetLastError());
-  ctx.sync();
-  ctx.raise_device_errors(host->err);
-  const uint64_t dropped = host->dropped;
-  if (dropped == 0) return;
-  const uint64_t kept = n - dropped;
-  Scratch<uint64_t> status(ctx, tiles);
-  Rel out = rel_alloc(ctx, r.ncols, kept);
-  for (uint32_t c = 0; c < r.ncols; ++c) a.out[c] = out.cols[c];
-  VG_CUDA(cudaMemsetAsync(status.get(), 0, tiles * sizeof(uint64_t), ctx.stream));
-  ctx.launch("unique_compact", 4.0 * (n + kept) * r.ncols, [&] {
-    unique_move_kernel<<<static_cast<unsigned>(tiles), kBlock, 0, ctx.stream>>>(a, tot.get(), status.get(),
-                                                                                 ctx.d_err);
+  ctx.launch("unique_flags", 4.0 * n, [&] {
+    unique_flags_kernel<<<grid, kBlock, 0, ctx.stream>>>(a, tot, reinterpret_cast<uint32_t*>(tot + 1), first.get(),
+                                                         static_cast<uint32_t>(tiles), ctx.d_err, host);
   });
   VG_CUDA(cudaGetLastError());
+  if (soon) move(0.0);
+  ctx.sync();
+  const uint64_t dropped = host->dropped, kept = n - dropped;
+  if (host->err.timeout || host->err.overflow || dropped == 0) {
+    free_rooms(ctx, r.ncols, rooms);
+    ctx.raise_device_errors(host->err);
+    return;
+  }
+  const double bytes = 4.0 * (n + kept) * r.ncols;
+  Rel out;
+  bool busy = true;
+  if (soon) {
+    ctx.add_bytes("unique_compact", bytes);
+    busy = keep_room(ctx, r.ncols, rooms, kept, out);
+  } else {
+    out = rel_alloc(ctx, r.ncols, kept);
+    rooms.n = 1;
+    rooms.rows[0] = kept;
+    std::copy(out.cols, out.cols + r.ncols, rooms.cols[0]);
+    move(bytes);
+  }
   rel_free(ctx, r);
   r = out;
-  ctx.check_device_errors();
+  if (busy) ctx.sync();
 }
 
 void download(Ctx& ctx, const uint32_t* dev, uint64_t n, uint32_t* host) {

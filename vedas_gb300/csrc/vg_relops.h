@@ -87,8 +87,9 @@ void sort_by_first(Ctx& ctx, Rel& r);
 // result and raises device errors.
 void sort_rows(Ctx& ctx, Rel& r);
 // Adjacent duplicate-row removal (synchronizes and raises device errors).  A
-// relation without any keeps its columns; views stay views.
-void unique_in_place(Ctx& ctx, Rel& r);
+// relation without any keeps its columns; views stay views.  repeats: whether
+// some are expected (for speed only).
+void unique_in_place(Ctx& ctx, Rel& r, bool repeats);
 
 // Copies `n` values of a device column to the host (synchronizes).
 void download(Ctx& ctx, const uint32_t* dev, uint64_t n, uint32_t* host);
