@@ -10,7 +10,7 @@
 //   by o: (o, s, p) = OSP,  by s: (s, o, p) = SOP.
 // Sorting each permutation by its whole key took 12 passes over 100M triples
 // (7 for PSO, 5 for POS from PSO) where this takes 8, and 40 where it takes
-// 15 for the full index of 3M triples.
+// 14 for the full index of 3M triples.
 //
 // One fused pass per permutation unpacks the sorted keys into the data
 // columns and run-length encodes the level-1 and level-2 boundaries into
@@ -595,7 +595,7 @@ class Permuter {
           start.get(), at.get(), groups, rows, static_cast<uint32_t>(bo), out.col2.ptr, keys);
     });
     VG_CUDA(cudaGetLastError());
-    if (radix_sort_u64(ctx, keys, alt, nullptr, nullptr, rows, bo + (groups > 1 ? bits_for(groups - 1) : 0), false))
+    if (radix_sort_u64(ctx, keys, alt, rows, bo + (groups > 1 ? bits_for(groups - 1) : 0)))
       std::swap(keys, alt);
     ctx.launch("index_big_groups", 12.0 * rows, [&] {
       big_move_kernel<true><<<grid_for(ctx, rows, 4), kBlock, 0, ctx.stream>>>(

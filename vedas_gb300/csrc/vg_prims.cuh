@@ -186,18 +186,6 @@ __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32
       : "memory");
 }
 
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// Bounded wait for phase `parity` of an mbarrier; false (and a recorded
-// timeout) when it did not complete.
 // Non-blocking test of phase `parity`.
 __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
@@ -209,8 +197,10 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Polls with non-blocking tests and short sleeps, so the bound is in time
-// (about kSpinLimit x 64 ns) and not in hardware suspend periods.
+// Bounded wait for phase `parity` of an mbarrier; false (and a recorded
+// timeout) when it did not complete.  Polls with non-blocking tests and short
+// sleeps, so the bound is in time (about kSpinLimit x 64 ns) and not in
+// hardware suspend periods.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, DeviceErrors* err) {
   for (uint32_t i = 0; i < kSpinLimit; ++i) {
     if (mbar_test_wait(bar, parity)) return true;
@@ -323,16 +313,7 @@ __device__ __forceinline__ void compact_store(const uint32_t* const* in, uint32_
   }
 }
 
-// Branch-free lower/upper bound over a sorted device array.
-template <typename T, typename V>
-__device__ __forceinline__ uint64_t lower_bound_dev(const T* a, uint64_t lo, uint64_t hi, V key) {
-  while (lo < hi) {
-    uint64_t mid = (lo + hi) >> 1;
-    if (a[mid] < key) lo = mid + 1;
-    else hi = mid;
-  }
-  return lo;
-}
+// Upper bound over a sorted device array.
 template <typename T, typename V>
 __device__ __forceinline__ uint64_t upper_bound_dev(const T* a, uint64_t lo, uint64_t hi, V key) {
   while (lo < hi) {

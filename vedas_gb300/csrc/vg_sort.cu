@@ -5,8 +5,9 @@
 // A tile is 256 threads x 16, 12, 8 or 4 keys; tiles take their index from an
 // atomic ticket in launch order, which guarantees that every look-back
 // predecessor is running.  Passes whose digit is the same for every key are
-// skipped (the permutation would be the identity), unless the caller asks for
-// the variant without a host round trip, which runs every pass.
+// skipped (the permutation would be the identity) where this file counts the
+// digits, at the price of a wait; sorts whose counts the caller made run every
+// pass and wait for nothing.
 #include "vg_sort.h"
 
 #include <algorithm>
@@ -22,7 +23,7 @@ constexpr int kRadix = kRadixValues;
 constexpr int kMaxPasses = kRadixMaxPasses;
 
 // Digit counts and bases of every pass in one read of the keys (16-byte
-// loads).
+// loads), and which digits are the same for every key (a bit each).
 template <typename K>
 __global__ void __launch_bounds__(kBlock) radix_hist_kernel(const K* __restrict__ keys, uint64_t n, DigitList dl,
                                                             unsigned long long* __restrict__ hist,
@@ -400,7 +401,7 @@ bool run_passes(Ctx& ctx, K* keys, K* keys_alt, uint32_t* vals, uint32_t* vals_a
 
 template <typename K>
 bool radix_sort_impl(Ctx& ctx, K* keys, K* keys_alt, uint32_t* vals, uint32_t* vals_alt, uint64_t n,
-                     const std::vector<RadixDigit>& digits, bool vals_iota, bool host_skip) {
+                     const std::vector<RadixDigit>& digits, bool vals_iota) {
   const bool has_v = vals != nullptr;
   if (n == 0) return false;
   if (n > 0xFFFFFFFFull && has_v) fail(VG_ERR_OVERFLOW, "radix sort values are 32-bit row ids");
@@ -423,18 +424,14 @@ bool radix_sort_impl(Ctx& ctx, K* keys, K* keys_alt, uint32_t* vals, uint32_t* v
   auto* whole = reinterpret_cast<uint32_t*>(ctx.h_small);
   ctx.launch("radix_histogram", static_cast<double>(n) * sizeof(K), [&] {
     radix_hist_kernel<K><<<static_cast<unsigned>(grid), kBlock, (passes ? passes : 1) * kRadix * sizeof(uint32_t),
-                           ctx.stream>>>(keys, n, dl, hist, bases, done, host_skip ? whole : nullptr);
+                           ctx.stream>>>(keys, n, dl, hist, bases, done, whole);
   });
   VG_CUDA(cudaGetLastError());
   std::vector<uint32_t> todo;
-  if (host_skip) {
-    // (the kernel stored the host's word: no copy, and nothing for a copy to be staged in)
-    ctx.sync();
-    for (uint32_t p = 0; p < passes; ++p)
-      if (!(*whole >> p & 1u)) todo.push_back(p);
-  } else {
-    for (uint32_t p = 0; p < passes; ++p) todo.push_back(p);
-  }
+  // (the kernel stored the host's word: no copy, and nothing for a copy to be staged in)
+  ctx.sync();
+  for (uint32_t p = 0; p < passes; ++p)
+    if (!(*whole >> p & 1u)) todo.push_back(p);
   if (todo.empty()) {
     if (has_v && vals_iota) fill_iota(ctx, vals, n);
     return false;
@@ -456,17 +453,16 @@ void radix_plan(std::vector<RadixDigit>& digits, int begin, int end) {
 }
 
 bool radix_sort_u32(Ctx& ctx, uint32_t* keys, uint32_t* keys_alt, uint32_t* vals, uint32_t* vals_alt,
-                    uint64_t n, int end_bit, bool vals_iota, bool host_skip) {
+                    uint64_t n, int end_bit, bool vals_iota) {
   std::vector<RadixDigit> digits;
   radix_plan(digits, 0, end_bit);
-  return radix_sort_impl<uint32_t>(ctx, keys, keys_alt, vals, vals_alt, n, digits, vals_iota, host_skip);
+  return radix_sort_impl<uint32_t>(ctx, keys, keys_alt, vals, vals_alt, n, digits, vals_iota);
 }
 
-bool radix_sort_u64(Ctx& ctx, uint64_t* keys, uint64_t* keys_alt, uint32_t* vals, uint32_t* vals_alt,
-                    uint64_t n, int end_bit, bool vals_iota, bool host_skip) {
+bool radix_sort_u64(Ctx& ctx, uint64_t* keys, uint64_t* keys_alt, uint64_t n, int end_bit) {
   std::vector<RadixDigit> digits;
   radix_plan(digits, 0, end_bit);
-  return radix_sort_impl<uint64_t>(ctx, keys, keys_alt, vals, vals_alt, n, digits, vals_iota, host_skip);
+  return radix_sort_impl<uint64_t>(ctx, keys, keys_alt, nullptr, nullptr, n, digits, false);
 }
 
 bool radix_sort_u64_counted(Ctx& ctx, uint64_t* keys, uint64_t* keys_alt, uint32_t* vals, uint32_t* vals_alt,
