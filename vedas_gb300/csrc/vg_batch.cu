@@ -1045,8 +1045,8 @@ void alloc_count(Ctx& ctx, const CountTables& ct, JoinBatch& jb) {
   const uint64_t groups = ct.rows / kJcKeys;
   jb.cnt.lo = ctx.alloc<uint32_t>(ct.rows);
   jb.cnt.offs = ctx.alloc<uint32_t>(ct.rows);
-  jb.cnt.start = ctx.alloc<uint32_t>(div_up(groups, 4) * 4 + div_up(groups, 16) * 4);   // and the match bits
-  jb.cnt.match = reinterpret_cast<uint8_t*>(jb.cnt.start + div_up(groups, 4) * 4);
+  jb.cnt.start = ctx.alloc<uint32_t>(groups + div_up(groups, 4));   // and the match bits
+  jb.cnt.match = reinterpret_cast<uint8_t*>(jb.cnt.start + groups);
   jb.d_totals = ctx.alloc<uint64_t>(jb.J + ct.T + ct.nsmall);
   jb.cnt.base = jb.d_totals + jb.J;
 }

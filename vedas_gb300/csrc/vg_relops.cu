@@ -131,9 +131,10 @@ __device__ __forceinline__ uint32_t unique_kept(const UniqueArgs& a, uint64_t r0
 
 // The flags, each tile's count of rows to drop, and (by the last block) every
 // tile's first output row, so that the move waits for nothing.
-__global__ void __launch_bounds__(kBlock, 6) unique_flags_kernel(const __grid_constant__ UniqueArgs a, UniqueTotal* tot, uint32_t* tile_drops,
-                                                              uint64_t* __restrict__ tile_first, uint32_t tiles,
-                                                              const DeviceErrors* err, UniqueHost* host) {
+__global__ void __launch_bounds__(kBlock, 6) unique_flags_kernel(const __grid_constant__ UniqueArgs a,
+                                                                 UniqueTotal* tot, uint32_t* tile_drops,
+                                                                 uint64_t* __restrict__ tile_first, uint32_t tiles,
+                                                                 const DeviceErrors* err, UniqueHost* host) {
   __shared__ uint64_t s_scan[kBlock / 32 + 1];
   __shared__ uint64_t s_dropped;
   uint32_t drop = 0;
@@ -244,7 +245,8 @@ __global__ void __launch_bounds__(kBlock, 5) unique_move_kernel(const __grid_con
 }
 
 // A relation of one tile, by one block.
-__global__ void __launch_bounds__(kBlock) unique_tile_kernel(const __grid_constant__ UniqueArgs a, const __grid_constant__ Rooms rooms,
+__global__ void __launch_bounds__(kBlock) unique_tile_kernel(const __grid_constant__ UniqueArgs a,
+                                                             const __grid_constant__ Rooms rooms,
                                                              const DeviceErrors* err, UniqueHost* host) {
   __shared__ uint32_t s_scan[kBlock / 32 + 1];
   __shared__ uint32_t s_keep[2 * kTileRows];
@@ -762,7 +764,7 @@ bool join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
   if (tiles > 0x7FFFFFFFull) fail(VG_ERR_OVERFLOW, "join: too many tiles");
   const uint64_t ngroups = div_up(l.nrows, kJcKeys);
   Scratch<uint32_t> lo(ctx, ngroups * kJcKeys), offs(ctx, ngroups * kJcKeys), start(ctx, ngroups);
-  Scratch<uint8_t> match(ctx, div_up(ngroups, 16) * 16);
+  Scratch<uint8_t> match(ctx, ngroups);
   Scratch<uint64_t> z(ctx, tiles + 2);   // first output row of every tile, total, tiles done
   uint64_t* total = z.get() + tiles;
   const JoinCounts<uint32_t> cnt{lo.get(), offs.get(), start.get(), match.get(), z.get()};

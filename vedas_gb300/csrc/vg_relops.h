@@ -55,9 +55,9 @@ bool join(Ctx& ctx, const Rel& l, const Rel& r, bool two_keys, Rel& out, JoinEnd
 // output offsets (offs) stored, a sector of 32 bytes each; start is the group's
 // first output row, for the searches.  offs and start count from the tile's
 // first output row, which is base[tile] (tiles of 2048 left rows).  The arrays
-// cover whole groups, match whole 16 of them; lo, offs and match start on 16
-// bytes.  (With an offset and a bound for every row instead, a wave of joins
-// of which few left rows match moved twice the bytes.)
+// cover whole groups; lo and offs start on 16 bytes.  (With an offset and a
+// bound for every row instead, a wave of joins of which few left rows match
+// moved twice the bytes.)
 // Off: 32 bits hold every offset of a join that is written (one with 2^32 rows
 // or more is refused, by its 64-bit total); 64 bits for the join that takes any.
 constexpr int kJoinGroup = 8;
